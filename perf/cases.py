@@ -88,13 +88,18 @@ def _random(shape, generator, normal):
     return t.normal_(0.0, SIGMA, generator=generator) if normal else t.uniform_(-1.0, 1.0, generator=generator)
 
 
+def _inputs(case, seed):
+    N, C, K, H, W = (case[k] for k in "NCKHW")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    x = _random((N, C, H, W) if case["entry"] == "nchw" else (C, H, W, N), gen, False)
+    return x, _random((C, 3, 3, K), gen, True)
+
+
 def prepare(case, seed):
     N, C, K, H, W = (case[k] for k in "NCKHW")
     entry, precision = case["entry"], case["precision"]
-    gen = torch.Generator(device="cuda")
-    gen.manual_seed(seed)
-    x = _random((N, C, H, W) if entry == "nchw" else (C, H, W, N), gen, False)
-    g = _random((C, 3, 3, K), gen, True)
+    x, g = _inputs(case, seed)
     s = {"entry": entry, "precision": precision, "size": (N, C, H, W, K),
          "stream": torch.cuda.current_stream().cuda_stream}
     if entry == "host":
@@ -153,3 +158,20 @@ def tolerance(case):
     """fp32: sums of 9 C products of 32-bit values.  TF32 and BF16: the operands carry 11 and 8
     significant bits; the sums are kept in 32."""
     return {"rel": {"fp32": 1e-5, "tf32": 1e-3, "bf16": 1e-2}[case["precision"]]}
+
+
+def exact(case, seed):
+    """The convolution of the unrounded inputs in 64 bits: one matrix product per filter tap."""
+    N, C, K, H, W = (case[k] for k in "NCKHW")
+    x, g = _inputs(case, seed)
+    if case["entry"] == "nchw":
+        x = x.permute(1, 2, 3, 0)
+    padded = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1))
+    y = torch.zeros((K, H * W * N), dtype=torch.float64, device="cuda")
+    for r in range(3):
+        for t in range(3):
+            y.addmm_(g[:, r, t].double().T, padded[:, r:r + H, t:t + W].reshape(C, H * W * N))
+    y = y.view(K, H, W, N)
+    if case["entry"] == "nchw":
+        return y.permute(3, 0, 1, 2).contiguous()
+    return y.cpu() if case["entry"] == "host" else y
