@@ -98,7 +98,7 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, u
 // True in exactly one lane of a fully converged warp.  Single-thread instructions that take their
 // operands from uniform registers (tcgen05.mma, TMA) are issued under this predicate by a warp
 // that executes the surrounding code convergently; issuing them from an `if (lane == 0)` branch
-// instead costs on the order of a hundred cycles per instruction.
+// instead costs tens of cycles per instruction.  The elected lane is the same every time.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

@@ -63,10 +63,8 @@ template <int DT, bool HU = false> struct TcCfg {
   static constexpr int kRawStages = (DT == kTcBf16 && !HU) ? 2 : 4;
   static constexpr uint32_t kUPosBytes = HU ? 2048 : 4096;           // one position of a U stage
   static constexpr uint32_t kUBytes = 16 * kUPosBytes;
-  // MMA-issuing threads (warp kTcMmaWarp and warps kTcMmaWarpB ..).  Two: one thread cannot issue
-  // these small MMAs faster than one per ~52 cycles, two keep the tensor pipe fed (40 cycles per
-  // MMA).  Four measured the same as two in BF16; in TF32 they cost more than they bring, because
-  // 18 warps leave the epilogue 96 registers per thread instead of 128 (3-7 % slower).
+  // MMA-issuing warps (kTcMmaWarp and kTcMmaWarpB ..).  Two, so that one's waits overlap the other's
+  // MMAs; four would leave the epilogue 96 registers per thread instead of 128 (3-7 % slower).
   static constexpr int kIssuers = 2;
   static constexpr int kThreads = (kTcMmaWarpB + kIssuers - 1) * 32;
   static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kTcStages * (kUBytes + kTcVBytes) + 1024;
@@ -265,7 +263,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   volatile int *dead = reinterpret_cast<volatile int *>(u_full + 9);
   uint64_t *mma_done = u_full + 10;                    // one per MMA-issuing thread: "all my MMAs have completed"
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
   const int my_tiles = (p.total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int cpt = p.chunks_per_tile;
   const int total_chunks = my_tiles * cpt;
@@ -358,14 +356,14 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     }
   } else if (warp == kTcMmaWarp || warp >= kTcMmaWarpB) {
     // ===================================== MMA issuers =========================================
-    // Two threads, each issuing the MMAs of eight positions (disjoint accumulator columns, so no
-    // ordering is needed between them).  One thread's waits and fences then overlap the other's
-    // issuing; with a single issuer its instruction stream (16 MMAs plus ~500 cycles of waits,
-    // fence and commit per K-step) was what bounded the main loop.
-    // The descriptors are built once and only advanced by constants inside the fully unrolled
-    // loop: building them per instruction made each of these small MMAs (N = 32 occupies the
-    // tensor pipe ~50 cycles) cost ~180 cycles.
-    if (lane == 0) {
+    // Two warps, each issuing the MMAs of eight positions (disjoint accumulator columns, so no
+    // ordering is needed between them).  A warp runs this loop convergently and elect.sync picks the
+    // issuing lane - always the same one, which is also the one whose MMAs its commits cover.  From an
+    // `if (lane == 0)` region, as this was before, every MMA pays for moving its operands to uniform
+    // registers one lane at a time: main loop without loads, transform and epilogue 224 -> 152 us on
+    // 64x1024x1024x14x14 in BF16 and 428 -> 284 in TF32, whole kernel 298 -> 284 and 556 -> 523.
+    // The descriptors are built once and only advanced by constants inside the unrolled loop.
+    {
       // A thread issues whole columns of the 4x4 positions (two columns each), column by column:
       // the epilogue hands the accumulators back per column, so the next tile's first MMAs start while the
       // other columns are still being read.
@@ -389,7 +387,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         const int s = g % kTcStages;
         const uint32_t use = g / kTcStages;
         // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-        if (!mbar_wait(smem_u32(u_full + s), use & 1, dead, p.status)) break;      // U landed and V written
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + s), use & 1, dead, p.status))) break;      // U landed and V written
         tc_fence_after();
         const uint64_t ad = ((dup || HU) ? a_desc0_dup : a_desc0) + (uint64_t)(s * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (Cfg::kUPosBytes >> 4)),
                        bd = b_desc0 + (uint64_t)(s * (kTcVBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
@@ -399,15 +397,15 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         for (int xo = 0; xo < kPer; ++xo) {
           const int xr = 4 * (xo & 3) + (xo >> 2);                          // position relative to col0: row xo & 3, column xo >> 2
           if ((xo & 3) == 0 && ci == 0 && seq > 0) {                         // first write to a column of a new tile: drained?
-            if (!mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status)) { ok = false; break; }
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
             tc_fence_after();
           }
-          tc_mma<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (Cfg::kUPosBytes >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate);
+          if (elect_one()) tc_mma<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (Cfg::kUPosBytes >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate);
         }
         if (!ok) break;
-        tc_commit(smem_u32(uv_empty + s));                 // stage reusable when these MMAs are done
+        if (elect_one()) tc_commit(smem_u32(uv_empty + s));                 // stage reusable when these MMAs are done
         if (++ci == cpt) {
-          tc_commit(smem_u32(acc_full));                   // tile finished
+          if (elect_one()) tc_commit(smem_u32(acc_full));                   // tile finished
           ci = 0;
           ++seq;
           if (seq < my_tiles) dup = tile_repeats_filters<DT>(p, decode_tile(p, (int)blockIdx.x + seq * (int)gridDim.x));
@@ -415,7 +413,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
       }
       // Tensor memory is freed at the end of the kernel: every MMA this thread issued must have
       // completed by then, also after a give-up (then nobody waited for acc_full).
-      tc_commit(smem_u32(mma_done + me));
+      if (elect_one()) tc_commit(smem_u32(mma_done + me));
       mbar_wait_drain(smem_u32(mma_done + me), 0);
     }
   } else {

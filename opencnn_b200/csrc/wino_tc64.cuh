@@ -72,7 +72,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 4);
   volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 5);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
   const int n_pairs = (p.n_blocks + 1) / 2;
   const int my_tiles = (p.total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int cpt = p.chunks_per_tile;                                   // K-steps per tile
@@ -167,8 +167,8 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       }
     }
   } else if (warp == kTcMmaWarp || warp == kTcMmaWarpB) {
-    // ===================================== MMA issuers (two threads, two position columns each) ==
-    if (lane == 0) {
+    // ===================================== MMA issuers (two warps, two position columns each; see wino_tc.cuh)
+    {
       const int me = warp == kTcMmaWarp ? 0 : 1;
       const int col0 = 2 * me;                         // columns col0, col0 + 1 of the 4x4 positions, column by column
       const uint32_t idesc = instr_desc<DT>();
@@ -195,8 +195,8 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       for (int g = 0; g < total_sub; ++g) {
         const int b = g & 1, su = (g >> 1) % SU, sv = g % SV;
         // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-        if (b == 0 && !mbar_wait(smem_u32(u_full + su), ((g >> 1) / SU) & 1, dead, p.status)) break;
-        if (!mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status)) break;
+        if (b == 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + su), ((g >> 1) / SU) & 1, dead, p.status))) break;
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status))) break;
         tc_fence_after();
         const uint64_t astep = b == 0 ? kTopPos : kBotPos;
         const uint64_t ad = (b == 0 ? a_top0 + (uint64_t)su * kTopStage : a_bot0 + (uint64_t)su * kBotStage) + (uint64_t)col0 * astep;
@@ -207,24 +207,24 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
         for (int xo = 0; xo < 8; ++xo) {
           const int xr = 4 * (xo & 3) + (xo >> 2);     // position relative to col0: row xo & 3, column xo >> 2
           if ((xo & 3) == 0 && b == 0 && ci == 0 && seq > 0) {   // first write to a column of a new tile: drained?
-            if (!mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status)) { ok = false; break; }
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
             tc_fence_after();
           }
-          tc_mma<DT>(d0 + xr * kTcN, ad + (uint64_t)xr * astep, bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate);
+          if (elect_one()) tc_mma<DT>(d0 + xr * kTcN, ad + (uint64_t)xr * astep, bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate);
         }
         if (!ok) break;
-        tc_commit(smem_u32(v_empty + sv));                 // V stage reusable when these MMAs are done
+        if (elect_one()) tc_commit(smem_u32(v_empty + sv));                 // V stage reusable when these MMAs are done
         if (b == 1) {
-          tc_commit(smem_u32(u_empty + su));               // and the filter slice after the second image block
+          if (elect_one()) tc_commit(smem_u32(u_empty + su));               // and the filter slice after the second image block
           if (++ci == cpt) {
-            tc_commit(smem_u32(acc_full));                 // tile finished
+            if (elect_one()) tc_commit(smem_u32(acc_full));                 // tile finished
             ci = 0;
             ++seq;
           }
         }
       }
       // Tensor memory is freed at the end of the kernel: every MMA this thread issued must have completed by then.
-      tc_commit(smem_u32(mma_done + me));
+      if (elect_one()) tc_commit(smem_u32(mma_done + me));
       mbar_wait_drain(smem_u32(mma_done + me), 0);
     }
   } else {
