@@ -14,7 +14,7 @@
 #include "layout.cuh"
 #include "wino_fp32.cuh"
 #include "wino_tc.cuh"
-#include "wino_tc2.cuh"
+#include "wino_pair.cuh"
 #include "wino_tc64.cuh"
 
 #if defined(BASE)
@@ -41,7 +41,7 @@ struct DeviceState {
   std::once_flag once;
   cudaError_t init_error = cudaSuccess;
   int sm_count = 0;
-  int max_clusters[2] = {0, 0};   // co-resident CTA pairs of wino_tc2_kernel<BF16 / TF32>
+  int max_clusters[2] = {0, 0};   // co-resident CTA pairs of wino_pair_kernel<BF16 / TF32>
   int *status_ptr = nullptr;
 };
 DeviceState g_dev[kMaxDevices];
@@ -101,26 +101,26 @@ cudaError_t device_state(DeviceState **out) {
       err = cudaFuncSetAttribute(ocb::wino_tc_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ocb::TcCfg<ocb::kTcTf32>::kSmemBytes);
     if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_tc2_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::P2Cfg<ocb::kTcBf16>::kSmemBytes);
+      err = cudaFuncSetAttribute(ocb::wino_pair_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ocb::PairCfg<ocb::kTcBf16>::kSmemBytes);
     if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_tc2_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::P2Cfg<ocb::kTcTf32>::kSmemBytes);
+      err = cudaFuncSetAttribute(ocb::wino_pair_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ocb::PairCfg<ocb::kTcTf32>::kSmemBytes);
     if (err == cudaSuccess) {
       // how many CTA pairs fit on the device at once (pairs must sit in one GPC)
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(2 * (unsigned)st.sm_count);
-      cfg.blockDim = dim3(ocb::kP2Threads);
+      cfg.blockDim = dim3(ocb::kPairThreads);
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
       attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
       cfg.attrs = &attr;
       cfg.numAttrs = 1;
-      cfg.dynamicSmemBytes = ocb::P2Cfg<ocb::kTcBf16>::kSmemBytes;
-      err = cudaOccupancyMaxActiveClusters(&st.max_clusters[0], ocb::wino_tc2_kernel<ocb::kTcBf16>, &cfg);
+      cfg.dynamicSmemBytes = ocb::PairCfg<ocb::kTcBf16>::kSmemBytes;
+      err = cudaOccupancyMaxActiveClusters(&st.max_clusters[0], ocb::wino_pair_kernel<ocb::kTcBf16>, &cfg);
       if (err == cudaSuccess) {
-        cfg.dynamicSmemBytes = ocb::P2Cfg<ocb::kTcTf32>::kSmemBytes;
-        err = cudaOccupancyMaxActiveClusters(&st.max_clusters[1], ocb::wino_tc2_kernel<ocb::kTcTf32>, &cfg);
+        cfg.dynamicSmemBytes = ocb::PairCfg<ocb::kTcTf32>::kSmemBytes;
+        err = cudaOccupancyMaxActiveClusters(&st.max_clusters[1], ocb::wino_pair_kernel<ocb::kTcTf32>, &cfg);
       }
     }
     if (err == cudaSuccess)
@@ -303,16 +303,16 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   return cudaGetLastError();
 }
 
-// Pair kernel: clusters of two CTAs share a tile of 128 filters x 64 images (wino_tc2.cuh).
+// CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).
 template <int DT>
-cudaError_t launch_wino_tc2(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
+cudaError_t launch_wino_pair(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
                             int K, cudaStream_t stream) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  constexpr int KC = ocb::P2Cfg<DT>::kKC;
+  constexpr int KC = ocb::PairCfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
   constexpr cuuint64_t esz = bf16 ? 2 : 4;
   constexpr cuuint32_t row_elems = bf16 ? 64 : 32;
@@ -323,7 +323,7 @@ cudaError_t launch_wino_tc2(const float *input, const float *workspace, float *o
   {
     cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
     cuuint64_t strides[3] = {(cuuint64_t)N * 4, (cuuint64_t)W * N * 4, (cuuint64_t)H * W * N * 4};
-    cuuint32_t box[4] = {(cuuint32_t)ocb::kP2N, 4, 3, (cuuint32_t)KC};   // three patch rows per CTA
+    cuuint32_t box[4] = {(cuuint32_t)ocb::kTcN, 4, 4, (cuuint32_t)KC};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -333,7 +333,7 @@ cudaError_t launch_wino_tc2(const float *input, const float *workspace, float *o
   {
     cuuint64_t dims[4] = {row_elems, (cuuint64_t)C, (cuuint64_t)K / row_elems, 16};
     cuuint64_t strides[3] = {(cuuint64_t)16 * K * esz, 128, (cuuint64_t)K * esz};
-    cuuint32_t box[4] = {row_elems, (cuuint32_t)KC, (cuuint32_t)(ocb::kTcM / row_elems), 8};
+    cuuint32_t box[4] = {row_elems, (cuuint32_t)KC, (cuuint32_t)(ocb::kPairFilters / row_elems), 16};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     if (enc(&tm_u, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
             const_cast<float *>(workspace), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -348,14 +348,16 @@ cudaError_t launch_wino_tc2(const float *input, const float *workspace, float *o
   p.tiles_w = (W + 1) / 2;
   p.n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
-  const long long tiles = (long long)p.tiles_h * p.tiles_w * ((p.n_blocks + 1) / 2) * p.k_blocks;
-  if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
+  const long long blocks = (long long)p.tiles_h * p.tiles_w * p.n_blocks;
+  const long long tiles = (blocks + 1) / 2 * p.k_blocks;
+  if (blocks > 0x7fffffffll / 8 || tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
+  p.blocks = (int)blocks;
   p.total_tiles = (int)tiles;
   p.split_from = p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  ocb::wino_tc2_kernel<DT><<<2 * clusters, ocb::kP2Threads, ocb::P2Cfg<DT>::kSmemBytes, stream>>>(tm_in, tm_u, p);
+  ocb::wino_pair_kernel<DT><<<2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream>>>(tm_in, tm_u, p);
   return cudaGetLastError();
 }
 
@@ -416,25 +418,42 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   return cudaGetLastError();
 }
 
-// Which tensor-core kernel a problem gets.  Both compute the same thing.  The CTA-pair kernel
-// (wino_tc2.cuh) has the cheaper main loop (half as many, twice as wide MMAs) but a dearer
-// epilogue (two CTAs meet through L2), so it wins where a tile has many K-steps and the MMAs are
-// many: in TF32 from 64 K-steps per tile (C >= 512: 6-20 % ahead).  In BF16 the single-CTA kernel
-// is level or ahead everywhere since it issues its MMAs from two threads (C = 1024: within 1 %),
-// so BF16 never takes the pair.
+// Which tensor-core kernel a problem gets.  All three give the same bits.  Medians, L2 flushed, bf16 / tf32 us.
+//   More than 64 filters: the CTA-pair kernel, except where the launch of clusters (2 us more) is not paid back -
+//   few K-steps and few tiles.  N x C x K x H x W, single : pair
+//     64x1024x1024x14x14 281 : 211 / 514 : 367    128x256x256x14x14 49 : 41 / 78 : 59    256x8x128x56x56 160 : 101 / 156 : 102
+//     32x64x128x9x9 (4 K-steps in BF16) 13.2 : 13.3 / 15.4 : 15.3    32x16x128x9x9 10.2 : 12.3 / 10.2 : 12.3
+//     64x16x128x28x28 (392 tiles) 15.4 : 17.4 / 17.3 : 17.4          64x3x128x56x56 (1568 tiles) 34.8 : 32.8 / 30.7 : 30.7
+//   At most 64 filters: the stacked kernel while there are few K-steps and more tiles than SMs (the other two leave half
+//   of the accumulator rows or of the pair idle), then the pair.  Single : pair : stacked
+//     128x64x64x56x56 96 : 94 : 78 / 135 : 127 : 122    128x128x64x28x28 (8 / 16 K-steps) 46 : 46 : 42 / 73 : 65 : 67
+//     64x192x64x28x28 35 : 35 : 39 / 56 : 48 : 63       128x128x64x7x7 (32 tiles) 14.3 : 15.4 : 18.4 / 19.5 : 17.4 : 25.6
+//     32x64x64x28x28 15.4 : 17.5 : 19.5 / 21.5 : 21.5 : 26.6    32x512x64x28x28 51 : 47 : 76 / 92 : 72 : 133
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
                       cudaStream_t stream, int kernel = OPENCNN_TC_AUTO) {
   if (kernel == OPENCNN_TC_SINGLE_CTA) return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream);
-  if (kernel == OPENCNN_TC_PAIR_LOCAL) return launch_wino_tc2<DT>(input, workspace, output, N, C, H, W, K, stream);
+  if (kernel == OPENCNN_TC_PAIR_LOCAL) return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream);
   if (kernel == OPENCNN_TC_STACKED_BLOCKS) return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream);
   if (kernel != OPENCNN_TC_AUTO) return cudaErrorInvalidValue;
-  // at most 64 filters and more than one 32-image block: two blocks share the accumulator rows
-  if (K <= 64 && N > ocb::kTcN) return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream);
+  DeviceState *st = nullptr;
+  cudaError_t e = device_state(&st);
+  if (e != cudaSuccess) return e;
+  constexpr bool bf16 = DT == ocb::kTcBf16;
   const int k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC;
-  const bool pair = DT == ocb::kTcTf32 && k_steps >= 64 && N >= 64;
-  return pair ? launch_wino_tc2<DT>(input, workspace, output, N, C, H, W, K, stream)
-              : launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream);
+  const long long tiles = (long long)((H + 1) / 2) * ((W + 1) / 2), n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
+  bool pair;
+  if (K <= 64) {
+    if (n_blocks > 1 && k_steps <= (bf16 ? 8 : 12) && tiles * ((n_blocks + 1) / 2) > st->sm_count)
+      return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream);
+    pair = k_steps >= (bf16 ? 16 : 8);
+  } else {
+    pair = k_steps >= 4 || tiles * n_blocks * ((K + ocb::kTcM - 1) / ocb::kTcM) >= 4ll * st->sm_count;
+  }
+  // (max_clusters is 0 only where no two CTAs of this size can be co-scheduled as a cluster)
+  return pair && st->max_clusters[bf16 ? 0 : 1] > 0
+             ? launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream)
+             : launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream);
 }
 
 cudaError_t forward(const float *input, const float *filter, float *output, float *workspace, int N, int C, int H,

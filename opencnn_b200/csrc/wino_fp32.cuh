@@ -79,6 +79,7 @@ struct WinoParams {
   // tile is two items, one per consumer group (see item_tile).  split_from == total_tiles and
   // total_items == total_tiles mean "no split".
   int split_from, total_items;
+  int blocks;          // CTA-pair kernel only: n_blocks * tiles_w * tiles_h
   int *status;         // device status word
 };
 

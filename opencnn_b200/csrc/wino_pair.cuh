@@ -1,0 +1,318 @@
+// Tensor-core Winograd kernel on CTA pairs (BF16 or TF32 operands): the MMAs of a pair run on both
+// SMs at once (tcgen05.mma.cta_group::2), each SM supplying half of each operand.
+//
+// Same operator as wino_tc.cuh (it replaces the reference's Winograd_kernel,
+// src/convolutionForward_32x64x8.cu:169-262, with the contraction on the tensor cores; the reference
+// has no tensor-core path).  All 16 accumulators of a tile have to stay in tensor memory until the
+// output transform, which leaves 32 accumulator columns per position.  One CTA on its own spends them
+// on 128 filters x 32 images: per K-step it loads a 64 KB filter slice for 32 KB (BF16) of patches,
+// and every MMA re-reads 4 KB of filters for 1 KB of images - shared-memory traffic and the two-deep
+// ring of 64 KB filter slices bound it, not the tensor pipe.  Here a pair computes
+//     128 filters x 64 images (two blocks of 32),   M = 128, N = 64 over two SMs:
+// CTA r holds the transformed filters 64*r .. 64*r+63 and transforms the patches of image block r,
+// and its tensor memory receives
+//     lanes  0-63   filters 64*r .. +63 of image block 0      32 columns per position
+//     lanes 64-127  the same filters of image block 1
+// (the M = 128 data-path layout of cta_group::2).  A square 64 x 64 share per CTA instead of 128 x 32:
+// the filter slice of a K-step is 32 KB instead of 64 KB, three or four of them fit, and nothing is
+// exchanged by the threads - each CTA has all 16 positions of its outputs and stores them on its own.
+//
+// The two image blocks need not belong together: block q of the list (tile row, tile column, image
+// block), image blocks fastest, pairs with block q + 1, so that only the very last pair can be half empty.
+//
+// Warp roles as in wino_tc.cuh (512 threads per CTA).  Barriers: the patches' ring is each CTA's own.
+// "Filter slice landed" and "V written" are barriers of the leading CTA (rank 0), whose two issuing
+// warps wait for both CTAs' halves there; the tensor core's commits reach the "free again" and "tile
+// finished" barriers of both CTAs (multicast arrive); a drained accumulator column is reported to the
+// leader.  All waits are bounded.  Both CTAs leave through a cluster barrier.
+#pragma once
+#include "wino_tc.cuh"
+
+namespace ocb {
+
+constexpr int kPairThreads = 512;
+constexpr int kPairFilters = 64;                 // per CTA
+template <int DT> struct PairCfg {
+  static constexpr int kKC = DT == kTcBf16 ? 16 : 8;                       // channels per K-step
+  static constexpr uint32_t kRawBytes = kKC * 16 * kTcN * 4;               // [c][4 h][4 w][32 n] fp32
+  static constexpr uint32_t kUPosBytes = 2048;                             // 64 filters x one K-step
+  static constexpr uint32_t kUBytes = 16 * kUPosBytes;
+  static constexpr int kRawStages = DT == kTcBf16 ? 3 : 4;
+  static constexpr int kUStages = 3;
+  static constexpr int kVStages = DT == kTcBf16 ? 2 : 4;
+  static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kUStages * kUBytes +
+                                       (size_t)kVStages * kTcVBytes + 512;
+  static_assert(kSmemBytes <= 232448, "shared memory");
+};
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address (shared::cluster window) of the object at the same shared-memory offset in CTA `rank`.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+// Arrive on a barrier given by its shared::cluster address, with the default release semantics.  What the arrival
+// stands for is never read by the other CTA's threads: V is read by the tensor core, for which the writer's
+// fence.proxy.async has made it visible, and a drained accumulator column has been read (tcgen05.wait::ld).  A
+// release at cluster scope would add a memory fence to every transform warp and K-step, and an acquire one to the
+// issuers: 510 instead of 212 us on 64x1024x1024x14x14 in BF16, 921 instead of 367 in TF32.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// TMA tiled load into this CTA's shared memory whose bytes are counted on a barrier of the pair's leader.
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap *map, uint32_t cluster_bar, int c0, int c1,
+                                                 int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(cluster_bar)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_512_pair(uint32_t smem_dst) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_dst) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_512_pair(uint32_t taddr) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(taddr) : "memory");
+}
+// Arrives on the barrier at this offset in both CTAs once all MMAs issued so far by this thread are complete.
+__device__ __forceinline__ void tc_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair_local(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+template <int DT>
+__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  if (DT == kTcBf16) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+  }
+}
+
+// One 32-image block of the input at one 2x2-output tile.
+struct PairBlock { int nb, tx, ty; };
+__device__ __forceinline__ PairBlock pair_block(const WinoParams &p, int q) {
+  PairBlock b;
+  b.nb = q % p.n_blocks; q /= p.n_blocks;
+  b.tx = q % p.tiles_w;
+  b.ty = q / p.tiles_w;
+  return b;
+}
+
+// p.n_blocks counts 32-image blocks, p.k_blocks 128-filter blocks, p.blocks blocks of images over all
+// tiles, p.total_tiles pair tiles (k_blocks times half of those).
+template <int DT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
+  using Cfg = PairCfg<DT>;
+  constexpr int SR = Cfg::kRawStages, SU = Cfg::kUStages, SV = Cfg::kVStages, KC = Cfg::kKC;
+  extern __shared__ __align__(1024) uint8_t psmem[];
+  uint8_t *raw_s = psmem;
+  uint8_t *u_s = raw_s + SR * Cfg::kRawBytes;
+  uint8_t *v_s = u_s + SU * Cfg::kUBytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(v_s + SV * kTcVBytes);
+  uint64_t *raw_full = bars, *raw_empty = raw_full + SR, *u_full = raw_empty + SR, *u_empty = u_full + SU,
+           *v_ready = u_empty + SU, *v_empty = v_ready + SV;
+  uint64_t *acc_full = v_empty + SV, *mma_done = acc_full + 1, *acc_empty = acc_full + 3;   // mma_done[2], acc_empty[4]
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 7);
+  volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 8);
+  static_assert((2 * SR + 2 * SU + 2 * SV + 9) * 8 <= 512, "barriers");
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
+  const uint32_t rank = cluster_ctarank();
+  const int cid = (int)blockIdx.x >> 1, n_clusters = (int)gridDim.x >> 1;
+  const int my_tiles = (p.total_tiles - cid + n_clusters - 1) / n_clusters;
+  const int blocks = p.blocks, pairs = (blocks + 1) / 2;
+  const int cpt = p.chunks_per_tile;
+  const int total_steps = my_tiles * cpt;
+
+  if (tid == 0) {
+    *dead = 0;
+    for (int s = 0; s < SR; ++s) {
+      mbar_init(smem_u32(raw_full + s), 1);
+      mbar_init(smem_u32(raw_empty + s), kTcTransformWarps);
+    }
+    for (int s = 0; s < SU; ++s) {
+      mbar_init(smem_u32(u_full + s), 1);                              // leader only: its loader, with both CTAs' bytes
+      mbar_init(smem_u32(u_empty + s), 2);                             // one commit per issuing warp
+    }
+    for (int s = 0; s < SV; ++s) {
+      mbar_init(smem_u32(v_ready + s), 2 * kTcTransformWarps);         // leader only: the transform warps of both CTAs
+      mbar_init(smem_u32(v_empty + s), 2);
+    }
+    mbar_init(smem_u32(acc_full), 2);
+    for (int j = 0; j < 4; ++j) mbar_init(smem_u32(acc_empty + j), 2 * kTcEpilogueWarps);   // leader only
+    mbar_init(smem_u32(mma_done + 0), 1);
+    mbar_init(smem_u32(mma_done + 1), 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  if (warp == kTcMmaWarp) tmem_alloc_512_pair(smem_u32(tmem_slot));
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                     // the peer's barriers exist before anything arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ===================================== patches =============================================
+    if (lane == 0) {
+      tma_prefetch_descriptor(&tm_in);
+      int g = 0;
+      bool ok = true;
+      for (int seq = 0; seq < my_tiles && ok; ++seq) {
+        const int q = 2 * ((cid + seq * n_clusters) % pairs) + (int)rank;
+        const PairBlock b = pair_block(p, q < blocks ? q : 0);         // an odd last block is paired with a spare one, not stored
+        for (int ci = 0; ci < cpt; ++ci, ++g) {
+          const int s = g % SR;
+          const uint32_t use = g / SR;
+          // A wait that gave up: stop issuing - the stage may still be in use.
+          if (use > 0 && !mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+          mbar_arrive_expect_tx(smem_u32(raw_full + s), Cfg::kRawBytes);
+          tma_load_4d(smem_u32(raw_s + s * Cfg::kRawBytes), &tm_in, smem_u32(raw_full + s), b.nb * kTcN, 2 * b.tx - 1,
+                      2 * b.ty - 1, ci * KC);
+        }
+      }
+      // No exit with bulk copies in flight (after a complete run these phases are long over).
+      for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
+    }
+  } else if (warp == kTcULoaderWarp) {
+    // ===================================== filter slices =======================================
+    if (lane == 0) {
+      tma_prefetch_descriptor(&tm_u);
+      constexpr int kRowBlocks = kPairFilters / (DT == kTcBf16 ? 64 : 32);   // 128-byte rows of a CTA's 64 filters
+      int g = 0;
+      bool ok = true;
+      for (int seq = 0; seq < my_tiles && ok; ++seq) {
+        const int kb = (cid + seq * n_clusters) / pairs;
+        for (int ci = 0; ci < cpt; ++ci, ++g) {
+          const int s = g % SU;
+          const uint32_t use = g / SU;
+          if (use > 0 && !mbar_wait(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(u_full + s), 2 * Cfg::kUBytes);
+          tma_load_4d_pair(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, map_to_rank(smem_u32(u_full + s), 0), 0, ci * KC,
+                           (2 * kb + (int)rank) * kRowBlocks, 0);
+        }
+      }
+      // The slices land before the MMAs that read them, whose completion is what these phases stand for.
+      for (int i = g > SU ? g - SU : 0; i < g; ++i) mbar_wait_drain(smem_u32(u_empty + i % SU), (i / SU) & 1);
+    }
+  } else if (warp <= kTcTransformWarps) {
+    // ===================================== input transform =====================================
+    const int t = tid - 32;                                            // 0..127: channel t >> 4 (BF16: and + 8), image pair t & 15
+    for (int g = 0; g < total_steps; ++g) {
+      const int sv = g % SV, sr = g % SR;
+      const uint32_t use = g / SV;
+      mbar_wait(smem_u32(raw_full + sr), (g / SR) & 1, dead, p.status);
+      if (use > 0) mbar_wait(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status);   // V stage free again
+      const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
+      if (DT == kTcBf16) transform_to_v_bf16_x2(raw, v_s + sv * kTcVBytes, t >> 4, t & 15);
+      else               transform_to_v_tf32_pair(raw, v_s + sv * kTcVBytes, t >> 4, t & 15);
+      fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(smem_u32(raw_empty + sr));
+        mbar_arrive_cluster(map_to_rank(smem_u32(v_ready + sv), 0));
+      }
+    }
+    // the leader's commits arrive here until the end: do not leave before the last ones have
+    for (int i = total_steps > SV ? total_steps - SV : 0; i < total_steps; ++i)
+      mbar_wait(smem_u32(v_empty + i % SV), (i / SV) & 1, dead, p.status);
+  } else if (warp == kTcMmaWarp || warp == kTcMmaWarpB) {
+    // ============================ MMA issuers (leader: two warps, two position columns each) ===
+    if (rank == 0) {
+      const int me = warp == kTcMmaWarp ? 0 : 1;
+      const int col0 = 2 * me;                         // columns col0, col0 + 1 of the 4x4 positions, column by column
+      constexpr uint32_t fmt = DT == kTcBf16 ? 1u : 2u;
+      // fp32 accumulate, both operands MN-major, M = 128 and N = 64 over the pair
+      constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) |
+                                 ((uint32_t)(2 * kTcN >> 3) << 17) | ((uint32_t)(2 * kPairFilters >> 4) << 24);
+      // A (this CTA's 64 filters; the peer's lie at the same offsets): BF16 rows of 128 B = all 64 filters (128-byte
+      // swizzle), 8-channel groups 1 KB apart; TF32 rows of 32 filters (128-byte swizzle with 32-byte atoms),
+      // 4-channel groups 512 B apart, the second 32 filters 1 KB further.  B (32 images) as in wino_tc.cuh.
+      const uint64_t a_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(u_s), 2048, 1024, 2) : smem_desc(smem_u32(u_s), 1024, 512, 1);
+      const uint64_t b_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(v_s), 512, 512, 4) : smem_desc(smem_u32(v_s), 1024, 512, 1);
+      int ci = 0, seq = 0;
+      for (int g = 0; g < total_steps; ++g) {
+        const int su = g % SU, sv = g % SV;
+        // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + su), (g / SU) & 1, dead, p.status))) break;
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status))) break;
+        tc_fence_after();
+        const uint64_t ad = a_desc0 + (uint64_t)(su * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (Cfg::kUPosBytes >> 4)),
+                       bd = b_desc0 + (uint64_t)(sv * (kTcVBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
+        const uint32_t accumulate = ci > 0 ? 1u : 0u, d0 = tmem_base + col0 * kTcN;
+        bool ok = true;
+#pragma unroll
+        for (int xo = 0; xo < 8; ++xo) {
+          const int xr = 4 * (xo & 3) + (xo >> 2);     // position relative to col0: row xo & 3, column xo >> 2
+          if ((xo & 3) == 0 && ci == 0 && seq > 0) {   // first write to a column of a new tile: drained in both CTAs?
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
+            tc_fence_after();
+          }
+          if (elect_one()) tc_mma_pair<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (Cfg::kUPosBytes >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc,
+                          accumulate);
+        }
+        if (!ok) break;
+        if (elect_one()) tc_commit_both(smem_u32(v_empty + sv));
+        if (elect_one()) tc_commit_both(smem_u32(u_empty + su));
+        if (++ci == cpt) {
+          if (elect_one()) tc_commit_both(smem_u32(acc_full));              // tile finished
+          ci = 0;
+          ++seq;
+        }
+      }
+      // Tensor memory is freed at the end of the kernel: every MMA this thread issued must have completed by then.
+      if (elect_one()) tc_commit_pair_local(smem_u32(mma_done + me));
+      mbar_wait_drain(smem_u32(mma_done + me), 0);
+    }
+  } else {
+    // ===================================== epilogue ============================================
+    const int quarter = warp & 3;                                        // TMEM lanes this warp may read
+    const int sub = (warp - kTcFirstEpilogueWarp) >> 2;                  // 0 / 1: which 16 of the block's 32 images
+    const int ib = quarter >> 1;                                         // image block of the pair
+    const uint32_t tcol = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * sub;
+    const size_t plane = (size_t)p.H * p.W * p.N;
+    const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
+    for (int seq = 0; seq < my_tiles; ++seq) {
+      const int t = cid + seq * n_clusters, q = 2 * (t % pairs) + ib;
+      const PairBlock b = pair_block(p, q < blocks ? q : 0);
+      const int k0 = (t / pairs) * 2 * kPairFilters + (int)rank * kPairFilters + 32 * (quarter & 1);
+      const int n0 = b.nb * kTcN + 16 * sub;
+      mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
+      tc_fence_after();
+      tc_epilogue_16x32(tcol, q < blocks && k0 < p.K, p, k0 + lane, n0, 2 * b.ty, 2 * b.tx,
+                        [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
+    }
+  }
+
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                     // nobody still reads or signals the other CTA's shared memory
+  if (warp == kTcMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc_512_pair(tmem_base);
+  }
+  __syncwarp();
+  cluster_sync_all();                     // both halves of the allocation are given back by running CTAs
+}
+
+}  // namespace ocb

@@ -238,6 +238,79 @@ __device__ __forceinline__ void transform_to_v_tf32_pair(const float *__restrict
     }
   }
 }
+// Epilogue of one warp: 32 filters (its TMEM lanes; `k` is this lane's) x 16 images (accumulator columns from
+// `tcol`, images from `n0`) of the 2x2-output tile at (oh0, ow0).  A warp that is not `active` only hands the
+// accumulators back.
+template <class Release>
+__device__ __forceinline__ void tc_epilogue_16x32(uint32_t tcol, bool active, const WinoParams &p, int k, int n0, int oh0, int ow0,
+                                                  Release release) {
+  const int lane = threadIdx.x & 31;
+  const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
+  const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = (size_t)p.H * dH;
+  float *ybase = p.y + (size_t)k * plane + ((size_t)oh0 * p.W + ow0) * p.N + n0;
+  // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
+  // row sums a[j], a[4+j] of output_transform, which are folded into the four outputs at once - the same
+  // operations in the same order.  After a column has been read it is handed back (release(j)), so the
+  // MMAs of the next tile into those four accumulators overlap the rest of this epilogue.
+  float y[4][4][4];                                                  // [image quad][output position][image]
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (active) {
+        float mm[2][4][4];                                           // [quad of this half][row][image]
+#pragma unroll
+        for (int q2 = 0; q2 < 2; ++q2)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) tmem_ld_x4(tcol + (4 * r + j) * kTcN + 8 * h + 4 * q2, mm[q2][r]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q2 = 0; q2 < 2; ++q2)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float lo = __fadd_rn(__fadd_rn(mm[q2][0][e], mm[q2][1][e]), mm[q2][2][e]);
+            const float hi = __fsub_rn(__fsub_rn(mm[q2][1][e], mm[q2][2][e]), mm[q2][3][e]);
+            float(&yy)[4][4] = y[2 * h + q2];
+            if (j == 0) { yy[0][e] = lo; yy[2][e] = hi; }
+            if (j == 1) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = lo; yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = hi; }
+            if (j == 2) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = __fsub_rn(yy[1][e], lo);
+                          yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = __fsub_rn(yy[3][e], hi); }
+            if (j == 3) { yy[1][e] = __fsub_rn(yy[1][e], lo); yy[3][e] = __fsub_rn(yy[3][e], hi); }
+          }
+      }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) release(j);
+  }
+  // Stores: neighbouring lanes (filters) swap halves of their 16 images, so that one instruction writes the
+  // 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter - 16 lines of
+  // two full sectors per instruction instead of 32 lines of one (see wino_tc_kernel).
+  if (active) {
+    const bool odd = (lane & 1) != 0;
+    float *pair_base = ybase - (odd ? plane : 0) + (odd ? 8 : 0);           // even filter of the pair, this lane's half
+    const bool n_ok = n0 + (odd ? 8 : 0) < p.N;            // N is a multiple of 8
+    const bool ok_even = n_ok && (k - (odd ? 1 : 0)) < p.K, ok_odd = n_ok && (k + (odd ? 0 : 1)) < p.K;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float ev[2][4], od[2][4];             // this lane's half of the even / odd filter's 64 bytes
+#pragma unroll
+      for (int q2 = 0; q2 < 2; ++q2)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float lo = y[q2][q][e], hi = y[2 + q2][q][e];                // images 0-7 / 8-15 of this lane's filter
+          const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
+          ev[q2][e] = odd ? got : lo;
+          od[q2][e] = odd ? hi : got;
+        }
+      const bool here = (q == 0) || (q == 1 && col1) || (q == 2 && row1) || (q == 3 && row1 && col1);
+      float *dst = pair_base + ((q & 1) ? dW : 0) + ((q & 2) ? dH : 0);
+      if (here && ok_even) st_global_v8(dst, ev[0], ev[1]);
+      if (here && ok_odd) st_global_v8(dst + plane, od[0], od[1]);
+    }
+  }
+}
+
 // True when the tile's accumulator rows 64-127 repeat rows 0-63 (see the MMA issuer).
 template <int DT> __device__ __forceinline__ bool tile_repeats_filters(const WinoParams &p, const TileCoord &tc) {
   return DT == kTcBf16 && p.K - tc.kb * kTcM <= 64;

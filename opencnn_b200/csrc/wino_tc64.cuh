@@ -32,9 +32,20 @@
 // positions each, warps 6-13 are the epilogue (quarters 0,1 store image block 0, quarters 2,3
 // image block 1).  All hand-offs are mbarriers with bounded waits.
 #pragma once
-#include "wino_tc2.cuh"   // P2Tile / p2_decode (tiles over pairs of image blocks), wino_tc.cuh
+#include "wino_tc.cuh"
 
 namespace ocb {
+
+// A tile over two 32-image blocks, 2*np and 2*np + 1.
+struct T64Tile { int np, tx, ty, kb; };
+__device__ __forceinline__ T64Tile t64_decode(const WinoParams &p, int t, int n_pairs) {
+  T64Tile tc;
+  tc.np = t % n_pairs; t /= n_pairs;
+  tc.tx = t % p.tiles_w; t /= p.tiles_w;
+  tc.ty = t % p.tiles_h;
+  tc.kb = t / p.tiles_h;
+  return tc;
+}
 
 constexpr int kT64RawStages = 3, kT64UStages = 2, kT64VStages = 3;
 constexpr uint32_t kT64ZeroBytes = 2048;                   // one empty half of an A operand (64 filter rows x one K-step)
@@ -117,7 +128,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     if (lane == 0) {
       tma_prefetch_descriptor(loads_u ? &tm_u : &tm_in);
       int seq = 0, ci = 0, issued = 0;
-      P2Tile tc = p2_decode(p, (int)blockIdx.x, n_pairs);
+      T64Tile tc = t64_decode(p, (int)blockIdx.x, n_pairs);
       const int ring = loads_u ? SU : SR;
       const int count = loads_u ? total_steps : total_sub;             // U once per K-step, patches once per sub-step
       for (int g = 0; g < count; ++g) {
@@ -139,7 +150,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
           if (++ci == cpt) {
             ci = 0;
             ++seq;
-            if (seq < my_tiles) tc = p2_decode(p, (int)blockIdx.x + seq * (int)gridDim.x, n_pairs);
+            if (seq < my_tiles) tc = t64_decode(p, (int)blockIdx.x + seq * (int)gridDim.x, n_pairs);
           }
         }
       }
@@ -234,79 +245,15 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     const int fq = quarter & 1, ib = quarter >> 1;                       // filters 32*fq .. +31 of image block ib
     const int k = fq * 32 + lane;
     const bool warp_valid = fq * 32 < p.K;
-    const size_t plane = (size_t)p.H * p.W * p.N;
-    const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N;
     const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
     for (int seq = 0; seq < my_tiles; ++seq) {
-      const P2Tile tc = p2_decode(p, (int)blockIdx.x + seq * (int)gridDim.x, n_pairs);
+      const T64Tile tc = t64_decode(p, (int)blockIdx.x + seq * (int)gridDim.x, n_pairs);
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
       const int nb = 2 * tc.np + ib;                                     // 32-image block this warp stores
-      const int oh0 = 2 * tc.ty, ow0 = 2 * tc.tx;
-      const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
-      float *ybase = p.y + (size_t)k * plane + ((size_t)oh0 * p.W + ow0) * p.N + (size_t)nb * kTcN + 16 * sub;
       const bool active = warp_valid && nb < p.n_blocks;
-      // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
-      // row sums a[j], a[4+j] of output_transform, which are folded into the four outputs at once - the same
-      // operations in the same order.  After a column has been read it is handed back (acc_empty[j]), so the
-      // MMAs of the next tile into those four accumulators overlap the rest of this epilogue.
-      float y[4][4][4];                                                  // [image quad][output position][image]
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (active) {
-            float mm[2][4][4];                                           // [quad of this half][row][image]
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-              for (int r = 0; r < 4; ++r) tmem_ld_x4(tlane + (4 * r + j) * kTcN + 16 * sub + 8 * h + 4 * q2, mm[q2][r]);
-            tmem_ld_wait();
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float lo = __fadd_rn(__fadd_rn(mm[q2][0][e], mm[q2][1][e]), mm[q2][2][e]);
-                const float hi = __fsub_rn(__fsub_rn(mm[q2][1][e], mm[q2][2][e]), mm[q2][3][e]);
-                float(&yy)[4][4] = y[2 * h + q2];
-                if (j == 0) { yy[0][e] = lo; yy[2][e] = hi; }
-                if (j == 1) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = lo; yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = hi; }
-                if (j == 2) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = __fsub_rn(yy[1][e], lo);
-                              yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = __fsub_rn(yy[3][e], hi); }
-                if (j == 3) { yy[1][e] = __fsub_rn(yy[1][e], lo); yy[3][e] = __fsub_rn(yy[3][e], hi); }
-              }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(acc_empty + j));
-      }
-      // Stores: neighbouring lanes (filters) swap halves of their 16 images, so that one instruction writes the
-      // 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter - 16 lines of
-      // two full sectors per instruction instead of 32 lines of one (see wino_tc_kernel).
-      if (active) {
-        const bool odd = (lane & 1) != 0;
-        float *pair_base = ybase - (odd ? plane : 0) + (odd ? 8 : 0);           // even filter of the pair, this lane's half
-        const bool n_ok = nb * kTcN + 16 * sub + (odd ? 8 : 0) < p.N;            // N is a multiple of 8
-        const bool ok_even = n_ok && (k - (odd ? 1 : 0)) < p.K, ok_odd = n_ok && (k + (odd ? 0 : 1)) < p.K;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float ev[2][4], od[2][4];             // this lane's half of the even / odd filter's 64 bytes
-#pragma unroll
-          for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float lo = y[q2][q][e], hi = y[2 + q2][q][e];                // images 0-7 / 8-15 of this lane's filter
-              const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
-              ev[q2][e] = odd ? got : lo;
-              od[q2][e] = odd ? hi : got;
-            }
-          const bool here = (q == 0) || (q == 1 && col1) || (q == 2 && row1) || (q == 3 && row1 && col1);
-          float *dst = pair_base + ((q & 1) ? dW : 0) + ((q & 2) ? dH : 0);
-          if (here && ok_even) st_global_v8(dst, ev[0], ev[1]);
-          if (here && ok_odd) st_global_v8(dst + plane, od[0], od[1]);
-        }
-      }
+      tc_epilogue_16x32(tlane + 16 * sub, active, p, k, nb * kTcN + 16 * sub, 2 * tc.ty, 2 * tc.tx,
+                        [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }
 

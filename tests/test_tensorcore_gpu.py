@@ -211,3 +211,26 @@ def test_stacked_blocks_kernel(oracle, libs, precision):
     # refused: more than 64 filters
     z = torch.zeros(1 << 16, device="cuda")
     assert api.winograd_forward_kernel(z, z, z, 64, 16, 4, 4, 128, precision=precision, kernel="stacked") != 0
+
+
+# The CTA-pair kernel against the single-CTA kernel, which issues the same products in the same order: one image block
+# (the pair's second half is empty), an odd number of them, a pair that spans two tiles, a second CTA without filters,
+# fewer K-steps than ring stages, more pairs than fit on the device at once.
+PAIR_SHAPES = [(8, 16, 128, 2, 2), (32, 24, 128, 5, 5), (40, 3, 192, 3, 5), (96, 72, 64, 3, 3), (24, 100, 320, 9, 4),
+               (160, 40, 192, 17, 23)]
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("shape", PAIR_SHAPES)
+def test_pair_kernel_gives_the_bits_of_the_single_cta_kernel(libs, precision, shape):
+    N, C, K, H, W = shape
+    x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
+    ws = torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(torch.randn((C, 3, 3, K), device="cuda") * 0.05, ws, C, K, precision=precision) == 0
+    out = {}
+    for kernel in ("single", "pair_local"):
+        out[kernel] = torch.full((K, H, W, N), float("nan"), device="cuda")
+        assert api.winograd_forward_kernel(x, ws, out[kernel], N, C, H, W, K, precision=precision, kernel=kernel) == 0
+        assert api.last_device_status() == 0
+    assert bool(torch.isfinite(out["single"]).all().item())
+    assert torch.equal(out["single"], out["pair_local"])
