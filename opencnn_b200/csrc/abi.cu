@@ -90,6 +90,11 @@ cudaError_t device_state(DeviceState **out) {
       if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_fp32_kernel<OCB_VARIANT, true>);
       if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
+      // the same for the CTA-pair kernel
+      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcBf16>);
+      if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcTf32>);
+      if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
     }
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_tc_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,

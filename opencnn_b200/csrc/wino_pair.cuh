@@ -20,7 +20,7 @@
 // The two image blocks need not belong together: block q of the list (tile row, tile column, image
 // block), image blocks fastest, pairs with block q + 1, so that only the very last pair can be half empty.
 //
-// Warp roles as in wino_tc.cuh (512 threads per CTA).  Barriers: the patches' ring is each CTA's own.
+// Barriers: the patches' ring is each CTA's own.
 // "Filter slice landed" and "V written" are barriers of the leading CTA (rank 0), whose two issuing
 // warps wait for both CTAs' halves there; the tensor core's commits reach the "free again" and "tile
 // finished" barriers of both CTAs (multicast arrive); a drained accumulator column is reported to the
@@ -30,16 +30,37 @@
 
 namespace ocb {
 
-constexpr int kPairThreads = 512;
+// What bounds it: the bytes in flight per SM - patches and filter slices of a K-step are 64 KB (BF16), the three-deep rings
+// of 96 KB each turn over in one load latency - and the transform's shared-memory round trip.  Kernel alone, four
+// transform warps (512 threads) -> eight: 64x1024x1024x14x14 199 -> 196 us in BF16 and 355 -> 321 in TF32,
+// 128x256x256x14x14 36.2 -> 35.4 and 56.0 -> 46.2, 128x64x128x56x56 93.5 -> 91.3 and 124 -> 115; a single K-step per
+// tile loses (256x8x128x56x56 91.0 -> 93.4 and 87.1 -> 90.8).  Handing the patches back as soon as they are in
+// registers, with a proxy fence of its own, gained nothing (203 / 323).
+// Five warpgroups: warps 0 and 1 load patches and filter slices, 2 and 3 issue the MMAs; warps 4-11 transform;
+// warps 12-19 are the epilogue.  Registers are shared out with setmaxnreg.
+constexpr int kPairThreads = 640;
+constexpr int kPairTransformWarps = 8, kPairFirstTransformWarp = 4, kPairFirstEpilogueWarp = 12, kPairMmaWarp = 2;
+constexpr int kPairLaunchRegs = 96, kPairIssueRegs = 64, kPairTransformRegs = 80, kPairEpilogueRegs = 128;
+static_assert(kPairIssueRegs + 2 * kPairTransformRegs + 2 * kPairEpilogueRegs <= 5 * kPairLaunchRegs,
+              "setmaxnreg budgets exceed the registers the CTA was launched with");
 constexpr int kPairFilters = 64;                 // per CTA
 template <int DT> struct PairCfg {
   static constexpr int kKC = DT == kTcBf16 ? 16 : 8;                       // channels per K-step
   static constexpr uint32_t kRawBytes = kKC * 16 * kTcN * 4;               // [c][4 h][4 w][32 n] fp32
   static constexpr uint32_t kUPosBytes = 2048;                             // 64 filters x one K-step
   static constexpr uint32_t kUBytes = 16 * kUPosBytes;
+  // Ring depths: what fits in 227 KB.  Fewer than three stages of patches starve the BF16 kernel (two: 229-270 us
+  // instead of 208 on 64x1024x1024x14x14), fewer than three of filters the TF32 kernel (two: 467 instead of 330).
   static constexpr int kRawStages = DT == kTcBf16 ? 3 : 4;
   static constexpr int kUStages = 3;
   static constexpr int kVStages = DT == kTcBf16 ? 2 : 4;
+  // Transform warps that share a K-step: all eight in BF16 (16 channels x 16 image pairs, one item per thread); in
+  // TF32 (8 channels) two groups of four take the K-steps in turn.
+  static constexpr int kStepWarps = DT == kTcBf16 ? 8 : 4;
+  // A group has to come back to the same stages: were a stage shared by two groups, a group could wait on it two phases
+  // ahead of the other, which the parity of a barrier does not tell from the phase before.
+  static constexpr int kGroups = kPairTransformWarps / kStepWarps;
+  static_assert(kRawStages % kGroups == 0 && kVStages % kGroups == 0, "ring depths are multiples of the group count");
   static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kUStages * kUBytes +
                                        (size_t)kVStages * kTcVBytes + 512;
   static_assert(kSmemBytes <= 232448, "shared memory");
@@ -147,14 +168,14 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     *dead = 0;
     for (int s = 0; s < SR; ++s) {
       mbar_init(smem_u32(raw_full + s), 1);
-      mbar_init(smem_u32(raw_empty + s), kTcTransformWarps);
+      mbar_init(smem_u32(raw_empty + s), Cfg::kStepWarps);
     }
     for (int s = 0; s < SU; ++s) {
       mbar_init(smem_u32(u_full + s), 1);                              // leader only: its loader, with both CTAs' bytes
       mbar_init(smem_u32(u_empty + s), 2);                             // one commit per issuing warp
     }
     for (int s = 0; s < SV; ++s) {
-      mbar_init(smem_u32(v_ready + s), 2 * kTcTransformWarps);         // leader only: the transform warps of both CTAs
+      mbar_init(smem_u32(v_ready + s), 2 * Cfg::kStepWarps);           // leader only: the transform warps of both CTAs
       mbar_init(smem_u32(v_empty + s), 2);
     }
     mbar_init(smem_u32(acc_full), 2);
@@ -164,132 +185,20 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     mbar_fence_init();
   }
   __syncwarp();
-  if (warp == kTcMmaWarp) tmem_alloc_512_pair(smem_u32(tmem_slot));
+  if (warp == kPairMmaWarp) tmem_alloc_512_pair(smem_u32(tmem_slot));
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                     // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    // ===================================== patches =============================================
-    if (lane == 0) {
-      tma_prefetch_descriptor(&tm_in);
-      int g = 0;
-      bool ok = true;
-      for (int seq = 0; seq < my_tiles && ok; ++seq) {
-        const int q = 2 * ((cid + seq * n_clusters) % pairs) + (int)rank;
-        const PairBlock b = pair_block(p, q < blocks ? q : 0);         // an odd last block is paired with a spare one, not stored
-        for (int ci = 0; ci < cpt; ++ci, ++g) {
-          const int s = g % SR;
-          const uint32_t use = g / SR;
-          // A wait that gave up: stop issuing - the stage may still be in use.
-          if (use > 0 && !mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
-          mbar_arrive_expect_tx(smem_u32(raw_full + s), Cfg::kRawBytes);
-          tma_load_4d(smem_u32(raw_s + s * Cfg::kRawBytes), &tm_in, smem_u32(raw_full + s), b.nb * kTcN, 2 * b.tx - 1,
-                      2 * b.ty - 1, ci * KC);
-        }
-      }
-      // No exit with bulk copies in flight (after a complete run these phases are long over).
-      for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
-    }
-  } else if (warp == kTcULoaderWarp) {
-    // ===================================== filter slices =======================================
-    if (lane == 0) {
-      tma_prefetch_descriptor(&tm_u);
-      constexpr int kRowBlocks = kPairFilters / (DT == kTcBf16 ? 64 : 32);   // 128-byte rows of a CTA's 64 filters
-      int g = 0;
-      bool ok = true;
-      for (int seq = 0; seq < my_tiles && ok; ++seq) {
-        const int kb = (cid + seq * n_clusters) / pairs;
-        for (int ci = 0; ci < cpt; ++ci, ++g) {
-          const int s = g % SU;
-          const uint32_t use = g / SU;
-          if (use > 0 && !mbar_wait(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
-          if (rank == 0) mbar_arrive_expect_tx(smem_u32(u_full + s), 2 * Cfg::kUBytes);
-          tma_load_4d_pair(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, map_to_rank(smem_u32(u_full + s), 0), 0, ci * KC,
-                           (2 * kb + (int)rank) * kRowBlocks, 0);
-        }
-      }
-      // The slices land before the MMAs that read them, whose completion is what these phases stand for.
-      for (int i = g > SU ? g - SU : 0; i < g; ++i) mbar_wait_drain(smem_u32(u_empty + i % SU), (i / SU) & 1);
-    }
-  } else if (warp <= kTcTransformWarps) {
-    // ===================================== input transform =====================================
-    const int t = tid - 32;                                            // 0..127: channel t >> 4 (BF16: and + 8), image pair t & 15
-    for (int g = 0; g < total_steps; ++g) {
-      const int sv = g % SV, sr = g % SR;
-      const uint32_t use = g / SV;
-      mbar_wait(smem_u32(raw_full + sr), (g / SR) & 1, dead, p.status);
-      if (use > 0) mbar_wait(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status);   // V stage free again
-      const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
-      if (DT == kTcBf16) transform_to_v_bf16_x2(raw, v_s + sv * kTcVBytes, t >> 4, t & 15);
-      else               transform_to_v_tf32_pair(raw, v_s + sv * kTcVBytes, t >> 4, t & 15);
-      fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(smem_u32(raw_empty + sr));
-        mbar_arrive_cluster(map_to_rank(smem_u32(v_ready + sv), 0));
-      }
-    }
-    // the leader's commits arrive here until the end: do not leave before the last ones have
-    for (int i = total_steps > SV ? total_steps - SV : 0; i < total_steps; ++i)
-      mbar_wait(smem_u32(v_empty + i % SV), (i / SV) & 1, dead, p.status);
-  } else if (warp == kTcMmaWarp || warp == kTcMmaWarpB) {
-    // ============================ MMA issuers (leader: two warps, two position columns each) ===
-    if (rank == 0) {
-      const int me = warp == kTcMmaWarp ? 0 : 1;
-      const int col0 = 2 * me;                         // columns col0, col0 + 1 of the 4x4 positions, column by column
-      constexpr uint32_t fmt = DT == kTcBf16 ? 1u : 2u;
-      // fp32 accumulate, both operands MN-major, M = 128 and N = 64 over the pair
-      constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) |
-                                 ((uint32_t)(2 * kTcN >> 3) << 17) | ((uint32_t)(2 * kPairFilters >> 4) << 24);
-      // A (this CTA's 64 filters; the peer's lie at the same offsets): BF16 rows of 128 B = all 64 filters (128-byte
-      // swizzle), 8-channel groups 1 KB apart; TF32 rows of 32 filters (128-byte swizzle with 32-byte atoms),
-      // 4-channel groups 512 B apart, the second 32 filters 1 KB further.  B (32 images) as in wino_tc.cuh.
-      const uint64_t a_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(u_s), 2048, 1024, 2) : smem_desc(smem_u32(u_s), 1024, 512, 1);
-      const uint64_t b_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(v_s), 512, 512, 4) : smem_desc(smem_u32(v_s), 1024, 512, 1);
-      int ci = 0, seq = 0;
-      for (int g = 0; g < total_steps; ++g) {
-        const int su = g % SU, sv = g % SV;
-        // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + su), (g / SU) & 1, dead, p.status))) break;
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status))) break;
-        tc_fence_after();
-        const uint64_t ad = a_desc0 + (uint64_t)(su * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (Cfg::kUPosBytes >> 4)),
-                       bd = b_desc0 + (uint64_t)(sv * (kTcVBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
-        const uint32_t accumulate = ci > 0 ? 1u : 0u, d0 = tmem_base + col0 * kTcN;
-        bool ok = true;
-#pragma unroll
-        for (int xo = 0; xo < 8; ++xo) {
-          const int xr = 4 * (xo & 3) + (xo >> 2);     // position relative to col0: row xo & 3, column xo >> 2
-          if ((xo & 3) == 0 && ci == 0 && seq > 0) {   // first write to a column of a new tile: drained in both CTAs?
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
-            tc_fence_after();
-          }
-          if (elect_one()) tc_mma_pair<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (Cfg::kUPosBytes >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc,
-                          accumulate);
-        }
-        if (!ok) break;
-        if (elect_one()) tc_commit_both(smem_u32(v_empty + sv));
-        if (elect_one()) tc_commit_both(smem_u32(u_empty + su));
-        if (++ci == cpt) {
-          if (elect_one()) tc_commit_both(smem_u32(acc_full));              // tile finished
-          ci = 0;
-          ++seq;
-        }
-      }
-      // Tensor memory is freed at the end of the kernel: every MMA this thread issued must have completed by then.
-      if (elect_one()) tc_commit_pair_local(smem_u32(mma_done + me));
-      mbar_wait_drain(smem_u32(mma_done + me), 0);
-    }
-  } else {
+  if (warp >= kPairFirstEpilogueWarp) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPairEpilogueRegs));
     // ===================================== epilogue ============================================
     const int quarter = warp & 3;                                        // TMEM lanes this warp may read
-    const int sub = (warp - kTcFirstEpilogueWarp) >> 2;                  // 0 / 1: which 16 of the block's 32 images
+    const int sub = (warp - kPairFirstEpilogueWarp) >> 2;                  // 0 / 1: which 16 of the block's 32 images
     const int ib = quarter >> 1;                                         // image block of the pair
     const uint32_t tcol = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * sub;
-    const size_t plane = (size_t)p.H * p.W * p.N;
     const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
     for (int seq = 0; seq < my_tiles; ++seq) {
       const int t = cid + seq * n_clusters, q = 2 * (t % pairs) + ib;
@@ -301,13 +210,133 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       tc_epilogue_16x32(tcol, q < blocks && k0 < p.K, p, k0 + lane, n0, 2 * b.ty, 2 * b.tx,
                         [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
     }
+  } else if (warp >= kPairFirstTransformWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairTransformRegs));
+    // ===================================== input transform =====================================
+    constexpr int kGroups = Cfg::kGroups;
+    const int t = (tid - 32 * kPairFirstTransformWarp) % (32 * Cfg::kStepWarps);      // channel t >> 4, image pair t & 15
+    for (int g = (warp - kPairFirstTransformWarp) / Cfg::kStepWarps; g < total_steps; g += kGroups) {
+      const int sv = g % SV, sr = g % SR;
+      const uint32_t use = g / SV;
+      mbar_wait(smem_u32(raw_full + sr), (g / SR) & 1, dead, p.status);
+      const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
+      uint8_t *vst = v_s + sv * kTcVBytes;
+      uint64_t d[16];
+      load_patch_pair(raw, t >> 4, t & 15, d);
+      if (use > 0) mbar_wait(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status);   // V stage free again
+      if (DT == kTcBf16) finish_v_bf16(d, vst, t >> 4, t & 15);
+      else               finish_v_tf32(d, vst, t >> 4, t & 15);
+      fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(smem_u32(raw_empty + sr));     // behind the fence: TMA refills the stage
+        mbar_arrive_cluster(map_to_rank(smem_u32(v_ready + sv), 0));
+      }
+    }
+    // the leader's commits arrive here until the end: do not leave before the last ones have
+    for (int i = total_steps > SV ? total_steps - SV : 0; i < total_steps; ++i)
+      mbar_wait(smem_u32(v_empty + i % SV), (i / SV) & 1, dead, p.status);
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairIssueRegs));
+    if (warp == 0) {
+      // ===================================== patches =============================================
+      if (lane == 0) {
+        tma_prefetch_descriptor(&tm_in);
+        int g = 0;
+        bool ok = true;
+        for (int seq = 0; seq < my_tiles && ok; ++seq) {
+          const int q = 2 * ((cid + seq * n_clusters) % pairs) + (int)rank;
+          const PairBlock b = pair_block(p, q < blocks ? q : 0);         // an odd last block is paired with a spare one, not stored
+          for (int ci = 0; ci < cpt; ++ci, ++g) {
+            const int s = g % SR;
+            const uint32_t use = g / SR;
+            // A wait that gave up: stop issuing - the stage may still be in use.
+            if (use > 0 && !mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+            mbar_arrive_expect_tx(smem_u32(raw_full + s), Cfg::kRawBytes);
+            tma_load_4d(smem_u32(raw_s + s * Cfg::kRawBytes), &tm_in, smem_u32(raw_full + s), b.nb * kTcN, 2 * b.tx - 1,
+                        2 * b.ty - 1, ci * KC);
+          }
+        }
+        // No exit with bulk copies in flight (after a complete run these phases are long over).
+        for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
+      }
+    } else if (warp == 1) {
+      // ===================================== filter slices =======================================
+      if (lane == 0) {
+        tma_prefetch_descriptor(&tm_u);
+        constexpr int kRowBlocks = kPairFilters / (DT == kTcBf16 ? 64 : 32);   // 128-byte rows of a CTA's 64 filters
+        int g = 0;
+        bool ok = true;
+        for (int seq = 0; seq < my_tiles && ok; ++seq) {
+          const int kb = (cid + seq * n_clusters) / pairs;
+          for (int ci = 0; ci < cpt; ++ci, ++g) {
+            const int s = g % SU;
+            const uint32_t use = g / SU;
+            if (use > 0 && !mbar_wait(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+            if (rank == 0) mbar_arrive_expect_tx(smem_u32(u_full + s), 2 * Cfg::kUBytes);
+            tma_load_4d_pair(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, map_to_rank(smem_u32(u_full + s), 0), 0, ci * KC,
+                             (2 * kb + (int)rank) * kRowBlocks, 0);
+          }
+        }
+        // The slices land before the MMAs that read them, whose completion is what these phases stand for.
+        for (int i = g > SU ? g - SU : 0; i < g; ++i) mbar_wait_drain(smem_u32(u_empty + i % SU), (i / SU) & 1);
+      }
+    } else {
+      // ============================ MMA issuers (leader: two warps, two position columns each) ===
+      if (rank == 0) {
+        const int me = warp - kPairMmaWarp;
+        const int col0 = 2 * me;                         // columns col0, col0 + 1 of the 4x4 positions, column by column
+        constexpr uint32_t fmt = DT == kTcBf16 ? 1u : 2u;
+        // fp32 accumulate, both operands MN-major, M = 128 and N = 64 over the pair
+        constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) |
+                                   ((uint32_t)(2 * kTcN >> 3) << 17) | ((uint32_t)(2 * kPairFilters >> 4) << 24);
+        // A (this CTA's 64 filters; the peer's lie at the same offsets): BF16 rows of 128 B = all 64 filters (128-byte
+        // swizzle), 8-channel groups 1 KB apart; TF32 rows of 32 filters (128-byte swizzle with 32-byte atoms),
+        // 4-channel groups 512 B apart, the second 32 filters 1 KB further.  B (32 images) as in wino_tc.cuh.
+        const uint64_t a_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(u_s), 2048, 1024, 2) : smem_desc(smem_u32(u_s), 1024, 512, 1);
+        const uint64_t b_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(v_s), 512, 512, 4) : smem_desc(smem_u32(v_s), 1024, 512, 1);
+        int ci = 0, seq = 0;
+        for (int g = 0; g < total_steps; ++g) {
+          const int su = g % SU, sv = g % SV;
+          // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
+          if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + su), (g / SU) & 1, dead, p.status))) break;
+          if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status))) break;
+          tc_fence_after();
+          const uint64_t ad = a_desc0 + (uint64_t)(su * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (Cfg::kUPosBytes >> 4)),
+                         bd = b_desc0 + (uint64_t)(sv * (kTcVBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
+          const uint32_t accumulate = ci > 0 ? 1u : 0u, d0 = tmem_base + col0 * kTcN;
+          bool ok = true;
+#pragma unroll
+          for (int xo = 0; xo < 8; ++xo) {
+            const int xr = 4 * (xo & 3) + (xo >> 2);     // position relative to col0: row xo & 3, column xo >> 2
+            if ((xo & 3) == 0 && ci == 0 && seq > 0) {   // first write to a column of a new tile: drained in both CTAs?
+              if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
+              tc_fence_after();
+            }
+            if (elect_one()) tc_mma_pair<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (Cfg::kUPosBytes >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc,
+                            accumulate);
+          }
+          if (!ok) break;
+          if (elect_one()) tc_commit_both(smem_u32(v_empty + sv));
+          if (elect_one()) tc_commit_both(smem_u32(u_empty + su));
+          if (++ci == cpt) {
+            if (elect_one()) tc_commit_both(smem_u32(acc_full));              // tile finished
+            ci = 0;
+            ++seq;
+          }
+        }
+        // Tensor memory is freed at the end of the kernel: every MMA this thread issued must have completed by then.
+        if (elect_one()) tc_commit_pair_local(smem_u32(mma_done + me));
+        mbar_wait_drain(smem_u32(mma_done + me), 0);
+      }
+    }
   }
 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                     // nobody still reads or signals the other CTA's shared memory
-  if (warp == kTcMmaWarp) {
+  if (warp == kPairMmaWarp) {
     tc_fence_after();
     tmem_dealloc_512_pair(tmem_base);
   }

@@ -164,6 +164,13 @@ __global__ void __launch_bounds__(128) fx_tc_kernel(const float4 *__restrict__ g
   }
 }
 
+// The 4x4 patches of two adjacent images (pair np) of one channel of a stage.
+__device__ __forceinline__ void load_patch_pair(const float *__restrict__ raw, int c, int np, uint64_t (&d)[16]) {
+  const uint64_t *R = reinterpret_cast<const uint64_t *>(raw + (c * 16) * kTcN + 2 * np);
+#pragma unroll
+  for (int q = 0; q < 16; ++q) d[q] = R[q * (kTcN / 2)];
+}
+
 // ---- input transform into the V operand --------------------------------------------------------
 // BF16: item = (channel c of the stage, image pair np); V tile of a position is [16 c][32 n] bf16,
 // rows of 64 bytes, 64-byte swizzle (16-byte chunk index ^= (c >> 1) & 3).
@@ -208,12 +215,8 @@ __device__ __forceinline__ void transform_to_v_bf16_x2(const float *__restrict__
 // need (32-byte chunk index ^= c & 3; the pattern repeats every 4 rows).
 // Packed form: one item = (channel c, image pair np); the two images of a pair are adjacent in a
 // V row, so each result is one 8-byte store.  Same operations per image as the scalar form.
-__device__ __forceinline__ void transform_to_v_tf32_pair(const float *__restrict__ raw, uint8_t *__restrict__ vst, int c, int np) {
-  constexpr int P = kTcN / 2;
-  const uint64_t *R = reinterpret_cast<const uint64_t *>(raw + (c * 16) * kTcN + 2 * np);
-  uint64_t d[16], b[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) d[q] = R[q * P];
+__device__ __forceinline__ void finish_v_tf32(const uint64_t (&d)[16], uint8_t *__restrict__ vst, int c, int np) {
+  uint64_t b[16];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     b[j] = sub2(d[j], d[8 + j]);
@@ -238,6 +241,12 @@ __device__ __forceinline__ void transform_to_v_tf32_pair(const float *__restrict
     }
   }
 }
+__device__ __forceinline__ void transform_to_v_tf32_pair(const float *__restrict__ raw, uint8_t *__restrict__ vst, int c, int np) {
+  uint64_t d[16];
+  load_patch_pair(raw, c, np, d);
+  finish_v_tf32(d, vst, c, np);
+}
+
 // Epilogue of one warp: 32 filters (its TMEM lanes; `k` is this lane's) x 16 images (accumulator columns from
 // `tcol`, images from `n0`) of the 2x2-output tile at (oh0, ow0).  A warp that is not `active` only hands the
 // accumulators back.
