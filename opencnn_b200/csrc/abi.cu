@@ -171,6 +171,27 @@ cudaError_t check_shape(int N, int C, int H, int W, int K, ShapeRule rule) {
   return cudaSuccess;
 }
 
+// Launches a kernel that reads the transformed filter.  `after_fx`: the filter transform was the launch before it on this
+// stream, by this call, so its set-up (barriers, tensor memory, descriptors, the first patches) may overlap it; the
+// kernels wait for the transform's completion before their first load of U, and all other data is older than the
+// transform, which itself is launched the ordinary way.  Whole calls: fp32 32x16x64x9x9 12.3 -> 10.2 us,
+// 32x64x64x56x56 81.9 -> 79.7; TF32 128x128x128x28x28 63.0 -> 59.8.
+template <class... P, class... A>
+cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, bool after_fx, const A &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after_fx ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_fx(const float *filter, float *workspace, int C, int K, cudaStream_t stream) {
   const int k4 = K / 4;
   const int total = C * k4;
@@ -180,7 +201,7 @@ cudaError_t launch_fx(const float *filter, float *workspace, int C, int K, cudaS
 }
 
 cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *output, int N, int C, int H,
-                             int W, int K, cudaStream_t stream) {
+                             int W, int K, cudaStream_t stream, bool after_fx) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -233,10 +254,9 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
     p.total_items = p.split_from + 2 * rest;
   }
   if (N % ocb::kBN == 0 && K % ocb::kBK == 0)
-    ocb::wino_fp32_kernel<OCB_VARIANT, false><<<grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream>>>(tm_in, tm_u, p);
-  else   // ragged last block of images or filters: stores masked
-    ocb::wino_fp32_kernel<OCB_VARIANT, true><<<grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream>>>(tm_in, tm_u, p);
-  return cudaGetLastError();
+    return launch_main(ocb::wino_fp32_kernel<OCB_VARIANT, false>, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
+  // ragged last block of images or filters: stores masked
+  return launch_main(ocb::wino_fp32_kernel<OCB_VARIANT, true>, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // Tensor-core path: filter transform rounded to the operand type, then the tcgen05 kernel.
@@ -250,7 +270,7 @@ cudaError_t launch_fx_tc(const float *filter, float *workspace, int C, int K, cu
 
 template <int DT>
 cudaError_t launch_wino_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                           int K, cudaStream_t stream) {
+                           int K, cudaStream_t stream, bool after_fx) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -301,17 +321,15 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
   if (bf16 && K <= 64)
-    ocb::wino_tc_kernel<ocb::kTcBf16, true><<<grid, ocb::TcCfg<ocb::kTcBf16, true>::kThreads,
-                                              ocb::TcCfg<ocb::kTcBf16, true>::kSmemBytes, stream>>>(tm_in, tm_u, p);
-  else
-    ocb::wino_tc_kernel<DT><<<grid, ocb::TcCfg<DT>::kThreads, ocb::TcCfg<DT>::kSmemBytes, stream>>>(tm_in, tm_u, p);
-  return cudaGetLastError();
+    return launch_main(ocb::wino_tc_kernel<ocb::kTcBf16, true>, grid, ocb::TcCfg<ocb::kTcBf16, true>::kThreads,
+                       ocb::TcCfg<ocb::kTcBf16, true>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+  return launch_main(ocb::wino_tc_kernel<DT>, grid, ocb::TcCfg<DT>::kThreads, ocb::TcCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).
 template <int DT>
 cudaError_t launch_wino_pair(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                            int K, cudaStream_t stream) {
+                            int K, cudaStream_t stream, bool after_fx) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -362,14 +380,13 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  ocb::wino_pair_kernel<DT><<<2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream>>>(tm_in, tm_u, p);
-  return cudaGetLastError();
+  return launch_main(ocb::wino_pair_kernel<DT>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // Layers with at most 64 filters: two 32-image blocks share the 128 accumulator rows (wino_tc64.cuh).
 template <int DT>
 cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                             int K, cudaStream_t stream) {
+                             int K, cudaStream_t stream, bool after_fx) {
   if (K > 64) return cudaErrorInvalidValue;
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
@@ -419,8 +436,7 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
-  ocb::wino_tc64_kernel<DT><<<grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream>>>(tm_in, tm_u, p);
-  return cudaGetLastError();
+  return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // Which tensor-core kernel a problem gets.  All three give the same bits.  Medians, L2 flushed, bf16 / tf32 us.
@@ -436,10 +452,10 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
 //     32x64x64x28x28 15.4 : 17.5 : 19.5 / 21.5 : 21.5 : 26.6    32x512x64x28x28 51 : 47 : 76 / 92 : 72 : 133
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
-                      cudaStream_t stream, int kernel = OPENCNN_TC_AUTO) {
-  if (kernel == OPENCNN_TC_SINGLE_CTA) return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream);
-  if (kernel == OPENCNN_TC_PAIR_LOCAL) return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream);
-  if (kernel == OPENCNN_TC_STACKED_BLOCKS) return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream);
+                      cudaStream_t stream, bool after_fx, int kernel = OPENCNN_TC_AUTO) {
+  if (kernel == OPENCNN_TC_SINGLE_CTA) return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+  if (kernel == OPENCNN_TC_PAIR_LOCAL) return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+  if (kernel == OPENCNN_TC_STACKED_BLOCKS) return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
   if (kernel != OPENCNN_TC_AUTO) return cudaErrorInvalidValue;
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
@@ -450,15 +466,15 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
   bool pair;
   if (K <= 64) {
     if (n_blocks > 1 && k_steps <= (bf16 ? 8 : 12) && tiles * ((n_blocks + 1) / 2) > st->sm_count)
-      return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream);
+      return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
     pair = k_steps >= (bf16 ? 16 : 8);
   } else {
     pair = k_steps >= 4 || tiles * n_blocks * ((K + ocb::kTcM - 1) / ocb::kTcM) >= 4ll * st->sm_count;
   }
   // (max_clusters is 0 only where no two CTAs of this size can be co-scheduled as a cluster)
   return pair && st->max_clusters[bf16 ? 0 : 1] > 0
-             ? launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream)
-             : launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream);
+             ? launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx)
+             : launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
 }
 
 cudaError_t forward(const float *input, const float *filter, float *output, float *workspace, int N, int C, int H,
@@ -472,17 +488,17 @@ cudaError_t forward(const float *input, const float *filter, float *output, floa
   if (precision == OPENCNN_BF16) {
     e = launch_fx_tc<ocb::kTcBf16>(filter, workspace, C, K, stream);
     if (e != cudaSuccess) return e;
-    return launch_tc<ocb::kTcBf16>(input, workspace, output, N, C, H, W, K, stream);
+    return launch_tc<ocb::kTcBf16>(input, workspace, output, N, C, H, W, K, stream, true);
   }
   if (precision == OPENCNN_TF32) {
     e = launch_fx_tc<ocb::kTcTf32>(filter, workspace, C, K, stream);
     if (e != cudaSuccess) return e;
-    return launch_tc<ocb::kTcTf32>(input, workspace, output, N, C, H, W, K, stream);
+    return launch_tc<ocb::kTcTf32>(input, workspace, output, N, C, H, W, K, stream, true);
   }
   if (precision != OPENCNN_FP32) return cudaErrorInvalidValue;
   e = launch_fx(filter, workspace, C, K, stream);
   if (e != cudaSuccess) return e;
-  return launch_wino_fp32(input, workspace, output, N, C, H, W, K, stream);
+  return launch_wino_fp32(input, workspace, output, N, C, H, W, K, stream, true);
 }
 
 // Scratch for opencnn_convolutionForward_noalloc: the transformed filter, [C][16][K] floats, for
@@ -574,11 +590,11 @@ int opencnn_winograd_forward(const float *input, const float *workspace, float *
   cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
   if (e != cudaSuccess) return (int)e;
   if (precision == OPENCNN_BF16)
-    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream);
+    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false);
   if (precision == OPENCNN_TF32)
-    return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream);
+    return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false);
   if (precision != OPENCNN_FP32) return (int)cudaErrorInvalidValue;
-  return (int)launch_wino_fp32(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream);
+  return (int)launch_wino_fp32(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false);
 }
 
 int opencnn_winograd_forward_kernel(const float *input, const float *workspace, float *output, int in_n, int in_c,
@@ -590,8 +606,8 @@ int opencnn_winograd_forward_kernel(const float *input, const float *workspace, 
   cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
   if (e != cudaSuccess) return (int)e;
   if (precision == OPENCNN_BF16)
-    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, kernel);
-  return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, kernel);
+    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, kernel);
+  return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, kernel);
 }
 
 int opencnn_convolutionForward_noalloc(const float *input, const float *filter, float *output, int in_n,
@@ -612,7 +628,7 @@ int opencnn_convolutionForward_noalloc(const float *input, const float *filter, 
   if (e != cudaSuccess) return (int)e;
   e = launch_fx(filter, ws, in_c, filt_k, (cudaStream_t)stream);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_wino_fp32(input, ws, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream);
+  return (int)launch_wino_fp32(input, ws, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, true);
 }
 
 int opencnn_nchw_to_chwn(const float *src, float *dst, int n, int c, int h, int w, opencnn_stream_t stream) {

@@ -8,7 +8,7 @@
 // reference's grouping, ((a + c) +/- b) * 0.5 with every operation rounded on its own, so the
 // workspace is bit-identical to the reference's.
 #pragma once
-#include <cuda_runtime.h>
+#include "ptx.cuh"
 
 namespace ocb {
 
@@ -40,6 +40,7 @@ __device__ __forceinline__ void fx_one(const float (&w)[9], float (&u)[16]) {
 
 // grid: ceil(C*K/4 / 128) blocks of 128 threads.  k4 = K/4.
 __global__ void __launch_bounds__(128) fx_kernel(const float4 *__restrict__ g, float4 *__restrict__ U, int C, int k4) {
+  grid_launch_dependents();                // the kernel that reads U may set itself up meanwhile
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= C * k4) return;
   const int c = idx / k4, kq = idx - c * k4;

@@ -95,6 +95,12 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, u
   }
 }
 
+// Programmatic dependent launch.  The first lets the next kernel of the stream start its set-up once every block of
+// this one has said so or is done; the second waits until the kernel before has completed and its writes are visible
+// (returns at once in a kernel that was launched the ordinary way).
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // True in exactly one lane of a fully converged warp.  Single-thread instructions that take their
 // operands from uniform registers (tcgen05.mma, TMA) are issued under this predicate by a warp
 // that executes the surrounding code convergently; issuing them from an `if (lane == 0)` branch

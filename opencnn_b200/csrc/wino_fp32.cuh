@@ -379,6 +379,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
           const uint32_t dst = smem_u32(stages + s * kStageFloats);
           mbar_arrive_expect_tx(bar, kStageBytes);
           tma_load_4d(dst, &tm_in, bar, tc.nb * kBN, 2 * tc.tx - 1, 2 * tc.ty - 1, ci * kBC);
+          if (g == 0) grid_dependency_wait();       // U is all that the kernel before this one writes
           tma_load_3d(dst + kVStageFloats * 4u, &tm_u, bar, tc.kb * kBK, 0, ci * kBC);
           issued = g + 1;
           if (++ci == cpt) {

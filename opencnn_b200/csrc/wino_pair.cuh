@@ -264,6 +264,7 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       // ===================================== filter slices =======================================
       if (lane == 0) {
         tma_prefetch_descriptor(&tm_u);
+        grid_dependency_wait();   // U is all that the kernel before this one writes
         constexpr int kRowBlocks = kPairFilters / (DT == kTcBf16 ? 64 : 32);   // 128-byte rows of a CTA's 64 filters
         int g = 0;
         bool ok = true;

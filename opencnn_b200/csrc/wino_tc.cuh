@@ -140,6 +140,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // BF16 packed, or fp32 words holding TF32 values (low 13 mantissa bits zero).
 template <int DT>
 __global__ void __launch_bounds__(128) fx_tc_kernel(const float4 *__restrict__ g, void *__restrict__ U, int C, int k4) {
+  grid_launch_dependents();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= C * k4) return;
   const int c = idx / k4, kq = idx - c * k4;
@@ -379,6 +380,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     const bool loads_u = warp != 0;
     if (lane == 0) {
       tma_prefetch_descriptor(loads_u ? &tm_u : &tm_in);
+      if (loads_u) grid_dependency_wait();   // U is all that the kernel before this one writes
       int seq = 0, ci = 0, issued = 0;
       TileCoord tc = decode_tile(p, (int)blockIdx.x);
       for (int g = 0; g < total_chunks; ++g) {

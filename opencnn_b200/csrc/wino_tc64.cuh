@@ -127,6 +127,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     const bool loads_u = warp != 0;
     if (lane == 0) {
       tma_prefetch_descriptor(loads_u ? &tm_u : &tm_in);
+      if (loads_u) grid_dependency_wait();   // U is all that the kernel before this one writes
       int seq = 0, ci = 0, issued = 0;
       T64Tile tc = t64_decode(p, (int)blockIdx.x, n_pairs);
       const int ring = loads_u ? SU : SR;
