@@ -124,10 +124,14 @@ template <int DT> __device__ __forceinline__ uint32_t instr_desc() {
          ((uint32_t)(kTcM >> 4) << 24);
 }
 
+// To the nearest TF32 value, ties to even; an infinity stays one and a NaN stays a NaN.  (Adding half a unit to the bits
+// and masking gives the same values for everything but NaNs: the NaN that arithmetic produces, 0x7FFFFFFF, carries
+// over into the sign and came out as -0, and took four instructions.  Fused kernel, 128x128x128x28x28: single CTA 71.8 ->
+// 67.8 us, CTA pair 54.7 -> 51.4; stacked 128x64x64x56x56: 116.9 -> 114.8.)
 __device__ __forceinline__ float round_tf32_rne(float v) {
-  uint32_t u = __float_as_uint(v);
-  u += 0xFFFu + ((u >> 13) & 1u);
-  return __uint_as_float(u & 0xFFFFE000u);
+  uint32_t u;
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
+  return __uint_as_float(u);
 }
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;

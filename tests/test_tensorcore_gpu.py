@@ -275,3 +275,30 @@ def test_transform_and_kernel_stay_ordered(libs, precision, shape):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, expect))
     assert api.last_device_status() == 0
+
+
+# An infinity or a NaN in the data must not come out as a number: the outputs that are not finite are those of the fp32 path,
+# which does the same additions (no transformed filter value is zero here, and none overflows).  The NaNs include the bit
+# patterns that rounding by integer addition would carry into the exponent or the sign.
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("bits", [0x7F800000, 0xFF800000, 0x7FC00000, 0x7FFFFFFF, 0xFFFFFFFF, 0x7F800001])
+def test_nonfinite_values_are_not_lost(libs, precision, bits):
+    N, C, K, H, W = 64, 24, 64, 7, 8
+    x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
+    g = torch.randn((C, 3, 3, K), device="cuda") * 0.05
+    for where in ("input", "filter"):
+        xb, gb = x.clone(), g.clone()
+        word = torch.tensor(bits - (1 << 32) if bits >= 1 << 31 else bits, dtype=torch.int32, device="cuda")
+        if where == "input":
+            xb.view(torch.int32)[3, 2, 5, 7] = word
+        else:
+            gb.view(torch.int32)[3, 0, 0, 9] = word          # the tap that the filter transform copies unchanged
+        finite = {}
+        for p in ("fp32", precision):
+            ws = torch.empty((C, 4, 4, K), device="cuda")
+            y = torch.zeros((K, H, W, N), device="cuda")
+            assert api.conv3x3(xb, gb, y, ws, N, C, H, W, K, precision=p) == 0
+            assert api.last_device_status() == 0
+            finite[p] = torch.isfinite(y)
+        assert not bool(finite["fp32"].all())
+        assert torch.equal(finite["fp32"], finite[precision]), where
