@@ -13,6 +13,11 @@
 // rows whose distance is a free field of the shared-memory descriptor (the leading-dimension byte
 // offset), so [U ; 0] is "first block at U, second block at a 2 KB region of zeros above all U
 // stages" and [0 ; U] is "first block at a region of zeros below them, second block at U".
+// Each MMA is told not to write the other image block's 64 accumulator rows (the mask operand of tcgen05.mma): added there,
+// the zeros would carry an infinity or a NaN of one image into the image 32 further on, because 0 * infinity is NaN.  The
+// rows that are not written are zeros all the same, because that is faster than U in both halves (128x128x64x28x28: 35.0 us
+// against 36.8 in BF16, 55.5 against 63.7 in TF32).  The mask itself costs 1.5 % where a tile has two K-steps
+// (256x32x64x112x112 in BF16 388 -> 394 us), nothing from four on (128x64x64x56x56 71.9 -> 71.9).
 // What it buys: one filter slice (32 KB per K-step) now serves 64 images instead of 32, and the
 // per-tile costs - the accumulator hand-over, the epilogue, the pipeline restart, which dominate
 // layers with few channels - are paid once per 64 images, with all 128 TMEM lanes doing useful
@@ -35,6 +40,24 @@
 #include "wino_tc.cuh"
 
 namespace ocb {
+
+// tc_mma (wino_tc.cuh) that leaves 64 of the 128 accumulator rows as they are: rows 0-63 if `skip_lo` is all ones,
+// rows 64-127 if `skip_hi` is (one mask bit per tensor-memory lane, set = not written).
+template <int DT>
+__device__ __forceinline__ void tc_mma_half(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                            uint32_t skip_lo, uint32_t skip_hi) {
+  if (DT == kTcBf16) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %6, %6}, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(skip_lo), "r"(skip_hi) : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %6, %6}, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(skip_lo), "r"(skip_hi) : "memory");
+  }
+}
 
 // A tile over two 32-image blocks, 2*np and 2*np + 1.
 struct T64Tile { int np, tx, ty, kb; };
@@ -213,7 +236,8 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
         const uint64_t astep = b == 0 ? kTopPos : kBotPos;
         const uint64_t ad = (b == 0 ? a_top0 + (uint64_t)su * kTopStage : a_bot0 + (uint64_t)su * kBotStage) + (uint64_t)col0 * astep;
         const uint64_t bd = b_desc0 + (uint64_t)(sv * (kTcVBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
-        const uint32_t accumulate = (ci > 0 || b > 0) ? 1u : 0u, d0 = tmem_base + col0 * kTcN;
+        const uint32_t accumulate = ci > 0 ? 1u : 0u, d0 = tmem_base + col0 * kTcN;
+        const uint32_t skip_lo = b == 0 ? 0u : 0xFFFFFFFFu, skip_hi = ~skip_lo;     // the other image block's rows
         bool ok = true;
 #pragma unroll
         for (int xo = 0; xo < 8; ++xo) {
@@ -222,7 +246,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
             if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
             tc_fence_after();
           }
-          if (elect_one()) tc_mma<DT>(d0 + xr * kTcN, ad + (uint64_t)xr * astep, bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate);
+          if (elect_one()) tc_mma_half<DT>(d0 + xr * kTcN, ad + (uint64_t)xr * astep, bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate, skip_lo, skip_hi);
         }
         if (!ok) break;
         if (elect_one()) tc_commit(smem_u32(v_empty + sv));                 // V stage reusable when these MMAs are done

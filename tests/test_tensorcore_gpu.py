@@ -302,3 +302,32 @@ def test_nonfinite_values_are_not_lost(libs, precision, bits):
             finite[p] = torch.isfinite(y)
         assert not bool(finite["fp32"].all())
         assert torch.equal(finite["fp32"], finite[precision]), where
+
+
+# Every image is a convolution of its own: an infinity or a NaN in one leaves the bits of all others as they are, whichever
+# of a tile's two image blocks it sits in and whether the tile's other rows are another block's (K = 64, stacked), a
+# repetition of the same filters (K = 64, single) or filters that do not exist (K = 192).  The large maps have more tiles
+# than the device has SMs, which is what the automatic choice asks for before it takes the stacked kernel.
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("kernel,shape", [("single", (64, 16, 64, 5, 6)), ("pair_local", (64, 24, 192, 5, 6)), ("stacked", (96, 24, 64, 5, 6)),
+                                          ("auto", (64, 16, 64, 31, 26)), ("auto", (64, 16, 128, 31, 26))])
+def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
+    N, C, K, H, W = shape
+    x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
+    ws = torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(torch.randn((C, 3, 3, K), device="cuda") * 0.05, ws, C, K, precision=precision) == 0
+
+    def run(x):
+        y = torch.zeros((K, H, W, N), device="cuda")
+        assert api.winograd_forward_kernel(x, ws, y, N, C, H, W, K, precision=precision, kernel=kernel) == 0
+        assert api.last_device_status() == 0
+        return y
+
+    clean = run(x)
+    for image, value in [(5, float("inf")), (40, float("-inf")), (N - 1, float("nan"))]:
+        bad = x.clone()
+        bad[C - 2, 3, 2, image] = value
+        y = run(bad)
+        assert not bool(torch.isfinite(y[..., image]).all())
+        others = [n for n in range(N) if n != image]
+        assert torch.equal(y[..., others], clean[..., others]), (image, value)
