@@ -95,6 +95,39 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, u
   }
 }
 
+// ---- pairs of CTAs (clusters of two) -----------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address (shared::cluster window) of the object at the same shared-memory offset in CTA `rank`.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+// mbar_wait for a thread that arrives on barriers of another CTA, whose address (shared::cluster) is `report`: once a wait
+// has given up these arrivals go to `nowhere`, a barrier of its own CTA that nobody waits for.  The `dead` word is each
+// CTA's own, so a CTA that carried on reporting would have the other one consume what was never written; this way the
+// other one's wait runs out as well.  (Changing the address keeps the step that arrives as it is: a predicate carried
+// through the loop took 2 % of 64x1024x1024x14x14 in BF16, a look at `dead` before the arrival 15 %.)
+__device__ __forceinline__ void mbar_wait_reporting(uint32_t bar, uint32_t parity, volatile int *dead, int *status, uint32_t &report,
+                                                    uint32_t nowhere, uint64_t limit_ns = 2000000000ull) {
+  if (!mbar_wait(bar, parity, dead, status, limit_ns)) report = nowhere;
+}
+// Arrive on a barrier given by its shared::cluster address, with the default release semantics.  What the
+// arrival stands for is never read by the other CTA's threads: V is read by the tensor core, for which the writer's
+// fence.proxy.async has made it visible, and a drained accumulator column has been read (tcgen05.wait::ld).  A release
+// at cluster scope would add a memory fence to every transform warp and K-step, and an acquire one to the issuers:
+// 510 instead of 212 us on 64x1024x1024x14x14 in BF16, 921 instead of 367 in TF32 (four transform warps).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
 // Programmatic dependent launch.  The first lets the next kernel of the stream start its set-up once every block of
 // this one has said so or is done; the second waits until the kernel before has completed and its writes are visible
 // (returns at once in a kernel that was launched the ordinary way).

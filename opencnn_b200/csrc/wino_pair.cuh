@@ -24,7 +24,8 @@
 // "Filter slice landed" and "V written" are barriers of the leading CTA (rank 0), whose two issuing
 // warps wait for both CTAs' halves there; the tensor core's commits reach the "free again" and "tile
 // finished" barriers of both CTAs (multicast arrive); a drained accumulator column is reported to the
-// leader.  All waits are bounded.  Both CTAs leave through a cluster barrier.
+// leader.  All waits are bounded, and a thread whose wait gave up reports nothing more to the leader, whose own waits
+// then run out too.  Both CTAs leave through a cluster barrier.
 #pragma once
 #include "wino_tc.cuh"
 
@@ -66,28 +67,6 @@ template <int DT> struct PairCfg {
   static_assert(kSmemBytes <= 232448, "shared memory");
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address (shared::cluster window) of the object at the same shared-memory offset in CTA `rank`.
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-  return r;
-}
-// Arrive on a barrier given by its shared::cluster address, with the default release semantics.  What the arrival
-// stands for is never read by the other CTA's threads: V is read by the tensor core, for which the writer's
-// fence.proxy.async has made it visible, and a drained accumulator column has been read (tcgen05.wait::ld).  A
-// release at cluster scope would add a memory fence to every transform warp and K-step, and an acquire one to the
-// issuers: 510 instead of 212 us on 64x1024x1024x14x14 in BF16, 921 instead of 367 in TF32.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
 // TMA tiled load into this CTA's shared memory whose bytes are counted on a barrier of the pair's leader.
 __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap *map, uint32_t cluster_bar, int c0, int c1,
                                                  int c2, int c3) {
@@ -154,7 +133,8 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   uint64_t *acc_full = v_empty + SV, *mma_done = acc_full + 1, *acc_empty = acc_full + 3;   // mma_done[2], acc_empty[4]
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 7);
   volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 8);
-  static_assert((2 * SR + 2 * SU + 2 * SV + 9) * 8 <= 512, "barriers");
+  uint64_t *nowhere = acc_full + 9;                    // [4]: nobody waits for these; where a thread that gave up arrives
+  static_assert(SV <= 4 && (2 * SR + 2 * SU + 2 * SV + 13) * 8 <= 512, "barriers");
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
   const uint32_t rank = cluster_ctarank();
@@ -180,6 +160,7 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     }
     mbar_init(smem_u32(acc_full), 2);
     for (int j = 0; j < 4; ++j) mbar_init(smem_u32(acc_empty + j), 2 * kTcEpilogueWarps);   // leader only
+    for (int j = 0; j < 4; ++j) mbar_init(smem_u32(nowhere + j), 1);
     mbar_init(smem_u32(mma_done + 0), 1);
     mbar_init(smem_u32(mma_done + 1), 1);
     mbar_fence_init();
@@ -199,13 +180,13 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     const int sub = (warp - kPairFirstEpilogueWarp) >> 2;                  // 0 / 1: which 16 of the block's 32 images
     const int ib = quarter >> 1;                                         // image block of the pair
     const uint32_t tcol = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * sub;
-    const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
+    uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
     for (int seq = 0; seq < my_tiles; ++seq) {
       const int t = cid + seq * n_clusters, q = 2 * (t % pairs) + ib;
       const PairBlock b = pair_block(p, q < blocks ? q : 0);
       const int k0 = (t / pairs) * 2 * kPairFilters + (int)rank * kPairFilters + 32 * (quarter & 1);
       const int n0 = b.nb * kTcN + 16 * sub;
-      mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
+      mbar_wait_reporting(smem_u32(acc_full), seq & 1, dead, p.status, acc_empty0, smem_u32(nowhere));
       tc_fence_after();
       tc_epilogue_16x32(tcol, q < blocks && k0 < p.K, p, k0 + lane, n0, 2 * b.ty, 2 * b.tx,
                         [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
@@ -215,22 +196,24 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     // ===================================== input transform =====================================
     constexpr int kGroups = Cfg::kGroups;
     const int t = (tid - 32 * kPairFirstTransformWarp) % (32 * Cfg::kStepWarps);      // channel t >> 4, image pair t & 15
+    uint32_t v_ready0 = map_to_rank(smem_u32(v_ready), 0);
     for (int g = (warp - kPairFirstTransformWarp) / Cfg::kStepWarps; g < total_steps; g += kGroups) {
       const int sv = g % SV, sr = g % SR;
       const uint32_t use = g / SV;
-      mbar_wait(smem_u32(raw_full + sr), (g / SR) & 1, dead, p.status);
+      mbar_wait_reporting(smem_u32(raw_full + sr), (g / SR) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
       const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
       uint8_t *vst = v_s + sv * kTcVBytes;
       uint64_t d[16];
       load_patch_pair(raw, t >> 4, t & 15, d);
-      if (use > 0) mbar_wait(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status);   // V stage free again
+      if (use > 0)                       // V stage free again
+        mbar_wait_reporting(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
       if (DT == kTcBf16) finish_v_bf16(d, vst, t >> 4, t & 15);
       else               finish_v_tf32(d, vst, t >> 4, t & 15);
       fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(raw_empty + sr));     // behind the fence: TMA refills the stage
-        mbar_arrive_cluster(map_to_rank(smem_u32(v_ready + sv), 0));
+        mbar_arrive_cluster(v_ready0 + 8 * sv);
       }
     }
     // the leader's commits arrive here until the end: do not leave before the last ones have
@@ -279,7 +262,8 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
                              (2 * kb + (int)rank) * kRowBlocks, 0);
           }
         }
-        // The slices land before the MMAs that read them, whose completion is what these phases stand for.
+        // The slices land before the MMAs that read them, whose completion is what these phases stand for.  (After a
+        // give-up nothing completes them: their limit, in both CTAs of the pair, is the time the copies get to land.)
         for (int i = g > SU ? g - SU : 0; i < g; ++i) mbar_wait_drain(smem_u32(u_empty + i % SU), (i / SU) & 1);
       }
     } else {

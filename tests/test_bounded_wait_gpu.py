@@ -58,3 +58,23 @@ def test_wait_that_runs_out_sets_status_and_returns(oracle, libs, probe):
     assert api.conv3x3(torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda(), dy, dws, N, C, H, W, K) == 0
     assert api.last_device_status() == 0
     assert np.array_equal(dy.cpu().numpy(), oracle.forward(x, g))
+
+
+@pytest.mark.parametrize("skip_arrive", [False, True])
+def test_wait_that_runs_out_in_one_cta_of_a_pair_ends_the_other(oracle, libs, probe, skip_arrive):
+    """A CTA that gave up no longer reports to the pair's leader, so that the leader's wait runs out as well (it must not
+    take what was never written for ready); both return, and the operator on CTA pairs still runs."""
+    out = (ctypes.c_longlong * 3)()
+    assert probe.wait_probe_pair_run(int(skip_arrive), LIMIT_NS, out) == 0
+    worker_ok, leader_ok, leader_wait_ns = list(out)
+    assert probe.wait_probe_last_status() == int(skip_arrive)
+    assert (worker_ok, leader_ok) == ((0, 0) if skip_arrive else (1, 1))
+    if skip_arrive:
+        assert 4 * LIMIT_NS <= leader_wait_ns < 200 * LIMIT_NS
+    N, C, K, H, W = 32, 64, 128, 4, 4
+    x, g = oracle.input_int(N, C, H, W), oracle.filter_int(C, K)
+    ws, dy = torch.empty((C, 4, 4, K), device="cuda"), torch.full((K, H, W, N), float("nan"), device="cuda")
+    assert api.filter_transform(torch.from_numpy(g).cuda(), ws, C, K, precision="bf16") == 0
+    assert api.winograd_forward_kernel(torch.from_numpy(x).cuda(), ws, dy, N, C, H, W, K, precision="bf16", kernel="pair_local") == 0
+    assert api.last_device_status() == 0
+    assert np.array_equal(dy.cpu().numpy().astype(np.float64), oracle.direct_f64(x, g))

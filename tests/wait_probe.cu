@@ -1,4 +1,4 @@
-// Test-only kernel for the bounded waits of opencnn_b200/csrc/ptx.cuh (mbar_wait, mbar_wait_drain).
+// Test-only kernels for the bounded waits of opencnn_b200/csrc/ptx.cuh (mbar_wait, mbar_wait_drain, mbar_wait_reporting).
 // The library's kernels never wait for ever: a wait that runs out sets the CTA's `dead` word and a
 // device status word, the thread that issues asynchronous work stops and drains, everybody else
 // falls through their later waits, and the kernel returns.  None of that can be seen in a
@@ -74,7 +74,72 @@ __global__ void __launch_bounds__(96, 1) wait_probe_kernel(ProbeOut *out, int sk
   __syncthreads();       // every thread gets here whatever the waits did
 }
 
+struct PairProbeOut {
+  int worker_ok;          // 1 if the wait of CTA 1's worker succeeded
+  int leader_ok;          // 1 if the leader's wait for the worker succeeded
+  long long leader_wait_ns;
+};
+
+// Two CTAs of 64 threads, the hand-over of wino_pair_kernel in miniature: warp 0 of CTA 1 waits for a barrier of its own
+// CTA (arrived on by its warp 1 unless `skip_arrive`) and reports to a barrier of the leader (CTA 0), on which warp 0 of the
+// leader waits four times as long.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64, 1)
+wait_probe_pair_kernel(PairProbeOut *out, int skip_arrive, unsigned long long limit_ns, int *status) {
+  __shared__ __align__(8) uint64_t bars[3];          // landed (each CTA's own), ready (the leader's), nowhere
+  __shared__ int dead_word;
+  volatile int *dead = &dead_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = ocb::cluster_ctarank();
+  if (threadIdx.x == 0) {
+    dead_word = 0;
+    ocb::mbar_init(ocb::smem_u32(bars + 0), 1);
+    ocb::mbar_init(ocb::smem_u32(bars + 1), 1);
+    ocb::mbar_init(ocb::smem_u32(bars + 2), 1);
+    ocb::mbar_fence_init();
+  }
+  __syncthreads();
+  ocb::cluster_sync_all();
+  if (lane == 0) {
+    if (rank == 1 && warp == 0) {
+      const uint32_t leaders = ocb::map_to_rank(ocb::smem_u32(bars + 1), 0);
+      uint32_t report = leaders;
+      ocb::mbar_wait_reporting(ocb::smem_u32(bars + 0), 0, dead, status, report, ocb::smem_u32(bars + 2), limit_ns);
+      out->worker_ok = report == leaders ? 1 : 0;
+      ocb::mbar_arrive_cluster(report);
+    } else if (rank == 1) {
+      if (!skip_arrive) ocb::mbar_arrive(ocb::smem_u32(bars + 0));
+    } else if (warp == 0) {
+      const uint64_t t0 = ocb::global_timer_ns();
+      out->leader_ok = ocb::mbar_wait(ocb::smem_u32(bars + 1), 0, dead, status, 4 * limit_ns) ? 1 : 0;
+      out->leader_wait_ns = (long long)(ocb::global_timer_ns() - t0);
+    }
+  }
+  __syncwarp();
+  ocb::cluster_sync_all();                           // every thread gets here whatever the waits did
+}
+
 }  // namespace
+
+// Runs the two-CTA probe once, synchronously.  out[3]: worker_ok, leader_ok, leader_wait_ns.  Returns a cudaError_t code.
+extern "C" int wait_probe_pair_run(int skip_arrive, unsigned long long limit_ns, long long *out3) {
+  if (!out3 || limit_ns == 0 || limit_ns > 100000000ull) return (int)cudaErrorInvalidValue;   // at most 0.4 s per wait
+  PairProbeOut *d = nullptr;
+  int *status = nullptr;
+  cudaError_t e = cudaMalloc(&d, sizeof(PairProbeOut));
+  if (e == cudaSuccess) e = cudaMemset(d, 0xff, sizeof(PairProbeOut));
+  if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void **>(&status), g_status);
+  if (e == cudaSuccess) {
+    wait_probe_pair_kernel<<<2, 64>>>(d, skip_arrive, limit_ns, status);
+    e = cudaGetLastError();
+  }
+  PairProbeOut h;
+  if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) {
+    out3[0] = h.worker_ok; out3[1] = h.leader_ok; out3[2] = h.leader_wait_ns;
+  }
+  if (d) cudaFree(d);
+  return (int)e;
+}
 
 // Runs the probe once, synchronously.  out[8]: issuer_ok, waiter_ok, waiter_second_ok, drain_ok,
 // drain_timeout_ok, issuer_wait_ns, waiter_second_ns, drain_timeout_ns.  Returns a cudaError_t code.
