@@ -439,17 +439,30 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
-// Which tensor-core kernel a problem gets.  All three give the same bits.  Medians, L2 flushed, bf16 / tf32 us.
-//   More than 64 filters: the CTA-pair kernel, except where the launch of clusters (2 us more) is not paid back -
-//   few K-steps and few tiles.  N x C x K x H x W, single : pair
-//     64x1024x1024x14x14 281 : 211 / 514 : 367    128x256x256x14x14 49 : 41 / 78 : 59    256x8x128x56x56 160 : 101 / 156 : 102
-//     32x64x128x9x9 (4 K-steps in BF16) 13.2 : 13.3 / 15.4 : 15.3    32x16x128x9x9 10.2 : 12.3 / 10.2 : 12.3
-//     64x16x128x28x28 (392 tiles) 15.4 : 17.4 / 17.3 : 17.4          64x3x128x56x56 (1568 tiles) 34.8 : 32.8 / 30.7 : 30.7
-//   At most 64 filters: the stacked kernel while there are few K-steps and more tiles than SMs (the other two leave half
-//   of the accumulator rows or of the pair idle), then the pair.  Single : pair : stacked
-//     128x64x64x56x56 96 : 94 : 78 / 135 : 127 : 122    128x128x64x28x28 (8 / 16 K-steps) 46 : 46 : 42 / 73 : 65 : 67
-//     64x192x64x28x28 35 : 35 : 39 / 56 : 48 : 63       128x128x64x7x7 (32 tiles) 14.3 : 15.4 : 18.4 / 19.5 : 17.4 : 25.6
-//     32x64x64x28x28 15.4 : 17.5 : 19.5 / 21.5 : 21.5 : 26.6    32x512x64x28x28 51 : 47 : 76 / 92 : 72 : 133
+// Which tensor-core kernel a problem gets.  All three give the same bits.  The measure is K-steps x rounds: what one SM
+// works through, a round being one tile of 32 images per SM.  Fused kernel alone, back to back, medians in us, measured at 720
+// sizes per type of 1 to 64 K-steps and 1 to 22 rounds; this rule is 0.1 % behind the best kernel of each on average.
+//   More than 64 filters: the CTA-pair kernel loads and multiplies faster, but costs about 2 us more to start.
+//     K-steps x rounds, single : pair   N x C x K x H x W in BF16 (TF32: half the channels)
+//      1 x 1   8.4 :  9.5 /  8.4 :  8.9   64x16x128x14x14         3 x 1   9.5 : 10.5 /  8.4 : 10.5   64x48x128x14x14
+//      4 x 2  14.6 : 14.6 / 13.4 : 12.5   64x64x128x20x20         8 x 1  12.5 : 12.5 / 12.4 : 11.9   64x128x128x14x14
+//      3 x 6  27.4 : 25.0 / 24.8 : 22.8   128x48x128x28x28        8 x 6  53.3 : 43.3 / 41.6 : 33.5   128x128x128x28x28
+//     fewer than three K-steps have little to gain:
+//      2 x 6  21.9 : 22.8 / 20.7 : 20.7   128x32x128x28x28        1 x 14 33.0 : 35.6 / 33.0 : 34.9   160x16x192x28x28
+//      1 x 22 70.7 : 51.6 / 51.5 : 49.4   128x16x128x56x56
+//   At most 64 filters: half of the rows of the pair's operand are empty, so it has to gain more; the stacked kernel does
+//   two blocks of images per step and needs 1.6 (few K-steps) to 1.9 (many) times as long for it, so it wants its rounds
+//   to be nearly half of the others'.  Single : pair : stacked, rounds of the first two / of the stacked
+//      4 x 2/1  12.5 : 14.6 : 11.5 / 12.5 : 12.9 : 11.0   64x64x64x20x20
+//      8 x 3/2  22.8 : 22.9 : 24.8 / 22.8 : 20.7 : 22.8   64x128x64x28x28
+//      4 x 6/3  28.8 : 28.9 : 22.8 / 25.5 : 24.8 : 21.8   128x64x64x28x28
+//      8 x 6/3  41.2 : 40.9 : 35.1 / 38.5 : 33.0 : 31.1   128x128x64x28x28
+//     24 x 6/3  92.2 : 90.0 : 88.5 / 90.4 : 67.2 : 85.2   128x384x64x28x28
+//      4 x 22/11 89.2 : 85.9 : 71.9 / 78.1 : 69.9 : 69.7  128x64x64x56x56
+//      8 x 22/11 134 : 131 : 119 / 126 : 103 : 115        128x128x64x56x56
+//     12 x 1/1  13.6 : 14.6 : 18.7 / 13.6 : 13.2 : 18.2   96x192x64x14x14
+//     16 x 3/2  35.2 : 35.1 : 40.5 / 35.1 : 27.9 : 36.9   64x256x64x28x28
+//     48 x 1/1  31.0 : 28.9 : 51.8 (BF16)                 32x768x64x4x4
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
                       cudaStream_t stream, bool after_fx, int kernel = OPENCNN_TC_AUTO) {
@@ -461,15 +474,18 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
   constexpr bool bf16 = DT == ocb::kTcBf16;
-  const int k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC;
+  const long long k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC;
   const long long tiles = (long long)((H + 1) / 2) * ((W + 1) / 2), n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
+  const auto rounds_of = [&](long long all_tiles) { return (all_tiles + st->sm_count - 1) / st->sm_count; };
+  const long long rounds = rounds_of(tiles * n_blocks * ((K + ocb::kTcM - 1) / ocb::kTcM));
   bool pair;
   if (K <= 64) {
-    if (n_blocks > 1 && k_steps <= (bf16 ? 8 : 12) && tiles * ((n_blocks + 1) / 2) > st->sm_count)
+    const long long stacked_rounds = rounds_of(tiles * ((n_blocks + 1) / 2));
+    if (4 * rounds >= 7 * stacked_rounds && (bf16 ? k_steps <= 24 : k_steps <= 4 || (k_steps <= 12 && k_steps * rounds <= 48)))
       return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-    pair = k_steps >= (bf16 ? 16 : 8);
+    pair = bf16 ? k_steps >= 16 && k_steps * rounds >= 32 : k_steps >= 3 && k_steps * rounds >= 12;
   } else {
-    pair = k_steps >= 4 || tiles * n_blocks * ((K + ocb::kTcM - 1) / ocb::kTcM) >= 4ll * st->sm_count;
+    pair = k_steps * rounds >= (k_steps >= 3 ? 8 : 20);
   }
   // (max_clusters is 0 only where no two CTAs of this size can be co-scheduled as a cluster)
   return pair && st->max_clusters[bf16 ? 0 : 1] > 0

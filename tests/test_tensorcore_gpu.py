@@ -306,11 +306,11 @@ def test_nonfinite_values_are_not_lost(libs, precision, bits):
 
 # Every image is a convolution of its own: an infinity or a NaN in one leaves the bits of all others as they are, whichever
 # of a tile's two image blocks it sits in and whether the tile's other rows are another block's (K = 64, stacked), a
-# repetition of the same filters (K = 64, single) or filters that do not exist (K = 192).  The large maps have more tiles
-# than the device has SMs, which is what the automatic choice asks for before it takes the stacked kernel.
+# repetition of the same filters (K = 64, single) or filters that do not exist (K = 192).  The large maps take the device
+# four rounds of tiles, enough for the automatic choice to take the stacked kernel and the CTA pair.
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
 @pytest.mark.parametrize("kernel,shape", [("single", (64, 16, 64, 5, 6)), ("pair_local", (64, 24, 192, 5, 6)), ("stacked", (96, 24, 64, 5, 6)),
-                                          ("auto", (64, 16, 64, 31, 26)), ("auto", (64, 16, 128, 31, 26))])
+                                          ("auto", (64, 16, 64, 31, 30)), ("auto", (64, 40, 128, 31, 30))])
 def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
     N, C, K, H, W = shape
     x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
@@ -331,3 +331,27 @@ def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
         assert not bool(torch.isfinite(y[..., image]).all())
         others = [n for n in range(N) if n != image]
         assert torch.equal(y[..., others], clean[..., others]), (image, value)
+
+
+# The automatic choice on both sides of its cut-offs (K-steps x rounds of tiles, B200: 148 SMs, 16 / 8 channels per K-step in
+# BF16 / TF32; rounds in the comment): the bits of the single-CTA kernel whatever it takes.
+CHOICES = [(32, 48, 128, 24, 12), (32, 128, 128, 24, 12), (64, 64, 192, 14, 20),                    # 1, 1, 2
+           (128, 16, 128, 41, 38), (128, 15, 256, 41, 39),                                        # 11, 23
+           (64, 64, 64, 16, 36), (64, 33, 64, 26, 26), (64, 33, 64, 30, 30), (200, 24, 64, 17, 23),  # 2 / 1, 3 / 2, 4 / 2, 6 / 3 stacked
+           (104, 100, 64, 30, 30), (40, 400, 64, 30, 30), (8, 200, 64, 7, 5)]                        # 7 / 4, 4 / 2, 1 / 1
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("shape", CHOICES)
+def test_automatic_choice_gives_the_bits_of_the_single_cta_kernel(libs, precision, shape):
+    N, C, K, H, W = shape
+    x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
+    ws = torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(torch.randn((C, 3, 3, K), device="cuda") * 0.05, ws, C, K, precision=precision) == 0
+    out = {}
+    for kernel in ("single", "auto"):
+        out[kernel] = torch.full((K, H, W, N), float("nan"), device="cuda")
+        assert api.winograd_forward_kernel(x, ws, out[kernel], N, C, H, W, K, precision=precision, kernel=kernel) == 0
+        assert api.last_device_status() == 0
+    assert bool(torch.isfinite(out["single"]).all().item())
+    assert torch.equal(out["single"], out["auto"])
