@@ -355,3 +355,58 @@ def test_automatic_choice_gives_the_bits_of_the_single_cta_kernel(libs, precisio
         assert api.last_device_status() == 0
     assert bool(torch.isfinite(out["single"]).all().item())
     assert torch.equal(out["single"], out["auto"])
+
+
+# The fused kernel reads its input before the transform it overlaps is over, so what it reads must be older than that
+# transform: on one stream and without synchronisation the input buffer is rewritten before every call, and every call's
+# output is the next one's input.  Sizes that reach each fused kernel (single CTA, CTA pair, stacked, fp32), ragged ones too.
+@pytest.mark.parametrize("precision,shape", [("fp32", (32, 64, 64, 9, 9)), ("fp32", (36, 20, 20, 6, 5)), ("bf16", (32, 64, 64, 6, 6)),
+                                             ("tf32", (40, 64, 64, 5, 5)), ("bf16", (64, 128, 128, 14, 20)), ("tf32", (72, 128, 128, 15, 20)),
+                                             ("bf16", (64, 64, 64, 31, 30)), ("tf32", (104, 64, 64, 22, 18)), ("noalloc", (32, 64, 64, 9, 9))])
+def test_input_written_just_before_the_call(libs, precision, shape):
+    N, C, K, H, W = shape
+    sources = [torch.rand((C, H, W, N), device="cuda") * 2 - 1 for _ in range(4)]
+    filters = [torch.randn((C, 3, 3, K), device="cuda") * 0.05 for _ in range(4)]
+    x, ws = torch.empty((C, H, W, N), device="cuda"), torch.empty((C, 4, 4, K), device="cuda")
+    stream = torch.cuda.Stream()
+
+    def conv(x, g, y, wait):
+        if precision == "noalloc":
+            assert api.conv3x3_noalloc(x, g, y, N, C, H, W, K, stream=stream.cuda_stream) == 0
+        else:
+            assert api.conv3x3(x, g, y, ws, N, C, H, W, K, precision=precision, stream=stream.cuda_stream) == 0
+        if wait:
+            torch.cuda.synchronize()
+
+    def calls(outs, wait):
+        with torch.cuda.stream(stream):
+            for s, g, y in zip(sources, filters, outs):
+                x.copy_(s)
+                if wait:
+                    torch.cuda.synchronize()
+                conv(x, g, y, wait)
+            for g, a, b in zip(filters, outs[3:], outs[4:]):      # a chain: C == K, so an output is an input as it lies
+                conv(a, g, b, wait)
+
+    expect = [torch.full((K, H, W, N), float("nan"), device="cuda") for _ in range(8)]
+    got = [torch.empty_like(y) for y in expect]
+    torch.cuda.synchronize()
+    calls(expect, wait=True)
+    assert all(bool(torch.isfinite(y).all()) for y in expect)
+    for _ in range(3):
+        for y in got:
+            y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        calls(got, wait=False)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, expect))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        calls(got, wait=False)
+    for _ in range(2):
+        for y in got:
+            y.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, expect))
+    assert api.last_device_status() == 0
