@@ -460,6 +460,7 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
 //     24 x 6/3  92.2 : 90.0 : 88.5 / 90.4 : 67.2 : 85.2   128x384x64x28x28
 //      4 x 22/11 89.2 : 85.9 : 71.9 / 78.1 : 69.9 : 69.7  128x64x64x56x56
 //      8 x 22/11 134 : 131 : 119 / 126 : 103 : 115        128x128x64x56x56
+//      2 x 170/85 820 : 417 : 394 (BF16), 4 x 170/85 569 : 486 : 500 (TF32)  256x32x64x112x112
 //     12 x 1/1  13.6 : 14.6 : 18.7 / 13.6 : 13.2 : 18.2   96x192x64x14x14
 //     16 x 3/2  35.2 : 35.1 : 40.5 / 35.1 : 27.9 : 36.9   64x256x64x28x28
 //     48 x 1/1  31.0 : 28.9 : 51.8 (BF16)                 32x768x64x4x4
@@ -481,7 +482,7 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
   bool pair;
   if (K <= 64) {
     const long long stacked_rounds = rounds_of(tiles * ((n_blocks + 1) / 2));
-    if (4 * rounds >= 7 * stacked_rounds && (bf16 ? k_steps <= 24 : k_steps <= 4 || (k_steps <= 12 && k_steps * rounds <= 48)))
+    if (4 * rounds >= 7 * stacked_rounds && (bf16 ? k_steps <= 24 : k_steps <= 3 || (k_steps <= 12 && k_steps * rounds <= 48)))
       return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
     pair = bf16 ? k_steps >= 16 && k_steps * rounds >= 32 : k_steps >= 3 && k_steps * rounds >= 12;
   } else {
