@@ -175,7 +175,9 @@ cudaError_t check_shape(int N, int C, int H, int W, int K, ShapeRule rule) {
 // stream, by this call, so its set-up (barriers, tensor memory, descriptors, the first patches) may overlap it; the
 // kernels wait for the transform's completion before their first load of U, and all other data is older than the
 // transform, which itself is launched the ordinary way.  Whole calls: fp32 32x16x64x9x9 12.3 -> 10.2 us,
-// 32x64x64x56x56 81.9 -> 79.7; TF32 128x128x128x28x28 63.0 -> 59.8.
+// 32x64x64x56x56 81.9 -> 79.7; TF32 128x128x128x28x28 63.0 -> 59.8 - with calls queued one behind the other.  On an idle
+// stream the transform is over before the host has encoded the tensor maps and launched the second kernel, and a small call
+// takes what it took: 9x9 27.1 -> 27.0 us from the call to the end of a synchronise.
 template <class... P, class... A>
 cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, bool after_fx, const A &...args) {
   cudaLaunchConfig_t cfg = {};

@@ -36,7 +36,8 @@ namespace ocb {
 // transform warps (512 threads) -> eight: 64x1024x1024x14x14 199 -> 196 us in BF16 and 355 -> 321 in TF32,
 // 128x256x256x14x14 36.2 -> 35.4 and 56.0 -> 46.2, 128x64x128x56x56 93.5 -> 91.3 and 124 -> 115; a single K-step per
 // tile loses (256x8x128x56x56 91.0 -> 93.4 and 87.1 -> 90.8).  Handing the patches back as soon as they are in
-// registers, with a proxy fence of its own, gained nothing (203 / 323).
+// registers, with a proxy fence of its own, gained nothing (203 / 323).  Since TF32 operands are rounded by one instruction:
+// 64x1024x1024x14x14 195 / 317, 128x256x256x14x14 34 / 43, 128x64x128x56x56 90 / 109, 256x8x128x56x56 92 / 88.
 // Five warpgroups: warps 0 and 1 load patches and filter slices, 2 and 3 issue the MMAs; warps 4-11 transform;
 // warps 12-19 are the epilogue.  Registers are shared out with setmaxnreg.
 constexpr int kPairThreads = 640;

@@ -449,7 +449,8 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     // issuing lane - always the same one, which is also the one whose MMAs its commits cover.  From an
     // `if (lane == 0)` region, as this was before, every MMA pays for moving its operands to uniform
     // registers one lane at a time: main loop without loads, transform and epilogue 224 -> 152 us on
-    // 64x1024x1024x14x14 in BF16 and 428 -> 284 in TF32, whole kernel 298 -> 284 and 556 -> 523.
+    // 64x1024x1024x14x14 in BF16 and 428 -> 284 in TF32, whole kernel 298 -> 284 and 556 -> 523
+    // (now 275 and 510).
     // The descriptors are built once and only advanced by constants inside the unrolled loop.
     {
       // A thread issues whole columns of the 4x4 positions (two columns each), column by column:

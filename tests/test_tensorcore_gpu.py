@@ -15,9 +15,9 @@ from opencnn_b200 import api  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
-# TF32 problems with >= 64 K-steps per tile (C >= 512) and >= 64 images take the CTA-pair kernel - the last five
-# here, also with an odd number of 32-image blocks and with K not a multiple of 128; everything else, and all of
-# BF16, the single-CTA kernel.
+# With more than 64 filters these small maps are one round of tiles: from eight K-steps of 16 (BF16) or 8 (TF32) channels on
+# they take the CTA-pair kernel - the four deep ones of that kind, in both types, also with an odd number of 32-image blocks
+# and with K not a multiple of 128 - and the others the single-CTA kernel; the deep one with 64 filters the pair, too.
 SHAPES = [(32, 16, 128, 8, 8), (32, 8, 64, 7, 7), (64, 40, 192, 5, 9), (32, 64, 64, 14, 14), (96, 32, 256, 6, 6),
           (64, 512, 128, 4, 4), (96, 512, 192, 3, 5), (128, 520, 64, 2, 2), (64, 1024, 128, 3, 3), (96, 1040, 192, 2, 3)]
 MODEL_REL = 2e-4                     # device vs model: fp32 accumulation order inside the tensor core
@@ -56,7 +56,7 @@ def test_tensor_core_path(oracle, libs, precision, shape):
     assert tworst <= TRUTH_REL[precision] * trms, f"vs fp64: {tworst / trms:.3e} of rms"
 
 
-# Ragged last image block (N % 8 == 0 on this path), single-CTA kernel and CTA-pair kernel (TF32, >= 64 K-steps, N >= 64).
+# Ragged last image block (N % 8 == 0 on this path), single-CTA kernel and (C >= 512) CTA-pair kernel.
 RAGGED = [(40, 16, 128, 6, 6), (72, 32, 64, 5, 7), (8, 16, 128, 4, 4), (72, 512, 128, 4, 4), (104, 512, 128, 3, 3),
           (72, 1024, 128, 2, 2),
           (32, 3, 64, 6, 6), (40, 21, 128, 5, 5), (64, 515, 128, 3, 3)]   # and channel counts that are not a multiple of 8
@@ -92,8 +92,7 @@ def test_integer_tensors_are_exact_on_tensor_cores(oracle, libs, precision):
 
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
 def test_tensor_core_results_are_repeatable(libs, precision):
-    """Same bits run after run, also from the CTA-pair kernel that deep TF32 problems take (its two partial
-    results are added by an L2 reduction, but two addends commute)."""
+    """Same bits run after run, from the single-CTA kernel (the first size) and the CTA-pair kernel (the other)."""
     for (N, C, K, H, W) in [(64, 64, 64, 9, 9), (64, 1024, 128, 3, 3)]:
         x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
         g = torch.randn((C, 3, 3, K), device="cuda") * 0.05
@@ -109,8 +108,8 @@ def test_tensor_core_results_are_repeatable(libs, precision):
 
 
 # The benchmark shapes at full size (the N=128 layer sweep and the two wide stress layers): error of both
-# operand types against 10^5 sampled fp64 outputs, relative to rms(truth).  The N=64 C=K=1024 layer takes the
-# CTA-pair kernel in TF32.
+# operand types against 10^5 sampled fp64 outputs, relative to rms(truth).  All take the CTA-pair kernel but, in BF16, the
+# two layers with 64 filters, which take the stacked one.
 FULL = [(128, 64, 64, 56), (128, 128, 128, 28), (128, 256, 256, 14), (128, 512, 512, 7), (64, 1024, 1024, 14),
         (256, 32, 64, 112)]
 
@@ -362,7 +361,7 @@ def test_automatic_choice_gives_the_bits_of_the_single_cta_kernel(libs, precisio
 # output is the next one's input.  Sizes that reach each fused kernel (single CTA, CTA pair, stacked, fp32), ragged ones too.
 @pytest.mark.parametrize("precision,shape", [("fp32", (32, 64, 64, 9, 9)), ("fp32", (36, 20, 20, 6, 5)), ("bf16", (32, 64, 64, 6, 6)),
                                              ("tf32", (40, 64, 64, 5, 5)), ("bf16", (64, 128, 128, 14, 20)), ("tf32", (72, 128, 128, 15, 20)),
-                                             ("bf16", (64, 64, 64, 31, 30)), ("tf32", (104, 64, 64, 22, 18)), ("noalloc", (32, 64, 64, 9, 9))])
+                                             ("bf16", (64, 64, 64, 31, 30)), ("tf32", (56, 64, 64, 31, 30)), ("noalloc", (32, 64, 64, 9, 9))])
 def test_input_written_just_before_the_call(libs, precision, shape):
     N, C, K, H, W = shape
     sources = [torch.rand((C, H, W, N), device="cuda") * 2 - 1 for _ in range(4)]
