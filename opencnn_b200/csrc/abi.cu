@@ -442,8 +442,8 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
 }
 
 // Which tensor-core kernel a problem gets.  All three give the same bits.  The measure is K-steps x rounds: what one SM
-// works through, a round being one tile of 32 images per SM.  Fused kernel alone, back to back, medians in us, measured at 720
-// sizes per type of 1 to 64 K-steps and 1 to 22 rounds; this rule is 0.1 % behind the best kernel of each on average.
+// works through, a round being one tile of 32 images per SM.  Fused kernel alone, back to back, medians in us, measured at 930
+// sizes per type of 1 to 64 K-steps and 1 to 45 rounds; this rule is 0.15 % behind the best kernel of each on average.
 //   More than 64 filters: the CTA-pair kernel loads and multiplies faster, but costs about 2 us more to start.
 //     K-steps x rounds, single : pair   N x C x K x H x W in BF16 (TF32: half the channels)
 //      1 x 1   8.4 :  9.5 /  8.4 :  8.9   64x16x128x14x14         3 x 1   9.5 : 10.5 /  8.4 : 10.5   64x48x128x14x14
@@ -453,10 +453,12 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
 //      2 x 6  21.9 : 22.8 / 20.7 : 20.7   128x32x128x28x28        1 x 14 33.0 : 35.6 / 33.0 : 34.9   160x16x192x28x28
 //      1 x 22 70.7 : 51.6 / 51.5 : 49.4   128x16x128x56x56
 //   At most 64 filters: half of the rows of the pair's operand are empty, so it has to gain more; the stacked kernel does
-//   two blocks of images per step and needs 1.6 (few K-steps) to 1.9 (many) times as long for it, so it wants its rounds
-//   to be nearly half of the others'.  Single : pair : stacked, rounds of the first two / of the stacked
+//   two blocks of images per step and needs 1.5 (one K-step) to almost 2 times (many) as long for it, so its rounds have to be
+//   nearly half of the others': their ratio at least 2 - 1.8 / K-steps in BF16 and 2 - 1 / K-steps in TF32.  Single : pair : stacked, rounds of the first two / of the stacked
 //      4 x 2/1  12.5 : 14.6 : 11.5 / 12.5 : 12.9 : 11.0   64x64x64x20x20
 //      8 x 3/2  22.8 : 22.9 : 24.8 / 22.8 : 20.7 : 22.8   64x128x64x28x28
+//      1 x 15/9 31.0 : 37.3 : 26.9 (BF16)                  1 x 20/12 40.4 : 45.0 : 33.4 (TF32)
+//     16 x 7/4  75.6 : 72.3 : 81.3 (BF16)                  3 x 5/3   20.7 : 22.8 : 20.7 (TF32)
 //      4 x 6/3  28.8 : 28.9 : 22.8 / 25.5 : 24.8 : 21.8   128x64x64x28x28
 //      8 x 6/3  41.2 : 40.9 : 35.1 / 38.5 : 33.0 : 31.1   128x128x64x28x28
 //     24 x 6/3  92.2 : 90.0 : 88.5 / 90.4 : 67.2 : 85.2   128x384x64x28x28
@@ -484,9 +486,10 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
   bool pair;
   if (K <= 64) {
     const long long stacked_rounds = rounds_of(tiles * ((n_blocks + 1) / 2));
-    if (4 * rounds >= 7 * stacked_rounds && (bf16 ? k_steps <= 24 : k_steps <= 3 || (k_steps <= 12 && k_steps * rounds <= 48)))
+    if (2 * rounds >= 3 * stacked_rounds && 5 * k_steps * (2 * stacked_rounds - rounds) <= (bf16 ? 9 : 5) * stacked_rounds &&
+        (bf16 ? k_steps <= 24 : k_steps <= 3 || (k_steps <= 12 && k_steps * rounds <= 48)))
       return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-    pair = bf16 ? k_steps >= 16 && k_steps * rounds >= 32 : k_steps >= 3 && k_steps * rounds >= 12;
+    pair = bf16 ? k_steps * rounds >= (k_steps >= 16 ? 32 : 48) : k_steps >= 10 || (k_steps >= 3 && k_steps * rounds >= 14);
   } else {
     pair = k_steps * rounds >= (k_steps >= 3 ? 8 : 20);
   }

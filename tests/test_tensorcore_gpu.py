@@ -337,7 +337,7 @@ def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
 CHOICES = [(32, 48, 128, 24, 12), (32, 128, 128, 24, 12), (64, 64, 192, 14, 20),                    # 1, 1, 2
            (128, 16, 128, 41, 38), (128, 15, 256, 41, 39),                                        # 11, 23
            (64, 64, 64, 16, 36), (64, 33, 64, 26, 26), (64, 33, 64, 30, 30), (200, 24, 64, 17, 23),  # 2 / 1, 3 / 2, 4 / 2, 6 / 3 stacked
-           (104, 100, 64, 30, 30), (40, 400, 64, 30, 30), (8, 200, 64, 7, 5)]                        # 7 / 4, 4 / 2, 1 / 1
+           (104, 100, 64, 30, 30), (160, 16, 64, 30, 30), (40, 400, 64, 30, 30), (8, 200, 64, 7, 5)]         # 7 / 4, 8 / 5, 4 / 2, 1 / 1
 
 
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
