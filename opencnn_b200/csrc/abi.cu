@@ -75,21 +75,21 @@ cudaError_t device_state(DeviceState **out) {
   std::call_once(st.once, [&] {
     cudaError_t err = cudaDeviceGetAttribute(&st.sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_fp32_kernel<OCB_VARIANT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::SmemLayout<OCB_VARIANT>::kBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_fp32_kernel<OCB_VARIANT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::SmemLayout<OCB_VARIANT>::kBytes);
+      for (const auto kernel : {ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>, ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>,
+                                ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>})
+        if (err == cudaSuccess)
+          err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ocb::SmemLayout<OCB_VARIANT>::kBytes);
     if (err == cudaSuccess) {
       // The kernel redistributes registers with setmaxnreg; that only works if the compiler gave
       // the CTA at least the pool the budgets add up to.  Refuse to run a build where it did not
       // (its consumer warps would wait for registers for ever).
       constexpr int kBudget = ocb::kConsumerThreads * ocb::kConsumerRegs + ocb::kProducerThreads * ocb::kProducerRegs;
       cudaFuncAttributes fa;
-      err = cudaFuncGetAttributes(&fa, ocb::wino_fp32_kernel<OCB_VARIANT, false>);
-      if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
-      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_fp32_kernel<OCB_VARIANT, true>);
-      if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
+      for (const auto kernel : {ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>, ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>,
+                                ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>}) {
+        if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, kernel);
+        if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
+      }
       // the same for the CTA-pair kernel
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcBf16>);
       if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
@@ -210,6 +210,7 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
 
+  const bool packed = N % ocb::kBN != 0, ragged = K % ocb::kBK != 0;      // which instantiation (see ocb::Shape)
   CUtensorMap tm_in, tm_u;
   {
     cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
@@ -234,31 +235,37 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
 
   ocb::WinoParams p;
   p.y = output;
+  p.x = input;
   p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
   p.tiles_h = (H + 1) / 2;
   p.tiles_w = (W + 1) / 2;
   p.n_blocks = (N + ocb::kBN - 1) / ocb::kBN;
   p.k_blocks = (K + ocb::kBK - 1) / ocb::kBK;
-  const long long tiles = (long long)p.tiles_h * p.tiles_w * p.n_blocks * p.k_blocks;
+  const long long blocks = ((long long)p.tiles_h * p.tiles_w * (N / 4) + 7) / 8;
+  const long long tiles = blocks * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
+  p.blocks = (int)blocks;
   p.total_tiles = (int)tiles;
   p.chunks_per_tile = (C + ocb::kBC - 1) / ocb::kBC;
+  p.ty0 = 0;
   p.status = st->status_ptr;
-  const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
-  // The last round of the persistent schedule is usually only partly filled.  If its tiles, cut in
-  // two (one item per consumer group), still fit on the SMs, cut them: that round then takes about
-  // half as long (see item_tile in wino_fp32.cuh).
-  const int full_rounds = p.total_tiles / grid, rest = p.total_tiles % grid;
-  p.split_from = p.total_tiles;
-  p.total_items = p.total_tiles;
-  if (rest > 0 && 2 * rest <= grid) {
-    p.split_from = full_rounds * grid;
-    p.total_items = p.split_from + 2 * rest;
-  }
-  if (N % ocb::kBN == 0 && K % ocb::kBK == 0)
-    return launch_main(ocb::wino_fp32_kernel<OCB_VARIANT, false>, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
-  // ragged last block of images or filters: stores masked
-  return launch_main(ocb::wino_fp32_kernel<OCB_VARIANT, true>, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
+  // The last round of the persistent schedule is usually only partly filled; cutting its tiles in
+  // two (one item per consumer group) pays if the halves still fit on the SMs (see item_tile).  The tiles of a last filter block
+  // with at most 32 filters are such halves already.  An SM's items are item, item + grid, ...: the first SM has most, and a
+  // half takes about 0.55 of a tile.
+  const long long sms = st->sm_count, halves = K % ocb::kBK && K % ocb::kBK <= ocb::kBK / 2 ? blocks : 0, wholes = tiles - halves;
+  const auto rounds = [&](long long items) { return (items + sms - 1) / sms; };
+  const auto cost = [&](long long split) { return 11 * rounds(tiles + split) + 9 * rounds(wholes - split); };
+  const long long rest = wholes % sms, split = cost(rest) < cost(0) ? rest : 0;
+  p.split_from = (int)(wholes - split);
+  p.split_tiles = (int)split;
+  p.half_from = (int)wholes;
+  p.total_items = (int)(tiles + split);
+  const int grid = p.total_items < st->sm_count ? p.total_items : st->sm_count;
+  const auto kernel = packed   ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>
+                      : ragged ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>
+                               : ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>;
+  return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // Tensor-core path: filter transform rounded to the operand type, then the tcgen05 kernel.
@@ -318,8 +325,9 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   const long long tiles = (long long)p.tiles_h * p.tiles_w * p.n_blocks * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.total_tiles = (int)tiles;
-  p.split_from = p.total_items = p.total_tiles;
+  p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
+  p.ty0 = 0;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
   if (bf16 && K <= 64)
@@ -378,8 +386,9 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   if (blocks > 0x7fffffffll / 8 || tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.blocks = (int)blocks;
   p.total_tiles = (int)tiles;
-  p.split_from = p.total_items = p.total_tiles;
+  p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
+  p.ty0 = 0;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
   return launch_main(ocb::wino_pair_kernel<DT>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
@@ -434,8 +443,9 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   const long long tiles = (long long)p.tiles_h * p.tiles_w * ((p.n_blocks + 1) / 2);
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.total_tiles = (int)tiles;
-  p.split_from = p.total_items = p.total_tiles;
+  p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
+  p.ty0 = 0;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
   return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);

@@ -32,6 +32,10 @@
 
 namespace ocb {
 
+// Exact: the batch and the filters fill the blocks of 32 images and 64 filters.  Ragged: the batch does, the filters do not.
+// Packed: the batch does not (see ColumnQuad).  (Channels beyond the end are loaded as zeros by all three.)
+enum Shape : int { kExact = 0, kRagged = 1, kPacked = 2 };
+
 enum Variant : int { kBase = 0, kOptSts64 = 1, kOptSts64Cmp = 2, kOptLds64 = 3 };
 
 constexpr int kBN = 32;                     // images per CTA tile
@@ -73,13 +77,14 @@ template <int V> struct SmemLayout {
 
 struct WinoParams {
   float *y;            // output, KHWN
+  const float *x;      // input, CHWN (read through the tensor map except by kernels that pack images)
   int N, C, K, H, W;
   int tiles_h, tiles_w, n_blocks, k_blocks, total_tiles, chunks_per_tile;
-  // fp32 kernel only: work items.  Items below split_from are whole tiles; from there on each
-  // tile is two items, one per consumer group (see item_tile).  split_from == total_tiles and
-  // total_items == total_tiles mean "no split".
-  int split_from, total_items;
-  int blocks;          // CTA-pair kernel only: n_blocks * tiles_w * tiles_h
+  // fp32 kernel only: work items.  The split_tiles tiles from split_from on are two items each, one per consumer
+  // group (see item_tile); all others are whole, those from half_from on with one group idle (see ragged_item).
+  int split_from, split_tiles, half_from, total_items;
+  int ty0;             // first tile row (tiles_h of them are computed)
+  int blocks;          // 32-column blocks of all tiles: n_blocks * tiles_w * tiles_h, or the packed count (see ColumnQuad)
   int *status;         // device status word
 };
 
@@ -89,25 +94,102 @@ __device__ __forceinline__ TileCoord decode_tile(const WinoParams &p, int t) {
   TileCoord tc;
   tc.nb = t % p.n_blocks; t /= p.n_blocks;
   tc.tx = t % p.tiles_w;  t /= p.tiles_w;
-  tc.ty = t % p.tiles_h;
+  tc.ty = p.ty0 + t % p.tiles_h;
   tc.kb = t / p.tiles_h;
   return tc;
 }
 
 // Work item -> tile and the consumer groups that compute it (bit 0 = group 0, bit 1 = group 1).
-// The tiles of the last, partly filled round of the persistent schedule are cut in two items of 32
+// Where that shortens the last, partly filled round of the persistent schedule, its tiles are cut in two items of 32
 // filters each and given to two SMs: a group that has the FMA pipe to itself runs almost twice as
 // fast, so that round takes about half as long.  The group that sits an item out only keeps the
 // ring moving (it hands every stage straight back).
 __device__ __forceinline__ int item_tile(const WinoParams &p, int item, int &groups) {
-  if (item < p.split_from) {
-    groups = 3;
-    return item;
-  }
   const int j = item - p.split_from;
+  groups = 3;
+  if (j < 0) return item;
+  if (j >= 2 * p.split_tiles) return item - p.split_tiles;
   groups = 1 << (j & 1);
   return p.split_from + (j >> 1);
 }
+
+// The same where the filters do not fill their last block of 64: tiles from half_from on have at most 32 filters, which is work
+// for group 0 alone.
+__device__ __forceinline__ int ragged_item(const WinoParams &p, int item, int &groups) {
+  const int t = item_tile(p, item, groups);
+  if (t >= p.half_from) groups = 1;
+  return t;
+}
+
+// Columns.  A block of 32 columns is eight quads (four images of one 2x2-output tile each) that follow one another in the list
+// (tile row, tile column, image quad), image quads fastest.  Where the batch is a multiple of 32 that makes a block 32 images of
+// one tile; where it is not, blocks run on from tile to tile ("packed"), and no column is empty but in the very last block.
+struct ColumnQuad { int tx, ty, n; bool valid; };
+__device__ __forceinline__ ColumnQuad column_quad(const WinoParams &p, int quad) {
+  const int per_tile = p.N >> 2;
+  ColumnQuad r;
+  int t = quad / per_tile;
+  r.n = 4 * (quad - t * per_tile);
+  r.ty = t / p.tiles_w;
+  r.tx = t - r.ty * p.tiles_w;
+  r.valid = r.ty < p.tiles_h;
+  r.ty += p.ty0;
+  return r;
+}
+
+// Loads the 4x4 patches of a packed block as TMA lays them out, [channel][4 h][4 w][32 columns]; all lanes of a warp.  A block
+// that lies in one tile comes by TMA all the same.  Else a lane copies one of the eight quads (16 bytes of an input row) of
+// one of the four pixel columns for every row and channel, zeros where there is no pixel, image or channel.
+struct PackedLoader {
+  const float *src[4];         // the lane's quad in each of the patch's rows, of the next channel
+  uint32_t outside;            // bit h: the image does not have row h of the patch, or not this pixel column
+  ColumnQuad first;
+  bool whole;
+  __device__ __forceinline__ void start(const WinoParams &p, int block) {
+    const int lane = threadIdx.x & 31, px = lane >> 3;
+    first = column_quad(p, 8 * block);
+    whole = first.n + 32 <= p.N && first.valid;
+    if (whole) return;
+    const ColumnQuad q = column_quad(p, 8 * block + (lane & 7));
+    const int w = 2 * q.tx - 1 + px, h0 = 2 * q.ty - 1;
+    outside = 0;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const bool out = !q.valid || w < 0 || w >= p.W || h0 + h < 0 || h0 + h >= p.H;
+      src[h] = p.x + (out ? 0 : ((long long)(h0 + h) * p.W + w) * p.N + q.n);
+      outside |= (uint32_t)out << h;
+    }
+  }
+  // One chunk of CH channels from `c0` on; `bar` expects 32 arrivals.  To be called for c0 = 0, CH, 2 CH ...
+  template <int CH>
+  __device__ __forceinline__ void chunk(const WinoParams &p, const CUtensorMap *tm_in, uint32_t dst, uint32_t bar, int c0) {
+    const int lane = threadIdx.x & 31;
+    if (whole) {
+      if (lane == 0) {
+        mbar_arrive_expect_tx(bar, CH * 16 * 32 * 4u);
+        tma_load_4d(dst, tm_in, bar, first.n, 2 * first.tx - 1, 2 * first.ty - 1, c0);
+      } else {
+        mbar_arrive(bar);
+      }
+      return;
+    }
+    const size_t plane = (size_t)p.H * p.W * p.N;
+    const int exist = p.C - c0;
+    const uint32_t at = dst + (lane >> 3) * 128u + (lane & 7) * 16u;
+    const bool out0 = outside & 1u, out1 = outside & 2u, out2 = outside & 4u, out3 = outside & 8u;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const bool none = c >= exist;
+      cp_async_16(at + (c * 16 + 0) * 128u, src[0], out0 || none);
+      cp_async_16(at + (c * 16 + 4) * 128u, src[1], out1 || none);
+      cp_async_16(at + (c * 16 + 8) * 128u, src[2], out2 || none);
+      cp_async_16(at + (c * 16 + 12) * 128u, src[3], out3 || none);
+#pragma unroll
+      for (int h = 0; h < 4; ++h) src[h] += plane;
+    }
+    cp_async_arrive(bar);
+  }
+};
 
 // ---------------------------------------------------------------------------------------------
 // Output transform Y = A^T M A for one (image, filter): rows first, then columns
@@ -171,23 +253,35 @@ __device__ __forceinline__ void group_barrier(int gi) {
 //   OPTLDS64      deposit as OPTSTS64, read back 16 x LDS.64, float2 stores
 // Only the group's own named barrier is used, so the other group keeps computing meanwhile.
 // ---------------------------------------------------------------------------------------------
-template <int V, bool RAGGED>
+template <int V, int SHAPE>
 __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, const WinoParams &p,
-                                         const TileCoord &tc, const LaneRole &role) {
+                                         int tile, const LaneRole &role) {
   const int lane = threadIdx.x & 31;
   constexpr int RF = Staging<V>::kRowFloats;
-
-  const int oh0 = 2 * tc.ty, ow0 = 2 * tc.tx;
+  constexpr bool RAGGED = SHAPE != kExact, PACKED = SHAPE == kPacked;
+  const int col = V == kOptLds64 ? 2 * (lane & 15) : lane;            // first column that this lane reads back and stores
+  // Packed kernel: every quad of columns has a place of its own in the output.  Columns and filters beyond the end are not
+  // stored.  (Instantiations of their own, so that the usual case pays nothing; its base address is the same in all lanes.)
+  int oh0, ow0, kb;
+  size_t at;                                                          // of output row oh0, column ow0 in a filter's plane
+  size_t at_lane = col;
+  bool n_ok = true;
+  if (PACKED) {
+    kb = tile / p.blocks;
+    const ColumnQuad q = column_quad(p, 8 * (tile - kb * p.blocks) + (col >> 2));
+    oh0 = 2 * q.ty; ow0 = 2 * q.tx; n_ok = q.valid;
+    at = 0;
+    at_lane = ((size_t)oh0 * p.W + ow0) * p.N + q.n + (col & 3);
+  } else {
+    const TileCoord tc = decode_tile(p, tile);
+    oh0 = 2 * tc.ty; ow0 = 2 * tc.tx; kb = tc.kb;
+    at = ((size_t)oh0 * p.W + ow0) * p.N + (size_t)tc.nb * kBN;
+  }
   const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
   const size_t plane = (size_t)p.H * p.W * p.N;                       // one filter's output
-  float *ybase = p.y + ((size_t)oh0 * p.W + ow0) * p.N + (size_t)tc.nb * kBN +
-                 ((size_t)tc.kb * kBK + 32 * role.gi) * plane;
+  float *ybase = p.y + at + ((size_t)kb * kBK + 32 * role.gi) * plane;
   const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N;
-  // Ragged last block of images or filters (N not a multiple of 32, K not of 64; its own kernel
-  // instantiation, so that the usual case pays nothing): what is missing was loaded as zeros and
-  // is not stored.  N is a multiple of 4, so an image pair is either inside or outside.
-  const bool n_ok = !RAGGED || (V == kOptLds64 ? 2 * (lane & 15) : lane) < p.N - tc.nb * kBN;
-  const int k_left = p.K - (tc.kb * kBK + 32 * role.gi);              // filters of this group's 32 that exist
+  const int k_left = p.K - (kb * kBK + 32 * role.gi);                 // filters of this group's 32 that exist
 
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -226,7 +320,7 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
       float y0[4], y1[4];
       output_transform(m0, y0);
       output_transform(m1, y1);
-      float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + 2 * np;
+      float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + at_lane;
       if (n_ok && (!RAGGED || round_filter<V>(kl, r) < k_left)) {
         *reinterpret_cast<float2 *>(dst) = make_float2(y0[0], y1[0]);
         if (col1) *reinterpret_cast<float2 *>(dst + dW) = make_float2(y0[1], y1[1]);
@@ -248,7 +342,7 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
         }
         float yy[4];
         output_transform(m, yy);
-        float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + lane;
+        float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + at_lane;
         if (n_ok && (!RAGGED || round_filter<V>(kl, r) < k_left)) {
           dst[0] = yy[0];
           if (col1) dst[dW] = yy[1];
@@ -333,11 +427,51 @@ __device__ __forceinline__ void fma_frag(uint64_t (&acc)[8][8], const Frag &f) {
     for (int qq = 0; qq < 8; ++qq) ffma2(acc[kk][qq], vv[qq], dup[kk]);
 }
 
-template <int V, bool RAGGED>
+// The packed kernel's loader (one whole warp).
+__device__ __forceinline__ void load_packed(const WinoParams &p, const CUtensorMap *tm_in, const CUtensorMap *tm_u, float *stages,
+                                            uint64_t *bar_full, uint64_t *bar_empty, int S, int my_tiles, volatile int *dead) {
+  const int lane = threadIdx.x & 31, cpt = p.chunks_per_tile;
+  if (lane == 0) {
+    tma_prefetch_descriptor(tm_in);
+    tma_prefetch_descriptor(tm_u);
+  }
+  int g = 0;
+  bool ok = true;
+  for (int seq = 0; seq < my_tiles && ok; ++seq) {
+    int groups_unused;
+    const int tile = ragged_item(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused);
+    const int kb = tile / p.blocks;
+    PackedLoader patches;
+    patches.start(p, tile - kb * p.blocks);
+    for (int ci = 0; ci < cpt; ++ci, ++g) {
+      const int s = g % S;
+      // A wait that gave up: stop issuing - the stage may still be in use.
+      if (g >= S && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(bar_empty + s), ((g / S) - 1) & 1, dead, p.status))) { ok = false; break; }
+      const uint32_t bar = smem_u32(bar_full + s), dst = smem_u32(stages + s * kStageFloats);
+      if (lane == 0) {
+        mbar_expect_tx(bar, kUStageFloats * 4u);
+        if (g > 0) tma_load_3d(dst + kVStageFloats * 4u, tm_u, bar, kb * kBK, 0, ci * kBC);
+      }
+      __syncwarp();
+      patches.chunk<kBC>(p, tm_in, dst, bar, ci * kBC);
+      if (g == 0 && lane == 0) {
+        grid_dependency_wait();                     // U is all that the kernel before this one writes
+        tma_load_3d(dst + kVStageFloats * 4u, tm_u, bar, kb * kBK, 0, ci * kBC);
+      }
+    }
+  }
+  // No exit with copies in flight (see the other loader).
+  cp_async_wait_all();
+  if (lane == 0)
+    for (int i = g > S ? g - S : 0; i < g; ++i) mbar_wait_drain(smem_u32(bar_full + i % S), (i / S) & 1);
+}
+
+template <int V, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 1)
 wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u,
                  const WinoParams p) {
   constexpr int S = SmemLayout<V>::kStages;
+  constexpr bool RAGGED = SHAPE != kExact, PACKED = SHAPE == kPacked;
   extern __shared__ __align__(1024) float smem[];
   float *stages = smem;
   float *stg = smem + S * kStageFloats;
@@ -353,7 +487,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   if (tid == 0) {
     *dead = 0;
     for (int s = 0; s < S; ++s) {
-      mbar_init(smem_u32(bar_full + s), 1);                       // the TMA issuer + its bytes
+      mbar_init(smem_u32(bar_full + s), PACKED ? 32 : 1);         // the TMA issuer and its bytes; packed: each lane of the loader
       mbar_init(smem_u32(bar_ready + s), kTransformThreads / 32);  // one arrive per transform warp
       mbar_init(smem_u32(bar_empty + s), kConsumerThreads / 32);   // one arrive per consumer warp
     }
@@ -365,8 +499,10 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     // =============================== producers ===============================================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
     if (warp == kConsumerThreads / 32) {
-      // ---- TMA issuer: one lane keeps the ring full ----
-      if (lane == 0) {
+      if (PACKED) {
+        load_packed(p, &tm_in, &tm_u, stages, bar_full, bar_empty, S, my_tiles, dead);
+      } else if (lane == 0) {
+        // ---- TMA issuer: one lane keeps the ring full ----
         tma_prefetch_descriptor(&tm_in);
         tma_prefetch_descriptor(&tm_u);
         int seq = 0, ci = 0, groups_unused, issued = 0;
@@ -436,7 +572,8 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   int g = 0;                                                       // chunk counter over all items of this CTA
   for (int seq = 0; seq < my_tiles; ++seq) {
     int groups;
-    const int tile = item_tile(p, (int)blockIdx.x + seq * (int)gridDim.x, groups);
+    const int item = (int)blockIdx.x + seq * (int)gridDim.x;
+    const int tile = RAGGED ? ragged_item(p, item, groups) : item_tile(p, item, groups);
     if ((groups >> role.gi) & 1) {
       // ---- this group computes the item ----
       for (int ci = 0; ci < cpt; ++ci, ++g) {
@@ -470,8 +607,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
           if (lane == 0) mbar_arrive(smem_u32(bar_empty + s));
         }
       }
-      const TileCoord tc = decode_tile(p, tile);
-      epilogue<V, RAGGED>(acc, my_stg, p, tc, role);
+      epilogue<V, SHAPE>(acc, my_stg, p, tile, role);
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll

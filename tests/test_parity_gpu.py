@@ -116,6 +116,22 @@ def test_any_channel_count_bit_for_bit(oracle, libs, variant, shape):
             "the tensor-core path keeps K % 64 == 0"
 
 
+# Packed columns (batches that are not a multiple of 32): blocks of 32 columns that lie in one tile, end in the next one, span
+# up to eight and run past the last; filters that leave the second group of the last block idle or not; channel counts that
+# leave the last chunk one to seven channels; fewer items than SMs, more, and a last round that is split.
+PACKED = [(4, 3, 20, 9, 7), (8, 5, 64, 12, 12), (12, 21, 100, 5, 9), (20, 10, 96, 31, 45), (28, 9, 36, 3, 3), (36, 13, 68, 6, 5),
+          (100, 4, 132, 13, 16), (116, 30, 64, 8, 9), (252, 7, 160, 3, 2), (32, 11, 96, 24, 17), (64, 23, 72, 19, 18)]
+
+
+@pytest.mark.parametrize("variant", build.VARIANTS)
+@pytest.mark.parametrize("shape", PACKED)
+def test_packed_columns_bit_for_bit(oracle, libs, variant, shape):
+    N, C, K, H, W = shape
+    x, g = oracle.input_chwn(N, C, H, W), oracle.filter_crsk(C, K)
+    y, _ = run(variant, x, g, "stream")
+    assert np.array_equal(y, oracle.forward(x, g))
+
+
 @pytest.mark.parametrize("variant", build.VARIANTS)
 def test_integer_known_answers_are_exact(oracle, libs, variant):
     for N, C, K, H, W in [(32, 8, 64, 5, 5), (64, 16, 64, 8, 8)]:
