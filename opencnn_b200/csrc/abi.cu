@@ -15,6 +15,7 @@
 #include "wino_fp32.cuh"
 #include "wino_tc.cuh"
 #include "wino_pair.cuh"
+#include "wino_img.cuh"
 #include "wino_tc64.cuh"
 
 #if defined(BASE)
@@ -41,7 +42,7 @@ struct DeviceState {
   std::once_flag once;
   cudaError_t init_error = cudaSuccess;
   int sm_count = 0;
-  int max_clusters[2] = {0, 0};   // co-resident CTA pairs of wino_pair_kernel<BF16 / TF32>
+  int max_clusters[2] = {0, 0};   // co-resident CTA pairs of wino_pair_kernel and wino_img_kernel, <BF16 / TF32>
   int *status_ptr = nullptr;
 };
 DeviceState g_dev[kMaxDevices];
@@ -90,7 +91,11 @@ cudaError_t device_state(DeviceState **out) {
         if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, kernel);
         if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
       }
-      // the same for the CTA-pair kernel
+      // the same for the CTA-pair kernels
+      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_img_kernel<ocb::kTcBf16>);
+      if (err == cudaSuccess && fa.numRegs < ocb::kImgLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_img_kernel<ocb::kTcTf32>);
+      if (err == cudaSuccess && fa.numRegs < ocb::kImgLaunchRegs) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcBf16>);
       if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcTf32>);
@@ -111,6 +116,12 @@ cudaError_t device_state(DeviceState **out) {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_pair_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ocb::PairCfg<ocb::kTcTf32>::kSmemBytes);
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(ocb::wino_img_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes);
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(ocb::wino_img_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes);
     if (err == cudaSuccess) {
       // how many CTA pairs fit on the device at once (pairs must sit in one GPC)
       cudaLaunchConfig_t cfg = {};
@@ -121,12 +132,17 @@ cudaError_t device_state(DeviceState **out) {
       attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
       cfg.attrs = &attr;
       cfg.numAttrs = 1;
-      cfg.dynamicSmemBytes = ocb::PairCfg<ocb::kTcBf16>::kSmemBytes;
-      err = cudaOccupancyMaxActiveClusters(&st.max_clusters[0], ocb::wino_pair_kernel<ocb::kTcBf16>, &cfg);
-      if (err == cudaSuccess) {
-        cfg.dynamicSmemBytes = ocb::PairCfg<ocb::kTcTf32>::kSmemBytes;
-        err = cudaOccupancyMaxActiveClusters(&st.max_clusters[1], ocb::wino_pair_kernel<ocb::kTcTf32>, &cfg);
-      }
+      const auto pairs = [&](auto kernel, size_t smem, int &clusters) {
+        int n = 0;
+        cfg.dynamicSmemBytes = smem;
+        if (err == cudaSuccess) err = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+        clusters = clusters == 0 || n < clusters ? n : clusters;
+      };
+      pairs(ocb::wino_pair_kernel<ocb::kTcBf16>, ocb::PairCfg<ocb::kTcBf16>::kSmemBytes, st.max_clusters[0]);
+      pairs(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes, st.max_clusters[1]);
+      cfg.blockDim = dim3(ocb::kImgThreads);
+      pairs(ocb::wino_img_kernel<ocb::kTcBf16>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.max_clusters[0]);
+      pairs(ocb::wino_img_kernel<ocb::kTcTf32>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, st.max_clusters[1]);
     }
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_tc64_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -194,6 +210,33 @@ cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem
   return cudaGetLastError();
 }
 
+// Tensor map of the input for the 4x4 patches of 32 images and `channels` channels.
+bool encode_patches(EncodeTiledFn enc, CUtensorMap *map, const float *input, int N, int C, int H, int W, int channels) {
+  cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
+  cuuint64_t strides[3] = {(cuuint64_t)N * 4, (cuuint64_t)W * N * 4, (cuuint64_t)H * W * N * 4};
+  cuuint32_t box[4] = {32, 4, 4, (cuuint32_t)channels};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Tensor map of the workspace [C][16][K] of a tensor-core precision, viewed as {filter within a row of `row_bytes`, channel, row,
+// position}: boxes of one K-step of channels, `rows` rows of filters and all positions, swizzled over a row.
+template <int DT>
+bool encode_filter(EncodeTiledFn enc, CUtensorMap *map, const float *workspace, int C, int K, int row_bytes, int rows) {
+  constexpr bool bf16 = DT == ocb::kTcBf16;
+  constexpr int esz = bf16 ? 2 : 4;
+  cuuint64_t dims[4] = {(cuuint64_t)(row_bytes / esz), (cuuint64_t)C, (cuuint64_t)K * esz / row_bytes, 16};
+  cuuint64_t strides[3] = {(cuuint64_t)16 * K * esz, (cuuint64_t)row_bytes, (cuuint64_t)K * esz};
+  cuuint32_t box[4] = {(cuuint32_t)(row_bytes / esz), (cuuint32_t)ocb::TcCfg<DT>::kKC, (cuuint32_t)rows, 16};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(workspace),
+             dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             !bf16 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 cudaError_t launch_fx(const float *filter, float *workspace, int C, int K, cudaStream_t stream) {
   const int k4 = K / 4;
   const int total = C * k4;
@@ -212,16 +255,7 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
 
   const bool packed = N % ocb::kBN != 0, ragged = K % ocb::kBK != 0;      // which instantiation (see ocb::Shape)
   CUtensorMap tm_in, tm_u;
-  {
-    cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
-    cuuint64_t strides[3] = {(cuuint64_t)N * 4, (cuuint64_t)W * N * 4, (cuuint64_t)H * W * N * 4};
-    cuuint32_t box[4] = {(cuuint32_t)ocb::kBN, 4, 4, (cuuint32_t)ocb::kBC};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
+  if (!encode_patches(enc, &tm_in, input, N, C, H, W, ocb::kBC)) return cudaErrorInvalidValue;
   {
     cuuint64_t dims[3] = {(cuuint64_t)K, 16, (cuuint64_t)C};
     cuuint64_t strides[2] = {(cuuint64_t)K * 4, (cuuint64_t)K * 16 * 4};
@@ -241,7 +275,9 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   p.tiles_w = (W + 1) / 2;
   p.n_blocks = (N + ocb::kBN - 1) / ocb::kBN;
   p.k_blocks = (K + ocb::kBK - 1) / ocb::kBK;
-  const long long blocks = ((long long)p.tiles_h * p.tiles_w * (N / 4) + 7) / 8;
+  p.packed = packed;
+  p.quads_per_tile = N / 4;
+  const long long blocks = ((long long)p.tiles_h * p.tiles_w * p.quads_per_tile + 7) / 8;
   const long long tiles = blocks * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.blocks = (int)blocks;
@@ -268,6 +304,24 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
+// Sizes of a problem for a tensor-core kernel, and its blocks of 32 columns (see ocb::ColumnQuad).
+long long column_blocks(int N, int H, int W) {
+  return (long long)((H + 1) / 2) * ((W + 1) / 2) * ((N + ocb::kTcN - 1) / ocb::kTcN);
+}
+bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K) {
+  const long long blocks = column_blocks(N, H, W);
+  p.x = input;
+  p.y = output;
+  p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
+  p.tiles_h = (H + 1) / 2;
+  p.tiles_w = (W + 1) / 2;
+  p.packed = false;
+  p.quads_per_tile = (N + ocb::kTcN - 1) / ocb::kTcN * (ocb::kTcN / 4);
+  p.blocks = (int)blocks;
+  p.ty0 = 0;
+  return blocks <= 0x7fffffffll / 16;
+}
+
 // Tensor-core path: filter transform rounded to the operand type, then the tcgen05 kernel.
 template <int DT>
 cudaError_t launch_fx_tc(const float *filter, float *workspace, int C, int K, cudaStream_t stream) {
@@ -287,47 +341,20 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   if (!enc) return cudaErrorNotSupported;
   constexpr int KC = ocb::TcCfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
-  constexpr cuuint64_t esz = bf16 ? 2 : 4;
-  constexpr cuuint32_t row_elems = bf16 ? 64 : 32;            // filters in one 128-byte row
+  constexpr int esz = bf16 ? 2 : 4;
 
   CUtensorMap tm_in, tm_u;
-  {
-    cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
-    cuuint64_t strides[3] = {(cuuint64_t)N * 4, (cuuint64_t)W * N * 4, (cuuint64_t)H * W * N * 4};
-    cuuint32_t box[4] = {(cuuint32_t)ocb::kTcN, 4, 4, (cuuint32_t)KC};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
-  {
-    // workspace [C][16][K] viewed as {filter within a 128-byte row, channel, 128-byte row, position}
-    cuuint64_t dims[4] = {row_elems, (cuuint64_t)C, (cuuint64_t)K / row_elems, 16};
-    cuuint64_t strides[3] = {(cuuint64_t)16 * K * esz, 128, (cuuint64_t)K * esz};
-    // BF16 with at most 64 filters: only the first 64-filter row block is loaded (wino_tc.cuh, "half U")
-    const bool half_u = bf16 && K <= 64;
-    cuuint32_t box[4] = {row_elems, (cuuint32_t)KC, half_u ? 1u : (cuuint32_t)(ocb::kTcM / row_elems), 16};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_u, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-            const_cast<float *>(workspace), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            bf16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
+  if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  // BF16 with at most 64 filters: only the first 64-filter row block is loaded (wino_tc.cuh, "half U")
+  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 && K <= 64 ? 1 : ocb::kTcM * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  p.y = output;
-  p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
-  p.tiles_h = (H + 1) / 2;
-  p.tiles_w = (W + 1) / 2;
-  p.n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
+  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
-  const long long tiles = (long long)p.tiles_h * p.tiles_w * p.n_blocks * p.k_blocks;
+  const long long tiles = (long long)p.blocks * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.total_tiles = (int)tiles;
   p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
-  p.ty0 = 0;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
   if (bf16 && K <= 64)
@@ -347,51 +374,53 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   if (!enc) return cudaErrorNotSupported;
   constexpr int KC = ocb::PairCfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
-  constexpr cuuint64_t esz = bf16 ? 2 : 4;
-  constexpr cuuint32_t row_elems = bf16 ? 64 : 32;
+  constexpr int esz = bf16 ? 2 : 4;
   const int max_clusters = st->max_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
 
   CUtensorMap tm_in, tm_u;
-  {
-    cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
-    cuuint64_t strides[3] = {(cuuint64_t)N * 4, (cuuint64_t)W * N * 4, (cuuint64_t)H * W * N * 4};
-    cuuint32_t box[4] = {(cuuint32_t)ocb::kTcN, 4, 4, (cuuint32_t)KC};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
-  {
-    cuuint64_t dims[4] = {row_elems, (cuuint64_t)C, (cuuint64_t)K / row_elems, 16};
-    cuuint64_t strides[3] = {(cuuint64_t)16 * K * esz, 128, (cuuint64_t)K * esz};
-    cuuint32_t box[4] = {row_elems, (cuuint32_t)KC, (cuuint32_t)(ocb::kPairFilters / row_elems), 16};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_u, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-            const_cast<float *>(workspace), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            bf16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
+  if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, ocb::kPairFilters * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  p.y = output;
-  p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
-  p.tiles_h = (H + 1) / 2;
-  p.tiles_w = (W + 1) / 2;
-  p.n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
+  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
-  const long long blocks = (long long)p.tiles_h * p.tiles_w * p.n_blocks;
-  const long long tiles = (blocks + 1) / 2 * p.k_blocks;
-  if (blocks > 0x7fffffffll / 8 || tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
-  p.blocks = (int)blocks;
+  const long long tiles = ((long long)p.blocks + 1) / 2 * p.k_blocks;
+  if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.total_tiles = (int)tiles;
   p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
-  p.ty0 = 0;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
   return launch_main(ocb::wino_pair_kernel<DT>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+}
+
+// Image columns in the accumulator rows: 64 filters x four blocks of 32 columns per cluster of two (wino_img.cuh).
+template <int DT>
+cudaError_t launch_wino_img(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
+                            int K, cudaStream_t stream, bool after_fx) {
+  DeviceState *st = nullptr;
+  cudaError_t e = device_state(&st);
+  if (e != cudaSuccess) return e;
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return cudaErrorNotSupported;
+  constexpr int KC = ocb::ImgCfg<DT>::kKC;
+  constexpr bool bf16 = DT == ocb::kTcBf16;
+  const int max_clusters = st->max_clusters[bf16 ? 0 : 1];
+  if (max_clusters <= 0) return cudaErrorNotSupported;
+  CUtensorMap tm_in, tm_u;
+  if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
+  ocb::WinoParams p;
+  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
+  p.k_blocks = K / ocb::kImgFilters;
+  const long long tiles = ((long long)p.blocks + 3) / 4 * p.k_blocks;
+  if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
+  p.total_tiles = (int)tiles;
+  p.total_items = p.total_tiles;
+  p.chunks_per_tile = (C + KC - 1) / KC;
+  p.status = st->status_ptr;
+  const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
+  return launch_main(ocb::wino_img_kernel<DT>, 2 * clusters, ocb::kImgThreads, ocb::ImgCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // Layers with at most 64 filters: two 32-image blocks share the 128 accumulator rows (wino_tc64.cuh).
@@ -407,106 +436,80 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   constexpr int KC = ocb::T64Cfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
   CUtensorMap tm_in, tm_u;
-  {
-    cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
-    cuuint64_t strides[3] = {(cuuint64_t)N * 4, (cuuint64_t)W * N * 4, (cuuint64_t)H * W * N * 4};
-    cuuint32_t box[4] = {(cuuint32_t)ocb::kTcN, 4, 4, (cuuint32_t)KC};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
-  {
-    // workspace [C][16][K] viewed as {filter within a 128-byte row, channel, 128-byte row, position}.
-    // BF16: one row block of 64 filters.  TF32: a box of four row blocks of 32 filters, of which two exist -
-    // the hardware fills the other two with zeros, which the kernel uses as the empty half of its A operand.
-    constexpr cuuint64_t esz = bf16 ? 2 : 4;
-    constexpr cuuint32_t row_elems = bf16 ? 64 : 32;
-    cuuint64_t dims[4] = {row_elems, (cuuint64_t)C, (cuuint64_t)K / row_elems, 16};
-    cuuint64_t strides[3] = {(cuuint64_t)16 * K * esz, 128, (cuuint64_t)K * esz};
-    cuuint32_t box[4] = {row_elems, (cuuint32_t)KC, bf16 ? 1u : 4u, 16};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_u, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-            const_cast<float *>(workspace), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            bf16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
-  }
+  if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  // BF16: one row block of 64 filters.  TF32: a box of four row blocks of 32 filters, of which two exist -
+  // the hardware fills the other two with zeros, which the kernel uses as the empty half of its A operand.
+  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 ? 1 : 4)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  p.y = output;
-  p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
-  p.tiles_h = (H + 1) / 2;
-  p.tiles_w = (W + 1) / 2;
-  p.n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
+  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
   p.k_blocks = 1;
-  const long long tiles = (long long)p.tiles_h * p.tiles_w * ((p.n_blocks + 1) / 2);
-  if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
-  p.total_tiles = (int)tiles;
+  p.total_tiles = (p.blocks + 1) / 2;
   p.total_items = p.total_tiles;
   p.chunks_per_tile = (C + KC - 1) / KC;
-  p.ty0 = 0;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
   return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
-// Which tensor-core kernel a problem gets.  All three give the same bits.  The measure is K-steps x rounds: what one SM
-// works through, a round being one tile of 32 images per SM.  Fused kernel alone, back to back, medians in us, measured at 930
-// sizes per type of 1 to 64 K-steps and 1 to 45 rounds; this rule is 0.15 % behind the best kernel of each on average.
-//   More than 64 filters: the CTA-pair kernel loads and multiplies faster, but costs about 2 us more to start.
-//     K-steps x rounds, single : pair   N x C x K x H x W in BF16 (TF32: half the channels)
-//      1 x 1   8.4 :  9.5 /  8.4 :  8.9   64x16x128x14x14         3 x 1   9.5 : 10.5 /  8.4 : 10.5   64x48x128x14x14
-//      4 x 2  14.6 : 14.6 / 13.4 : 12.5   64x64x128x20x20         8 x 1  12.5 : 12.5 / 12.4 : 11.9   64x128x128x14x14
-//      3 x 6  27.4 : 25.0 / 24.8 : 22.8   128x48x128x28x28        8 x 6  53.3 : 43.3 / 41.6 : 33.5   128x128x128x28x28
-//     fewer than three K-steps have little to gain:
-//      2 x 6  21.9 : 22.8 / 20.7 : 20.7   128x32x128x28x28        1 x 14 33.0 : 35.6 / 33.0 : 34.9   160x16x192x28x28
-//      1 x 22 70.7 : 51.6 / 51.5 : 49.4   128x16x128x56x56
-//   At most 64 filters: half of the rows of the pair's operand are empty, so it has to gain more; the stacked kernel does
-//   two blocks of images per step and needs 1.5 (one K-step) to almost 2 times (many) as long for it, so its rounds have to be
-//   nearly half of the others': their ratio at least 2 - 1.8 / K-steps in BF16 and 2 - 1 / K-steps in TF32.  Single : pair : stacked, rounds of the first two / of the stacked
-//      4 x 2/1  12.5 : 14.6 : 11.5 / 12.5 : 12.9 : 11.0   64x64x64x20x20
-//      8 x 3/2  22.8 : 22.9 : 24.8 / 22.8 : 20.7 : 22.8   64x128x64x28x28
-//      1 x 15/9 31.0 : 37.3 : 26.9 (BF16)                  1 x 20/12 40.4 : 45.0 : 33.4 (TF32)
-//     16 x 7/4  75.6 : 72.3 : 81.3 (BF16)                  3 x 5/3   20.7 : 22.8 : 20.7 (TF32)
-//      4 x 6/3  28.8 : 28.9 : 22.8 / 25.5 : 24.8 : 21.8   128x64x64x28x28
-//      8 x 6/3  41.2 : 40.9 : 35.1 / 38.5 : 33.0 : 31.1   128x128x64x28x28
-//     24 x 6/3  92.2 : 90.0 : 88.5 / 90.4 : 67.2 : 85.2   128x384x64x28x28
-//      4 x 22/11 89.2 : 85.9 : 71.9 / 78.1 : 69.9 : 69.7  128x64x64x56x56
-//      8 x 22/11 134 : 131 : 119 / 126 : 103 : 115        128x128x64x56x56
-//      2 x 170/85 820 : 417 : 394 (BF16), 4 x 170/85 569 : 486 : 500 (TF32)  256x32x64x112x112
-//     12 x 1/1  13.6 : 14.6 : 18.7 / 13.6 : 13.2 : 18.2   96x192x64x14x14
-//     16 x 3/2  35.2 : 35.1 : 40.5 / 35.1 : 27.9 : 36.9   64x256x64x28x28
-//     48 x 1/1  31.0 : 28.9 : 51.8 (BF16)                 32x768x64x4x4
+// Which tensor-core kernel a problem gets: the one with the least estimated time.  All give the same bits.  An SM (or a CTA
+// pair) works through its tiles one after the other, so a kernel takes
+//     start + rounds x (round + step x K-steps),   K-steps = channels / 16 (BF16) or 8 (TF32),
+// and a problem much larger than L2 no less than its bytes at the rate the kernel's stores and loads were seen to reach.  The constants are
+// least squares through the fused kernels' times, back to back, at 260 random sizes per type (8 to 256 images, 64 to 1024
+// filters, 1 to 1024 channels, maps of 4 to 112); the estimates are 4 to 6 % off in the mean, and the kernel chosen by them is 0.4 %
+// behind the fastest one in the mean, 3 % at the 95th percentile.  Both sides of it, us, single : pair : stacked : image rows:
+//   few K-steps or rounds      128x32x128x28x28  BF16 22.6 : 22.6 : - : 25.2    TF32 28.7 : 24.8 : - : 28.7
+//                              128x64x64x14x14   BF16 12.3 : 14.4 : 10.3 : 12.3  TF32 16.4 : 16.4 : 14.4 : 12.3
+//   64 filters                 128x64x64x56x56   BF16 83.8 : 86.1 : 71.8 : 67.6  TF32 124 : 105 : 113 : 72.1
+//                              256x32x64x112x112 BF16 814 : 413 : 390 : 277      TF32 553 : 486 : 491 : 303
+//                              128x512x64x14x14  BF16 41.5 : 40.8 : 41.0 : 30.8  TF32 77.3 : 51.3 : 61.6 : 39.0
+//   more filters, deep         128x256x256x14x14 BF16 41.0 : 34.9 : - : 45.4    TF32 63.1 : 43.3 : - : 57.5
+//                              64x1024x1024x14x14 BF16 278 : 200 : - : 300      TF32 506 : 325 : - : 469
+//   more filters, large output 96x4x128x99x99    BF16 174 : 131 : - : 122       TF32 188 : 131 : - : 111
+struct KernelCost {
+  double start, round, step;    // us
+  double rate;                  // MB per us
+};
+constexpr double kL2Bound = 200.0;   // MB of input and output from which on the rate counts
+struct TcCosts { KernelCost single, single64, pair, stacked, image_rows; };   // single64: at most 64 filters
+constexpr TcCosts kTcCosts[2] = {   // BF16, TF32
+    {{5.8, 1.29, 0.672, 2.9}, {4.9, 1.16, 0.57, 2.9}, {6.8, 1.53, 0.487, 4.1}, {5.2, 1.63, 1.043, 4.1}, {7.1, 1.61, 0.741, 4.5}},
+    {{5.3, 1.32, 0.576, 2.9}, {5, 1.32, 0.557, 2.9}, {6.8, 1.6, 0.338, 4.2}, {5.2, 1.79, 0.883, 4.1}, {7.1, 1.61, 0.493, 5.1}},
+};
+
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
                       cudaStream_t stream, bool after_fx, int kernel = OPENCNN_TC_AUTO) {
-  if (kernel == OPENCNN_TC_SINGLE_CTA) return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-  if (kernel == OPENCNN_TC_PAIR_LOCAL) return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-  if (kernel == OPENCNN_TC_STACKED_BLOCKS) return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-  if (kernel != OPENCNN_TC_AUTO) return cudaErrorInvalidValue;
-  DeviceState *st = nullptr;
-  cudaError_t e = device_state(&st);
-  if (e != cudaSuccess) return e;
-  constexpr bool bf16 = DT == ocb::kTcBf16;
-  const long long k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC;
-  const long long tiles = (long long)((H + 1) / 2) * ((W + 1) / 2), n_blocks = (N + ocb::kTcN - 1) / ocb::kTcN;
-  const auto rounds_of = [&](long long all_tiles) { return (all_tiles + st->sm_count - 1) / st->sm_count; };
-  const long long rounds = rounds_of(tiles * n_blocks * ((K + ocb::kTcM - 1) / ocb::kTcM));
-  bool pair;
-  if (K <= 64) {
-    const long long stacked_rounds = rounds_of(tiles * ((n_blocks + 1) / 2));
-    if (2 * rounds >= 3 * stacked_rounds && 5 * k_steps * (2 * stacked_rounds - rounds) <= (bf16 ? 9 : 5) * stacked_rounds &&
-        (bf16 ? k_steps <= 24 : k_steps <= 3 || (k_steps <= 12 && k_steps * rounds <= 48)))
-      return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-    pair = bf16 ? k_steps * rounds >= (k_steps >= 16 ? 32 : 48) : k_steps >= 10 || (k_steps >= 3 && k_steps * rounds >= 14);
-  } else {
-    pair = k_steps * rounds >= (k_steps >= 3 ? 8 : 20);
+  if (kernel == OPENCNN_TC_AUTO) {
+    DeviceState *st = nullptr;
+    const cudaError_t e = device_state(&st);
+    if (e != cudaSuccess) return e;
+    constexpr bool bf16 = DT == ocb::kTcBf16;
+    const TcCosts &costs = kTcCosts[bf16 ? 0 : 1];
+    const double k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC, mb = 4e-6 * N * H * W * ((double)C + K);
+    double best = 0;
+    const auto consider = [&](int which, const KernelCost &c, long long tiles, int at_once) {
+      if (at_once <= 0) return;             // (no two CTAs of this size can be co-scheduled as a cluster)
+      double t = c.start + (double)((tiles + at_once - 1) / at_once) * (c.round + c.step * k_steps);
+      if (mb > kL2Bound && t < mb / c.rate) t = mb / c.rate;
+      if (kernel != OPENCNN_TC_AUTO && t >= best) return;
+      best = t;
+      kernel = which;
+    };
+    const long long blocks = column_blocks(N, H, W), wide = (K + ocb::kTcM - 1) / ocb::kTcM;
+    const int clusters = st->max_clusters[bf16 ? 0 : 1];
+    consider(OPENCNN_TC_SINGLE_CTA, K <= 64 ? costs.single64 : costs.single, blocks * wide, st->sm_count);
+    consider(OPENCNN_TC_PAIR_LOCAL, costs.pair, (blocks + 1) / 2 * wide, clusters);
+    if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, costs.stacked, (blocks + 1) / 2, st->sm_count);
+    consider(OPENCNN_TC_IMAGE_ROWS, costs.image_rows, (blocks + 3) / 4 * (K / ocb::kImgFilters), clusters);
   }
-  // (max_clusters is 0 only where no two CTAs of this size can be co-scheduled as a cluster)
-  return pair && st->max_clusters[bf16 ? 0 : 1] > 0
-             ? launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx)
-             : launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+  switch (kernel) {
+    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+    case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+    case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+    case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t forward(const float *input, const float *filter, float *output, float *workspace, int N, int C, int H,

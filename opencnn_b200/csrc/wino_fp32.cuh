@@ -83,6 +83,9 @@ struct WinoParams {
   // fp32 kernel only: work items.  The split_tiles tiles from split_from on are two items each, one per consumer
   // group (see item_tile); all others are whole, those from half_from on with one group idle (see ragged_item).
   int split_from, split_tiles, half_from, total_items;
+  // how the columns' list is made (see ColumnQuad): image quads per tile, and whether that is all of a batch that is not a multiple of 32
+  int quads_per_tile;
+  bool packed;
   int ty0;             // first tile row (tiles_h of them are computed)
   int blocks;          // 32-column blocks of all tiles: n_blocks * tiles_w * tiles_h, or the packed count (see ColumnQuad)
   int *status;         // device status word
@@ -123,19 +126,23 @@ __device__ __forceinline__ int ragged_item(const WinoParams &p, int item, int &g
 
 // Columns.  A block of 32 columns is eight quads (four images of one 2x2-output tile each) that follow one another in the list
 // (tile row, tile column, image quad), image quads fastest.  Where the batch is a multiple of 32 that makes a block 32 images of
-// one tile; where it is not, blocks run on from tile to tile ("packed"), and no column is empty but in the very last block.
+// one tile.  Where it is not, either blocks run on from tile to tile ("packed"), and no column is empty but in the very last
+// block; or every tile's quads are made up to a multiple of eight with quads of no image.
 struct ColumnQuad { int tx, ty, n; bool valid; };
 __device__ __forceinline__ ColumnQuad column_quad(const WinoParams &p, int quad) {
-  const int per_tile = p.N >> 2;
+  const int per_tile = p.quads_per_tile;
   ColumnQuad r;
   int t = quad / per_tile;
   r.n = 4 * (quad - t * per_tile);
   r.ty = t / p.tiles_w;
   r.tx = t - r.ty * p.tiles_w;
-  r.valid = r.ty < p.tiles_h;
+  r.valid = r.ty < p.tiles_h && r.n < p.N;
   r.ty += p.ty0;
   return r;
 }
+
+// First quad of a block: all there is to know of it unless blocks are packed.
+__device__ __forceinline__ ColumnQuad column_block(const WinoParams &p, int block) { return column_quad(p, 8 * block); }
 
 // Loads the 4x4 patches of a packed block as TMA lays them out, [channel][4 h][4 w][32 columns]; all lanes of a warp.  A block
 // that lies in one tile comes by TMA all the same.  Else a lane copies one of the eight quads (16 bytes of an input row) of
@@ -147,7 +154,7 @@ struct PackedLoader {
   bool whole;
   __device__ __forceinline__ void start(const WinoParams &p, int block) {
     const int lane = threadIdx.x & 31, px = lane >> 3;
-    first = column_quad(p, 8 * block);
+    first = column_block(p, block);
     whole = first.n + 32 <= p.N && first.valid;
     if (whole) return;
     const ColumnQuad q = column_quad(p, 8 * block + (lane & 7));

@@ -107,18 +107,7 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uin
   }
 }
 
-// One 32-image block of the input at one 2x2-output tile.
-struct PairBlock { int nb, tx, ty; };
-__device__ __forceinline__ PairBlock pair_block(const WinoParams &p, int q) {
-  PairBlock b;
-  b.nb = q % p.n_blocks; q /= p.n_blocks;
-  b.tx = q % p.tiles_w;
-  b.ty = q / p.tiles_w;
-  return b;
-}
-
-// p.n_blocks counts 32-image blocks, p.k_blocks 128-filter blocks, p.blocks blocks of images over all
-// tiles, p.total_tiles pair tiles (k_blocks times half of those).
+// p.k_blocks counts 128-filter blocks, p.blocks blocks of 32 columns, p.total_tiles pair tiles (k_blocks times half of those).
 template <int DT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
@@ -184,13 +173,12 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
     for (int seq = 0; seq < my_tiles; ++seq) {
       const int t = cid + seq * n_clusters, q = 2 * (t % pairs) + ib;
-      const PairBlock b = pair_block(p, q < blocks ? q : 0);
+      const ColumnQuad c = column_quad(p, 8 * q + 4 * sub + 2 * (lane & 1));
       const int k0 = (t / pairs) * 2 * kPairFilters + (int)rank * kPairFilters + 32 * (quarter & 1);
-      const int n0 = b.nb * kTcN + 16 * sub;
       mbar_wait_reporting(smem_u32(acc_full), seq & 1, dead, p.status, acc_empty0, smem_u32(nowhere));
       tc_fence_after();
-      tc_epilogue_16x32(tcol, q < blocks && k0 < p.K, p, k0 + lane, n0, 2 * b.ty, 2 * b.tx,
-                        [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
+      tc_epilogue<false>(tcol, q < blocks && k0 < p.K ? 2 : 0, p, k0 + lane, c,
+                         [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
     }
   } else if (warp >= kPairFirstTransformWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairTransformRegs));
@@ -224,26 +212,9 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairIssueRegs));
     if (warp == 0) {
       // ===================================== patches =============================================
-      if (lane == 0) {
-        tma_prefetch_descriptor(&tm_in);
-        int g = 0;
-        bool ok = true;
-        for (int seq = 0; seq < my_tiles && ok; ++seq) {
-          const int q = 2 * ((cid + seq * n_clusters) % pairs) + (int)rank;
-          const PairBlock b = pair_block(p, q < blocks ? q : 0);         // an odd last block is paired with a spare one, not stored
-          for (int ci = 0; ci < cpt; ++ci, ++g) {
-            const int s = g % SR;
-            const uint32_t use = g / SR;
-            // A wait that gave up: stop issuing - the stage may still be in use.
-            if (use > 0 && !mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
-            mbar_arrive_expect_tx(smem_u32(raw_full + s), Cfg::kRawBytes);
-            tma_load_4d(smem_u32(raw_s + s * Cfg::kRawBytes), &tm_in, smem_u32(raw_full + s), b.nb * kTcN, 2 * b.tx - 1,
-                        2 * b.ty - 1, ci * KC);
-          }
-        }
-        // No exit with bulk copies in flight (after a complete run these phases are long over).
-        for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
-      }
+      if (lane == 0)
+        load_patches<KC, SR, 1>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,      // an odd last block is paired with one that does not exist
+                           [&](int seq, int) { return 2 * ((cid + seq * n_clusters) % pairs) + (int)rank; });
     } else if (warp == 1) {
       // ===================================== filter slices =======================================
       if (lane == 0) {

@@ -252,16 +252,25 @@ __device__ __forceinline__ void transform_to_v_tf32_pair(const float *__restrict
   finish_v_tf32(d, vst, c, np);
 }
 
-// Epilogue of one warp: 32 filters (its TMEM lanes; `k` is this lane's) x 16 images (accumulator columns from
-// `tcol`, images from `n0`) of the 2x2-output tile at (oh0, ow0).  A warp that is not `active` only hands the
-// accumulators back.
-template <class Release>
-__device__ __forceinline__ void tc_epilogue_16x32(uint32_t tcol, bool active, const WinoParams &p, int k, int n0, int oh0, int ow0,
-                                                  Release release) {
+// Column j of the 4x4 accumulators of one output tile (rows 0-3: m0 .. m3) folded into element e of its four outputs: the two row
+// sums of output_transform, then its column sums, in its order.
+__device__ __forceinline__ void fold_column(float (&yy)[4][4], int j, int e, float m0, float m1, float m2, float m3) {
+  const float lo = __fadd_rn(__fadd_rn(m0, m1), m2);
+  const float hi = __fsub_rn(__fsub_rn(m1, m2), m3);
+  if (j == 0) { yy[0][e] = lo; yy[2][e] = hi; }
+  if (j == 1) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = lo; yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = hi; }
+  if (j == 2) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = __fsub_rn(yy[1][e], lo);
+                yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = __fsub_rn(yy[3][e], hi); }
+  if (j == 3) { yy[1][e] = __fsub_rn(yy[1][e], lo); yy[3][e] = __fsub_rn(yy[3][e], hi); }
+}
+
+// Epilogue of one warp: 32 filters (its TMEM lanes; `k` is this lane's) x 16 columns (accumulator columns from `tcol`) of
+// a block; `q` is the quad of columns that this lane stores from on: the first of the 16 for an even lane, the ninth column's for an odd
+// one (see the stores).  HALF: the warp may have 8 columns only, `octets` = 1, which every lane stores from `q` on; with
+// `octets` = 0 it only hands the accumulators back.
+template <bool HALF, class Release>
+__device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const WinoParams &p, int k, const ColumnQuad &q, Release release) {
   const int lane = threadIdx.x & 31;
-  const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
-  const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = (size_t)p.H * dH;
-  float *ybase = p.y + (size_t)k * plane + ((size_t)oh0 * p.W + ow0) * p.N + n0;
   // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
   // row sums a[j], a[4+j] of output_transform, which are folded into the four outputs at once - the same
   // operations in the same order.  After a column has been read it is handed back (release(j)), so the
@@ -271,7 +280,7 @@ __device__ __forceinline__ void tc_epilogue_16x32(uint32_t tcol, bool active, co
   for (int j = 0; j < 4; ++j) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      if (active) {
+      if (HALF ? h < octets : octets != 0) {
         float mm[2][4][4];                                           // [quad of this half][row][image]
 #pragma unroll
         for (int q2 = 0; q2 < 2; ++q2)
@@ -281,16 +290,8 @@ __device__ __forceinline__ void tc_epilogue_16x32(uint32_t tcol, bool active, co
 #pragma unroll
         for (int q2 = 0; q2 < 2; ++q2)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float lo = __fadd_rn(__fadd_rn(mm[q2][0][e], mm[q2][1][e]), mm[q2][2][e]);
-            const float hi = __fsub_rn(__fsub_rn(mm[q2][1][e], mm[q2][2][e]), mm[q2][3][e]);
-            float(&yy)[4][4] = y[2 * h + q2];
-            if (j == 0) { yy[0][e] = lo; yy[2][e] = hi; }
-            if (j == 1) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = lo; yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = hi; }
-            if (j == 2) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = __fsub_rn(yy[1][e], lo);
-                          yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = __fsub_rn(yy[3][e], hi); }
-            if (j == 3) { yy[1][e] = __fsub_rn(yy[1][e], lo); yy[3][e] = __fsub_rn(yy[3][e], hi); }
-          }
+          for (int e = 0; e < 4; ++e)
+            fold_column(y[2 * h + q2], j, e, mm[q2][0][e], mm[q2][1][e], mm[q2][2][e], mm[q2][3][e]);
       }
     }
     tc_fence_before();
@@ -300,25 +301,38 @@ __device__ __forceinline__ void tc_epilogue_16x32(uint32_t tcol, bool active, co
   // Stores: neighbouring lanes (filters) swap halves of their 16 images, so that one instruction writes the
   // 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter - 16 lines of
   // two full sectors per instruction instead of 32 lines of one (see wino_tc_kernel).
-  if (active) {
+  const int oh0 = 2 * q.ty, ow0 = 2 * q.tx;
+  const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
+  const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = (size_t)p.H * dH;
+  if (HALF && octets == 1) {
+    if (q.valid && k < p.K) {             // one full 32-byte sector per lane and store
+      float *dst = p.y + (size_t)k * plane + ((size_t)oh0 * p.W + ow0) * p.N + q.n;
+      st_global_v8(dst, y[0][0], y[1][0]);
+      if (col1) st_global_v8(dst + dW, y[0][1], y[1][1]);
+      if (row1) {
+        st_global_v8(dst + dH, y[0][2], y[1][2]);
+        if (col1) st_global_v8(dst + dH + dW, y[0][3], y[1][3]);
+      }
+    }
+  } else if (octets != 0) {
     const bool odd = (lane & 1) != 0;
-    float *pair_base = ybase - (odd ? plane : 0) + (odd ? 8 : 0);           // even filter of the pair, this lane's half
-    const bool n_ok = n0 + (odd ? 8 : 0) < p.N;            // N is a multiple of 8
-    const bool ok_even = n_ok && (k - (odd ? 1 : 0)) < p.K, ok_odd = n_ok && (k + (odd ? 0 : 1)) < p.K;
+    // even filter of the pair, this lane's half: eight columns, which are images of one tile (N is a multiple of 8)
+    float *pair_base = p.y + (size_t)(k - (odd ? 1 : 0)) * plane + ((size_t)oh0 * p.W + ow0) * p.N + q.n;
+    const bool ok_even = q.valid && (k - (odd ? 1 : 0)) < p.K, ok_odd = q.valid && (k + (odd ? 0 : 1)) < p.K;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int o = 0; o < 4; ++o) {
       float ev[2][4], od[2][4];             // this lane's half of the even / odd filter's 64 bytes
 #pragma unroll
       for (int q2 = 0; q2 < 2; ++q2)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float lo = y[q2][q][e], hi = y[2 + q2][q][e];                // images 0-7 / 8-15 of this lane's filter
+          const float lo = y[q2][o][e], hi = y[2 + q2][o][e];                // columns 0-7 / 8-15 of this lane's filter
           const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
           ev[q2][e] = odd ? got : lo;
           od[q2][e] = odd ? hi : got;
         }
-      const bool here = (q == 0) || (q == 1 && col1) || (q == 2 && row1) || (q == 3 && row1 && col1);
-      float *dst = pair_base + ((q & 1) ? dW : 0) + ((q & 2) ? dH : 0);
+      const bool here = (o == 0) || (o == 1 && col1) || (o == 2 && row1) || (o == 3 && row1 && col1);
+      float *dst = pair_base + ((o & 1) ? dW : 0) + ((o & 2) ? dH : 0);
       if (here && ok_even) st_global_v8(dst, ev[0], ev[1]);
       if (here && ok_odd) st_global_v8(dst + plane, od[0], od[1]);
     }
@@ -326,11 +340,39 @@ __device__ __forceinline__ void tc_epilogue_16x32(uint32_t tcol, bool active, co
 }
 
 // True when the tile's accumulator rows 64-127 repeat rows 0-63 (see the MMA issuer).
-template <int DT> __device__ __forceinline__ bool tile_repeats_filters(const WinoParams &p, const TileCoord &tc) {
-  return DT == kTcBf16 && p.K - tc.kb * kTcM <= 64;
+template <int DT> __device__ __forceinline__ bool tile_repeats_filters(const WinoParams &p, int kb) {
+  return DT == kTcBf16 && p.K - kb * kTcM <= 64;
 }
 
-// p.k_blocks counts 128-filter blocks here.
+// The loader of the raw patches (one thread), which is the same in all tensor-core kernels: every K-step of KC channels of
+// each of this CTA's `my_tiles` tiles takes the patches of PER_STEP blocks of 32 columns, block_of(tile, i), into a ring of SR stages.
+template <int KC, int SR, int PER_STEP, class BlockOf>
+__device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensorMap *tm_in, uint8_t *raw_s, uint64_t *raw_full,
+                                             uint64_t *raw_empty, int my_tiles, volatile int *dead, BlockOf block_of) {
+  constexpr uint32_t kBytes = KC * 16 * kTcN * 4;
+  static_assert(PER_STEP == 1 || PER_STEP == 2, "blocks of a K-step");
+  const int cpt = p.chunks_per_tile;
+  tma_prefetch_descriptor(tm_in);
+  int g = 0;
+  bool ok = true;
+  for (int seq = 0; seq < my_tiles && ok; ++seq) {
+    const ColumnQuad b0 = column_block(p, block_of(seq, 0)), b1 = column_block(p, block_of(seq, PER_STEP - 1));
+    for (int i = 0; i < cpt * PER_STEP; ++i, ++g) {
+      const int s = g % SR;
+      const uint32_t use = g / SR;
+      const ColumnQuad &b = i % PER_STEP ? b1 : b0;
+      // A wait that gave up: stop issuing - the stage may still be in use.
+      if (use > 0 && !mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+      mbar_arrive_expect_tx(smem_u32(raw_full + s), kBytes);
+      // (a block past the last one lies below the image: zeros)
+      tma_load_4d(smem_u32(raw_s + s * kBytes), tm_in, smem_u32(raw_full + s), b.n, 2 * b.tx - 1, 2 * b.ty - 1, i / PER_STEP * KC);
+    }
+  }
+  // No exit with bulk copies in flight (after a complete run these phases are long over).
+  for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
+}
+
+// p.k_blocks counts 128-filter blocks here; tiles are (filter block, block of 32 columns).
 template <int DT, bool HU = false>
 __global__ void __launch_bounds__(TcCfg<DT, HU>::kThreads, 1)
 wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
@@ -376,49 +418,41 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0 || warp == kTcULoaderWarp) {
-    // ===================================== TMA producers =======================================
+  if (warp == 0) {
+    // ===================================== patches =============================================
     // Two independent loaders, so that the input patches (needed early, by the transform) never
-    // wait behind the filter slices (whose stage is released late, by the MMAs): warp 0 loads the
-    // raw patches, the last warp loads U.
-    const bool loads_u = warp != 0;
+    // wait behind the filter slices (whose stage is released late, by the MMAs): this warp loads the
+    // raw patches, the next one U.
+    if (lane == 0)
+      load_patches<KC, SR, 1>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
+                              [&](int seq, int) { return ((int)blockIdx.x + seq * (int)gridDim.x) % p.blocks; });
+  } else if (warp == kTcULoaderWarp) {
+    // ===================================== filter slices =======================================
     if (lane == 0) {
-      tma_prefetch_descriptor(loads_u ? &tm_u : &tm_in);
-      if (loads_u) grid_dependency_wait();   // U is all that the kernel before this one writes
-      int seq = 0, ci = 0, issued = 0;
-      TileCoord tc = decode_tile(p, (int)blockIdx.x);
+      tma_prefetch_descriptor(&tm_u);
+      grid_dependency_wait();   // U is all that the kernel before this one writes
+      int seq = 0, ci = 0, issued = 0, kb = (int)blockIdx.x / p.blocks;
       for (int g = 0; g < total_chunks; ++g) {
         const int s = g % kTcStages;
         const uint32_t use = g / kTcStages;
         // A wait that gave up: stop issuing - the stage may still be in use.
-        if (!loads_u) {
-          const int sr = g % SR;
-          const uint32_t use_r = g / SR;
-          if (use_r > 0 && !mbar_wait(smem_u32(raw_empty + sr), (use_r - 1) & 1, dead, p.status)) break;
-          mbar_arrive_expect_tx(smem_u32(raw_full + sr), Cfg::kRawBytes);
-          tma_load_4d(smem_u32(raw_s + sr * Cfg::kRawBytes), &tm_in, smem_u32(raw_full + sr), tc.nb * kTcN,
-                      2 * tc.tx - 1, 2 * tc.ty - 1, ci * KC);
-        } else {
-          if (use > 0 && !mbar_wait(smem_u32(uv_empty + s), (use - 1) & 1, dead, p.status)) break;
-          mbar_arrive_expect_tx(smem_u32(u_full + s), Cfg::kUBytes);
-          // U viewed as {filters within a 128-byte row, channel, 128-byte row of the filter axis, position}
-          tma_load_4d(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC,
-                      tc.kb * (DT == kTcBf16 ? 2 : 4), 0);
-        }
+        if (use > 0 && !mbar_wait(smem_u32(uv_empty + s), (use - 1) & 1, dead, p.status)) break;
+        mbar_arrive_expect_tx(smem_u32(u_full + s), Cfg::kUBytes);
+        // U viewed as {filters within a 128-byte row, channel, 128-byte row of the filter axis, position}
+        tma_load_4d(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, kb * (DT == kTcBf16 ? 2 : 4), 0);
         issued = g + 1;
         if (++ci == cpt) {
           ci = 0;
           ++seq;
-          if (seq < my_tiles) tc = decode_tile(p, (int)blockIdx.x + seq * (int)gridDim.x);
+          kb = ((int)blockIdx.x + seq * (int)gridDim.x) / p.blocks;
         }
       }
       // No exit with bulk copies in flight: wait (with a limit of its own) for the last loads of
       // every stage.  After a complete run these phases are long over.  u_full also counts the
       // transform warps' arrivals; after a give-up those may be missing, and then the limit ends
       // the wait.
-      const int ring = loads_u ? kTcStages : SR;
-      for (int g = issued > ring ? issued - ring : 0; g < issued; ++g)
-        mbar_wait_drain(smem_u32((loads_u ? u_full : raw_full) + g % ring), (g / ring) & 1);
+      for (int g = issued > kTcStages ? issued - kTcStages : 0; g < issued; ++g)
+        mbar_wait_drain(smem_u32(u_full + g % kTcStages), (g / kTcStages) & 1);
     }
   } else if (warp <= kTcTransformWarps) {
     // ===================================== input transform =====================================
@@ -469,7 +503,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
       // A operand is made to alias the first (block stride 0): accumulator rows 64-127 then repeat rows 0-63,
       // and the epilogue warps that own those TMEM lanes take half of the images instead of idling.
       const uint64_t a_desc0_dup = smem_desc(smem_u32(u_s), 0, 1024, 2);
-      bool dup = tile_repeats_filters<DT>(p, decode_tile(p, (int)blockIdx.x));
+      bool dup = tile_repeats_filters<DT>(p, (int)blockIdx.x / p.blocks);
       const uint64_t b_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(v_s), 512, 512, 4) : smem_desc(smem_u32(v_s), 1024, 512, 1);
       int ci = 0, seq = 0;
       for (int g = 0; g < total_chunks; ++g) {
@@ -497,7 +531,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
           if (elect_one()) tc_commit(smem_u32(acc_full));                   // tile finished
           ci = 0;
           ++seq;
-          if (seq < my_tiles) dup = tile_repeats_filters<DT>(p, decode_tile(p, (int)blockIdx.x + seq * (int)gridDim.x));
+          dup = tile_repeats_filters<DT>(p, ((int)blockIdx.x + seq * (int)gridDim.x) / p.blocks);
         }
       }
       // Tensor memory is freed at the end of the kernel: every MMA this thread issued must have
@@ -509,104 +543,20 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     // ===================================== epilogue ============================================
     const int quarter = warp & 3;                                        // TMEM lanes this warp may read
     const int sub = (warp - kTcFirstEpilogueWarp) >> 2;                  // 0 / 1: the two warps of a lane quarter
-    const size_t plane = (size_t)p.H * p.W * p.N;
-    const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N;
     for (int seq = 0; seq < my_tiles; ++seq) {
-      const TileCoord tc = decode_tile(p, (int)blockIdx.x + seq * (int)gridDim.x);
+      const int t = (int)blockIdx.x + seq * (int)gridDim.x, kb = t / p.blocks;
+      // Usually the quarter's lanes are filters 32*quarter .. +31 and the two warps of a quarter split the 32
+      // columns 16 / 16 (two steps of 8).  With repeated filters, quarters 2 and 3 hold filters 0-63 again, so
+      // the eight warps split the columns 8 each (one step).
+      const bool dup = tile_repeats_filters<DT>(p, kb);
+      const int k0 = kb * kTcM + 32 * (dup ? (quarter & 1) : quarter);   // filter block of 32 this warp stores
+      const int quad0 = dup ? 2 * (2 * (quarter >> 1) + sub) : 4 * sub;  // this warp's first quad of columns
+      const ColumnQuad q = column_quad(p, 8 * (t - kb * p.blocks) + quad0 + (!dup && (lane & 1) ? 2 : 0));
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
-      // Usually the quarter's lanes are filters 32*quarter .. +31 and the two warps of a quarter split the 32
-      // images 16 / 16 (two steps of 8).  With repeated filters, quarters 2 and 3 hold filters 0-63 again, so
-      // the eight warps split the images 8 each (one step).
-      const bool dup = tile_repeats_filters<DT>(p, tc);
-      const int fq = dup ? (quarter & 1) : quarter;                      // filter block of 32 this warp stores
-      const int m = fq * 32 + lane;                                      // filter within the tile
-      const int k = tc.kb * kTcM + m;
-      const bool valid = k < p.K;
-      const int oh0 = 2 * tc.ty, ow0 = 2 * tc.tx;
-      const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
-      float *ybase = p.y + (size_t)k * plane + ((size_t)oh0 * p.W + ow0) * p.N + (size_t)tc.nb * kTcN;
-      const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
       // Warps whose 32 filters all lie beyond K (K = 64 layers) have nothing to read or store.
-      const bool warp_valid = (tc.kb * kTcM + fq * 32) < p.K;
-      // this warp's share of the 32 images: image quads jbase .. jbase + nq - 1
-      const int nq = dup ? 2 : 4;
-      const int jbase = dup ? 2 * (2 * (quarter >> 1) + sub) : 4 * sub;
-      // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
-      // row sums a[j], a[4+j] of output_transform, which are folded into the four outputs at once - the same
-      // operations in the same order.  After a column has been read it is handed back (acc_empty[j]), so the
-      // MMAs of the next tile into those four accumulators overlap the rest of this epilogue.
-      float y[4][4][4];                         // [image quad][output position][image]
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (warp_valid && 2 * h < nq) {
-            float mm[2][4][4];                  // [quad of this half][row][image]
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-              for (int r = 0; r < 4; ++r) tmem_ld_x4(tlane + (4 * r + j) * kTcN + 4 * (jbase + 2 * h + q2), mm[q2][r]);
-            tmem_ld_wait();
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float lo = __fadd_rn(__fadd_rn(mm[q2][0][e], mm[q2][1][e]), mm[q2][2][e]);
-                const float hi = __fsub_rn(__fsub_rn(mm[q2][1][e], mm[q2][2][e]), mm[q2][3][e]);
-                float(&yy)[4][4] = y[2 * h + q2];
-                if (j == 0) { yy[0][e] = lo; yy[2][e] = hi; }
-                if (j == 1) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = lo; yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = hi; }
-                if (j == 2) { yy[0][e] = __fadd_rn(yy[0][e], lo); yy[1][e] = __fsub_rn(yy[1][e], lo);
-                              yy[2][e] = __fadd_rn(yy[2][e], hi); yy[3][e] = __fsub_rn(yy[3][e], hi); }
-                if (j == 3) { yy[1][e] = __fsub_rn(yy[1][e], lo); yy[3][e] = __fsub_rn(yy[3][e], hi); }
-              }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(acc_empty + j));
-      }
-      // Stores.  Lanes are filters, i.e. different output rows, so a warp-wide store touches 32 lines however it
-      // is arranged; what can be halved is the number of lines per byte.  A lane holds 16 consecutive images
-      // (64 bytes) of its filter per output position: neighbouring lanes swap halves, so that one instruction
-      // writes the 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter -
-      // 16 lines of two full sectors per instruction instead of 32 lines of one.  (Measured on the 56x56 layer:
-      // 7 % of the kernel; the memory pipe is shared with the transform warps' shared-memory traffic.)
-      if (warp_valid) {
-        if (nq == 4) {
-          const bool odd = (lane & 1) != 0;
-          float *pair_base = ybase - (odd ? plane : 0) + 16 * sub + (odd ? 8 : 0);   // even filter of the pair, this lane's half
-          const bool n_ok = tc.nb * kTcN + 16 * sub + (odd ? 8 : 0) < p.N;         // N is a multiple of 8
-          const bool ok_even = n_ok && (k - (odd ? 1 : 0)) < p.K, ok_odd = n_ok && (k + (odd ? 0 : 1)) < p.K;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            float ev[2][4], od[2][4];           // this lane's half of the even / odd filter's 64 bytes
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float lo = y[q2][q][e], hi = y[2 + q2][q][e];              // images 0-7 / 8-15 of this lane's filter
-                const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? lo : hi, 1);
-                ev[q2][e] = odd ? got : lo;
-                od[q2][e] = odd ? hi : got;
-              }
-            const bool here = (q == 0) || (q == 1 && col1) || (q == 2 && row1) || (q == 3 && row1 && col1);
-            float *dst = pair_base + ((q & 1) ? dW : 0) + ((q & 2) ? dH : 0);
-            if (here && ok_even) st_global_v8(dst, ev[0], ev[1]);
-            if (here && ok_odd) st_global_v8(dst + plane, od[0], od[1]);
-          }
-        } else if (valid && tc.nb * kTcN + 4 * jbase < p.N) {
-          // eight images per lane (repeated-filter tiles): one full 32-byte sector per lane and store
-          float *dst = ybase + 4 * jbase;
-          st_global_v8(dst, y[0][0], y[1][0]);
-          if (col1) st_global_v8(dst + dW, y[0][1], y[1][1]);
-          if (row1) {
-            st_global_v8(dst + dH, y[0][2], y[1][2]);
-            if (col1) st_global_v8(dst + dH + dW, y[0][3], y[1][3]);
-          }
-        }
-      }
+      tc_epilogue<true>(tmem_base + ((uint32_t)(quarter * 32) << 16) + 4 * quad0, k0 >= p.K ? 0 : dup ? 1 : 2, p, k0 + lane, q,
+                        [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }
 

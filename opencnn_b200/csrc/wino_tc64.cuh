@@ -59,17 +59,6 @@ __device__ __forceinline__ void tc_mma_half(uint32_t tmem_d, uint64_t adesc, uin
   }
 }
 
-// A tile over two 32-image blocks, 2*np and 2*np + 1.
-struct T64Tile { int np, tx, ty, kb; };
-__device__ __forceinline__ T64Tile t64_decode(const WinoParams &p, int t, int n_pairs) {
-  T64Tile tc;
-  tc.np = t % n_pairs; t /= n_pairs;
-  tc.tx = t % p.tiles_w; t /= p.tiles_w;
-  tc.ty = t % p.tiles_h;
-  tc.kb = t / p.tiles_h;
-  return tc;
-}
-
 constexpr int kT64RawStages = 3, kT64UStages = 2, kT64VStages = 3;
 constexpr uint32_t kT64ZeroBytes = 2048;                   // one empty half of an A operand (64 filter rows x one K-step)
 constexpr int kT64Threads = 512;
@@ -84,7 +73,7 @@ template <int DT> struct T64Cfg {
   static_assert(kSmemBytes <= 232448, "shared memory");
 };
 
-// p.n_blocks counts 32-image blocks; p.total_tiles counts 64-image tiles; p.k_blocks is 1.
+// p.blocks counts blocks of 32 columns; tile t is blocks 2t and 2t + 1; p.k_blocks is 1.
 template <int DT>
 __global__ void __launch_bounds__(kT64Threads, 1)
 wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
@@ -107,7 +96,6 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 5);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
-  const int n_pairs = (p.n_blocks + 1) / 2;
   const int my_tiles = (p.total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int cpt = p.chunks_per_tile;                                   // K-steps per tile
   const int total_steps = my_tiles * cpt;                              // K-steps of this CTA
@@ -145,42 +133,29 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0 || warp == kTcULoaderWarp) {
-    // ===================================== TMA loaders =========================================
-    const bool loads_u = warp != 0;
+  if (warp == 0) {
+    // ===================================== patches: one block per sub-step =====================
+    if (lane == 0)
+        load_patches<KC, SR, 2>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
+                         [&](int seq, int i) { return 2 * ((int)blockIdx.x + seq * (int)gridDim.x) + i; });
+  } else if (warp == kTcULoaderWarp) {
+    // ===================================== filter slices: one per K-step =======================
     if (lane == 0) {
-      tma_prefetch_descriptor(loads_u ? &tm_u : &tm_in);
-      if (loads_u) grid_dependency_wait();   // U is all that the kernel before this one writes
-      int seq = 0, ci = 0, issued = 0;
-      T64Tile tc = t64_decode(p, (int)blockIdx.x, n_pairs);
-      const int ring = loads_u ? SU : SR;
-      const int count = loads_u ? total_steps : total_sub;             // U once per K-step, patches once per sub-step
-      for (int g = 0; g < count; ++g) {
-        const int s = g % ring;
-        const uint32_t use = g / ring;
+      tma_prefetch_descriptor(&tm_u);
+      grid_dependency_wait();   // U is all that the kernel before this one writes
+      int ci = 0, issued = 0;
+      for (int g = 0; g < total_steps; ++g) {
+        const int s = g % SU;
+        const uint32_t use = g / SU;
         // A wait that gave up: stop issuing - the stage may still be in use.
-        if (use > 0 && !mbar_wait(smem_u32((loads_u ? u_empty : raw_empty) + s), (use - 1) & 1, dead, p.status)) break;
-        if (loads_u) {
-          mbar_arrive_expect_tx(smem_u32(u_full + s), kT64UBytes);
-          tma_load_4d(smem_u32(u_s + s * kT64UBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, 0, 0);
-        } else {
-          const int b = g & 1;
-          mbar_arrive_expect_tx(smem_u32(raw_full + s), kT64RawBytes);
-          tma_load_4d(smem_u32(raw_s + s * kT64RawBytes), &tm_in, smem_u32(raw_full + s), (2 * tc.np + b) * kTcN,
-                      2 * tc.tx - 1, 2 * tc.ty - 1, ci * KC);
-        }
+        if (use > 0 && !mbar_wait(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) break;
+        mbar_arrive_expect_tx(smem_u32(u_full + s), kT64UBytes);
+        tma_load_4d(smem_u32(u_s + s * kT64UBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, 0, 0);
         issued = g + 1;
-        if (loads_u || (g & 1)) {                                      // next K-step
-          if (++ci == cpt) {
-            ci = 0;
-            ++seq;
-            if (seq < my_tiles) tc = t64_decode(p, (int)blockIdx.x + seq * (int)gridDim.x, n_pairs);
-          }
-        }
+        if (++ci == cpt) ci = 0;
       }
       // No exit with bulk copies in flight (after a complete run these phases are long over).
-      for (int g = issued > ring ? issued - ring : 0; g < issued; ++g)
-        mbar_wait_drain(smem_u32((loads_u ? u_full : raw_full) + g % ring), (g / ring) & 1);
+      for (int g = issued > SU ? issued - SU : 0; g < issued; ++g) mbar_wait_drain(smem_u32(u_full + g % SU), (g / SU) & 1);
     }
   } else if (warp <= kTcTransformWarps) {
     // ===================================== input transform =====================================
@@ -272,13 +247,11 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     const bool warp_valid = fq * 32 < p.K;
     const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
     for (int seq = 0; seq < my_tiles; ++seq) {
-      const T64Tile tc = t64_decode(p, (int)blockIdx.x + seq * (int)gridDim.x, n_pairs);
+      const int block = 2 * ((int)blockIdx.x + seq * (int)gridDim.x) + ib;   // block of columns this warp stores
+      const ColumnQuad q = column_quad(p, 8 * block + 4 * sub + 2 * (lane & 1));
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
-      const int nb = 2 * tc.np + ib;                                     // 32-image block this warp stores
-      const bool active = warp_valid && nb < p.n_blocks;
-      tc_epilogue_16x32(tlane + 16 * sub, active, p, k, nb * kTcN + 16 * sub, 2 * tc.ty, 2 * tc.tx,
-                        [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
+      tc_epilogue<false>(tlane + 16 * sub, warp_valid && block < p.blocks ? 2 : 0, p, k, q, [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }
 

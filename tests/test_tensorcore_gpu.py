@@ -235,6 +235,29 @@ def test_pair_kernel_gives_the_bits_of_the_single_cta_kernel(libs, precision, sh
     assert torch.equal(out["single"], out["pair_local"])
 
 
+# The kernel with the images in the accumulator rows (code 4 of the C ABI), likewise: one block of columns (three quarters of the
+# pair's tile empty), five, a tile that spans two output tiles, more filter blocks than one, fewer K-steps than ring stages, more
+# tiles than pairs fit on the device at once.
+IMAGE_ROWS_SHAPES = [(8, 16, 64, 2, 2), (32, 24, 128, 5, 5), (40, 3, 192, 3, 5), (96, 72, 64, 3, 3), (24, 100, 320, 9, 4), (160, 40, 64, 17, 23),
+                     (64, 16, 64, 31, 30)]
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("shape", IMAGE_ROWS_SHAPES)
+def test_image_rows_kernel_gives_the_bits_of_the_single_cta_kernel(libs, precision, shape):
+    N, C, K, H, W = shape
+    x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
+    ws = torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(torch.randn((C, 3, 3, K), device="cuda") * 0.05, ws, C, K, precision=precision) == 0
+    single, rows = (torch.full((K, H, W, N), float("nan"), device="cuda") for _ in range(2))
+    assert api.winograd_forward_kernel(x, ws, single, N, C, H, W, K, precision=precision, kernel="single") == 0
+    assert libs["OPTSTS64"].opencnn_winograd_forward_kernel(x.data_ptr(), ws.data_ptr(), rows.data_ptr(), N, C, H, W, K,
+                                                            api.PRECISIONS[precision], 4, None) == 0
+    assert api.last_device_status() == 0
+    assert bool(torch.isfinite(single).all().item())
+    assert torch.equal(single, rows)
+
+
 # The fused kernel is launched so that its set-up overlaps the filter transform: back-to-back calls that reuse one
 # workspace with other filters, and the same under stream capture, give what a transform waited for gives.
 @pytest.mark.parametrize("precision,shape", [("fp32", (32, 16, 64, 9, 9)), ("fp32", (36, 5, 68, 6, 5)), ("bf16", (64, 16, 64, 30, 30)),
