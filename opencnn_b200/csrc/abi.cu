@@ -304,22 +304,31 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
-// Sizes of a problem for a tensor-core kernel, and its blocks of 32 columns (see ocb::ColumnQuad).
-long long column_blocks(int N, int H, int W) {
-  return (long long)((H + 1) / 2) * ((W + 1) / 2) * ((N + ocb::kTcN - 1) / ocb::kTcN);
+// Blocks of 32 columns of a problem (see ocb::ColumnQuad), with every tile's images filled up to a multiple of 32 or packed.
+struct Columns {
+  bool packed;
+  int quads_per_tile;
+  long long blocks;
+};
+Columns columns_of(int N, int H, int W, bool packed) {
+  Columns c;
+  c.packed = packed;
+  c.quads_per_tile = packed ? N / 4 : (N + ocb::kTcN - 1) / ocb::kTcN * (ocb::kTcN / 4);
+  c.blocks = ((long long)((H + 1) / 2) * ((W + 1) / 2) * c.quads_per_tile + 7) / 8;
+  return c;
 }
-bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K) {
-  const long long blocks = column_blocks(N, H, W);
+bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K, bool packed) {
+  const Columns c = columns_of(N, H, W, packed);
   p.x = input;
   p.y = output;
   p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
   p.tiles_h = (H + 1) / 2;
   p.tiles_w = (W + 1) / 2;
-  p.packed = false;
-  p.quads_per_tile = (N + ocb::kTcN - 1) / ocb::kTcN * (ocb::kTcN / 4);
-  p.blocks = (int)blocks;
+  p.packed = c.packed;
+  p.quads_per_tile = c.quads_per_tile;
+  p.blocks = (int)c.blocks;
   p.ty0 = 0;
-  return blocks <= 0x7fffffffll / 16;
+  return c.blocks <= 0x7fffffffll / 16;
 }
 
 // Tensor-core path: filter transform rounded to the operand type, then the tcgen05 kernel.
@@ -333,7 +342,7 @@ cudaError_t launch_fx_tc(const float *filter, float *workspace, int C, int K, cu
 
 template <int DT>
 cudaError_t launch_wino_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                           int K, cudaStream_t stream, bool after_fx) {
+                           int K, cudaStream_t stream, bool after_fx, bool packed) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -348,7 +357,7 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   // BF16 with at most 64 filters: only the first 64-filter row block is loaded (wino_tc.cuh, "half U")
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 && K <= 64 ? 1 : ocb::kTcM * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, packed)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
   const long long tiles = (long long)p.blocks * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
@@ -382,7 +391,7 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, ocb::kPairFilters * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, false)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
   const long long tiles = ((long long)p.blocks + 1) / 2 * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
@@ -411,7 +420,7 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, false)) return cudaErrorInvalidValue;
   p.k_blocks = K / ocb::kImgFilters;
   const long long tiles = ((long long)p.blocks + 3) / 4 * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
@@ -441,7 +450,7 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   // the hardware fills the other two with zeros, which the kernel uses as the empty half of its A operand.
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 ? 1 : 4)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, false)) return cudaErrorInvalidValue;
   p.k_blocks = 1;
   p.total_tiles = (p.blocks + 1) / 2;
   p.total_items = p.total_tiles;
@@ -471,15 +480,16 @@ struct KernelCost {
   double rate;                  // MB per us
 };
 constexpr double kL2Bound = 200.0;   // MB of input and output from which on the rate counts
-struct TcCosts { KernelCost single, single64, pair, stacked, image_rows; };   // single64: at most 64 filters
+struct TcCosts { KernelCost single, single64, pair, stacked, image_rows, packed, packed64; };   // single64: at most 64 filters
 constexpr TcCosts kTcCosts[2] = {   // BF16, TF32
-    {{5.8, 1.29, 0.672, 2.9}, {4.9, 1.16, 0.57, 2.9}, {6.8, 1.53, 0.487, 4.1}, {5.2, 1.63, 1.043, 4.1}, {7.1, 1.61, 0.741, 4.5}},
-    {{5.3, 1.32, 0.576, 2.9}, {5, 1.32, 0.557, 2.9}, {6.8, 1.6, 0.338, 4.2}, {5.2, 1.79, 0.883, 4.1}, {7.1, 1.61, 0.493, 5.1}},
+    {{5.8, 1.29, 0.672, 2.9}, {4.9, 1.16, 0.57, 2.9}, {6.8, 1.53, 0.487, 4.1}, {5.2, 1.63, 1.043, 4.1}, {7.1, 1.61, 0.741, 4.5}, {6.6, 1.27, 0.826, 2.9}, {6.4, 0.99, 0.65, 2.9}},
+    {{5.3, 1.32, 0.576, 2.9}, {5, 1.32, 0.557, 2.9}, {6.8, 1.6, 0.338, 4.2}, {5.2, 1.79, 0.883, 4.1}, {7.1, 1.61, 0.493, 5.1}, {6.2, 1.34, 0.603, 2.9}, {6, 1.15, 0.591, 2.9}},
 };
 
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
                       cudaStream_t stream, bool after_fx, int kernel = OPENCNN_TC_AUTO) {
+  bool packed = false;
   if (kernel == OPENCNN_TC_AUTO) {
     DeviceState *st = nullptr;
     const cudaError_t e = device_state(&st);
@@ -488,23 +498,26 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
     const TcCosts &costs = kTcCosts[bf16 ? 0 : 1];
     const double k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC, mb = 4e-6 * N * H * W * ((double)C + K);
     double best = 0;
-    const auto consider = [&](int which, const KernelCost &c, long long tiles, int at_once) {
+    const auto consider = [&](int which, bool as_packed, const KernelCost &c, long long tiles, int at_once) {
       if (at_once <= 0) return;             // (no two CTAs of this size can be co-scheduled as a cluster)
       double t = c.start + (double)((tiles + at_once - 1) / at_once) * (c.round + c.step * k_steps);
       if (mb > kL2Bound && t < mb / c.rate) t = mb / c.rate;
       if (kernel != OPENCNN_TC_AUTO && t >= best) return;
       best = t;
       kernel = which;
+      packed = as_packed;
     };
-    const long long blocks = column_blocks(N, H, W), wide = (K + ocb::kTcM - 1) / ocb::kTcM;
+    const long long blocks = columns_of(N, H, W, false).blocks, wide = (K + ocb::kTcM - 1) / ocb::kTcM;
     const int clusters = st->max_clusters[bf16 ? 0 : 1];
-    consider(OPENCNN_TC_SINGLE_CTA, K <= 64 ? costs.single64 : costs.single, blocks * wide, st->sm_count);
-    consider(OPENCNN_TC_PAIR_LOCAL, costs.pair, (blocks + 1) / 2 * wide, clusters);
-    if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, costs.stacked, (blocks + 1) / 2, st->sm_count);
-    consider(OPENCNN_TC_IMAGE_ROWS, costs.image_rows, (blocks + 3) / 4 * (K / ocb::kImgFilters), clusters);
+    const KernelCost &single = K <= 64 ? costs.single64 : costs.single, &packed_single = K <= 64 ? costs.packed64 : costs.packed;
+    consider(OPENCNN_TC_SINGLE_CTA, false, single, blocks * wide, st->sm_count);
+    if (N % ocb::kTcN) consider(OPENCNN_TC_SINGLE_CTA, true, packed_single, columns_of(N, H, W, true).blocks * wide, st->sm_count);
+    consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, clusters);
+    if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, false, costs.stacked, (blocks + 1) / 2, st->sm_count);
+    consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (blocks + 3) / 4 * (K / ocb::kImgFilters), clusters);
   }
   switch (kernel) {
-    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, packed);
     case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
     case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
     case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);

@@ -372,6 +372,30 @@ __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensor
   for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
 }
 
+// The same for packed columns (one whole warp), in the single-CTA kernel.
+template <int KC, int SR>
+__device__ __forceinline__ void load_packed_patches(const WinoParams &p, const CUtensorMap *tm_in, uint8_t *raw_s, uint64_t *raw_full,
+                                                    uint64_t *raw_empty, int my_tiles, volatile int *dead) {
+  constexpr uint32_t kBytes = KC * 16 * kTcN * 4;
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) tma_prefetch_descriptor(tm_in);
+  int g = 0;
+  bool ok = true;
+  for (int seq = 0; seq < my_tiles && ok; ++seq) {
+    PackedLoader patches;
+    patches.start(p, ((int)blockIdx.x + seq * (int)gridDim.x) % p.blocks);
+    for (int ci = 0; ci < p.chunks_per_tile; ++ci, ++g) {
+      const int s = g % SR;
+      const uint32_t use = g / SR;
+      if (use > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status))) { ok = false; break; }
+      patches.chunk<KC>(p, tm_in, smem_u32(raw_s + s * kBytes), smem_u32(raw_full + s), ci * KC);
+    }
+  }
+  cp_async_wait_all();
+  if (lane == 0)
+    for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
+}
+
 // p.k_blocks counts 128-filter blocks here; tiles are (filter block, block of 32 columns).
 template <int DT, bool HU = false>
 __global__ void __launch_bounds__(TcCfg<DT, HU>::kThreads, 1)
@@ -400,7 +424,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   if (tid == 0) {
     *dead = 0;
     for (int s = 0; s < SR; ++s) {
-      mbar_init(smem_u32(raw_full + s), 1);
+      mbar_init(smem_u32(raw_full + s), p.packed ? 32 : 1);
       mbar_init(smem_u32(raw_empty + s), kTcTransformWarps);
     }
     for (int s = 0; s < kTcStages; ++s) {
@@ -423,7 +447,9 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     // Two independent loaders, so that the input patches (needed early, by the transform) never
     // wait behind the filter slices (whose stage is released late, by the MMAs): this warp loads the
     // raw patches, the next one U.
-    if (lane == 0)
+    if (p.packed)
+      load_packed_patches<KC, SR>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead);
+    else if (lane == 0)
       load_patches<KC, SR, 1>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
                               [&](int seq, int) { return ((int)blockIdx.x + seq * (int)gridDim.x) % p.blocks; });
   } else if (warp == kTcULoaderWarp) {

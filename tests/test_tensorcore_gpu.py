@@ -258,6 +258,31 @@ def test_image_rows_kernel_gives_the_bits_of_the_single_cta_kernel(libs, precisi
     assert torch.equal(single, rows)
 
 
+# Batches that are not a multiple of 32 and whose blocks of columns the automatic choice packs (single-CTA kernel): the bits that the
+# same images have in a batch filled up to a multiple of 32.  Blocks within one tile, across two and across four; odd maps.
+PACKED = [(8, 40, 128, 28, 28), (8, 3, 64, 57, 56), (16, 66, 192, 39, 38), (24, 64, 128, 28, 28), (40, 20, 64, 35, 31), (72, 24, 64, 33, 30)]
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("shape", PACKED)
+def test_packed_columns_give_the_bits_of_a_full_batch(libs, precision, shape):
+    N, C, K, H, W = shape
+    full = (N + 31) // 32 * 32
+    x = torch.zeros((C, H, W, full), device="cuda")
+    x[..., :N] = torch.rand((C, H, W, N), device="cuda") * 2 - 1
+    ws = torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(torch.randn((C, 3, 3, K), device="cuda") * 0.05, ws, C, K, precision=precision) == 0
+    expect = torch.empty((K, H, W, full), device="cuda")
+    assert api.winograd_forward_kernel(x, ws, expect, full, C, H, W, K, precision=precision, kernel="single") == 0
+    guard = 4096                                    # floats after the output that must stay untouched
+    flat = torch.full((K * H * W * N + guard,), float("nan"), device="cuda")
+    y = flat[:K * H * W * N].view(K, H, W, N)
+    assert api.winograd_forward(x[..., :N].contiguous(), ws, y, N, C, H, W, K, precision=precision) == 0
+    assert api.last_device_status() == 0
+    assert torch.equal(y, expect[..., :N])
+    assert bool(torch.isnan(flat[K * H * W * N:]).all())
+
+
 # The fused kernel is launched so that its set-up overlaps the filter transform: back-to-back calls that reuse one
 # workspace with other filters, and the same under stream capture, give what a transform waited for gives.
 @pytest.mark.parametrize("precision,shape", [("fp32", (32, 16, 64, 9, 9)), ("fp32", (36, 5, 68, 6, 5)), ("bf16", (64, 16, 64, 30, 30)),
