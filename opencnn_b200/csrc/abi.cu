@@ -187,6 +187,10 @@ cudaError_t check_shape(int N, int C, int H, int W, int K, ShapeRule rule) {
   return cudaSuccess;
 }
 
+// Rows of 2x2-output tiles that a launch computes.
+struct TileRows { int first, count; };
+TileRows all_rows(int H) { return {0, (H + 1) / 2}; }
+
 // Launches a kernel that reads the transformed filter.  `after_fx`: the filter transform was the launch before it on this
 // stream, by this call, so its set-up (barriers, tensor memory, descriptors, the first patches) may overlap it; the
 // kernels wait for the transform's completion before their first load of U, and all other data is older than the
@@ -246,7 +250,7 @@ cudaError_t launch_fx(const float *filter, float *workspace, int C, int K, cudaS
 }
 
 cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *output, int N, int C, int H,
-                             int W, int K, cudaStream_t stream, bool after_fx) {
+                             int W, int K, cudaStream_t stream, bool after_fx, TileRows rows) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -271,7 +275,8 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   p.y = output;
   p.x = input;
   p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
-  p.tiles_h = (H + 1) / 2;
+  p.ty0 = rows.first;
+  p.tiles_h = rows.count;
   p.tiles_w = (W + 1) / 2;
   p.n_blocks = (N + ocb::kBN - 1) / ocb::kBN;
   p.k_blocks = (K + ocb::kBK - 1) / ocb::kBK;
@@ -283,7 +288,6 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   p.blocks = (int)blocks;
   p.total_tiles = (int)tiles;
   p.chunks_per_tile = (C + ocb::kBC - 1) / ocb::kBC;
-  p.ty0 = 0;
   p.status = st->status_ptr;
   // The last round of the persistent schedule is usually only partly filled; cutting its tiles in
   // two (one item per consumer group) pays if the halves still fit on the SMs (see item_tile).  The tiles of a last filter block
@@ -310,24 +314,25 @@ struct Columns {
   int quads_per_tile;
   long long blocks;
 };
-Columns columns_of(int N, int H, int W, bool packed) {
+Columns columns_of(int N, TileRows rows, int W, bool packed) {
   Columns c;
   c.packed = packed;
   c.quads_per_tile = packed ? N / 4 : (N + ocb::kTcN - 1) / ocb::kTcN * (ocb::kTcN / 4);
-  c.blocks = ((long long)((H + 1) / 2) * ((W + 1) / 2) * c.quads_per_tile + 7) / 8;
+  c.blocks = ((long long)rows.count * ((W + 1) / 2) * c.quads_per_tile + 7) / 8;
   return c;
 }
-bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K, bool packed) {
-  const Columns c = columns_of(N, H, W, packed);
+bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K, TileRows rows,
+                 bool packed) {
+  const Columns c = columns_of(N, rows, W, packed);
   p.x = input;
   p.y = output;
   p.N = N; p.C = C; p.K = K; p.H = H; p.W = W;
-  p.tiles_h = (H + 1) / 2;
+  p.ty0 = rows.first;
+  p.tiles_h = rows.count;
   p.tiles_w = (W + 1) / 2;
   p.packed = c.packed;
   p.quads_per_tile = c.quads_per_tile;
   p.blocks = (int)c.blocks;
-  p.ty0 = 0;
   return c.blocks <= 0x7fffffffll / 16;
 }
 
@@ -342,7 +347,7 @@ cudaError_t launch_fx_tc(const float *filter, float *workspace, int C, int K, cu
 
 template <int DT>
 cudaError_t launch_wino_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                           int K, cudaStream_t stream, bool after_fx, bool packed) {
+                           int K, cudaStream_t stream, bool after_fx, TileRows rows, bool packed) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -357,7 +362,7 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   // BF16 with at most 64 filters: only the first 64-filter row block is loaded (wino_tc.cuh, "half U")
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 && K <= 64 ? 1 : ocb::kTcM * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K, packed)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, rows, packed)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
   const long long tiles = (long long)p.blocks * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
@@ -375,7 +380,7 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
 // CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).
 template <int DT>
 cudaError_t launch_wino_pair(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                            int K, cudaStream_t stream, bool after_fx) {
+                            int K, cudaStream_t stream, bool after_fx, TileRows rows) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -391,7 +396,7 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, ocb::kPairFilters * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K, false)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
   const long long tiles = ((long long)p.blocks + 1) / 2 * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
@@ -406,7 +411,7 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
 // Image columns in the accumulator rows: 64 filters x four blocks of 32 columns per cluster of two (wino_img.cuh).
 template <int DT>
 cudaError_t launch_wino_img(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                            int K, cudaStream_t stream, bool after_fx) {
+                            int K, cudaStream_t stream, bool after_fx, TileRows rows) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -420,7 +425,7 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K, false)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
   p.k_blocks = K / ocb::kImgFilters;
   const long long tiles = ((long long)p.blocks + 3) / 4 * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
@@ -435,7 +440,7 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
 // Layers with at most 64 filters: two 32-image blocks share the 128 accumulator rows (wino_tc64.cuh).
 template <int DT>
 cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                             int K, cudaStream_t stream, bool after_fx) {
+                             int K, cudaStream_t stream, bool after_fx, TileRows rows) {
   if (K > 64) return cudaErrorInvalidValue;
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
@@ -450,7 +455,7 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   // the hardware fills the other two with zeros, which the kernel uses as the empty half of its A operand.
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 ? 1 : 4)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
-  if (!set_problem(p, input, output, N, C, H, W, K, false)) return cudaErrorInvalidValue;
+  if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
   p.k_blocks = 1;
   p.total_tiles = (p.blocks + 1) / 2;
   p.total_items = p.total_tiles;
@@ -488,7 +493,7 @@ constexpr TcCosts kTcCosts[2] = {   // BF16, TF32
 
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
-                      cudaStream_t stream, bool after_fx, int kernel = OPENCNN_TC_AUTO) {
+                      cudaStream_t stream, bool after_fx, TileRows rows, int kernel = OPENCNN_TC_AUTO) {
   bool packed = false;
   if (kernel == OPENCNN_TC_AUTO) {
     DeviceState *st = nullptr;
@@ -496,7 +501,7 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
     if (e != cudaSuccess) return e;
     constexpr bool bf16 = DT == ocb::kTcBf16;
     const TcCosts &costs = kTcCosts[bf16 ? 0 : 1];
-    const double k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC, mb = 4e-6 * N * H * W * ((double)C + K);
+    const double k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC, mb = 8e-6 * N * rows.count * W * ((double)C + K);
     double best = 0;
     const auto consider = [&](int which, bool as_packed, const KernelCost &c, long long tiles, int at_once) {
       if (at_once <= 0) return;             // (no two CTAs of this size can be co-scheduled as a cluster)
@@ -507,20 +512,20 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
       kernel = which;
       packed = as_packed;
     };
-    const long long blocks = columns_of(N, H, W, false).blocks, wide = (K + ocb::kTcM - 1) / ocb::kTcM;
+    const long long blocks = columns_of(N, rows, W, false).blocks, wide = (K + ocb::kTcM - 1) / ocb::kTcM;
     const int clusters = st->max_clusters[bf16 ? 0 : 1];
     const KernelCost &single = K <= 64 ? costs.single64 : costs.single, &packed_single = K <= 64 ? costs.packed64 : costs.packed;
     consider(OPENCNN_TC_SINGLE_CTA, false, single, blocks * wide, st->sm_count);
-    if (N % ocb::kTcN) consider(OPENCNN_TC_SINGLE_CTA, true, packed_single, columns_of(N, H, W, true).blocks * wide, st->sm_count);
+    if (N % ocb::kTcN) consider(OPENCNN_TC_SINGLE_CTA, true, packed_single, columns_of(N, rows, W, true).blocks * wide, st->sm_count);
     consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, clusters);
     if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, false, costs.stacked, (blocks + 1) / 2, st->sm_count);
     consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (blocks + 3) / 4 * (K / ocb::kImgFilters), clusters);
   }
   switch (kernel) {
-    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, packed);
-    case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-    case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
-    case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx);
+    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows, packed);
+    case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows);
+    case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows);
+    case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -536,17 +541,17 @@ cudaError_t forward(const float *input, const float *filter, float *output, floa
   if (precision == OPENCNN_BF16) {
     e = launch_fx_tc<ocb::kTcBf16>(filter, workspace, C, K, stream);
     if (e != cudaSuccess) return e;
-    return launch_tc<ocb::kTcBf16>(input, workspace, output, N, C, H, W, K, stream, true);
+    return launch_tc<ocb::kTcBf16>(input, workspace, output, N, C, H, W, K, stream, true, all_rows(H));
   }
   if (precision == OPENCNN_TF32) {
     e = launch_fx_tc<ocb::kTcTf32>(filter, workspace, C, K, stream);
     if (e != cudaSuccess) return e;
-    return launch_tc<ocb::kTcTf32>(input, workspace, output, N, C, H, W, K, stream, true);
+    return launch_tc<ocb::kTcTf32>(input, workspace, output, N, C, H, W, K, stream, true, all_rows(H));
   }
   if (precision != OPENCNN_FP32) return cudaErrorInvalidValue;
   e = launch_fx(filter, workspace, C, K, stream);
   if (e != cudaSuccess) return e;
-  return launch_wino_fp32(input, workspace, output, N, C, H, W, K, stream, true);
+  return launch_wino_fp32(input, workspace, output, N, C, H, W, K, stream, true, all_rows(H));
 }
 
 // Scratch for opencnn_convolutionForward_noalloc: the transformed filter, [C][16][K] floats, for
@@ -577,11 +582,93 @@ cudaError_t noalloc_workspace(float **out) {
   return st.error;
 }
 
+// Host-buffer front end.  The upload of the input, the kernel and the download of the output are done in `bands` bands of tile rows, so that
+// both directions of the host link are busy at once: the kernel of a band follows the rows that it reads (two more than its
+// own), its output leaves while the next band's input arrives.
 struct HostPlan {
-  int N, C, H, W, K, precision;
+  int N, C, H, W, K, precision, bands;
   float *d_in = nullptr, *d_filt = nullptr, *d_out = nullptr, *d_ws = nullptr;
-  cudaStream_t stream = nullptr;
+  cudaStream_t stream = nullptr, up = nullptr, down = nullptr;      // up, down, events: only with more than one band
+  cudaEvent_t landed = nullptr, computed = nullptr, left = nullptr, finished = nullptr;
 };
+
+// A band is at least kBandBytes of input and output, and its rows of one plane at least kBandRowBytes in a row (a strided
+// copy is made of such pieces).  One call, us, by the number of bands (1: as one upload, kernel, download), fp32:
+//     32x64x64x56x56    1: 1025   2: 828   4: 785   8: 819   12: 748   16: 844
+//     8x32x64x112x56    1: 403    2: 355   4: 334   8: 329   12: 355   16: 369
+//     32x256x256x14x14  1: 381    2: 309   4: 290   7: 334 (pieces of 3.6 KB)
+//     16x16x32x40x40    1: 137    2: 127   4: 125   8: 138   16: 182
+constexpr size_t kBandBytes = 2400000, kBandRowBytes = 6u << 10;
+constexpr int kMaxBands = 12;
+int band_count(int N, int C, int H, int W, int K) {
+  const size_t row = (size_t)W * N * 4, bytes = row * H * (C + K);
+  const int tile_rows = (H + 1) / 2;
+  long long bands = (long long)(bytes / kBandBytes);
+  if (bands > (long long)(row * H / kBandRowBytes)) bands = (long long)(row * H / kBandRowBytes);
+  if (bands > tile_rows) bands = tile_rows;
+  if (bands > kMaxBands) bands = kMaxBands;
+  if (row * H > 0x7fffffffu) bands = 1;            // pitch of a strided copy
+  return bands < 1 ? 1 : (int)bands;
+}
+
+// Asynchronous copies need page-locked memory at both ends.
+bool page_locked(const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+cudaError_t transform_filter(const float *filter, float *workspace, int C, int K, int precision, cudaStream_t stream) {
+  if (precision == OPENCNN_BF16) return launch_fx_tc<ocb::kTcBf16>(filter, workspace, C, K, stream);
+  if (precision == OPENCNN_TF32) return launch_fx_tc<ocb::kTcTf32>(filter, workspace, C, K, stream);
+  return launch_fx(filter, workspace, C, K, stream);
+}
+
+cudaError_t convolve_rows(const HostPlan *hp, TileRows rows) {
+  const auto run = [&](auto launch) { return launch(hp->d_in, hp->d_ws, hp->d_out, hp->N, hp->C, hp->H, hp->W, hp->K, hp->stream, false, rows); };
+  if (hp->precision == OPENCNN_BF16) return run([](auto... a) { return launch_tc<ocb::kTcBf16>(a...); });
+  if (hp->precision == OPENCNN_TF32) return run([](auto... a) { return launch_tc<ocb::kTcTf32>(a...); });
+  return run([](auto... a) { return launch_wino_fp32(a...); });
+}
+
+// Rows [r0, r1) of every plane of a CHWN / KHWN tensor.
+cudaError_t copy_rows(float *dst, const float *src, int planes, int r0, int r1, const HostPlan *hp, cudaMemcpyKind kind, cudaStream_t stream) {
+  const size_t row = (size_t)hp->W * hp->N, pitch = row * hp->H * 4;
+  return cudaMemcpy2DAsync(dst + r0 * row, pitch, src + r0 * row, pitch, (r1 - r0) * row * 4, planes, kind, stream);
+}
+
+cudaError_t run_bands(HostPlan *hp, const float *input_host, const float *filter_host, float *output_host, bool kernels) {
+  const size_t f_b = (size_t)hp->C * 9 * hp->K * 4;
+  const int tile_rows = (hp->H + 1) / 2;
+  // the run before this one must be through with the device buffers
+  cudaError_t e = cudaStreamWaitEvent(hp->up, hp->finished, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, hp->up);
+  if (e == cudaSuccess) e = cudaEventRecord(hp->landed, hp->up);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
+  if (e == cudaSuccess && kernels) e = transform_filter(hp->d_filt, hp->d_ws, hp->C, hp->K, hp->precision, hp->stream);
+  for (int b = 0, up_to = 0; b < hp->bands && e == cudaSuccess; ++b) {
+    const int t0 = (int)((long long)tile_rows * b / hp->bands), t1 = (int)((long long)tile_rows * (b + 1) / hp->bands);
+    const int need = 2 * t1 + 1 < hp->H ? 2 * t1 + 1 : hp->H, end = 2 * t1 < hp->H ? 2 * t1 : hp->H;
+    e = copy_rows(hp->d_in, input_host, hp->C, up_to, need, hp, cudaMemcpyHostToDevice, hp->up);
+    up_to = need;
+    if (e == cudaSuccess) e = cudaEventRecord(hp->landed, hp->up);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
+    if (e == cudaSuccess && kernels) e = convolve_rows(hp, {t0, t1 - t0});
+    if (e == cudaSuccess) e = cudaEventRecord(hp->computed, hp->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->down, hp->computed, 0);
+    if (e == cudaSuccess) e = copy_rows(output_host, hp->d_out, hp->K, 2 * t0, end, hp, cudaMemcpyDeviceToHost, hp->down);
+  }
+  // `stream` ends where everything has: it is what the caller waits for, and the next run.  After an error, too.
+  cudaError_t j = cudaEventRecord(hp->landed, hp->up);
+  if (j == cudaSuccess) j = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
+  if (j == cudaSuccess) j = cudaEventRecord(hp->left, hp->down);
+  if (j == cudaSuccess) j = cudaStreamWaitEvent(hp->stream, hp->left, 0);
+  if (j == cudaSuccess) j = cudaEventRecord(hp->finished, hp->stream);
+  return e != cudaSuccess ? e : j;
+}
 
 }  // namespace
 
@@ -638,11 +725,11 @@ int opencnn_winograd_forward(const float *input, const float *workspace, float *
   cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
   if (e != cudaSuccess) return (int)e;
   if (precision == OPENCNN_BF16)
-    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false);
+    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h));
   if (precision == OPENCNN_TF32)
-    return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false);
+    return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h));
   if (precision != OPENCNN_FP32) return (int)cudaErrorInvalidValue;
-  return (int)launch_wino_fp32(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false);
+  return (int)launch_wino_fp32(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h));
 }
 
 int opencnn_winograd_forward_kernel(const float *input, const float *workspace, float *output, int in_n, int in_c,
@@ -654,8 +741,8 @@ int opencnn_winograd_forward_kernel(const float *input, const float *workspace, 
   cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
   if (e != cudaSuccess) return (int)e;
   if (precision == OPENCNN_BF16)
-    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, kernel);
-  return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, kernel);
+    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h), kernel);
+  return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h), kernel);
 }
 
 int opencnn_convolutionForward_noalloc(const float *input, const float *filter, float *output, int in_n,
@@ -676,7 +763,7 @@ int opencnn_convolutionForward_noalloc(const float *input, const float *filter, 
   if (e != cudaSuccess) return (int)e;
   e = launch_fx(filter, ws, in_c, filt_k, (cudaStream_t)stream);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_wino_fp32(input, ws, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, true);
+  return (int)launch_wino_fp32(input, ws, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, true, all_rows(in_h));
 }
 
 int opencnn_nchw_to_chwn(const float *src, float *dst, int n, int c, int h, int w, opencnn_stream_t stream) {
@@ -719,6 +806,7 @@ int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w
   HostPlan *hp = new (std::nothrow) HostPlan;
   if (!hp) return (int)cudaErrorMemoryAllocation;
   hp->N = in_n; hp->C = in_c; hp->H = in_h; hp->W = in_w; hp->K = filt_k; hp->precision = precision;
+  hp->bands = band_count(in_n, in_c, in_h, in_w, filt_k);
   const size_t in_b = (size_t)in_n * in_c * in_h * in_w * 4, f_b = (size_t)in_c * 9 * filt_k * 4;
   const size_t out_b = (size_t)in_n * filt_k * in_h * in_w * 4;
   e = cudaMalloc(&hp->d_in, in_b);
@@ -726,6 +814,12 @@ int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w
   if (e == cudaSuccess) e = cudaMalloc(&hp->d_out, out_b);
   if (e == cudaSuccess) e = cudaMalloc(&hp->d_ws, opencnn_workspace_bytes(in_c, filt_k));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&hp->stream, cudaStreamNonBlocking);
+  if (hp->bands > 1) {
+    for (cudaStream_t *st : {&hp->up, &hp->down})
+      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+    for (cudaEvent_t *ev : {&hp->landed, &hp->computed, &hp->left, &hp->finished})
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  }
   if (e != cudaSuccess) {
     opencnn_host_plan_destroy(hp);
     return (int)e;
@@ -734,30 +828,30 @@ int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w
   return 0;
 }
 
-int opencnn_host_plan_run_async(void *plan, const float *input_host, const float *filter_host,
-                                float *output_host) {
+static int host_plan_async(void *plan, const float *input_host, const float *filter_host, float *output_host, bool kernels) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
+  if (hp->bands > 1 && page_locked(input_host) && page_locked(output_host))
+    return (int)run_bands(hp, input_host, filter_host, output_host, kernels);
   const size_t in_b = (size_t)hp->N * hp->C * hp->H * hp->W * 4, f_b = (size_t)hp->C * 9 * hp->K * 4;
   const size_t out_b = (size_t)hp->N * hp->K * hp->H * hp->W * 4;
   cudaError_t e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, hp->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_in, input_host, in_b, cudaMemcpyHostToDevice, hp->stream);
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && kernels)
     e = forward(hp->d_in, hp->d_filt, hp->d_out, hp->d_ws, hp->N, hp->C, hp->H, hp->W, hp->K, hp->precision, hp->stream,
                 shape_rule(hp->precision));
   if (e == cudaSuccess) e = cudaMemcpyAsync(output_host, hp->d_out, out_b, cudaMemcpyDeviceToHost, hp->stream);
+  if (e == cudaSuccess && hp->finished) e = cudaEventRecord(hp->finished, hp->stream);
   return (int)e;
 }
 
+int opencnn_host_plan_run_async(void *plan, const float *input_host, const float *filter_host,
+                                float *output_host) {
+  return host_plan_async(plan, input_host, filter_host, output_host, true);
+}
+
 int opencnn_host_plan_copy_async(void *plan, const float *input_host, const float *filter_host, float *output_host) {
-  HostPlan *hp = static_cast<HostPlan *>(plan);
-  if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
-  const size_t in_b = (size_t)hp->N * hp->C * hp->H * hp->W * 4, f_b = (size_t)hp->C * 9 * hp->K * 4;
-  const size_t out_b = (size_t)hp->N * hp->K * hp->H * hp->W * 4;
-  cudaError_t e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, hp->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_in, input_host, in_b, cudaMemcpyHostToDevice, hp->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(output_host, hp->d_out, out_b, cudaMemcpyDeviceToHost, hp->stream);
-  return (int)e;
+  return host_plan_async(plan, input_host, filter_host, output_host, false);
 }
 
 int opencnn_host_plan_wait(void *plan) {
@@ -774,6 +868,12 @@ int opencnn_host_plan_run(void *plan, const float *input_host, const float *filt
 int opencnn_host_plan_destroy(void *plan) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp) return 0;
+  // (the copies of a run that was not waited for end before their streams and buffers go)
+  if (hp->finished) cudaStreamSynchronize(hp->stream);
+  for (cudaEvent_t ev : {hp->landed, hp->computed, hp->left, hp->finished})
+    if (ev) cudaEventDestroy(ev);
+  if (hp->up) cudaStreamDestroy(hp->up);
+  if (hp->down) cudaStreamDestroy(hp->down);
   if (hp->d_in) cudaFree(hp->d_in);
   if (hp->d_filt) cudaFree(hp->d_filt);
   if (hp->d_out) cudaFree(hp->d_out);

@@ -228,3 +228,31 @@ def test_host_buffer_plan(oracle, libs):
         assert plan.run(hx.data_ptr(), hg.data_ptr(), hy.data_ptr()) == 0
         assert np.array_equal(hy.numpy(), oracle.forward(x, g))
     plan.close()
+
+
+# Plans large enough to be run in bands of rows: the bits of the operator on device tensors, twice without a wait in between (the
+# second run's filter differs), and the same from memory that is not page-locked.  Odd and even heights, ragged batches.
+@pytest.mark.parametrize("precision,shape", [("fp32", (32, 24, 64, 41, 40)), ("fp32", (36, 20, 68, 37, 33)), ("tf32", (64, 32, 64, 30, 31)),
+                                             ("bf16", (24, 40, 128, 45, 28)), ("fp32", (128, 64, 64, 3, 20))])
+def test_host_plan_in_bands(libs, precision, shape):
+    N, C, K, H, W = shape
+    x = torch.rand((C, H, W, N)) * 2 - 1
+    filters = [torch.randn((C, 3, 3, K)) * 0.05 for _ in range(2)]
+    expect = []
+    for g in filters:
+        y, ws = torch.empty((K, H, W, N), device="cuda"), torch.empty((C, 4, 4, K), device="cuda")
+        dx, dg = x.cuda(), g.cuda()
+        assert api.conv3x3(dx, dg, y, ws, N, C, H, W, K, precision=precision) == 0
+        expect.append(y.cpu())
+    plan = api.HostPlan(N, C, H, W, K, precision=precision)
+    for pinned in (True, False):
+        place = (lambda t: t.pin_memory()) if pinned else (lambda t: t.clone())
+        hx, hg = place(x), [place(g) for g in filters]
+        hy = [place(torch.full((K, H, W, N), float("nan"))) for _ in filters]
+        for g, y in zip(hg, hy):
+            assert plan.run_async(hx.data_ptr(), g.data_ptr(), y.data_ptr()) == 0
+        assert plan.wait() == 0
+        assert all(torch.equal(a, b) for a, b in zip(hy, expect)), pinned
+        assert plan.copy_async(hx.data_ptr(), hg[0].data_ptr(), hy[0].data_ptr()) == 0 and plan.wait() == 0
+        assert torch.equal(hy[0], expect[1]), "copy_async brings back what the plan's output buffer holds"
+    plan.close()
