@@ -93,9 +93,9 @@ cudaError_t device_state(DeviceState **out) {
       }
       // the same for the CTA-pair kernels
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_img_kernel<ocb::kTcBf16>);
-      if (err == cudaSuccess && fa.numRegs < ocb::kImgLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcBf16>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_img_kernel<ocb::kTcTf32>);
-      if (err == cudaSuccess && fa.numRegs < ocb::kImgLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcTf32>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcBf16>);
       if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcTf32>);
@@ -140,8 +140,9 @@ cudaError_t device_state(DeviceState **out) {
       };
       pairs(ocb::wino_pair_kernel<ocb::kTcBf16>, ocb::PairCfg<ocb::kTcBf16>::kSmemBytes, st.max_clusters[0]);
       pairs(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes, st.max_clusters[1]);
-      cfg.blockDim = dim3(ocb::kImgThreads);
+      cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcBf16>::kThreads);
       pairs(ocb::wino_img_kernel<ocb::kTcBf16>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.max_clusters[0]);
+      cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcTf32>::kThreads);
       pairs(ocb::wino_img_kernel<ocb::kTcTf32>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, st.max_clusters[1]);
     }
     if (err == cudaSuccess)
@@ -434,7 +435,7 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  return launch_main(ocb::wino_img_kernel<DT>, 2 * clusters, ocb::kImgThreads, ocb::ImgCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+  return launch_main(ocb::wino_img_kernel<DT>, 2 * clusters, ocb::ImgCfg<DT>::kThreads, ocb::ImgCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
 // Layers with at most 64 filters: two 32-image blocks share the 128 accumulator rows (wino_tc64.cuh).

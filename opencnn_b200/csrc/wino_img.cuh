@@ -29,20 +29,22 @@ template <int DT> struct ImgCfg {
   static constexpr int kRawStages = DT == kTcBf16 ? 4 : 8;
   static constexpr int kUStages = 2;
   static constexpr int kVStages = 2;
-  // BF16: all eight transform warps work on one block after the other (16 channels x 16 column pairs, one item per thread);
-  // TF32 (8 channels): four warps per block.
-  static constexpr int kBlockWarps = DT == kTcBf16 ? 8 : 4;
+  // Transform warps: four per block of columns, a thread one channel and column pair (BF16, 16 channels: two).  In TF32 a second set of
+  // eight takes every other K-step (256x32x64x112x112 325 -> 302 us); in BF16 that gains nothing on shallow layers, and the registers
+  // are better spent on an epilogue that reads 16 accumulator columns at a time (276 -> 266, 128x512x64x14x14 30.8 -> 29.0).
+  static constexpr int kBlockWarps = 4;
+  static constexpr int kTransformWarps = DT == kTcBf16 ? 8 : 16, kFirstEpilogueWarp = kPairFirstTransformWarp + kTransformWarps;
+  static constexpr int kThreads = (kFirstEpilogueWarp + kTcEpilogueWarps) * 32;
+  static constexpr int kEpilogueLoad = DT == kTcBf16 ? 16 : 8;       // accumulator columns per load
+  static constexpr int kLaunchRegs = DT == kTcBf16 ? 96 : 72, kIssueRegs = DT == kTcBf16 ? 64 : 72,
+                       kTransformRegs = 48, kEpilogueRegs = DT == kTcBf16 ? 160 : 120;
+  static_assert(4 * kIssueRegs + kTransformWarps * kTransformRegs + kTcEpilogueWarps * kEpilogueRegs <= kThreads / 32 * kLaunchRegs,
+                "setmaxnreg budgets exceed the registers the CTA was launched with");
   static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kUStages * kUBytes +
                                        (size_t)kVStages * kVBytes + 512;
   static_assert(kRawStages % 2 == 0 && kSmemBytes <= 232448, "shared memory");
 };
 constexpr int kImgFilters = 64;                  // per tile
-// Seven warpgroups: warps 0-3 as in wino_pair.cuh, 16 transform warps, eight epilogue warps.
-constexpr int kImgThreads = 896, kImgTransformWarps = 16, kImgFirstEpilogueWarp = 20;
-constexpr int kImgLaunchRegs = 72, kImgIssueRegs = 72, kImgTransformRegs = 48, kImgEpilogueRegs = 120;
-static_assert(kImgIssueRegs + 4 * kImgTransformRegs + 2 * kImgEpilogueRegs <= 7 * kImgLaunchRegs,
-              "setmaxnreg budgets exceed the registers the CTA was launched with");
-
 // Transformed values of a column pair in the operand layout: as finish_v_bf16 / finish_v_tf32, but a position holds 64 columns
 // (2 KB).  BF16: rows of 128 bytes, 128-byte swizzle (16-byte chunk index ^= c & 7).  TF32: the two blocks' rows of 128 bytes
 // are 1 KB apart.
@@ -79,32 +81,11 @@ __device__ __forceinline__ void finish_v_wide(const uint64_t (&d)[16], uint8_t *
 // Epilogue of one warp: 32 columns (its tensor-memory lanes; `q` is the quad of this lane's, `n` its image) x 16 filters
 // (accumulator columns from `tcol`, filters from `k0`).  The same operations in the same order as tc_epilogue; every store is
 // 32 lanes of one output row.
-template <class Release>
+template <int W, class Release>
 __device__ __forceinline__ void img_epilogue(uint32_t tcol, bool active, const WinoParams &p, int k0, const ColumnQuad &q, int n,
                                              Release release) {
-  const int lane = threadIdx.x & 31;
   float y[4][4][4];                                                  // [filter quad][output position][filter]
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (active) {
-        float mm[2][4][4];                                           // [quad of this half][row][filter]
-#pragma unroll
-        for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) tmem_ld_x4(tcol + (4 * r + j) * kTcN + 8 * h + 4 * q2, mm[q2][r]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) fold_column(y[2 * h + q2], j, e, mm[q2][0][e], mm[q2][1][e], mm[q2][2][e], mm[q2][3][e]);
-      }
-    }
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) release(j);
-  }
+  read_accumulators<W>(tcol, active, y, release);
   if (active && q.valid) {
     const int oh0 = 2 * q.ty, ow0 = 2 * q.tx;
     const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
@@ -125,7 +106,7 @@ __device__ __forceinline__ void img_epilogue(uint32_t tcol, bool active, const W
 // p.k_blocks counts 64-filter blocks, p.blocks blocks of 32 columns, p.total_tiles pair tiles (k_blocks times a quarter of
 // those).
 template <int DT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kImgThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ImgCfg<DT>::kThreads, 1)
 wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
   using Cfg = ImgCfg<DT>;
   constexpr int SR = Cfg::kRawStages, SU = Cfg::kUStages, SV = Cfg::kVStages, KC = Cfg::kKC;
@@ -161,7 +142,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
       mbar_init(smem_u32(u_empty + s), 2);                             // one commit per issuing warp
     }
     for (int s = 0; s < SV; ++s) {
-      mbar_init(smem_u32(v_ready + s), 2 * (DT == kTcBf16 ? 16 : 8));       // leader only: the transform warps of both CTAs
+      mbar_init(smem_u32(v_ready + s), 2 * 8);       // leader only: the transform warps of both CTAs
       mbar_init(smem_u32(v_empty + s), 2);
     }
     mbar_init(smem_u32(acc_full), 2);
@@ -179,11 +160,11 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp >= kImgFirstEpilogueWarp) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kImgEpilogueRegs));
+  if (warp >= Cfg::kFirstEpilogueWarp) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kEpilogueRegs));
     // ===================================== epilogue ============================================
     const int quarter = warp & 3;                                        // TMEM lanes this warp may read
-    const int sub = (warp - kImgFirstEpilogueWarp) >> 2;                // 0 / 1: which 16 of the quarter's 32 filters
+    const int sub = (warp - Cfg::kFirstEpilogueWarp) >> 2;                // 0 / 1: which 16 of the quarter's 32 filters
     const uint32_t tcol = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * sub;
     uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
     for (int seq = 0; seq < my_tiles; ++seq) {
@@ -192,28 +173,42 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
       const ColumnQuad q = column_quad(p, 8 * block + (lane >> 2));
       mbar_wait_reporting(smem_u32(acc_full), seq & 1, dead, p.status, acc_empty0, smem_u32(nowhere));
       tc_fence_after();
-      img_epilogue(tcol, block < p.blocks, p, kb * kImgFilters + 32 * (quarter >> 1) + 16 * sub, q, q.n + (lane & 3),
+      img_epilogue<Cfg::kEpilogueLoad>(tcol, block < p.blocks, p, kb * kImgFilters + 32 * (quarter >> 1) + 16 * sub, q, q.n + (lane & 3),
                    [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
     }
   } else if (warp >= kPairFirstTransformWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kImgTransformRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kTransformRegs));
     // ===================================== input transform =====================================
     const int t = (tid - 32 * kPairFirstTransformWarp) % (32 * Cfg::kBlockWarps), np = t & 15;   // column pair
     // BF16: the two channels of a warp are four apart, so that their 64-byte halves of a row lie in different banks.
-    const int c = DT == kTcBf16 ? ((t >> 5) & 3) + 8 * (t >> 7) + 4 * ((t >> 4) & 1) : t >> 4;
+    const int c = DT == kTcBf16 ? (t >> 5) + 4 * ((t >> 4) & 1) : t >> 4;
     uint32_t v_ready0 = map_to_rank(smem_u32(v_ready), 0);
-    // Groups of kBlockWarps: BF16, one for each block of a K-step; TF32, also for every other K-step.
+    // Groups of kBlockWarps: one for each block of a K-step (TF32: of every other K-step).
     const int group = (warp - kPairFirstTransformWarp) / Cfg::kBlockWarps, b = group & 1;
-    constexpr int kStepGroups = kImgTransformWarps / Cfg::kBlockWarps / 2;
+    constexpr int kStepGroups = Cfg::kTransformWarps / Cfg::kBlockWarps / 2;
     for (int g = group >> 1; g < total_steps; g += kStepGroups) {
       const int sv = g % SV, r = 2 * g + b, sr = r % SR;
       const uint32_t use = g / SV;
       mbar_wait_reporting(smem_u32(raw_full + sr), (r / SR) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
-      uint64_t d[16];
-      load_patch_pair(reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes), c, np, d);
-      if (use > 0)                       // V stage free again
-        mbar_wait_reporting(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
-      finish_v_wide<DT>(d, v_s + sv * Cfg::kVBytes, b, c, np);
+      const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
+      uint8_t *vst = v_s + sv * Cfg::kVBytes;
+      const auto wait_for_stage = [&] {              // V stage free again
+        if (use > 0) mbar_wait_reporting(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
+      };
+      if (KC == 8) {
+        uint64_t d[16];
+        load_patch_pair(raw, c, np, d);
+        wait_for_stage();                            // (before the load: 36 -> 40 us on 128x128x64x28x28)
+        finish_v_wide<DT>(d, vst, b, c, np);
+      } else {
+        wait_for_stage();
+#pragma unroll 1                                     // (unrolled, the second patch's registers spill: 266 -> 277 us on 256x32x64x112x112)
+        for (int i = 0; i < KC; i += 8) {
+          uint64_t d[16];
+          load_patch_pair(raw, c + i, np, d);
+          finish_v_wide<DT>(d, vst, b, c + i, np);
+        }
+      }
       fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
       __syncwarp();
       if (lane == 0) {
@@ -225,7 +220,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     for (int i = total_steps > SV ? total_steps - SV : 0; i < total_steps; ++i)
       mbar_wait(smem_u32(v_empty + i % SV), (i / SV) & 1, dead, p.status);
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kImgIssueRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kIssueRegs));
     if (warp == 0) {
       // ===================================== patches =============================================
       if (lane == 0)

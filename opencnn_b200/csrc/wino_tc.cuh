@@ -103,6 +103,17 @@ __device__ __forceinline__ void tmem_ld_x4(uint32_t taddr, float (&v)[4]) {
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(taddr) : "memory");
   v[0] = __uint_as_float(r0); v[1] = __uint_as_float(r1); v[2] = __uint_as_float(r2); v[3] = __uint_as_float(r3);
 }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr) : "memory");
+}
 // 256-bit global store (one full 32-byte sector per lane); `p` must be 32-byte aligned.
 __device__ __forceinline__ void st_global_v8(float *p, const float (&a)[4], const float (&b)[4]) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a[0]), "f"(a[1]), "f"(a[2]),
@@ -264,11 +275,43 @@ __device__ __forceinline__ void fold_column(float (&yy)[4][4], int j, int e, flo
   if (j == 3) { yy[1][e] = __fsub_rn(yy[1][e], lo); yy[3][e] = __fsub_rn(yy[3][e], hi); }
 }
 
+// Reads a warp's 16 accumulator columns position column by position column, W at a time, and folds them into y [quad][output
+// position][element].  A position column is handed back (release(j)) as soon as it is in registers, before it is folded: the next tile's
+// MMAs wait for nothing else.  W consecutive registers per load is what the single-CTA and the stacked kernel (128 registers per
+// thread) have no room for: they spill, 71 -> 73 us on 128x64x64x56x56 (stacked, BF16).
+template <int W, class Release>
+__device__ __forceinline__ void read_accumulators(uint32_t tcol, bool active, float (&y)[4][4][4], Release release) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int h = 0; h < 16 / W; ++h) {
+      uint32_t mm[4][W];                                             // [row][column]
+      if (active) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) tmem_ld(tcol + (4 * r + j) * kTcN + W * h, mm[r]);
+        tmem_ld_wait();
+      }
+      if (h == 16 / W - 1) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) release(j);
+      }
+      if (active) {
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+          fold_column(y[(W * h + i) >> 2], j, i & 3, __uint_as_float(mm[0][i]), __uint_as_float(mm[1][i]), __uint_as_float(mm[2][i]),
+                      __uint_as_float(mm[3][i]));
+      }
+    }
+  }
+}
+
 // Epilogue of one warp: 32 filters (its TMEM lanes; `k` is this lane's) x 16 columns (accumulator columns from `tcol`) of
 // a block; `q` is the quad of columns that this lane stores from on: the first of the 16 for an even lane, the ninth column's for an odd
 // one (see the stores).  HALF: the warp may have 8 columns only, `octets` = 1, which every lane stores from `q` on; with
-// `octets` = 0 it only hands the accumulators back.
-template <bool HALF, class Release>
+// `octets` = 0 it only hands the accumulators back.  WIDE: see read_accumulators.
+template <bool HALF, bool WIDE, class Release>
 __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const WinoParams &p, int k, const ColumnQuad &q, Release release) {
   const int lane = threadIdx.x & 31;
   // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
@@ -276,27 +319,31 @@ __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const Win
   // operations in the same order.  After a column has been read it is handed back (release(j)), so the
   // MMAs of the next tile into those four accumulators overlap the rest of this epilogue.
   float y[4][4][4];                                                  // [image quad][output position][image]
+  if (WIDE) {
+    read_accumulators<8>(tcol, octets != 0, y, release);
+  } else {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 4; ++j) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (HALF ? h < octets : octets != 0) {
-        float mm[2][4][4];                                           // [quad of this half][row][image]
+      for (int h = 0; h < 2; ++h) {
+        if (HALF ? h < octets : octets != 0) {
+          float mm[2][4][4];                                           // [quad of this half][row][image]
 #pragma unroll
-        for (int q2 = 0; q2 < 2; ++q2)
+          for (int q2 = 0; q2 < 2; ++q2)
 #pragma unroll
-          for (int r = 0; r < 4; ++r) tmem_ld_x4(tcol + (4 * r + j) * kTcN + 8 * h + 4 * q2, mm[q2][r]);
-        tmem_ld_wait();
+            for (int r = 0; r < 4; ++r) tmem_ld_x4(tcol + (4 * r + j) * kTcN + 8 * h + 4 * q2, mm[q2][r]);
+          tmem_ld_wait();
 #pragma unroll
-        for (int q2 = 0; q2 < 2; ++q2)
+          for (int q2 = 0; q2 < 2; ++q2)
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            fold_column(y[2 * h + q2], j, e, mm[q2][0][e], mm[q2][1][e], mm[q2][2][e], mm[q2][3][e]);
+            for (int e = 0; e < 4; ++e)
+              fold_column(y[2 * h + q2], j, e, mm[q2][0][e], mm[q2][1][e], mm[q2][2][e], mm[q2][3][e]);
+        }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) release(j);
     }
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) release(j);
   }
   // Stores: neighbouring lanes (filters) swap halves of their 16 images, so that one instruction writes the
   // 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter - 16 lines of
@@ -581,7 +628,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
       // Warps whose 32 filters all lie beyond K (K = 64 layers) have nothing to read or store.
-      tc_epilogue<true>(tmem_base + ((uint32_t)(quarter * 32) << 16) + 4 * quad0, k0 >= p.K ? 0 : dup ? 1 : 2, p, k0 + lane, q,
+      tc_epilogue<true, false>(tmem_base + ((uint32_t)(quarter * 32) << 16) + 4 * quad0, k0 >= p.K ? 0 : dup ? 1 : 2, p, k0 + lane, q,
                         [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }

@@ -251,7 +251,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       const ColumnQuad q = column_quad(p, 8 * block + 4 * sub + 2 * (lane & 1));
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
-      tc_epilogue<false>(tlane + 16 * sub, warp_valid && block < p.blocks ? 2 : 0, p, k, q, [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
+      tc_epilogue<false, false>(tlane + 16 * sub, warp_valid && block < p.blocks ? 2 : 0, p, k, q, [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }
 
