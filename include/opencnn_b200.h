@@ -143,9 +143,10 @@ int opencnn_convolutionForward_noalloc(const float *input, const float *filter, 
  * (src/openCNN_winograd.cu:300-316 allocation, :470-472 copy back): a plan owns device buffers
  * for one problem size; run copies input and filter host->device, runs the operator, copies the
  * output device->host and synchronises.  Host pointers; pinned memory makes the copies
- * asynchronous but is not required.  Where input and output are pinned and large enough, the work
- * is done in bands of image rows, so that a band's output leaves while the next one's input arrives;
- * the results have the same bits. */
+ * asynchronous but is not required.  Where input and output are pinned and both are large enough,
+ * opencnn_host_plan_run works in bands of image rows, so that a band's output leaves while the next one's input
+ * arrives; the results have the same bits.  (The first such plan on a device makes the two copy streams that
+ * all of them use; the process keeps them.) */
 int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w, int filt_k, int precision);
 int opencnn_host_plan_run(void *plan, const float *input_host, const float *filter_host, float *output_host);
 /* The same work enqueued on the plan's own stream without waiting, and the matching wait: plans
@@ -154,8 +155,8 @@ int opencnn_host_plan_run(void *plan, const float *input_host, const float *filt
 int opencnn_host_plan_run_async(void *plan, const float *input_host, const float *filter_host,
                                 float *output_host);
 int opencnn_host_plan_wait(void *plan);
-/* The copies of opencnn_host_plan_run_async, on the same streams and in the same bands, without the kernels between
- * them: what a step costs when the GPU work is free.  A measurement aid - the floor an
+/* The three copies of opencnn_host_plan_run_async without the kernels between them, on the same
+ * stream: what a step costs when the GPU work is free.  A measurement aid - the floor an
  * end-to-end time can be compared with; the output buffer receives whatever the plan's device
  * buffer holds.  The reference's main() has the same copies around its timed loop
  * (src/openCNN_winograd.cu:300-316, :470-472) and never times them. */

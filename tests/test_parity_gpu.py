@@ -230,8 +230,9 @@ def test_host_buffer_plan(oracle, libs):
     plan.close()
 
 
-# Plans large enough to be run in bands of rows: the bits of the operator on device tensors, twice without a wait in between (the
-# second run's filter differs), and the same from memory that is not page-locked.  Odd and even heights, ragged batches.
+# Plans large enough to be run in bands of rows: the bits of the operator on device tensors, in bands (page-locked memory) and in one
+# piece (other memory), and behind a run of the same plan that was not waited for.  Odd and even heights, ragged batches, and a
+# plan of two tile rows.
 @pytest.mark.parametrize("precision,shape", [("fp32", (32, 24, 64, 41, 40)), ("fp32", (36, 20, 68, 37, 33)), ("tf32", (64, 32, 64, 30, 31)),
                                              ("bf16", (24, 40, 128, 45, 28)), ("fp32", (128, 64, 64, 3, 20))])
 def test_host_plan_in_bands(libs, precision, shape):
@@ -249,10 +250,10 @@ def test_host_plan_in_bands(libs, precision, shape):
         place = (lambda t: t.pin_memory()) if pinned else (lambda t: t.clone())
         hx, hg = place(x), [place(g) for g in filters]
         hy = [place(torch.full((K, H, W, N), float("nan"))) for _ in filters]
-        for g, y in zip(hg, hy):
-            assert plan.run_async(hx.data_ptr(), g.data_ptr(), y.data_ptr()) == 0
-        assert plan.wait() == 0
+        assert plan.run_async(hx.data_ptr(), hg[0].data_ptr(), hy[0].data_ptr()) == 0
+        assert plan.run(hx.data_ptr(), hg[1].data_ptr(), hy[1].data_ptr()) == 0
         assert all(torch.equal(a, b) for a, b in zip(hy, expect)), pinned
-        assert plan.copy_async(hx.data_ptr(), hg[0].data_ptr(), hy[0].data_ptr()) == 0 and plan.wait() == 0
-        assert torch.equal(hy[0], expect[1]), "copy_async brings back what the plan's output buffer holds"
+        hy[0].fill_(float("nan"))
+        assert plan.run(hx.data_ptr(), hg[0].data_ptr(), hy[0].data_ptr()) == 0
+        assert torch.equal(hy[0], expect[0]), pinned
     plan.close()
