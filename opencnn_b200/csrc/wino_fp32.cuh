@@ -32,8 +32,9 @@
 
 namespace ocb {
 
-// Exact: the batch and the filters fill the blocks of 32 images and 64 filters.  Ragged: the batch does, the filters do not.
-// Packed: the batch does not (see ColumnQuad).  (Channels beyond the end are loaded as zeros by all three.)
+// Exact: the batch and the filters fill the blocks of 32 images and 64 filters.  Ragged: one of them does not; missing images
+// and filters are loaded as zeros and not stored.  Packed: the batch does not, and its images are packed (see ColumnQuad).
+// (Channels beyond the end are loaded as zeros by all three.)
 enum Shape : int { kExact = 0, kRagged = 1, kPacked = 2 };
 
 enum Variant : int { kBase = 0, kOptSts64 = 1, kOptSts64Cmp = 2, kOptLds64 = 3 };
@@ -283,6 +284,7 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
     const TileCoord tc = decode_tile(p, tile);
     oh0 = 2 * tc.ty; ow0 = 2 * tc.tx; kb = tc.kb;
     at = ((size_t)oh0 * p.W + ow0) * p.N + (size_t)tc.nb * kBN;
+    n_ok = !RAGGED || col < p.N - tc.nb * kBN;                        // N is a multiple of 4: a pair of columns is inside or outside
   }
   const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
   const size_t plane = (size_t)p.H * p.W * p.N;                       // one filter's output

@@ -118,9 +118,11 @@ def test_any_channel_count_bit_for_bit(oracle, libs, variant, shape):
 
 # Packed columns (batches that are not a multiple of 32): blocks of 32 columns that lie in one tile, end in the next one, span
 # up to eight and run past the last; filters that leave the second group of the last block idle or not; channel counts that
-# leave the last chunk one to seven channels; fewer items than SMs, more, and a last round that is split.
+# leave the last chunk one to seven channels; fewer items than SMs, more, and a last round that is split.  Those of one round either
+# way are not packed but filled up.
 PACKED = [(4, 3, 20, 9, 7), (8, 5, 64, 12, 12), (12, 21, 100, 5, 9), (20, 10, 96, 31, 45), (28, 9, 36, 3, 3), (36, 13, 68, 6, 5),
-          (100, 4, 132, 13, 16), (116, 30, 64, 8, 9), (252, 7, 160, 3, 2), (32, 11, 96, 24, 17), (64, 23, 72, 19, 18)]
+          (100, 4, 132, 13, 16), (116, 30, 64, 8, 9), (252, 7, 160, 3, 2), (32, 11, 96, 24, 17), (64, 23, 72, 19, 18),
+          (4, 3, 20, 45, 47), (8, 5, 64, 40, 41), (12, 9, 36, 30, 31)]
 
 
 @pytest.mark.parametrize("variant", build.VARIANTS)

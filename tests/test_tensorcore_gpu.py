@@ -15,9 +15,8 @@ from opencnn_b200 import api  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
-# With more than 64 filters these small maps are one round of tiles: from eight K-steps of 16 (BF16) or 8 (TF32) channels on
-# they take the CTA-pair kernel - the four deep ones of that kind, in both types, also with an odd number of 32-image blocks
-# and with K not a multiple of 128 - and the others the single-CTA kernel; the deep one with 64 filters the pair, too.
+# These small maps are one round of tiles: the deep ones take the CTA-pair kernel in both types, also with an odd number of 32-image
+# blocks, with K not a multiple of 128 and with 64 filters, the others the single-CTA kernel.
 SHAPES = [(32, 16, 128, 8, 8), (32, 8, 64, 7, 7), (64, 40, 192, 5, 9), (32, 64, 64, 14, 14), (96, 32, 256, 6, 6),
           (64, 512, 128, 4, 4), (96, 512, 192, 3, 5), (128, 520, 64, 2, 2), (64, 1024, 128, 3, 3), (96, 1040, 192, 2, 3)]
 MODEL_REL = 2e-4                     # device vs model: fp32 accumulation order inside the tensor core
@@ -108,8 +107,8 @@ def test_tensor_core_results_are_repeatable(libs, precision):
 
 
 # The benchmark shapes at full size (the N=128 layer sweep and the two wide stress layers): error of both
-# operand types against 10^5 sampled fp64 outputs, relative to rms(truth).  All take the CTA-pair kernel but, in BF16, the
-# two layers with 64 filters, which take the stacked one.
+# operand types against 10^5 sampled fp64 outputs, relative to rms(truth).  All take the CTA-pair kernel but the
+# two layers with 64 filters, which take the image-rows kernel.
 FULL = [(128, 64, 64, 56), (128, 128, 128, 28), (128, 256, 256, 14), (128, 512, 512, 7), (64, 1024, 1024, 14),
         (256, 32, 64, 112)]
 
@@ -380,8 +379,9 @@ def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
         assert torch.equal(y[..., others], clean[..., others]), (image, value)
 
 
-# The automatic choice on both sides of its cut-offs (K-steps x rounds of tiles, B200: 148 SMs, 16 / 8 channels per K-step in
-# BF16 / TF32; rounds in the comment): the bits of the single-CTA kernel whatever it takes.
+# The automatic choice on both sides of its cut-offs (148 SMs, 16 / 8 channels per K-step in BF16 / TF32; rounds of tiles in the
+# comment): the bits of the single-CTA kernel whatever it takes.  In BF16 / TF32 these are the single-CTA kernel for 5 / 1 of them (packed
+# columns for 2 / 0 more), the CTA pair for 2 / 5, the stacked kernel for 4 / 0 and the image-rows kernel for 0 / 7.
 CHOICES = [(32, 48, 128, 24, 12), (32, 128, 128, 24, 12), (64, 64, 192, 14, 20),                    # 1, 1, 2
            (128, 16, 128, 41, 38), (128, 15, 256, 41, 39),                                        # 11, 23
            (64, 64, 64, 16, 36), (64, 33, 64, 26, 26), (64, 33, 64, 30, 30), (200, 24, 64, 17, 23),  # 2 / 1, 3 / 2, 4 / 2, 6 / 3 stacked
