@@ -491,16 +491,20 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
 //     start + rounds x (round + step x K-steps),   K-steps = channels / 16 (BF16) or 8 (TF32),
 // and a problem much larger than L2 no less than its bytes at the rate the kernel's stores and loads were seen to reach.  The constants are
 // least squares through the fused kernels' times, back to back, at 260 random sizes per type (8 to 256 images, 64 to 1024
-// filters, 1 to 1024 channels, maps of 4 to 112); the estimates are 4 to 6 % off in the mean, and the kernel chosen by them is 0.4 %
-// behind the fastest one in the mean, 3 % at the 95th percentile.  Both sides of it, us, single : pair : stacked : image rows:
+// filters, 1 to 1024 channels, maps of 4 to 112); the estimates are 4 to 6 % off in the mean.  At 350 other random sizes per type the
+// kernel chosen by them was 0.15 % behind the fastest one in the mean, and 13 % at most.  Both sides of it, us,
+// single : pair : stacked : image rows:
 //   few K-steps or rounds      128x32x128x28x28  BF16 22.6 : 22.6 : - : 25.2    TF32 28.7 : 24.8 : - : 28.7
-//                              128x64x64x14x14   BF16 12.3 : 14.4 : 10.3 : 12.3  TF32 16.4 : 16.4 : 14.4 : 12.3
-//   64 filters                 128x64x64x56x56   BF16 83.8 : 86.1 : 71.8 : 67.6  TF32 124 : 105 : 113 : 72.1
-//                              256x32x64x112x112 BF16 814 : 413 : 390 : 277      TF32 553 : 486 : 491 : 303
-//                              128x512x64x14x14  BF16 41.5 : 40.8 : 41.0 : 30.8  TF32 77.3 : 51.3 : 61.6 : 39.0
-//   more filters, deep         128x256x256x14x14 BF16 41.0 : 34.9 : - : 45.4    TF32 63.1 : 43.3 : - : 57.5
-//                              64x1024x1024x14x14 BF16 278 : 200 : - : 300      TF32 506 : 325 : - : 469
+//                              128x64x64x14x14   BF16 12.3 : 14.4 : 10.3 : 12.3  TF32 16.4 : 15.0 : 14.4 : 12.3
+//   64 filters                 128x64x64x56x56   BF16 81.8 : 82.7 : 71.1 : 65.9  TF32 123 : 103 : 111 : 71.8
+//                              256x32x64x112x112 BF16 813 : 413 : 392 : 267      TF32 552 : 477 : 490 : 300
+//                              128x512x64x14x14  BF16 41.1 : 39.0 : 39.1 : 29.4  TF32 76.4 : 50.8 : 60.5 : 40.0
+//   more filters, deep         128x256x256x14x14 BF16 41.0 : 33.4 : - : 43.0    TF32 62.5 : 43.0 : - : 57.4
+//                              64x1024x1024x14x14 BF16 279 : 196 : - : 276      TF32 512 : 322 : - : 459
 //   more filters, large output 96x4x128x99x99    BF16 174 : 131 : - : 122       TF32 188 : 131 : - : 111
+// Packed columns (single-CTA kernel, batch not a multiple of 32), filled up : packed
+//                              8x66x192x38x38    BF16 24.6 : 18.6               TF32 34.9 : 20.5
+//                              48x83x64x9x39     BF16 14.3 : 14.6               TF32 18.7 : 20.4
 struct KernelCost {
   double start, round, step;    // us
   double rate;                  // MB per us
