@@ -83,7 +83,7 @@ struct WinoParams {
   int N, C, K, H, W;
   int tiles_h, tiles_w, n_blocks, k_blocks, total_tiles, chunks_per_tile;
   // fp32 kernel only: work items.  The split_tiles tiles from split_from on are two items each, one per consumer
-  // group (see item_tile); all others are whole, those from half_from on with one group idle (see ragged_item).
+  // group (see item_tile); all others are whole, those from half_from on with one group idle.
   int split_from, split_tiles, half_from, total_items;
   // how the columns' list is made (see ColumnQuad): image quads per tile, and whether that is all of a batch that is not a multiple of 32
   int quads_per_tile;
@@ -109,20 +109,36 @@ __device__ __forceinline__ TileCoord decode_tile(const WinoParams &p, int t) {
 // filters each and given to two SMs: a group that has the FMA pipe to itself runs almost twice as
 // fast, so that round takes about half as long.  The group that sits an item out only keeps the
 // ring moving (it hands every stage straight back).
+// HALVES: the tiles from half_from on, behind the split ones, are those of a last filter block of at most 32 filters, which is work for
+// group 0 alone.  The kernel whose filters fill their blocks has none and does without the test.
+template <bool HALVES>
 __device__ __forceinline__ int item_tile(const WinoParams &p, int item, int &groups) {
   const int j = item - p.split_from;
   groups = 3;
   if (j < 0) return item;
-  if (j >= 2 * p.split_tiles) return item - p.split_tiles;
   groups = 1 << (j & 1);
-  return p.split_from + (j >> 1);
+  const int t = p.split_from + (j >> 1);
+  if (HALVES && t >= p.half_from) {                 // beyond the split tiles: an item for each
+    groups = 1;
+    return item - p.split_tiles;
+  }
+  return t;
 }
-
-// The same where the filters do not fill their last block of 64: tiles from half_from on have at most 32 filters, which is work
-// for group 0 alone.
-__device__ __forceinline__ int ragged_item(const WinoParams &p, int item, int &groups) {
-  const int t = item_tile(p, item, groups);
-  if (t >= p.half_from) groups = 1;
+// The same in one piece, whose results the compiler can't take apart (see where the consumers use it).
+template <bool HALVES>
+__device__ __forceinline__ int pinned_item_tile(const WinoParams &p, int item, int &groups) {
+  const int j = item - p.split_from;
+  int t = item, g = 3;
+  if (j >= 0) {
+    t = p.split_from + (j >> 1);
+    g = 1 << (j & 1);
+  }
+  if (HALVES && j >= 2 * p.split_tiles) {
+    t = item - p.split_tiles;
+    g = 1;
+  }
+  asm volatile("" : "+r"(t), "+r"(g));
+  groups = g;
   return t;
 }
 
@@ -250,6 +266,17 @@ __device__ __forceinline__ void group_barrier(int gi) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + gi), "n"(kGroupThreads) : "memory");
 }
 
+// Where a lane's columns of a tile go: the tile and its image block, or, packed, the tile of the lane's own quad of columns and the image of
+// its first column.
+template <int V, bool PACKED>
+__device__ __forceinline__ TileCoord output_place(const WinoParams &p, int tile) {
+  if (!PACKED) return decode_tile(p, tile);
+  const int lane = threadIdx.x & 31, col = V == kOptLds64 ? 2 * (lane & 15) : lane;
+  const int kb = tile / p.blocks;
+  const ColumnQuad q = column_quad(p, 8 * (tile - kb * p.blocks) + (col >> 2));
+  return {q.n + (col & 3), q.tx, q.ty, kb};
+}
+
 // ---------------------------------------------------------------------------------------------
 // Epilogue of one consumer group (128 threads): transpose the group's accumulators through its
 // own staging buffer so that one thread holds all 16 Winograd positions of an (image, filter),
@@ -266,34 +293,21 @@ __device__ __forceinline__ void group_barrier(int gi) {
 // ---------------------------------------------------------------------------------------------
 template <int V, int SHAPE>
 __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, const WinoParams &p,
-                                         int tile, const LaneRole &role) {
+                                         const TileCoord &tc, const LaneRole &role) {
   const int lane = threadIdx.x & 31;
   constexpr int RF = Staging<V>::kRowFloats;
   constexpr bool RAGGED = SHAPE != kExact, PACKED = SHAPE == kPacked;
   const int col = V == kOptLds64 ? 2 * (lane & 15) : lane;            // first column that this lane reads back and stores
-  // Packed kernel: every quad of columns has a place of its own in the output.  Columns and filters beyond the end are not
-  // stored.  (Instantiations of their own, so that the usual case pays nothing; its base address is the same in all lanes.)
-  int oh0, ow0, kb;
-  size_t at;                                                          // of output row oh0, column ow0 in a filter's plane
-  size_t at_lane = col;
-  bool n_ok = true;
-  if (PACKED) {
-    kb = tile / p.blocks;
-    const ColumnQuad q = column_quad(p, 8 * (tile - kb * p.blocks) + (col >> 2));
-    oh0 = 2 * q.ty; ow0 = 2 * q.tx; n_ok = q.valid;
-    at = 0;
-    at_lane = ((size_t)oh0 * p.W + ow0) * p.N + q.n + (col & 3);
-  } else {
-    const TileCoord tc = decode_tile(p, tile);
-    oh0 = 2 * tc.ty; ow0 = 2 * tc.tx; kb = tc.kb;
-    at = ((size_t)oh0 * p.W + ow0) * p.N + (size_t)tc.nb * kBN;
-    n_ok = !RAGGED || col < p.N - tc.nb * kBN;                        // N is a multiple of 4: a pair of columns is inside or outside
-  }
+  const int oh0 = 2 * tc.ty, ow0 = 2 * tc.tx;
   const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
   const size_t plane = (size_t)p.H * p.W * p.N;                       // one filter's output
-  float *ybase = p.y + at + ((size_t)kb * kBK + 32 * role.gi) * plane;
+  float *ybase = p.y + ((size_t)oh0 * p.W + ow0) * p.N + (size_t)tc.nb * (PACKED ? 1 : kBN) +
+                 ((size_t)tc.kb * kBK + 32 * role.gi) * plane;
   const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N;
-  const int k_left = p.K - (kb * kBK + 32 * role.gi);                 // filters of this group's 32 that exist
+  // Columns and filters beyond the end were loaded as zeros and are not stored.  (Instantiations of their own, so that the usual case pays
+  // nothing.  N is a multiple of 4: a pair of columns is inside or outside.)
+  const bool n_ok = PACKED ? tc.ty < p.ty0 + p.tiles_h : !RAGGED || col < p.N - tc.nb * kBN;
+  const int k_left = p.K - (tc.kb * kBK + 32 * role.gi);              // filters of this group's 32 that exist
 
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -332,7 +346,7 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
       float y0[4], y1[4];
       output_transform(m0, y0);
       output_transform(m1, y1);
-      float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + at_lane;
+      float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + (PACKED ? 0 : 2 * np);
       if (n_ok && (!RAGGED || round_filter<V>(kl, r) < k_left)) {
         *reinterpret_cast<float2 *>(dst) = make_float2(y0[0], y1[0]);
         if (col1) *reinterpret_cast<float2 *>(dst + dW) = make_float2(y0[1], y1[1]);
@@ -354,7 +368,7 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
         }
         float yy[4];
         output_transform(m, yy);
-        float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + at_lane;
+        float *dst = ybase + (size_t)round_filter<V>(kl, r) * plane + (PACKED ? 0 : lane);
         if (n_ok && (!RAGGED || round_filter<V>(kl, r) < k_left)) {
           dst[0] = yy[0];
           if (col1) dst[dW] = yy[1];
@@ -370,11 +384,9 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
 }
 
 // ---------------------------------------------------------------------------------------------
-// In-place input transform V = B^T d B of two adjacent images of one channel inside a pipeline
-// stage: columns first, then rows (operation order of src/convolutionForward_32x64x8.cu:59-80),
-// with packed add/sub (each half rounded exactly like the scalar operation).  The stage holds
-// the raw patches as [c][h][w][n]; afterwards the same slots hold [c][xi][n].
-// `t` in 0..127: channel t >> 4, image pair t & 15.
+// In-place input transform V = B^T d B of one image and channel inside a pipeline stage: columns first, then rows (operation order
+// of src/convolutionForward_32x64x8.cu:59-80).  The stage holds the raw patches as [c][h][w][n]; afterwards the same slots hold
+// [c][xi][n].  add2 and sub2 are the tensor-core kernels' packed form: each half is rounded like the scalar operation.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   uint64_t r;
@@ -386,7 +398,7 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// Scalar form: one (image, channel) patch, `patch` = c * 32 + n.
+// `patch` = c * 32 + n.
 __device__ __forceinline__ void transform_patch(float *vstage, int patch) {
   float *R = vstage + ((patch >> 5) * 16) * kBN + (patch & 31);
   float d[16], b[16];
@@ -451,7 +463,7 @@ __device__ __forceinline__ void load_packed(const WinoParams &p, const CUtensorM
   bool ok = true;
   for (int seq = 0; seq < my_tiles && ok; ++seq) {
     int groups_unused;
-    const int tile = ragged_item(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused);
+    const int tile = item_tile<true>(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused);
     const int kb = tile / p.blocks;
     PackedLoader patches;
     patches.start(p, tile - kb * p.blocks);
@@ -518,7 +530,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
         tma_prefetch_descriptor(&tm_in);
         tma_prefetch_descriptor(&tm_u);
         int seq = 0, ci = 0, groups_unused, issued = 0;
-        TileCoord tc = decode_tile(p, item_tile(p, (int)blockIdx.x, groups_unused));
+        TileCoord tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x, groups_unused));
         for (int g = 0; g < total_chunks; ++g) {
           const int s = g % S;
           // A wait that gave up: stop issuing - the stage may still be in use.
@@ -533,7 +545,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
           if (++ci == cpt) {
             ci = 0;
             ++seq;
-            if (seq < my_tiles) tc = decode_tile(p, item_tile(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused));
+            if (seq < my_tiles) tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused));
           }
         }
         // The CTA must not exit with bulk copies in flight.  After a complete run the last loads
@@ -585,7 +597,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   for (int seq = 0; seq < my_tiles; ++seq) {
     int groups;
     const int item = (int)blockIdx.x + seq * (int)gridDim.x;
-    const int tile = RAGGED ? ragged_item(p, item, groups) : item_tile(p, item, groups);
+    const int tile = S < 4 && !PACKED ? pinned_item_tile<RAGGED>(p, item, groups) : item_tile<RAGGED>(p, item, groups);
     if ((groups >> role.gi) & 1) {
       // ---- this group computes the item ----
       for (int ci = 0; ci < cpt; ++ci, ++g) {
@@ -619,7 +631,12 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
           if (lane == 0) mbar_arrive(smem_u32(bar_empty + s));
         }
       }
-      epilogue<V, SHAPE>(acc, my_stg, p, tile, role);
+      // (Where this arithmetic stands and what of it the compiler moves decides how it schedules the main loop: with the packed kernel's
+      // places in the others' epilogue as well, the others were 1 to 2.5 % slower, OPTSTS64 152x55x108x83x85 1400 -> 1381 us, 128x8x448x7x7
+      // 14.8 -> 14.4.  With three stages pinned registers are better still, BASE 64x512x512x14x14 542 -> 529, with four they are worse by 1 %.)
+      TileCoord tc = output_place<V, PACKED>(p, tile);
+      if (S < 4) asm volatile("" : "+r"(tc.nb), "+r"(tc.tx), "+r"(tc.ty), "+r"(tc.kb));
+      epilogue<V, SHAPE>(acc, my_stg, p, tc, role);
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
