@@ -101,15 +101,15 @@ cudaError_t device_state(DeviceState **out) {
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcTf32>);
       if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
     }
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_tc_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::TcCfg<ocb::kTcBf16>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_tc_kernel<ocb::kTcBf16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::TcCfg<ocb::kTcBf16, true>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_tc_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::TcCfg<ocb::kTcTf32>::kSmemBytes);
+    const auto large_smem = [&](auto kernel, size_t bytes) {
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    large_smem(ocb::wino_tc_kernel<ocb::kTcBf16>, ocb::TcCfg<ocb::kTcBf16>::kSmemBytes);
+    large_smem(ocb::wino_tc_kernel<ocb::kTcBf16, true>, ocb::TcCfg<ocb::kTcBf16, true>::kSmemBytes);
+    large_smem(ocb::wino_tc_kernel<ocb::kTcTf32>, ocb::TcCfg<ocb::kTcTf32>::kSmemBytes);
+    large_smem(ocb::wino_tc_kernel<ocb::kTcBf16, false, true>, ocb::TcCfg<ocb::kTcBf16>::kSmemBytes);
+    large_smem(ocb::wino_tc_kernel<ocb::kTcBf16, true, true>, ocb::TcCfg<ocb::kTcBf16, true>::kSmemBytes);
+    large_smem(ocb::wino_tc_kernel<ocb::kTcTf32, false, true>, ocb::TcCfg<ocb::kTcTf32>::kSmemBytes);
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_pair_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ocb::PairCfg<ocb::kTcBf16>::kSmemBytes);
@@ -315,7 +315,6 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   }
   const bool ragged = N % ocb::kBN || K % ocb::kBK;
   if (plan.tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
-  p.packed = packed;
   p.blocks = (int)plan.blocks;
   p.total_tiles = (int)plan.tiles;
   p.split_from = (int)(plan.wholes - plan.split);
@@ -331,13 +330,11 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
 
 // Blocks of 32 columns of a problem (see ocb::ColumnQuad), with every tile's images filled up to a multiple of 32 or packed.
 struct Columns {
-  bool packed;
   int quads_per_tile;
   long long blocks;
 };
 Columns columns_of(int N, TileRows rows, int W, bool packed) {
   Columns c;
-  c.packed = packed;
   c.quads_per_tile = packed ? N / 4 : (N + ocb::kTcN - 1) / ocb::kTcN * (ocb::kTcN / 4);
   c.blocks = ((long long)rows.count * ((W + 1) / 2) * c.quads_per_tile + 7) / 8;
   return c;
@@ -351,7 +348,6 @@ bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, i
   p.ty0 = rows.first;
   p.tiles_h = rows.count;
   p.tiles_w = (W + 1) / 2;
-  p.packed = c.packed;
   p.quads_per_tile = c.quads_per_tile;
   p.blocks = (int)c.blocks;
   return c.blocks <= 0x7fffffffll / 16;
@@ -392,10 +388,14 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
-  if (bf16 && K <= 64)
-    return launch_main(ocb::wino_tc_kernel<ocb::kTcBf16, true>, grid, ocb::TcCfg<ocb::kTcBf16, true>::kThreads,
-                       ocb::TcCfg<ocb::kTcBf16, true>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
-  return launch_main(ocb::wino_tc_kernel<DT>, grid, ocb::TcCfg<DT>::kThreads, ocb::TcCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+  constexpr int threads = ocb::TcCfg<DT>::kThreads;
+  if constexpr (bf16) {
+    if (K <= 64)
+      return launch_main(packed ? ocb::wino_tc_kernel<DT, true, true> : ocb::wino_tc_kernel<DT, true>, grid, threads, ocb::TcCfg<DT, true>::kSmemBytes, stream,
+                         after_fx, tm_in, tm_u, p);
+  }
+  return launch_main(packed ? ocb::wino_tc_kernel<DT, false, true> : ocb::wino_tc_kernel<DT>, grid, threads, ocb::TcCfg<DT>::kSmemBytes, stream, after_fx,
+                     tm_in, tm_u, p);
 }
 
 // CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).

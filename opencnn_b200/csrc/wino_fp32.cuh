@@ -85,9 +85,7 @@ struct WinoParams {
   // fp32 kernel only: work items.  The split_tiles tiles from split_from on are two items each, one per consumer
   // group (see item_tile); all others are whole, those from half_from on with one group idle.
   int split_from, split_tiles, half_from, total_items;
-  // how the columns' list is made (see ColumnQuad): image quads per tile, and whether that is all of a batch that is not a multiple of 32
-  int quads_per_tile;
-  bool packed;
+  int quads_per_tile;  // how the columns' list is made (see ColumnQuad): image quads per tile
   int ty0;             // first tile row (tiles_h of them are computed)
   int blocks;          // 32-column blocks of all tiles: n_blocks * tiles_w * tiles_h, or the packed count (see ColumnQuad)
   int *status;         // device status word

@@ -307,13 +307,30 @@ __device__ __forceinline__ void read_accumulators(uint32_t tcol, bool active, fl
   }
 }
 
+// Where the outputs of a filter and a quad of columns start, and which of the tile's second row and column exist.
+struct OutputSpot {
+  float *first;
+  size_t plane;       // one filter's output
+  bool row1, col1;
+};
+__device__ __forceinline__ OutputSpot output_spot(const WinoParams &p, int filter, const ColumnQuad &q) {
+  const int oh0 = 2 * q.ty, ow0 = 2 * q.tx;
+  const size_t plane = (size_t)p.H * p.W * p.N;
+  return {p.y + (size_t)filter * plane + ((size_t)oh0 * p.W + ow0) * p.N + q.n, plane, (oh0 + 1) < p.H, (ow0 + 1) < p.W};
+}
+
 // Epilogue of one warp: 32 filters (its TMEM lanes; `k` is this lane's) x 16 columns (accumulator columns from `tcol`) of
 // a block; `q` is the quad of columns that this lane stores from on: the first of the 16 for an even lane, the ninth column's for an odd
 // one (see the stores).  HALF: the warp may have 8 columns only, `octets` = 1, which every lane stores from `q` on; with
 // `octets` = 0 it only hands the accumulators back.  WIDE: see read_accumulators.
 template <bool HALF, bool WIDE, class Release>
 __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const WinoParams &p, int k, const ColumnQuad &q, Release release) {
+  static_assert(!(HALF && WIDE), "the one with half a share of columns has its place from before the accumulators");
   const int lane = threadIdx.x & 31;
+  // Worked out before the accumulators are read where there are registers for it: a tile's last step is its stores (TF32 single CTA
+  // 128x20x64x12x12 7.7 -> 7.4 us; the wide loads of the CTA pair lose by it, BF16 128x256x256x14x14 31.3 -> 31.7).
+  OutputSpot at;
+  if (!WIDE) at = output_spot(p, k, q);
   // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
   // row sums a[j], a[4+j] of output_transform, which are folded into the four outputs at once - the same
   // operations in the same order.  After a column has been read it is handed back (release(j)), so the
@@ -349,11 +366,11 @@ __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const Win
   // 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter - 16 lines of
   // two full sectors per instruction instead of 32 lines of one (see wino_tc_kernel).
   const int oh0 = 2 * q.ty, ow0 = 2 * q.tx;
-  const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
-  const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = (size_t)p.H * dH;
+  const bool row1 = WIDE ? (oh0 + 1) < p.H : at.row1, col1 = WIDE ? (ow0 + 1) < p.W : at.col1;
+  const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = WIDE ? (size_t)p.H * dH : at.plane;
   if (HALF && octets == 1) {
     if (q.valid && k < p.K) {             // one full 32-byte sector per lane and store
-      float *dst = p.y + (size_t)k * plane + ((size_t)oh0 * p.W + ow0) * p.N + q.n;
+      float *dst = at.first;
       st_global_v8(dst, y[0][0], y[1][0]);
       if (col1) st_global_v8(dst + dW, y[0][1], y[1][1]);
       if (row1) {
@@ -364,7 +381,7 @@ __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const Win
   } else if (octets != 0) {
     const bool odd = (lane & 1) != 0;
     // even filter of the pair, this lane's half: eight columns, which are images of one tile (N is a multiple of 8)
-    float *pair_base = p.y + (size_t)(k - (odd ? 1 : 0)) * plane + ((size_t)oh0 * p.W + ow0) * p.N + q.n;
+    float *pair_base = WIDE ? p.y + (size_t)(k - (odd ? 1 : 0)) * plane + ((size_t)oh0 * p.W + ow0) * p.N + q.n : at.first - (odd ? plane : 0);
     const bool ok_even = q.valid && (k - (odd ? 1 : 0)) < p.K, ok_odd = q.valid && (k + (odd ? 0 : 1)) < p.K;
 #pragma unroll
     for (int o = 0; o < 4; ++o) {
@@ -443,8 +460,9 @@ __device__ __forceinline__ void load_packed_patches(const WinoParams &p, const C
     for (int i = g > SR ? g - SR : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SR), (i / SR) & 1);
 }
 
-// p.k_blocks counts 128-filter blocks here; tiles are (filter block, block of 32 columns).
-template <int DT, bool HU = false>
+// p.k_blocks counts 128-filter blocks here; tiles are (filter block, block of 32 columns).  PACKED: the columns are packed.  Instantiations of
+// their own: a kernel that holds both loaders makes the other batches pay, BF16 128x20x64x12x12 5.8 -> 6.4 us, 56x23x128x16x16 7.1 -> 7.6.
+template <int DT, bool HU = false, bool PACKED = false>
 __global__ void __launch_bounds__(TcCfg<DT, HU>::kThreads, 1)
 wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
   using Cfg = TcCfg<DT, HU>;
@@ -471,7 +489,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   if (tid == 0) {
     *dead = 0;
     for (int s = 0; s < SR; ++s) {
-      mbar_init(smem_u32(raw_full + s), p.packed ? 32 : 1);
+      mbar_init(smem_u32(raw_full + s), PACKED ? 32 : 1);
       mbar_init(smem_u32(raw_empty + s), kTcTransformWarps);
     }
     for (int s = 0; s < kTcStages; ++s) {
@@ -494,7 +512,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     // Two independent loaders, so that the input patches (needed early, by the transform) never
     // wait behind the filter slices (whose stage is released late, by the MMAs): this warp loads the
     // raw patches, the next one U.
-    if (p.packed)
+    if (PACKED)
       load_packed_patches<KC, SR>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead);
     else if (lane == 0)
       load_patches<KC, SR, 1>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,

@@ -248,7 +248,11 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16);
     for (int seq = 0; seq < my_tiles; ++seq) {
       const int block = 2 * ((int)blockIdx.x + seq * (int)gridDim.x) + ib;   // block of columns this warp stores
-      const ColumnQuad q = column_quad(p, 8 * block + 4 * sub + 2 * (lane & 1));
+      // All of the block's columns lie in one tile, which is the same for all lanes: with a tile worked out per lane the stores of shallow
+      // layers cost 3 to 5 %, BF16 104x7x64x13x96 16.1 -> 16.9 us, 48x3x64x72x72 23.9 -> 25.1.
+      ColumnQuad q = column_block(p, block);
+      q.n += 16 * sub + 8 * (lane & 1);
+      q.valid = q.n < p.N;
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
       tc_epilogue<false, false>(tlane + 16 * sub, warp_valid && block < p.blocks ? 2 : 0, p, k, q, [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
