@@ -1,0 +1,205 @@
+// Host-buffer front end (opencnn_host_plan_*): device buffers for one problem size, copies and launches.  Host code only, so that it can be
+// compiled and tested without a GPU.  Included by abi.cu, which declares what it uses: check_shape, shape_rule, TileRows, kMaxDevices,
+//     cudaError_t forward(input, filter, output, workspace, N, C, H, W, K, precision, stream, rule)             the whole operator
+//     cudaError_t transform_filter(filter, workspace, C, K, precision, stream)
+//     cudaError_t convolve_rows(input, workspace, output, N, C, H, W, K, precision, stream, rows)               some rows of tiles
+#pragma once
+
+namespace {
+
+// The streams on which all plans of a device copy in bands.  The link has one engine per direction, so more would not copy faster, and a
+// stream takes more than 2 ms to create (a plan of its own 5.9 -> 10.5 ms): two per device, made for the first such plan and kept
+// until the process exits.  What a plan enqueues waits only for what the same plan enqueued before.
+struct LinkStreams {
+  std::once_flag once;
+  cudaError_t error = cudaSuccess;
+  cudaStream_t up = nullptr, down = nullptr;
+};
+LinkStreams g_link[kMaxDevices];
+
+cudaError_t link_streams(LinkStreams **out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+  LinkStreams &l = g_link[dev];
+  std::call_once(l.once, [&] {
+    l.error = cudaStreamCreateWithFlags(&l.up, cudaStreamNonBlocking);
+    if (l.error == cudaSuccess) l.error = cudaStreamCreateWithFlags(&l.down, cudaStreamNonBlocking);
+  });
+  *out = &l;
+  return l.error;
+}
+
+// Host-buffer front end.  A run that is waited for does the upload of the input, the kernel and the download of the output in `bands` bands of
+// tile rows, so that both directions of the host link are busy at once: the kernel of a band follows the rows that it reads (two
+// more than its own), its output leaves while the next band's input arrives.  Runs that are only enqueued overlap with those of other
+// plans and do better in one piece: four layers in rotation copy 88 GB/s so, 81 in bands.
+struct HostPlan {
+  int N, C, H, W, K, precision, bands;
+  float *d_in = nullptr, *d_filt = nullptr, *d_out = nullptr, *d_ws = nullptr;
+  cudaStream_t stream = nullptr;
+  cudaStream_t up = nullptr, down = nullptr;                        // of LinkStreams; these and the events only with more than one band
+  cudaEvent_t landed = nullptr, computed = nullptr, left = nullptr;
+};
+
+// What bands can hide is the shorter of the two copies, so a band is at least kBandBytes of twice that one, and its rows of one plane at
+// least kBandRowBytes in a row (a strided copy is made of such pieces).  One call, us, by the number of bands (1: as one upload,
+// kernel, download):
+//     fp32 32x64x64x56x56    1: 1025   2: 828   4: 785   8: 819   12: 748   16: 844
+//     fp32 8x32x64x112x56    1: 403    2: 355   4: 334   8: 329   12: 355   16: 369
+//     fp32 32x256x256x14x14  1: 381    2: 309   4: 290   7: 334 (pieces of 3.6 KB)
+//     fp32 16x16x32x40x40    1: 137    2: 127   4: 125   8: 138   16: 182
+//     bf16 40x7x192x38x38    1: 877   12: 932 (1.6 MB in, 44 MB out: nothing to hide)
+constexpr size_t kBandBytes = 2400000, kBandRowBytes = 6u << 10;
+constexpr int kMaxBands = 12;
+int band_count(int N, int C, int H, int W, int K) {
+  const size_t row = (size_t)W * N * 4, bytes = 2 * row * H * (C < K ? C : K);
+  const int tile_rows = (H + 1) / 2;
+  long long bands = (long long)(bytes / kBandBytes);
+  if (bands > (long long)(row * H / kBandRowBytes)) bands = (long long)(row * H / kBandRowBytes);
+  if (bands > tile_rows) bands = tile_rows;
+  if (bands > kMaxBands) bands = kMaxBands;
+  if (row * H > 0x7fffffffu) bands = 1;            // pitch of a strided copy
+  return bands < 1 ? 1 : (int)bands;
+}
+
+// Asynchronous copies need page-locked memory at both ends.
+bool page_locked(const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+// Rows [r0, r1) of every plane of a CHWN / KHWN tensor.
+cudaError_t copy_rows(float *dst, const float *src, int planes, int r0, int r1, const HostPlan *hp, cudaMemcpyKind kind, cudaStream_t stream) {
+  const size_t row = (size_t)hp->W * hp->N, pitch = row * hp->H * 4;
+  if (r1 <= r0) return cudaSuccess;
+  return cudaMemcpy2DAsync(dst + r0 * row, pitch, src + r0 * row, pitch, (r1 - r0) * row * 4, planes, kind, stream);
+}
+
+cudaError_t run_bands(HostPlan *hp, const float *input_host, const float *filter_host, float *output_host) {
+  const size_t f_b = (size_t)hp->C * 9 * hp->K * 4;
+  const int tile_rows = (hp->H + 1) / 2;
+  // what was enqueued on the plan before must be through with the device buffers
+  cudaError_t e = cudaEventRecord(hp->landed, hp->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->up, hp->landed, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, hp->up);
+  if (e == cudaSuccess) e = cudaEventRecord(hp->landed, hp->up);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
+  if (e == cudaSuccess) e = transform_filter(hp->d_filt, hp->d_ws, hp->C, hp->K, hp->precision, hp->stream);
+  for (int b = 0, up_to = 0; b < hp->bands && e == cudaSuccess; ++b) {
+    const int t0 = (int)((long long)tile_rows * b / hp->bands), t1 = (int)((long long)tile_rows * (b + 1) / hp->bands);
+    const int need = 2 * t1 + 1 < hp->H ? 2 * t1 + 1 : hp->H, end = 2 * t1 < hp->H ? 2 * t1 : hp->H;
+    e = copy_rows(hp->d_in, input_host, hp->C, up_to, need, hp, cudaMemcpyHostToDevice, hp->up);
+    up_to = need;
+    if (e == cudaSuccess) e = cudaEventRecord(hp->landed, hp->up);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
+    if (e == cudaSuccess) e = convolve_rows(hp->d_in, hp->d_ws, hp->d_out, hp->N, hp->C, hp->H, hp->W, hp->K, hp->precision, hp->stream, {t0, t1 - t0});
+    if (e == cudaSuccess) e = cudaEventRecord(hp->computed, hp->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->down, hp->computed, 0);
+    if (e == cudaSuccess) e = copy_rows(output_host, hp->d_out, hp->K, 2 * t0, end, hp, cudaMemcpyDeviceToHost, hp->down);
+  }
+  // `stream` ends where everything has: it is what is waited for, here and by the next run.  After an error, too.
+  cudaError_t j = cudaEventRecord(hp->landed, hp->up);
+  if (j == cudaSuccess) j = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
+  if (j == cudaSuccess) j = cudaEventRecord(hp->left, hp->down);
+  if (j == cudaSuccess) j = cudaStreamWaitEvent(hp->stream, hp->left, 0);
+  return e != cudaSuccess ? e : j;
+}
+
+}  // namespace
+
+extern "C" {
+
+int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w, int filt_k, int precision) {
+  if (!plan) return (int)cudaErrorInvalidValue;
+  *plan = nullptr;
+  if (precision != OPENCNN_FP32 && precision != OPENCNN_TF32 && precision != OPENCNN_BF16) return (int)cudaErrorInvalidValue;
+  cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
+  if (e != cudaSuccess) return (int)e;
+  HostPlan *hp = new (std::nothrow) HostPlan;
+  if (!hp) return (int)cudaErrorMemoryAllocation;
+  hp->N = in_n; hp->C = in_c; hp->H = in_h; hp->W = in_w; hp->K = filt_k; hp->precision = precision;
+  hp->bands = band_count(in_n, in_c, in_h, in_w, filt_k);
+  const size_t in_b = (size_t)in_n * in_c * in_h * in_w * 4, f_b = (size_t)in_c * 9 * filt_k * 4;
+  const size_t out_b = (size_t)in_n * filt_k * in_h * in_w * 4;
+  e = cudaMalloc(&hp->d_in, in_b);
+  if (e == cudaSuccess) e = cudaMalloc(&hp->d_filt, f_b);
+  if (e == cudaSuccess) e = cudaMalloc(&hp->d_out, out_b);
+  if (e == cudaSuccess) e = cudaMalloc(&hp->d_ws, opencnn_workspace_bytes(in_c, filt_k));
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&hp->stream, cudaStreamNonBlocking);
+  if (hp->bands > 1) {
+    LinkStreams *link = nullptr;
+    if (e == cudaSuccess) e = link_streams(&link);
+    if (e == cudaSuccess) {
+      hp->up = link->up;
+      hp->down = link->down;
+    }
+    for (cudaEvent_t *ev : {&hp->landed, &hp->computed, &hp->left})
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  }
+  if (e != cudaSuccess) {
+    opencnn_host_plan_destroy(hp);
+    return (int)e;
+  }
+  *plan = hp;
+  return 0;
+}
+
+static int host_plan_async(void *plan, const float *input_host, const float *filter_host, float *output_host, bool kernels) {
+  HostPlan *hp = static_cast<HostPlan *>(plan);
+  if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
+  const size_t in_b = (size_t)hp->N * hp->C * hp->H * hp->W * 4, f_b = (size_t)hp->C * 9 * hp->K * 4;
+  const size_t out_b = (size_t)hp->N * hp->K * hp->H * hp->W * 4;
+  cudaError_t e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, hp->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_in, input_host, in_b, cudaMemcpyHostToDevice, hp->stream);
+  if (e == cudaSuccess && kernels)
+    e = forward(hp->d_in, hp->d_filt, hp->d_out, hp->d_ws, hp->N, hp->C, hp->H, hp->W, hp->K, hp->precision, hp->stream,
+                shape_rule(hp->precision));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(output_host, hp->d_out, out_b, cudaMemcpyDeviceToHost, hp->stream);
+  return (int)e;
+}
+
+int opencnn_host_plan_run_async(void *plan, const float *input_host, const float *filter_host,
+                                float *output_host) {
+  return host_plan_async(plan, input_host, filter_host, output_host, true);
+}
+
+int opencnn_host_plan_copy_async(void *plan, const float *input_host, const float *filter_host, float *output_host) {
+  return host_plan_async(plan, input_host, filter_host, output_host, false);
+}
+
+int opencnn_host_plan_wait(void *plan) {
+  HostPlan *hp = static_cast<HostPlan *>(plan);
+  if (!hp) return (int)cudaErrorInvalidValue;
+  return (int)cudaStreamSynchronize(hp->stream);
+}
+
+int opencnn_host_plan_run(void *plan, const float *input_host, const float *filter_host, float *output_host) {
+  HostPlan *hp = static_cast<HostPlan *>(plan);
+  if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
+  const bool bands = hp->bands > 1 && page_locked(input_host) && page_locked(output_host);
+  const int e = bands ? (int)run_bands(hp, input_host, filter_host, output_host)
+                      : host_plan_async(plan, input_host, filter_host, output_host, true);
+  return e != 0 ? e : opencnn_host_plan_wait(plan);
+}
+
+int opencnn_host_plan_destroy(void *plan) {
+  HostPlan *hp = static_cast<HostPlan *>(plan);
+  if (!hp) return 0;
+  for (cudaEvent_t ev : {hp->landed, hp->computed, hp->left})
+    if (ev) cudaEventDestroy(ev);
+  if (hp->d_in) cudaFree(hp->d_in);
+  if (hp->d_filt) cudaFree(hp->d_filt);
+  if (hp->d_out) cudaFree(hp->d_out);
+  if (hp->d_ws) cudaFree(hp->d_ws);
+  if (hp->stream) cudaStreamDestroy(hp->stream);
+  delete hp;
+  return 0;
+}
+
+}  // extern "C"
