@@ -183,9 +183,16 @@ int opencnn_host_plan_run(void *plan, const float *input_host, const float *filt
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
   const bool bands = hp->bands > 1 && page_locked(input_host) && page_locked(output_host);
-  const int e = bands ? (int)run_bands(hp, input_host, filter_host, output_host)
-                      : host_plan_async(plan, input_host, filter_host, output_host, true);
-  return e != 0 ? e : opencnn_host_plan_wait(plan);
+  const cudaError_t e = bands ? run_bands(hp, input_host, filter_host, output_host)
+                              : (cudaError_t)host_plan_async(plan, input_host, filter_host, output_host, true);
+  // What was enqueued before an error still reads and writes the caller's memory: wait for it, too.  (run_bands may not have joined its streams.)
+  cudaError_t w = cudaStreamSynchronize(hp->stream);
+  if (bands && (e != cudaSuccess || w != cudaSuccess))
+    for (cudaStream_t s : {hp->up, hp->down}) {
+      const cudaError_t ws = cudaStreamSynchronize(s);
+      if (w == cudaSuccess) w = ws;
+    }
+  return (int)(e != cudaSuccess ? e : w);
 }
 
 int opencnn_host_plan_destroy(void *plan) {
