@@ -7,28 +7,80 @@
 
 namespace {
 
-// The streams on which all plans of a device copy in bands.  The link has one engine per direction, so more would not copy faster, and a
-// stream takes more than 2 ms to create (a plan of its own 5.9 -> 10.5 ms): two per device, made for the first such plan and kept
-// until the process exits.  What a plan enqueues waits only for what the same plan enqueued before.
-struct LinkStreams {
-  std::once_flag once;
-  cudaError_t error = cudaSuccess;
-  cudaStream_t up = nullptr, down = nullptr;
+// The two streams on which a run copies in bands, one per direction.  A run has them to itself from its first copy until it has been waited for,
+// so it waits for nothing that another plan enqueued; plans that run one after the other use the same pair.  (One pair for all plans of a
+// device: four threads' runs stood in one queue, and a run beside a plan with work of 8 ms enqueued took up to 7.9 ms, 1.1 as here.)
+// A device has at most a pair for each plan that runs in bands, eight at most; the last one is kept for the next plan until the process
+// exits.  Where there is none to be had, a run is one piece.
+struct LinkStreams { cudaStream_t up = nullptr, down = nullptr; };
+constexpr int kMaxLinkPairs = 8;
+struct LinkPool {
+  std::mutex mutex;
+  LinkStreams idle[kMaxLinkPairs];
+  int idle_count = 0, made = 0, plans = 0;          // made: idle or in use; plans: with more than one band
 };
-LinkStreams g_link[kMaxDevices];
+LinkPool g_link[kMaxDevices];
 
-cudaError_t link_streams(LinkStreams **out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-  LinkStreams &l = g_link[dev];
-  std::call_once(l.once, [&] {
-    l.error = cudaStreamCreateWithFlags(&l.up, cudaStreamNonBlocking);
-    if (l.error == cudaSuccess) l.error = cudaStreamCreateWithFlags(&l.down, cudaStreamNonBlocking);
-  });
-  *out = &l;
-  return l.error;
+void destroy_pair(const LinkStreams &pair) {
+  if (pair.up) cudaStreamDestroy(pair.up);
+  if (pair.down) cudaStreamDestroy(pair.down);
+}
+
+// With the device current.
+bool take_link(LinkPool &pool, LinkStreams *out) {
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    if (pool.idle_count > 0) {
+      *out = pool.idle[--pool.idle_count];
+      return true;
+    }
+    if (pool.made >= kMaxLinkPairs || pool.made >= pool.plans) return false;
+    ++pool.made;
+  }
+  LinkStreams pair;
+  if (cudaStreamCreateWithFlags(&pair.up, cudaStreamNonBlocking) == cudaSuccess &&
+      cudaStreamCreateWithFlags(&pair.down, cudaStreamNonBlocking) == cudaSuccess) {
+    *out = pair;
+    return true;
+  }
+  cudaGetLastError();
+  destroy_pair(pair);
+  std::lock_guard<std::mutex> lock(pool.mutex);
+  --pool.made;
+  return false;
+}
+
+void give_link(LinkPool &pool, const LinkStreams &pair) {
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    if (pool.made == 1 || pool.made <= pool.plans) {
+      pool.idle[pool.idle_count++] = pair;
+      return;
+    }
+    --pool.made;
+  }
+  destroy_pair(pair);
+}
+
+void add_plan(LinkPool &pool) {
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    ++pool.plans;
+  }
+  LinkStreams pair;                                 // so that the first run does not wait for it
+  if (take_link(pool, &pair)) give_link(pool, pair);
+}
+
+void remove_plan(LinkPool &pool) {
+  LinkStreams pair;
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    --pool.plans;
+    if (pool.idle_count == 0 || pool.made <= 1 || pool.made <= pool.plans) return;
+    pair = pool.idle[--pool.idle_count];
+    --pool.made;
+  }
+  destroy_pair(pair);
 }
 
 // Host-buffer front end.  A run that is waited for does the upload of the input, the kernel and the download of the output in `bands` bands of
@@ -39,7 +91,8 @@ struct HostPlan {
   int N, C, H, W, K, precision, bands;
   float *d_in = nullptr, *d_filt = nullptr, *d_out = nullptr, *d_ws = nullptr;
   cudaStream_t stream = nullptr;
-  cudaStream_t up = nullptr, down = nullptr;                        // of LinkStreams; these and the events only with more than one band
+  int device = 0;
+  LinkPool *link = nullptr;                                         // this and the events only with more than one band
   cudaEvent_t landed = nullptr, computed = nullptr, left = nullptr;
 };
 
@@ -81,32 +134,32 @@ cudaError_t copy_rows(float *dst, const float *src, int planes, int r0, int r1, 
   return cudaMemcpy2DAsync(dst + r0 * row, pitch, src + r0 * row, pitch, (r1 - r0) * row * 4, planes, kind, stream);
 }
 
-cudaError_t run_bands(HostPlan *hp, const float *input_host, const float *filter_host, float *output_host) {
+cudaError_t run_bands(HostPlan *hp, const LinkStreams &link, const float *input_host, const float *filter_host, float *output_host) {
   const size_t f_b = (size_t)hp->C * 9 * hp->K * 4;
   const int tile_rows = (hp->H + 1) / 2;
   // what was enqueued on the plan before must be through with the device buffers
   cudaError_t e = cudaEventRecord(hp->landed, hp->stream);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->up, hp->landed, 0);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, hp->up);
-  if (e == cudaSuccess) e = cudaEventRecord(hp->landed, hp->up);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(link.up, hp->landed, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(hp->d_filt, filter_host, f_b, cudaMemcpyHostToDevice, link.up);
+  if (e == cudaSuccess) e = cudaEventRecord(hp->landed, link.up);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
   if (e == cudaSuccess) e = transform_filter(hp->d_filt, hp->d_ws, hp->C, hp->K, hp->precision, hp->stream);
   for (int b = 0, up_to = 0; b < hp->bands && e == cudaSuccess; ++b) {
     const int t0 = (int)((long long)tile_rows * b / hp->bands), t1 = (int)((long long)tile_rows * (b + 1) / hp->bands);
     const int need = 2 * t1 + 1 < hp->H ? 2 * t1 + 1 : hp->H, end = 2 * t1 < hp->H ? 2 * t1 : hp->H;
-    e = copy_rows(hp->d_in, input_host, hp->C, up_to, need, hp, cudaMemcpyHostToDevice, hp->up);
+    e = copy_rows(hp->d_in, input_host, hp->C, up_to, need, hp, cudaMemcpyHostToDevice, link.up);
     up_to = need;
-    if (e == cudaSuccess) e = cudaEventRecord(hp->landed, hp->up);
+    if (e == cudaSuccess) e = cudaEventRecord(hp->landed, link.up);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
     if (e == cudaSuccess) e = convolve_rows(hp->d_in, hp->d_ws, hp->d_out, hp->N, hp->C, hp->H, hp->W, hp->K, hp->precision, hp->stream, {t0, t1 - t0});
     if (e == cudaSuccess) e = cudaEventRecord(hp->computed, hp->stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->down, hp->computed, 0);
-    if (e == cudaSuccess) e = copy_rows(output_host, hp->d_out, hp->K, 2 * t0, end, hp, cudaMemcpyDeviceToHost, hp->down);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(link.down, hp->computed, 0);
+    if (e == cudaSuccess) e = copy_rows(output_host, hp->d_out, hp->K, 2 * t0, end, hp, cudaMemcpyDeviceToHost, link.down);
   }
   // `stream` ends where everything has: it is what is waited for, here and by the next run.  After an error, too.
-  cudaError_t j = cudaEventRecord(hp->landed, hp->up);
+  cudaError_t j = cudaEventRecord(hp->landed, link.up);
   if (j == cudaSuccess) j = cudaStreamWaitEvent(hp->stream, hp->landed, 0);
-  if (j == cudaSuccess) j = cudaEventRecord(hp->left, hp->down);
+  if (j == cudaSuccess) j = cudaEventRecord(hp->left, link.down);
   if (j == cudaSuccess) j = cudaStreamWaitEvent(hp->stream, hp->left, 0);
   return e != cudaSuccess ? e : j;
 }
@@ -132,15 +185,15 @@ int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w
   if (e == cudaSuccess) e = cudaMalloc(&hp->d_out, out_b);
   if (e == cudaSuccess) e = cudaMalloc(&hp->d_ws, opencnn_workspace_bytes(in_c, filt_k));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&hp->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaGetDevice(&hp->device);
+  if (hp->device < 0 || hp->device >= kMaxDevices) hp->bands = 1;
   if (hp->bands > 1) {
-    LinkStreams *link = nullptr;
-    if (e == cudaSuccess) e = link_streams(&link);
-    if (e == cudaSuccess) {
-      hp->up = link->up;
-      hp->down = link->down;
-    }
     for (cudaEvent_t *ev : {&hp->landed, &hp->computed, &hp->left})
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) {
+      hp->link = &g_link[hp->device];
+      add_plan(*hp->link);
+    }
   }
   if (e != cudaSuccess) {
     opencnn_host_plan_destroy(hp);
@@ -182,22 +235,29 @@ int opencnn_host_plan_wait(void *plan) {
 int opencnn_host_plan_run(void *plan, const float *input_host, const float *filter_host, float *output_host) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
-  const bool bands = hp->bands > 1 && page_locked(input_host) && page_locked(output_host);
-  const cudaError_t e = bands ? run_bands(hp, input_host, filter_host, output_host)
+  LinkStreams link;
+  int device = -1;
+  const bool bands = hp->bands > 1 && page_locked(input_host) && page_locked(output_host) && cudaGetDevice(&device) == cudaSuccess &&
+                     device == hp->device && take_link(*hp->link, &link);
+  const cudaError_t e = bands ? run_bands(hp, link, input_host, filter_host, output_host)
                               : (cudaError_t)host_plan_async(plan, input_host, filter_host, output_host, true);
   // What was enqueued before an error still reads and writes the caller's memory: wait for it, too.  (run_bands may not have joined its streams.)
   cudaError_t w = cudaStreamSynchronize(hp->stream);
-  if (bands && (e != cudaSuccess || w != cudaSuccess))
-    for (cudaStream_t s : {hp->up, hp->down}) {
-      const cudaError_t ws = cudaStreamSynchronize(s);
-      if (w == cudaSuccess) w = ws;
-    }
+  if (bands) {
+    if (e != cudaSuccess || w != cudaSuccess)
+      for (cudaStream_t s : {link.up, link.down}) {
+        const cudaError_t ws = cudaStreamSynchronize(s);
+        if (w == cudaSuccess) w = ws;
+      }
+    give_link(*hp->link, link);
+  }
   return (int)(e != cudaSuccess ? e : w);
 }
 
 int opencnn_host_plan_destroy(void *plan) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp) return 0;
+  if (hp->link) remove_plan(*hp->link);
   for (cudaEvent_t ev : {hp->landed, hp->computed, hp->left})
     if (ev) cudaEventDestroy(ev);
   if (hp->d_in) cudaFree(hp->d_in);

@@ -3,6 +3,7 @@
 // a missing wait shows as wrong numbers; any call can be made to fail.  No GPU, no CUDA library.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <cstdio>
@@ -33,7 +34,8 @@ std::mutex g_m;
 std::condition_variable g_cv;
 std::vector<Stream *> g_streams;
 unsigned g_seed = 1;
-int g_fail_in = -1, g_copies_2d = 0, g_streams_alive = 0, g_stream_creations_to_fail = 0;
+std::atomic<int> g_copies_2d{0};
+int g_fail_in = -1, g_streams_alive = 0, g_stream_creations_to_fail = 0;
 std::set<const void *> g_pageable;
 
 unsigned pick(unsigned n) {
@@ -102,12 +104,17 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
     n = ev->recorded + 1;
   }
   const cudaError_t err = push(s, {[ev, n] { if (ev->done < n) ev->done = n; }, {}, false});
+  std::lock_guard<std::mutex> l(g_m);
   if (err == cudaSuccess) ev->recorded = n;
   return err;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
   Event *ev = as_event(e);
-  const long n = ev->recorded;
+  long n;
+  {
+    std::lock_guard<std::mutex> l(g_m);
+    n = ev->recorded;
+  }
   return push(s, {{}, [ev, n] { return ev->done >= n; }, false});
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
@@ -241,9 +248,80 @@ void errors() {
     }
 }
 
+// A run waits for nothing of another plan: one whose work does not come to an end (here: is held back) keeps no other from it.
+void apart() {
+  Problem a(32, 24, 40, 40, 28), b(32, 24, 41, 40, 28, 3);
+  void *pa = a.plan(), *pb = b.plan();
+  CHECK(static_cast<HostPlan *>(pa)->bands > 1 && static_cast<HostPlan *>(pb)->bands > 1);
+  bool open = false;
+  int ea = -1;
+  CHECK(push(static_cast<HostPlan *>(pa)->stream, {{}, [&open] { return open; }, false}) == cudaSuccess);
+  std::thread t([&] { ea = a.run(pa); });
+  for (int n = 0; n < 1000; ++n) {                  // until all of it is enqueued: the join of the download waits on a's stream
+    std::this_thread::sleep_for(std::chrono::milliseconds(1));
+    std::lock_guard<std::mutex> l(g_m);
+    if (as_stream(static_cast<HostPlan *>(pa)->stream)->ops.size() > 10) break;
+  }
+  std::this_thread::sleep_for(std::chrono::milliseconds(100));
+  for (int n = 0; n < 3; ++n) {
+    std::fill(b.y.begin(), b.y.end(), -1.f);
+    CHECK(b.run(pb) == 0 && b.y == b.expect);
+  }
+  {
+    std::lock_guard<std::mutex> l(g_m);
+    open = true;
+    g_cv.notify_all();
+  }
+  t.join();
+  CHECK(ea == 0 && a.y == a.expect);
+  CHECK(opencnn_host_plan_destroy(pa) == 0 && opencnn_host_plan_destroy(pb) == 0);
+}
+
+// Copy streams: at most a pair for each plan that runs in bands, one pair when there is none, and a plan whose pair cannot be made
+// runs in one piece - until it can.
+void streams() {
+  Problem a(32, 24, 40, 40, 28);
+  g_streams_alive = 1;                              // so that the plan's own stream is not the one that fails
+  g_stream_creations_to_fail = 0;
+  void *warm = a.plan();
+  CHECK(a.run(warm) == 0 && a.y == a.expect);
+  const int base = g_streams_alive;
+  CHECK(base <= 4);                                 // 1, the plan's, a pair
+  std::vector<Problem> many(6, a);
+  std::vector<void *> plans;
+  for (Problem &q : many) plans.push_back(q.plan());
+  std::vector<std::thread> ts;
+  std::vector<int> bad(many.size(), 0);
+  for (size_t i = 0; i < many.size(); ++i)
+    ts.emplace_back([&, i] {
+      for (int n = 0; n < 5; ++n) {
+        std::fill(many[i].y.begin(), many[i].y.end(), -1.f);
+        bad[i] += many[i].run(plans[i]) != 0 || many[i].y != many[i].expect;
+      }
+    });
+  for (std::thread &t : ts) t.join();
+  for (int n : bad) CHECK(n == 0);
+  CHECK(g_streams_alive <= 1 + 3 * 7);
+  for (void *p : plans) CHECK(opencnn_host_plan_destroy(p) == 0);
+  CHECK(g_streams_alive == base);
+  CHECK(opencnn_host_plan_destroy(warm) == 0);
+  CHECK(g_streams_alive <= 3);
+}
+void no_streams() {
+  Problem a(32, 24, 40, 40, 28);
+  g_stream_creations_to_fail = 3;                   // at the plan's creation, and at its first runs
+  void *p = a.plan();
+  for (int n = 0; n < 4; ++n) {
+    std::fill(a.y.begin(), a.y.end(), -1.f);
+    CHECK(a.run(p) == 0 && a.y == a.expect);
+  }
+  CHECK(g_stream_creations_to_fail == 0 && g_copies_2d > 0);
+  CHECK(opencnn_host_plan_destroy(p) == 0);
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const std::map<std::string, void (*)()> checks = {{"results", results}, {"errors", errors}};
+  const std::map<std::string, void (*)()> checks = {{"results", results}, {"errors", errors}, {"apart", apart}, {"streams", streams}, {"no_streams", no_streams}};
   if (what == "bands" && argc == 7) {               // bands N C H W K
     std::printf("%d\n", band_count(atoi(argv[2]), atoi(argv[3]), atoi(argv[4]), atoi(argv[5]), atoi(argv[6])));
     return 0;

@@ -18,6 +18,13 @@ def host_plan(tmp_path_factory):
     return lambda *args: subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=120).stdout.strip()
 
 
-@pytest.mark.parametrize("check", ["results", "errors"])
+@pytest.mark.parametrize("check", ["results", "errors", "apart", "streams", "no_streams"])
 def test_host_plan(host_plan, check):
     assert host_plan(check) == "ok"
+
+
+def test_the_banded_plans_of_the_gpu_tests_are(host_plan):
+    from test_parity_gpu import BANDED
+    for _, (N, C, K, H, W) in BANDED:
+        assert int(host_plan("bands", N, C, H, W, K)) > 1, (N, C, K, H, W)
+    assert int(host_plan("bands", 32, 16, 12, 12, 64)) == 1

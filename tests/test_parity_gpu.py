@@ -2,6 +2,7 @@
 truth, the golden fixtures and (when built) the reference's own kernels on the same device."""
 import glob
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -234,9 +235,12 @@ def test_host_buffer_plan(oracle, libs):
 
 # Plans large enough to be run in bands of rows: the bits of the operator on device tensors, in bands (page-locked memory) and in one
 # piece (other memory), and behind a run of the same plan that was not waited for.  Odd and even heights, ragged batches, and a
-# plan of two tile rows.
-@pytest.mark.parametrize("precision,shape", [("fp32", (32, 24, 64, 41, 40)), ("fp32", (36, 20, 68, 37, 33)), ("tf32", (64, 32, 64, 30, 31)),
-                                             ("bf16", (24, 40, 128, 45, 28)), ("fp32", (128, 64, 64, 3, 20))])
+# plan of two tile rows.  (test_host_plan_cpu.py checks that all of them have more than one band.)
+BANDED = [("fp32", (32, 24, 64, 41, 40)), ("fp32", (36, 20, 68, 37, 33)), ("tf32", (64, 32, 64, 30, 31)), ("bf16", (24, 40, 128, 45, 28)),
+          ("fp32", (128, 96, 96, 3, 20))]
+
+
+@pytest.mark.parametrize("precision,shape", BANDED)
 def test_host_plan_in_bands(libs, precision, shape):
     N, C, K, H, W = shape
     x = torch.rand((C, H, W, N)) * 2 - 1
@@ -259,3 +263,33 @@ def test_host_plan_in_bands(libs, precision, shape):
         assert plan.run(hx.data_ptr(), hg[0].data_ptr(), hy[0].data_ptr()) == 0
         assert torch.equal(hy[0], expect[0]), pinned
     plan.close()
+
+
+def test_host_plans_in_several_threads(libs):
+    """Runs in bands of three plans at once, each in a thread of its own, and behind enqueued work of one of them."""
+    jobs = []
+    for precision, (N, C, K, H, W) in BANDED[:3]:
+        x, g = torch.rand((C, H, W, N)) * 2 - 1, torch.randn((C, 3, 3, K)) * 0.05
+        y, ws = torch.empty((K, H, W, N), device="cuda"), torch.empty((C, 4, 4, K), device="cuda")
+        dx, dg = x.cuda(), g.cuda()
+        assert api.conv3x3(dx, dg, y, ws, N, C, H, W, K, precision=precision) == 0
+        jobs.append((api.HostPlan(N, C, H, W, K, precision=precision), x.pin_memory(), g.pin_memory(),
+                     torch.empty((K, H, W, N)).pin_memory(), y.cpu()))
+    bad = []
+
+    def work(plan, x, g, y, expect, enqueue):
+        for _ in range(8):
+            if enqueue:
+                bad.append(plan.run_async(x.data_ptr(), g.data_ptr(), y.data_ptr()))
+            y.fill_(float("nan")) if not enqueue else None
+            bad.append(plan.run(x.data_ptr(), g.data_ptr(), y.data_ptr()))
+            bad.append(not torch.equal(y, expect))
+
+    threads = [threading.Thread(target=work, args=(*job, i == 0)) for i, job in enumerate(jobs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for job in jobs:
+        job[0].close()
+    assert len(bad) >= 48 and not any(bad)
