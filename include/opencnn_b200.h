@@ -145,9 +145,9 @@ int opencnn_convolutionForward_noalloc(const float *input, const float *filter, 
  * output device->host and synchronises.  Host pointers; pinned memory makes the copies
  * asynchronous but is not required.  Where input and output are pinned and both are large enough,
  * opencnn_host_plan_run works in bands of image rows, so that a band's output leaves while the next one's input
- * arrives; the results have the same bits.  Such runs copy on
- * two streams of their own, from a pool that holds at most a pair for each plan of this kind and keeps one when there is none left;
- * runs of different plans in different threads do not wait for each other.  A run that fails returns when its copies are over. */
+ * arrives; the results have the same bits.  Such a run has two copy streams to itself, which the process keeps; one that
+ * finds them taken by a run of another thread is in one piece and waits for nothing of it.  A run that fails returns when its
+ * copies are over. */
 int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w, int filt_k, int precision);
 int opencnn_host_plan_run(void *plan, const float *input_host, const float *filter_host, float *output_host);
 /* The same work enqueued on the plan's own stream without waiting, and the matching wait: plans

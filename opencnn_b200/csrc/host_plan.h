@@ -7,80 +7,34 @@
 
 namespace {
 
-// The two streams on which a run copies in bands, one per direction.  A run has them to itself from its first copy until it has been waited for,
-// so it waits for nothing that another plan enqueued; plans that run one after the other use the same pair.  (One pair for all plans of a
-// device: four threads' runs stood in one queue, and a run beside a plan with work of 8 ms enqueued took up to 7.9 ms, 1.1 as here.)
-// A device has at most a pair for each plan that runs in bands, eight at most; the last one is kept for the next plan until the process
-// exits.  Where there is none to be had, a run is one piece.
-struct LinkStreams { cudaStream_t up = nullptr, down = nullptr; };
-constexpr int kMaxLinkPairs = 8;
-struct LinkPool {
+// The two streams on which a run copies in bands, one per direction: a pair per device, made when a plan first needs it and kept until the
+// process exits.  A run has it to itself from its first copy until it has been waited for, so it waits for nothing that another plan
+// enqueued.  A run that finds it taken, or that it can't be made, is in one piece: the other run and its own copies in one stream keep both
+// directions busy already.  Runs of 32x64x64x56x56 and 32x128x128x28x28 in two threads take 940 us a pair so, 1090 with a pair of streams for
+// each and 1160 with both in one queue (in one piece, both: 1165); with a third thread (64x128x128x14x14) 1180, 1300, 1365 (1195).
+struct LinkStreams {
   std::mutex mutex;
-  LinkStreams idle[kMaxLinkPairs];
-  int idle_count = 0, made = 0, plans = 0;          // made: idle or in use; plans: with more than one band
+  bool taken = false;
+  cudaStream_t up = nullptr, down = nullptr;
 };
-LinkPool g_link[kMaxDevices];
-
-void destroy_pair(const LinkStreams &pair) {
-  if (pair.up) cudaStreamDestroy(pair.up);
-  if (pair.down) cudaStreamDestroy(pair.down);
-}
+LinkStreams g_link[kMaxDevices];
 
 // With the device current.
-bool take_link(LinkPool &pool, LinkStreams *out) {
-  {
-    std::lock_guard<std::mutex> lock(pool.mutex);
-    if (pool.idle_count > 0) {
-      *out = pool.idle[--pool.idle_count];
-      return true;
+bool take_link(LinkStreams &link) {
+  std::lock_guard<std::mutex> lock(link.mutex);
+  if (link.taken) return false;
+  for (cudaStream_t *s : {&link.up, &link.down})
+    if (!*s && cudaStreamCreateWithFlags(s, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaGetLastError();
+      *s = nullptr;
+      return false;
     }
-    if (pool.made >= kMaxLinkPairs || pool.made >= pool.plans) return false;
-    ++pool.made;
-  }
-  LinkStreams pair;
-  if (cudaStreamCreateWithFlags(&pair.up, cudaStreamNonBlocking) == cudaSuccess &&
-      cudaStreamCreateWithFlags(&pair.down, cudaStreamNonBlocking) == cudaSuccess) {
-    *out = pair;
-    return true;
-  }
-  cudaGetLastError();
-  destroy_pair(pair);
-  std::lock_guard<std::mutex> lock(pool.mutex);
-  --pool.made;
-  return false;
+  return link.taken = true;
 }
 
-void give_link(LinkPool &pool, const LinkStreams &pair) {
-  {
-    std::lock_guard<std::mutex> lock(pool.mutex);
-    if (pool.made == 1 || pool.made <= pool.plans) {
-      pool.idle[pool.idle_count++] = pair;
-      return;
-    }
-    --pool.made;
-  }
-  destroy_pair(pair);
-}
-
-void add_plan(LinkPool &pool) {
-  {
-    std::lock_guard<std::mutex> lock(pool.mutex);
-    ++pool.plans;
-  }
-  LinkStreams pair;                                 // so that the first run does not wait for it
-  if (take_link(pool, &pair)) give_link(pool, pair);
-}
-
-void remove_plan(LinkPool &pool) {
-  LinkStreams pair;
-  {
-    std::lock_guard<std::mutex> lock(pool.mutex);
-    --pool.plans;
-    if (pool.idle_count == 0 || pool.made <= 1 || pool.made <= pool.plans) return;
-    pair = pool.idle[--pool.idle_count];
-    --pool.made;
-  }
-  destroy_pair(pair);
+void give_link(LinkStreams &link) {
+  std::lock_guard<std::mutex> lock(link.mutex);
+  link.taken = false;
 }
 
 // Host-buffer front end.  A run that is waited for does the upload of the input, the kernel and the download of the output in `bands` bands of
@@ -92,7 +46,7 @@ struct HostPlan {
   float *d_in = nullptr, *d_filt = nullptr, *d_out = nullptr, *d_ws = nullptr;
   cudaStream_t stream = nullptr;
   int device = 0;
-  LinkPool *link = nullptr;                                         // this and the events only with more than one band
+  LinkStreams *link = nullptr;                                      // this and the events only with more than one band
   cudaEvent_t landed = nullptr, computed = nullptr, left = nullptr;
 };
 
@@ -134,7 +88,8 @@ cudaError_t copy_rows(float *dst, const float *src, int planes, int r0, int r1, 
   return cudaMemcpy2DAsync(dst + r0 * row, pitch, src + r0 * row, pitch, (r1 - r0) * row * 4, planes, kind, stream);
 }
 
-cudaError_t run_bands(HostPlan *hp, const LinkStreams &link, const float *input_host, const float *filter_host, float *output_host) {
+cudaError_t run_bands(HostPlan *hp, const float *input_host, const float *filter_host, float *output_host) {
+  const LinkStreams &link = *hp->link;
   const size_t f_b = (size_t)hp->C * 9 * hp->K * 4;
   const int tile_rows = (hp->H + 1) / 2;
   // what was enqueued on the plan before must be through with the device buffers
@@ -192,7 +147,7 @@ int opencnn_host_plan_create(void **plan, int in_n, int in_c, int in_h, int in_w
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     if (e == cudaSuccess) {
       hp->link = &g_link[hp->device];
-      add_plan(*hp->link);
+      if (take_link(*hp->link)) give_link(*hp->link);                // so that the first run does not wait for it
     }
   }
   if (e != cudaSuccess) {
@@ -235,21 +190,20 @@ int opencnn_host_plan_wait(void *plan) {
 int opencnn_host_plan_run(void *plan, const float *input_host, const float *filter_host, float *output_host) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
-  LinkStreams link;
   int device = -1;
   const bool bands = hp->bands > 1 && page_locked(input_host) && page_locked(output_host) && cudaGetDevice(&device) == cudaSuccess &&
-                     device == hp->device && take_link(*hp->link, &link);
-  const cudaError_t e = bands ? run_bands(hp, link, input_host, filter_host, output_host)
+                     device == hp->device && take_link(*hp->link);
+  const cudaError_t e = bands ? run_bands(hp, input_host, filter_host, output_host)
                               : (cudaError_t)host_plan_async(plan, input_host, filter_host, output_host, true);
   // What was enqueued before an error still reads and writes the caller's memory: wait for it, too.  (run_bands may not have joined its streams.)
   cudaError_t w = cudaStreamSynchronize(hp->stream);
   if (bands) {
     if (e != cudaSuccess || w != cudaSuccess)
-      for (cudaStream_t s : {link.up, link.down}) {
+      for (cudaStream_t s : {hp->link->up, hp->link->down}) {
         const cudaError_t ws = cudaStreamSynchronize(s);
         if (w == cudaSuccess) w = ws;
       }
-    give_link(*hp->link, link);
+    give_link(*hp->link);
   }
   return (int)(e != cudaSuccess ? e : w);
 }
@@ -257,7 +211,6 @@ int opencnn_host_plan_run(void *plan, const float *input_host, const float *filt
 int opencnn_host_plan_destroy(void *plan) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp) return 0;
-  if (hp->link) remove_plan(*hp->link);
   for (cudaEvent_t ev : {hp->landed, hp->computed, hp->left})
     if (ev) cudaEventDestroy(ev);
   if (hp->d_in) cudaFree(hp->d_in);
