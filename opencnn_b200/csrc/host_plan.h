@@ -53,13 +53,19 @@ struct HostPlan {
 // What bands can hide is the shorter of the two copies, so a band is at least kBandBytes of twice that one, and its rows of one plane at
 // least kBandRowBytes in a row (a strided copy is made of such pieces).  One call, us, by the number of bands (1: as one upload,
 // kernel, download):
-//     fp32 32x64x64x56x56    1: 1025   2: 828   4: 785   8: 819   12: 748   16: 844
-//     fp32 8x32x64x112x56    1: 403    2: 355   4: 334   8: 329   12: 355   16: 369
-//     fp32 32x256x256x14x14  1: 381    2: 309   4: 290   7: 334 (pieces of 3.6 KB)
-//     fp32 16x16x32x40x40    1: 137    2: 127   4: 125   8: 138   16: 182
-//     bf16 40x7x192x38x38    1: 877   12: 932 (1.6 MB in, 44 MB out: nothing to hide)
+//     fp32 32x64x64x56x56     1: 1028  2: 827   4: 787   6: 787   7: 814   8: 820   12: 780 to 842
+//     fp32 8x32x64x112x56     1: 401   2: 355   4: 335   6: 333   7: 335   8: 334   12: 334
+//     fp32 32x256x256x14x14   1: 384   2: 303   4: 290   6: 340 (pieces of 4.2 KB)
+//     fp32 32x128x128x28x28   1: 590   4: 469   6: 440   7: 399   8: 420   10: 433
+//     tf32 64x64x64x56x56     1: 1918  2: 1525  4: 1390  6: 1370  7: 1386  8: 1413  12: 1500
+//     bf16 16x64x64x60x90     1: 860   4: 664   6: 681   7: 685   8: 706   12: 749
+//     fp32 64x100x64x33x37                      6: 782   7: 843   8: 859   12: 811
+//     bf16 128x128x128x28x14                    6: 800   7: 813   8: 804   12: 776
+//     bf16 40x7x192x38x38     1: 877  12: 932 (1.6 MB in, 44 MB out: nothing to hide)
+// No number is the best for all; with six, ten of thirteen sizes were the same or up to 9 % faster than with twelve, and none more than 3 %
+// slower.
 constexpr size_t kBandBytes = 2400000, kBandRowBytes = 6u << 10;
-constexpr int kMaxBands = 12;
+constexpr int kMaxBands = 6;
 int band_count(int N, int C, int H, int W, int K) {
   const size_t row = (size_t)W * N * 4, bytes = 2 * row * H * (C < K ? C : K);
   const int tile_rows = (H + 1) / 2;
