@@ -4,6 +4,7 @@
 //     cudaError_t transform_filter(filter, workspace, C, K, precision, stream)
 //     cudaError_t convolve_rows(input, workspace, output, N, C, H, W, K, precision, stream, rows)               some rows of tiles
 #pragma once
+#include <functional>
 
 namespace {
 
@@ -92,6 +93,12 @@ cudaError_t copy_rows(float *dst, const float *src, int planes, int r0, int r1, 
   const size_t row = (size_t)hp->W * hp->N, pitch = row * hp->H * 4;
   if (r1 <= r0) return cudaSuccess;
   return cudaMemcpy2DAsync(dst + r0 * row, pitch, src + r0 * row, pitch, (r1 - r0) * row * 4, planes, kind, stream);
+}
+
+// Whether a band's output may be written before the next band's input is read: the arrays have nothing in common, or start at the same place,
+// where an output row lies over the same row of the input, which no later band reads from there.
+bool bands_apart(const float *in, size_t in_n, const float *out, size_t out_n) {
+  return in == out || std::less_equal<>()(in + in_n, out) || std::less_equal<>()(out + out_n, in);
 }
 
 cudaError_t run_bands(HostPlan *hp, const float *input_host, const float *filter_host, float *output_host) {
@@ -196,9 +203,11 @@ int opencnn_host_plan_wait(void *plan) {
 int opencnn_host_plan_run(void *plan, const float *input_host, const float *filter_host, float *output_host) {
   HostPlan *hp = static_cast<HostPlan *>(plan);
   if (!hp || !input_host || !filter_host || !output_host) return (int)cudaErrorInvalidValue;
+  const size_t plane = (size_t)hp->N * hp->H * hp->W;
   int device = -1;
-  const bool bands = hp->bands > 1 && page_locked(input_host) && page_locked(output_host) && cudaGetDevice(&device) == cudaSuccess &&
-                     device == hp->device && take_link(*hp->link);
+  const bool bands = hp->bands > 1 && bands_apart(input_host, hp->C * plane, output_host, hp->K * plane) && page_locked(input_host) &&
+                     page_locked(output_host) && cudaGetDevice(&device) == cudaSuccess && device == hp->device &&
+                     take_link(*hp->link);
   const cudaError_t e = bands ? run_bands(hp, input_host, filter_host, output_host)
                               : (cudaError_t)host_plan_async(plan, input_host, filter_host, output_host, true);
   // What was enqueued before an error still reads and writes the caller's memory: wait for it, too.  (run_bands may not have joined its streams.)

@@ -310,9 +310,28 @@ void no_streams() {
   CHECK(opencnn_host_plan_destroy(p) == 0);
 }
 
+// Input and output in one array: the input has been read where the output is written, wherever the two start.
+void overlap() {
+  Problem a(32, 24, 40, 40, 28);
+  const size_t row = (size_t)a.W * a.N;
+  for (long shift : {0l, (long)row, -(long)row, 5l * (long)row, -17l * (long)row, (long)a.x.size() / 2, -(long)a.y.size() / 2, (long)a.x.size()})
+    for (int trial = 0; trial < 4; ++trial) {
+      g_seed = 11 + trial;
+      std::vector<float> both(a.x.size() + 2 * a.y.size(), -1.f);
+      float *x = both.data() + a.y.size(), *y = x + shift;
+      std::copy(a.x.begin(), a.x.end(), x);
+      void *p = a.plan();
+      const int copies = g_copies_2d;
+      CHECK(opencnn_host_plan_run(p, x, a.f.data(), y) == 0);
+      CHECK(std::equal(a.expect.begin(), a.expect.end(), y));
+      CHECK((g_copies_2d > copies) == (shift == 0 || shift == (long)a.x.size()));
+      CHECK(opencnn_host_plan_destroy(p) == 0);
+    }
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const std::map<std::string, void (*)()> checks = {{"results", results}, {"errors", errors}, {"apart", apart}, {"streams", streams}, {"no_streams", no_streams}};
+  const std::map<std::string, void (*)()> checks = {{"results", results}, {"errors", errors}, {"apart", apart}, {"streams", streams}, {"no_streams", no_streams}, {"overlap", overlap}};
   if (what == "bands" && argc == 7) {               // bands N C H W K
     std::printf("%d\n", band_count(atoi(argv[2]), atoi(argv[3]), atoi(argv[4]), atoi(argv[5]), atoi(argv[6])));
     return 0;

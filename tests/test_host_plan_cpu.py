@@ -18,7 +18,7 @@ def host_plan(tmp_path_factory):
     return lambda *args: subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=120).stdout.strip()
 
 
-@pytest.mark.parametrize("check", ["results", "errors", "apart", "streams", "no_streams"])
+@pytest.mark.parametrize("check", ["results", "errors", "apart", "streams", "no_streams", "overlap"])
 def test_host_plan(host_plan, check):
     assert host_plan(check) == "ok"
 
