@@ -180,7 +180,7 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       const int k0 = (t / pairs) * 2 * kPairFilters + (int)rank * kPairFilters + 32 * (quarter & 1);
       mbar_wait_reporting(smem_u32(acc_full), seq & 1, dead, p.status, acc_empty0, smem_u32(nowhere));
       tc_fence_after();
-      tc_epilogue<false, true>(tcol, q < blocks && k0 < p.K ? 2 : 0, p, k0 + lane, c,
+      tc_epilogue<false, true, false>(tcol, q < blocks && k0 < p.K ? 2 : 0, p, k0 + lane, c,
                          [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
     }
   } else if (warp >= kPairFirstTransformWarp) {

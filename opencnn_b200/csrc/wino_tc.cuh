@@ -323,14 +323,15 @@ __device__ __forceinline__ OutputSpot output_spot(const WinoParams &p, int filte
 // a block; `q` is the quad of columns that this lane stores from on: the first of the 16 for an even lane, the ninth column's for an odd
 // one (see the stores).  HALF: the warp may have 8 columns only, `octets` = 1, which every lane stores from `q` on; with
 // `octets` = 0 it only hands the accumulators back.  WIDE: see read_accumulators.
-template <bool HALF, bool WIDE, class Release>
+template <bool HALF, bool WIDE, bool EARLY, class Release>
 __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const WinoParams &p, int k, const ColumnQuad &q, Release release) {
-  static_assert(!(HALF && WIDE), "the one with half a share of columns has its place from before the accumulators");
+  static_assert(!(EARLY && WIDE) && !(HALF && WIDE), "no such kernel");
   const int lane = threadIdx.x & 31;
-  // Worked out before the accumulators are read where there are registers for it: a tile's last step is its stores (TF32 single CTA
-  // 128x20x64x12x12 7.7 -> 7.4 us; the wide loads of the CTA pair lose by it, BF16 128x256x256x14x14 31.3 -> 31.7).
+  // EARLY: before the accumulators are read, a tile's last step being its stores.  Single CTA, TF32 128x20x64x12x12 7.7 -> 7.4 us, more than 64
+  // filters 1 % in the mean of 200 sizes; BF16 with 64 filters, which has a third of the work per tile, loses 1 %, and so does the CTA
+  // pair, BF16 128x256x256x14x14 31.3 -> 31.7.
   OutputSpot at;
-  if (!WIDE) at = output_spot(p, k, q);
+  if (EARLY) at = output_spot(p, k, q);
   // Y = A^T M A column by column of the 4x4 positions: column j (positions j, 4+j, 8+j, 12+j) gives the two
   // row sums a[j], a[4+j] of output_transform, which are folded into the four outputs at once - the same
   // operations in the same order.  After a column has been read it is handed back (release(j)), so the
@@ -365,6 +366,7 @@ __device__ __forceinline__ void tc_epilogue(uint32_t tcol, int octets, const Win
   // Stores: neighbouring lanes (filters) swap halves of their 16 images, so that one instruction writes the
   // 64 bytes of the pair's even filter (32 bytes per lane) and the next those of the odd filter - 16 lines of
   // two full sectors per instruction instead of 32 lines of one (see wino_tc_kernel).
+  if (!EARLY && !WIDE) at = output_spot(p, k, q);
   const int oh0 = 2 * q.ty, ow0 = 2 * q.tx;
   const bool row1 = WIDE ? (oh0 + 1) < p.H : at.row1, col1 = WIDE ? (ow0 + 1) < p.W : at.col1;
   const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = WIDE ? (size_t)p.H * dH : at.plane;
@@ -646,7 +648,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
       // Warps whose 32 filters all lie beyond K (K = 64 layers) have nothing to read or store.
-      tc_epilogue<true, false>(tmem_base + ((uint32_t)(quarter * 32) << 16) + 4 * quad0, k0 >= p.K ? 0 : dup ? 1 : 2, p, k0 + lane, q,
+      tc_epilogue<true, false, !HU>(tmem_base + ((uint32_t)(quarter * 32) << 16) + 4 * quad0, k0 >= p.K ? 0 : dup ? 1 : 2, p, k0 + lane, q,
                         [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }

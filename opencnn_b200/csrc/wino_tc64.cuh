@@ -255,7 +255,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       q.valid = q.n < p.N;
       mbar_wait(smem_u32(acc_full), seq & 1, dead, p.status);
       tc_fence_after();
-      tc_epilogue<false, false>(tlane + 16 * sub, warp_valid && block < p.blocks ? 2 : 0, p, k, q, [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
+      tc_epilogue<false, false, true>(tlane + 16 * sub, warp_valid && block < p.blocks ? 2 : 0, p, k, q, [&](int j) { mbar_arrive(smem_u32(acc_empty + j)); });
     }
   }
 
