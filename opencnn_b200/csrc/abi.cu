@@ -17,6 +17,7 @@
 #include "wino_pair.cuh"
 #include "wino_img.cuh"
 #include "wino_tc64.cuh"
+#include "dispatch.h"
 
 #if defined(BASE)
 #define OCB_VARIANT ocb::kBase
@@ -33,6 +34,10 @@
 #endif
 
 namespace {
+
+// What dispatch.h, which knows no kernels, says of them.
+static_assert(kColumns == ocb::kBN && kColumns == ocb::kTcN && kFp32Filters == ocb::kBK && kTcFilters == ocb::kTcM && kTcFilters == 2 * ocb::kPairFilters &&
+              kImgRowFilters == ocb::kImgFilters && kStepBf16 == ocb::TcCfg<ocb::kTcBf16>::kKC && kStepTf32 == ocb::TcCfg<ocb::kTcTf32>::kKC, "block sizes");
 
 __device__ int g_status = 0;
 
@@ -188,10 +193,6 @@ cudaError_t check_shape(int N, int C, int H, int W, int K, ShapeRule rule) {
   return cudaSuccess;
 }
 
-// Rows of 2x2-output tiles that a launch computes.
-struct TileRows { int first, count; };
-TileRows all_rows(int H) { return {0, (H + 1) / 2}; }
-
 // Launches a kernel that reads the transformed filter.  `after_fx`: the filter transform was the launch before it on this
 // stream, by this call, so its set-up (barriers, tensor memory, descriptors, the first patches) may overlap it; the
 // kernels wait for the transform's completion before their first load of U, and all other data is older than the
@@ -282,37 +283,9 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   p.k_blocks = (K + ocb::kBK - 1) / ocb::kBK;
   p.chunks_per_tile = (C + ocb::kBC - 1) / ocb::kBC;
   p.status = st->status_ptr;
-  // An SM's items are item, item + grid, ...: the first SM has most.  The last round of this schedule is usually only partly filled; cutting its
-  // whole tiles in two (one item per consumer group) pays if the halves still fit on the SMs (see item_tile), and the
-  // tiles of a last filter block with at most 32 filters are such halves already.  A half takes about 0.55 of a tile.
-  struct Schedule { long long blocks, tiles, wholes, split, cost; };
-  const auto schedule = [&](long long quads) {
-    const long long sms = st->sm_count;
-    const auto rounds = [&](long long items) { return (items + sms - 1) / sms; };
-    Schedule s;
-    s.blocks = (quads + 7) / 8;
-    s.tiles = s.blocks * p.k_blocks;
-    s.wholes = s.tiles - (K % ocb::kBK && K % ocb::kBK <= ocb::kBK / 2 ? s.blocks : 0);
-    const auto cost = [&](long long split) { return 11 * rounds(s.tiles + split) + 9 * rounds(s.wholes - split); };
-    const long long rest = s.wholes % sms;
-    s.split = cost(rest) < cost(0) ? rest : 0;
-    s.cost = cost(s.split);
-    return s;
-  };
-  // A ragged batch is packed where that shortens the schedule by more than the 4 to 7 % that the copies of its crossing blocks cost the main
-  // loop: 48x748x352x18x7 405 -> 358 us, but 28x24x396x7x7, one round either way, 10.9 -> 12.3.
-  const long long tile_count = (long long)p.tiles_h * p.tiles_w;
-  Schedule plan = schedule(tile_count * 8 * p.n_blocks);
-  p.quads_per_tile = 8 * p.n_blocks;
-  bool packed = false;
-  if (N % ocb::kBN) {
-    const Schedule tight = schedule(tile_count * (N / 4));
-    packed = 106 * tight.cost < 100 * plan.cost;
-    if (packed) {
-      plan = tight;
-      p.quads_per_tile = N / 4;
-    }
-  }
+  const Fp32Schedule plan = schedule_fp32(N, rows, W, K, st->sm_count);
+  const bool packed = plan.packed;
+  p.quads_per_tile = packed ? N / 4 : 8 * p.n_blocks;
   const bool ragged = N % ocb::kBN || K % ocb::kBK;
   if (plan.tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.blocks = (int)plan.blocks;
@@ -328,17 +301,6 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
-// Blocks of 32 columns of a problem (see ocb::ColumnQuad), with every tile's images filled up to a multiple of 32 or packed.
-struct Columns {
-  int quads_per_tile;
-  long long blocks;
-};
-Columns columns_of(int N, TileRows rows, int W, bool packed) {
-  Columns c;
-  c.quads_per_tile = packed ? N / 4 : (N + ocb::kTcN - 1) / ocb::kTcN * (ocb::kTcN / 4);
-  c.blocks = ((long long)rows.count * ((W + 1) / 2) * c.quads_per_tile + 7) / 8;
-  return c;
-}
 bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K, TileRows rows,
                  bool packed) {
   const Columns c = columns_of(N, rows, W, packed);
@@ -486,36 +448,6 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
 }
 
-// Which tensor-core kernel a problem gets: the one with the least estimated time.  All give the same bits.  An SM (or a CTA
-// pair) works through its tiles one after the other, so a kernel takes
-//     start + rounds x (round + step x K-steps),   K-steps = channels / 16 (BF16) or 8 (TF32),
-// and a problem much larger than L2 no less than its bytes at the rate the kernel's stores and loads were seen to reach.  The constants are
-// least squares through the fused kernels' times, back to back, at 260 random sizes per type (8 to 256 images, 64 to 1024
-// filters, 1 to 1024 channels, maps of 4 to 112); the estimates are 4 to 6 % off in the mean.  At 350 other random sizes per type the
-// kernel chosen by them was 0.15 % behind the fastest one in the mean, and 13 % at most.  Both sides of it, us,
-// single : pair : stacked : image rows:
-//   few K-steps or rounds      128x32x128x28x28  BF16 22.6 : 22.6 : - : 25.2    TF32 28.7 : 24.8 : - : 28.7
-//                              128x64x64x14x14   BF16 12.3 : 14.4 : 10.3 : 12.3  TF32 16.4 : 15.0 : 14.4 : 12.3
-//   64 filters                 128x64x64x56x56   BF16 81.8 : 82.7 : 71.1 : 65.9  TF32 123 : 103 : 111 : 71.8
-//                              256x32x64x112x112 BF16 813 : 413 : 392 : 267      TF32 552 : 477 : 490 : 300
-//                              128x512x64x14x14  BF16 41.1 : 39.0 : 39.1 : 29.4  TF32 76.4 : 50.8 : 60.5 : 40.0
-//   more filters, deep         128x256x256x14x14 BF16 41.0 : 33.4 : - : 43.0    TF32 62.5 : 43.0 : - : 57.4
-//                              64x1024x1024x14x14 BF16 279 : 196 : - : 276      TF32 512 : 322 : - : 459
-//   more filters, large output 96x4x128x99x99    BF16 174 : 131 : - : 122       TF32 188 : 131 : - : 111
-// Packed columns (single-CTA kernel, batch not a multiple of 32), filled up : packed
-//                              8x66x192x38x38    BF16 24.6 : 18.6               TF32 34.9 : 20.5
-//                              48x83x64x9x39     BF16 14.3 : 14.6               TF32 18.7 : 20.4
-struct KernelCost {
-  double start, round, step;    // us
-  double rate;                  // MB per us
-};
-constexpr double kL2Bound = 200.0;   // MB of input and output from which on the rate counts
-struct TcCosts { KernelCost single, single64, pair, stacked, image_rows, packed, packed64; };   // single64: at most 64 filters
-constexpr TcCosts kTcCosts[2] = {   // BF16, TF32
-    {{5.8, 1.29, 0.672, 2.9}, {4.9, 1.16, 0.57, 2.9}, {6.8, 1.53, 0.487, 4.1}, {5.2, 1.63, 1.043, 4.1}, {7.1, 1.61, 0.741, 4.5}, {6.6, 1.27, 0.826, 2.9}, {6.4, 0.99, 0.65, 2.9}},
-    {{5.3, 1.32, 0.576, 2.9}, {5, 1.32, 0.557, 2.9}, {6.8, 1.6, 0.338, 4.2}, {5.2, 1.79, 0.883, 4.1}, {7.1, 1.61, 0.493, 5.1}, {6.2, 1.34, 0.603, 2.9}, {6, 1.15, 0.591, 2.9}},
-};
-
 template <int DT>
 cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
                       cudaStream_t stream, bool after_fx, TileRows rows, int kernel = OPENCNN_TC_AUTO) {
@@ -525,26 +457,9 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
     const cudaError_t e = device_state(&st);
     if (e != cudaSuccess) return e;
     constexpr bool bf16 = DT == ocb::kTcBf16;
-    const TcCosts &costs = kTcCosts[bf16 ? 0 : 1];
-    const double k_steps = (C + ocb::TcCfg<DT>::kKC - 1) / ocb::TcCfg<DT>::kKC, mb = 8e-6 * N * rows.count * W * ((double)C + K);
-    double best = 0;
-    const auto consider = [&](int which, bool as_packed, const KernelCost &c, long long tiles, int at_once) {
-      if (at_once <= 0) return;             // (no two CTAs of this size can be co-scheduled as a cluster)
-      double t = c.start + (double)((tiles + at_once - 1) / at_once) * (c.round + c.step * k_steps);
-      if (mb > kL2Bound && t < mb / c.rate) t = mb / c.rate;
-      if (kernel != OPENCNN_TC_AUTO && t >= best) return;
-      best = t;
-      kernel = which;
-      packed = as_packed;
-    };
-    const long long blocks = columns_of(N, rows, W, false).blocks, wide = (K + ocb::kTcM - 1) / ocb::kTcM;
-    const int clusters = st->max_clusters[bf16 ? 0 : 1];
-    const KernelCost &single = K <= 64 ? costs.single64 : costs.single, &packed_single = K <= 64 ? costs.packed64 : costs.packed;
-    consider(OPENCNN_TC_SINGLE_CTA, false, single, blocks * wide, st->sm_count);
-    if (N % ocb::kTcN) consider(OPENCNN_TC_SINGLE_CTA, true, packed_single, columns_of(N, rows, W, true).blocks * wide, st->sm_count);
-    consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, clusters);
-    if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, false, costs.stacked, (blocks + 1) / 2, st->sm_count);
-    consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (blocks + 3) / 4 * (K / ocb::kImgFilters), clusters);
+    const TcChoice choice = choose_tc_kernel(bf16, N, C, rows, W, K, st->sm_count, st->max_clusters[bf16 ? 0 : 1]);
+    kernel = choice.kernel;
+    packed = choice.packed;
   }
   switch (kernel) {
     case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows, packed);
