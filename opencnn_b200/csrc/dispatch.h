@@ -63,33 +63,53 @@ Fp32Schedule schedule_fp32(int N, TileRows rows, int W, int K, int sms) {
 // ---- tensor cores ----
 // Which tensor-core kernel a problem gets: the one with the least estimated time.  All give the same bits.  An SM (or a CTA
 // pair) works through its tiles one after the other, so a kernel takes
-//     start + rounds x (round + step x K-steps),   K-steps = channels / 16 (BF16) or 8 (TF32),
-// and a problem much larger than L2 no less than its bytes at the rate the kernel's stores and loads were seen to reach.  The constants are
-// least squares through the fused kernels' times, back to back, at 260 random sizes per type (8 to 256 images, 64 to 1024
-// filters, 1 to 1024 channels, maps of 4 to 112); the estimates are 4 to 6 % off in the mean.  At 350 other random sizes per type the
-// kernel chosen by them was 0.15 % behind the fastest one in the mean, and 13 % at most.  Both sides of it, us,
+//     start + rounds x (round + images x full + crossing x cross + (step + crossing_step x cross) x K-steps)
+// with K-steps = channels / 16 (BF16) or 8 (TF32), full: the share of the columns that are images (they alone are stored), cross: the share of
+// packed blocks that lie in more than one tile (they are copied by threads); and a problem much larger than L2 no less than its bytes at
+// the rate the kernel's stores and loads were seen to reach.  The constants are least squares through the fused kernels' times, back to
+// back in a graph, at 1800 random sizes per type (8 to 256 images, 64 to 1024 filters, 1 to 1024 channels, maps of 4 to 112), on
+// 148 SMs at 1.9 GHz; the estimates are 3 to 6 % off in the mean.  At 1600 other sizes the kernel chosen by them was 0.35 % behind the fastest
+// one in the mean, and more than 10 % at 8.  Those are layers of one or two K-steps with an output that is many times L2, which the CTA
+// pair may write at 3.3 instead of 4.1 MB per us, for a reason not found (TF32 104x6x1024x54x54 377 us against 265, BF16 104x7x256x111x111 483
+// against 347), and small ones where two kernels' rounds end at about the same time (BF16 232x4x128x23x23 23.9 against 21.5).  Both sides of it, us,
 // single : pair : stacked : image rows:
-//   few K-steps or rounds      128x32x128x28x28  BF16 22.6 : 22.6 : - : 25.2    TF32 28.7 : 24.8 : - : 28.7
-//                              128x64x64x14x14   BF16 12.3 : 14.4 : 10.3 : 12.3  TF32 16.4 : 15.0 : 14.4 : 12.3
-//   64 filters                 128x64x64x56x56   BF16 81.8 : 82.7 : 71.1 : 65.9  TF32 123 : 103 : 111 : 71.8
-//                              256x32x64x112x112 BF16 813 : 413 : 392 : 267      TF32 552 : 477 : 490 : 300
-//                              128x512x64x14x14  BF16 41.1 : 39.0 : 39.1 : 29.4  TF32 76.4 : 50.8 : 60.5 : 40.0
-//   more filters, deep         128x256x256x14x14 BF16 41.0 : 33.4 : - : 43.0    TF32 62.5 : 43.0 : - : 57.4
-//                              64x1024x1024x14x14 BF16 279 : 196 : - : 276      TF32 512 : 322 : - : 459
-//   more filters, large output 96x4x128x99x99    BF16 174 : 131 : - : 122       TF32 188 : 131 : - : 111
-// Packed columns (single-CTA kernel, batch not a multiple of 32), filled up : packed
-//                              8x66x192x38x38    BF16 24.6 : 18.6               TF32 34.9 : 20.5
-//                              48x83x64x9x39     BF16 14.3 : 14.6               TF32 18.7 : 20.4
+//   few K-steps or rounds      128x32x128x28x28  BF16 20.3 : 19.8 : - : 22.0    TF32 26.0 : 22.1 : - : 25.8
+//                              128x64x64x14x14   BF16 10.1 : 11.4 : 9.2 : 9.2   TF32 14.1 : 13.1 : 12.3 : 10.4
+//   64 filters                 128x64x64x56x56   BF16 80.9 : 80.6 : 68.6 : 63.6  TF32 124 : 103 : 112 : 70.4
+//                              256x32x64x112x112 BF16 811 : 415 : 390 : 265      TF32 570 : 497 : 506 : 308
+//                              128x512x64x14x14  BF16 41.2 : 38.4 : 39.3 : 27.1  TF32 74.7 : 48.0 : 58.4 : 36.3
+//   more filters, deep         128x256x256x14x14 BF16 38.5 : 31.3 : - : 40.4    TF32 60.0 : 40.1 : - : 54.7
+//                              64x1024x1024x14x14 BF16 275 : 194 : - : 275      TF32 524 : 328 : - : 468
+//   more filters, large output 96x4x128x99x99    BF16 182 : 135 : - : 110       TF32 192 : 132 : - : 105
+// Packed columns (single-CTA kernel, batch not a multiple of 32), filled up : packed : the best of the others
+//                              8x66x192x38x38    BF16 22.9 : 16.5 : 20.8        TF32 32.1 : 18.1 : 23.9
+//                              48x83x64x9x39     BF16 11.7 : 12.3 : 10.2        TF32 17.2 : 17.8 : 11.5
+//                              24x20x960x58x60   BF16 130 packed, 113 the CTA pair
 struct KernelCost {
-  double start, round, step;    // us
-  double rate;                  // MB per us
+  double start, round, images, step;    // us
+  double rate;                          // MB per us
+  double crossing, crossing_step;       // us, packed columns only
 };
 constexpr double kL2Bound = 200.0;   // MB of input and output from which on the rate counts
 struct TcCosts { KernelCost single, single64, pair, stacked, image_rows, packed, packed64; };   // single64: at most 64 filters
 constexpr TcCosts kTcCosts[2] = {   // BF16, TF32
-    {{5.8, 1.29, 0.672, 2.9}, {4.9, 1.16, 0.57, 2.9}, {6.8, 1.53, 0.487, 4.1}, {5.2, 1.63, 1.043, 4.1}, {7.1, 1.61, 0.741, 4.5}, {6.6, 1.27, 0.826, 2.9}, {6.4, 0.99, 0.65, 2.9}},
-    {{5.3, 1.32, 0.576, 2.9}, {5, 1.32, 0.557, 2.9}, {6.8, 1.6, 0.338, 4.2}, {5.2, 1.79, 0.883, 4.1}, {7.1, 1.61, 0.493, 5.1}, {6.2, 1.34, 0.603, 2.9}, {6, 1.15, 0.591, 2.9}},
+    {{3.81, 0.712, 0.815, 0.659, 2.9, 0, 0}, {3.30, 0.428, 0.787, 0.545, 2.9, 0, 0}, {4.84, 0.935, 0.658, 0.469, 4.1, 0, 0},
+     {3.44, 0.776, 0.847, 1.020, 4.1, 0, 0}, {4.71, 1.141, 0.424, 0.723, 4.5, 0, 0}, {4.10, 1.354, 0, 0.756, 2.9, 0.167, 0.116},
+     {3.59, 1.035, 0, 0.604, 2.9, 0.183, 0.052}},
+    {{3.54, 0.719, 0.680, 0.561, 2.9, 0, 0}, {3.23, 1.069, 0.211, 0.540, 2.9, 0, 0}, {4.77, 0.887, 0.761, 0.330, 4.2, 0, 0},
+     {3.45, 0.947, 0.896, 0.866, 4.1, 0, 0}, {4.83, 1.128, 0.542, 0.482, 5.1, 0, 0}, {3.94, 1.320, 0, 0.585, 2.9, 0.226, 0.012},
+     {3.61, 1.210, 0, 0.555, 2.9, 0.078, 0.027}},
 };
+// Share of packed blocks of eight quads that run from one tile into the next, a tile having `quads` of them.
+double crossing_share(int quads) {
+  int unit = quads;                        // the common divisor of eight and the quads: where in a tile blocks may begin
+  for (int e = 8; e != 0;) {
+    const int r = unit % e;
+    unit = e;
+    e = r;
+  }
+  return quads <= 8 - unit ? 1.0 : (double)(8 - unit) / quads;
+}
 
 struct TcChoice { int kernel; bool packed; };
 // sms: SMs; clusters: CTA pairs that fit on the device at once.
@@ -97,11 +117,14 @@ TcChoice choose_tc_kernel(bool bf16, int N, int C, TileRows rows, int W, int K, 
   const TcCosts &costs = kTcCosts[bf16 ? 0 : 1];
   const int step = bf16 ? kStepBf16 : kStepTf32;
   const double k_steps = (C + step - 1) / step, mb = 8e-6 * N * rows.count * W * ((double)C + K);
+  const double full = (double)N / (columns_of(N, rows, W, false).quads_per_tile * 4), crossing = crossing_share(N / 4);
   TcChoice best = {OPENCNN_TC_AUTO, false};
   double best_time = 0;
   const auto consider = [&](int kernel, bool packed, const KernelCost &c, long long tiles, int at_once) {
     if (at_once <= 0) return;             // (no two CTAs of this size can be co-scheduled as a cluster)
-    double t = c.start + (double)((tiles + at_once - 1) / at_once) * (c.round + c.step * k_steps);
+    const double cross = packed ? crossing : 0;
+    double t = c.start + (double)((tiles + at_once - 1) / at_once) *
+                             (c.round + c.images * full + c.crossing * cross + (c.step + c.crossing_step * cross) * k_steps);
     if (mb > kL2Bound && t < mb / c.rate) t = mb / c.rate;
     if (best.kernel != OPENCNN_TC_AUTO && t >= best_time) return;
     best_time = t;

@@ -1,0 +1,41 @@
+"""The dispatch rules (opencnn_b200/csrc/dispatch.h) without a GPU: tests/dispatch_probe.cpp prints what they choose for a B200."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="session")
+def choose(tmp_path_factory):
+    """choose([(precision, (N, C, K, H, W)), ...]) -> the chosen routes."""
+    exe = str(tmp_path_factory.mktemp("dispatch") / "dispatch_probe")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-o", exe, os.path.join(HERE, "dispatch_probe.cpp")], check=True)
+
+    def ask(problems):
+        args = [str(a) for precision, shape in problems for a in (precision, *shape)]
+        out = subprocess.run([exe, *args], capture_output=True, text=True, check=True).stdout.splitlines()
+        assert len(out) == len(problems)
+        return out
+    return ask
+
+
+# Sizes at which two kernels' times are far apart (us, chosen : other, measured on a B200).  Among them batches of 24, 72 and 104 whose packed blocks
+# nearly all cross tiles.
+FAR_APART = [("bf16", (24, 20, 960, 58, 60), "pair_local"),      # 113 : 130 packed
+             ("tf32", (24, 18, 320, 92, 92), "pair_local"),      # 104 : 123 packed
+             ("tf32", (24, 48, 512, 70, 36), "pair_local"),      # 66.5 : 77.9 packed
+             ("tf32", (24, 31, 576, 66, 66), "pair_local"),      # 105 : 123 packed
+             ("bf16", (72, 41, 896, 58, 54), "pair_local"),      # 322 : 359 packed
+             ("bf16", (8, 66, 192, 38, 38), "packed"),           # 16.5 : 20.8 CTA pair
+             ("tf32", (8, 66, 192, 38, 38), "packed"),           # 18.1 : 23.9
+             ("bf16", (48, 83, 64, 9, 39), "image_rows"),        # 10.2 : 12.3 packed
+             ("tf32", (48, 83, 64, 9, 39), "image_rows"),        # 11.5 : 17.8
+             ("bf16", (128, 256, 256, 14, 14), "pair_local"),    # 31.3 : 38.5 single
+             ("tf32", (128, 64, 64, 56, 56), "image_rows")]      # 70.4 : 103 CTA pair
+
+
+def test_the_faster_kernel_is_chosen(choose):
+    got = choose([(precision, shape) for precision, shape, _ in FAR_APART])
+    assert got == [kernel for _, _, kernel in FAR_APART]
