@@ -47,7 +47,7 @@ struct DeviceState {
   std::once_flag once;
   cudaError_t init_error = cudaSuccess;
   int sm_count = 0;
-  int max_clusters[2] = {0, 0};   // co-resident CTA pairs of wino_pair_kernel and wino_img_kernel, <BF16 / TF32>
+  int pair_clusters[2] = {0, 0}, img_clusters[2] = {0, 0};   // co-resident CTA pairs of wino_pair_kernel and wino_img_kernel, <BF16 / TF32>
   int *status_ptr = nullptr;
 };
 DeviceState g_dev[kMaxDevices];
@@ -138,17 +138,15 @@ cudaError_t device_state(DeviceState **out) {
       cfg.attrs = &attr;
       cfg.numAttrs = 1;
       const auto pairs = [&](auto kernel, size_t smem, int &clusters) {
-        int n = 0;
         cfg.dynamicSmemBytes = smem;
-        if (err == cudaSuccess) err = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-        clusters = clusters == 0 || n < clusters ? n : clusters;
+        if (err == cudaSuccess) err = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
       };
-      pairs(ocb::wino_pair_kernel<ocb::kTcBf16>, ocb::PairCfg<ocb::kTcBf16>::kSmemBytes, st.max_clusters[0]);
-      pairs(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes, st.max_clusters[1]);
+      pairs(ocb::wino_pair_kernel<ocb::kTcBf16>, ocb::PairCfg<ocb::kTcBf16>::kSmemBytes, st.pair_clusters[0]);
+      pairs(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes, st.pair_clusters[1]);
       cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcBf16>::kThreads);
-      pairs(ocb::wino_img_kernel<ocb::kTcBf16>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.max_clusters[0]);
+      pairs(ocb::wino_img_kernel<ocb::kTcBf16>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.img_clusters[0]);
       cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcTf32>::kThreads);
-      pairs(ocb::wino_img_kernel<ocb::kTcTf32>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, st.max_clusters[1]);
+      pairs(ocb::wino_img_kernel<ocb::kTcTf32>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, st.img_clusters[1]);
     }
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_tc64_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -372,7 +370,7 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   constexpr int KC = ocb::PairCfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
   constexpr int esz = bf16 ? 2 : 4;
-  const int max_clusters = st->max_clusters[bf16 ? 0 : 1];
+  const int max_clusters = st->pair_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
 
   CUtensorMap tm_in, tm_u;
@@ -402,7 +400,7 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   if (!enc) return cudaErrorNotSupported;
   constexpr int KC = ocb::ImgCfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
-  const int max_clusters = st->max_clusters[bf16 ? 0 : 1];
+  const int max_clusters = st->img_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
   CUtensorMap tm_in, tm_u;
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
@@ -457,7 +455,7 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
     const cudaError_t e = device_state(&st);
     if (e != cudaSuccess) return e;
     constexpr bool bf16 = DT == ocb::kTcBf16;
-    const TcChoice choice = choose_tc_kernel(bf16, N, C, rows, W, K, st->sm_count, st->max_clusters[bf16 ? 0 : 1]);
+    const TcChoice choice = choose_tc_kernel(bf16, N, C, rows, W, K, st->sm_count, st->pair_clusters[bf16 ? 0 : 1], st->img_clusters[bf16 ? 0 : 1]);
     kernel = choice.kernel;
     packed = choice.packed;
   }

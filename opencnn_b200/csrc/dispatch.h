@@ -112,8 +112,8 @@ double crossing_share(int quads) {
 }
 
 struct TcChoice { int kernel; bool packed; };
-// sms: SMs; clusters: CTA pairs that fit on the device at once.
-TcChoice choose_tc_kernel(bool bf16, int N, int C, TileRows rows, int W, int K, int sms, int clusters) {
+// sms: SMs; pairs, img_pairs: CTA pairs of the two kernels that fit on the device at once (none: the kernel is not for it).
+TcChoice choose_tc_kernel(bool bf16, int N, int C, TileRows rows, int W, int K, int sms, int pairs, int img_pairs) {
   const TcCosts &costs = kTcCosts[bf16 ? 0 : 1];
   const int step = bf16 ? kStepBf16 : kStepTf32;
   const double k_steps = (C + step - 1) / step, mb = 8e-6 * N * rows.count * W * ((double)C + K);
@@ -133,9 +133,9 @@ TcChoice choose_tc_kernel(bool bf16, int N, int C, TileRows rows, int W, int K, 
   const long long blocks = columns_of(N, rows, W, false).blocks, wide = (K + kTcFilters - 1) / kTcFilters;
   consider(OPENCNN_TC_SINGLE_CTA, false, K <= 64 ? costs.single64 : costs.single, blocks * wide, sms);
   if (N % kColumns) consider(OPENCNN_TC_SINGLE_CTA, true, K <= 64 ? costs.packed64 : costs.packed, columns_of(N, rows, W, true).blocks * wide, sms);
-  consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, clusters);
+  consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, pairs);
   if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, false, costs.stacked, (blocks + 1) / 2, sms);
-  consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (blocks + 3) / 4 * (K / kImgRowFilters), clusters);
+  consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (blocks + 3) / 4 * (K / kImgRowFilters), img_pairs);
   return best;
 }
 

@@ -1,5 +1,6 @@
 // The rules of opencnn_b200/csrc/dispatch.h from the command line: `fp32 N C K H W` prints "filled" or "packed" and the rounds of items,
-// `tf32 | bf16 N C K H W` the kernel.  For a device of 148 SMs, 74 CTA pairs at once.
+// `tf32 | bf16 N C K H W` the kernel; `fits P I 0 0 0`: from here on P CTA pairs of the pair kernel and I of the image-rows kernel fit on the
+// device, which has 148 SMs (74 of each).
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -7,6 +8,7 @@
 #include "../opencnn_b200/csrc/dispatch.h"
 
 int main(int argc, char **argv) {
+  int pairs = 74, img_pairs = 74;
   for (int i = 1; i + 5 < argc; i += 6) {
     const int N = atoi(argv[i + 1]), C = atoi(argv[i + 2]), K = atoi(argv[i + 3]), H = atoi(argv[i + 4]), W = atoi(argv[i + 5]);
     if (!strcmp(argv[i], "fp32")) {
@@ -14,7 +16,13 @@ int main(int argc, char **argv) {
       std::printf("%s%s%s\n", s.packed ? "packed" : "filled", s.split ? " split" : "", s.wholes < s.tiles ? " halves" : "");
       continue;
     }
-    const TcChoice c = choose_tc_kernel(!strcmp(argv[i], "bf16"), N, C, all_rows(H), W, K, 148, 74);
+    if (!strcmp(argv[i], "fits")) {
+      pairs = N;
+      img_pairs = C;
+      std::printf("fits\n");
+      continue;
+    }
+    const TcChoice c = choose_tc_kernel(!strcmp(argv[i], "bf16"), N, C, all_rows(H), W, K, 148, pairs, img_pairs);
     const char *const names[] = {"auto", "single", "pair_local", "stacked", "image_rows"};
     std::printf("%s\n", c.packed ? "packed" : names[c.kernel]);
   }

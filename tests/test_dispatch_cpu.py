@@ -39,3 +39,12 @@ FAR_APART = [("bf16", (24, 20, 960, 58, 60), "pair_local"),      # 113 : 130 pac
 def test_the_faster_kernel_is_chosen(choose):
     got = choose([(precision, shape) for precision, shape, _ in FAR_APART])
     assert got == [kernel for _, _, kernel in FAR_APART]
+
+
+def test_a_kernel_that_does_not_fit_is_not_chosen(choose):
+    """No CTA pairs of one kernel at once: the other one's count does not stand in for it."""
+    problems = [(precision, shape) for precision, shape, _ in FAR_APART]
+    for pairs, img_pairs, never in ((0, 74, "pair_local"), (74, 0, "image_rows")):
+        got = choose([("fits", (pairs, img_pairs, 0, 0, 0)), *problems])[1:]
+        assert never not in got and set(got) & {"pair_local", "image_rows"}
+    assert not set(choose([("fits", (0, 0, 0, 0, 0)), *problems])) & {"pair_local", "image_rows"}
