@@ -47,7 +47,10 @@ template <int DT> struct ImgCfg {
                 "setmaxnreg budgets exceed the registers the CTA was launched with");
   static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kUStages * kUBytes +
                                        (size_t)kVStages * kVBytes + 512;
-  static_assert(kRawStages % 2 == 0 && kSmemBytes <= 232448, "shared memory");
+  static_assert(kSmemBytes <= 232448, "shared memory");
+  // Transform groups of a block that take K-steps in turn.  A group has to come back to the same stages (see PairCfg::kGroups).
+  static constexpr int kStepGroups = kTransformWarps / kBlockWarps / 2;
+  static_assert(kRawStages % (2 * kStepGroups) == 0 && kVStages % kStepGroups == 0, "ring depths are multiples of the group count");
 };
 constexpr int kImgFilters = 64;                  // per tile
 // Transformed values of a column pair in the operand layout: as finish_v_bf16 / finish_v_tf32, but a position holds 64 columns
@@ -190,7 +193,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     uint32_t v_ready0 = map_to_rank(smem_u32(v_ready), 0);
     // Groups of kBlockWarps: one for each block of a K-step (TF32: of every other K-step).
     const int group = (warp - kPairFirstTransformWarp) / Cfg::kBlockWarps, b = group & 1;
-    constexpr int kStepGroups = Cfg::kTransformWarps / Cfg::kBlockWarps / 2;
+    constexpr int kStepGroups = Cfg::kStepGroups;
     for (int g = group >> 1; g < total_steps; g += kStepGroups) {
       const int sv = g % SV, r = 2 * g + b, sr = r % SR;
       const uint32_t use = g / SV;
