@@ -87,7 +87,7 @@ def winograd_forward(input_chwn, workspace, output_khwn, N, C, H, W, K, *, preci
                                                        H, W, K, PRECISIONS[precision], stream)
 
 
-TC_KERNELS = {"auto": 0, "single": 1, "pair_local": 2, "stacked": 3}
+TC_KERNELS = {"auto": 0, "single": 1, "pair_local": 2, "stacked": 3, "image_rows": 4}
 
 
 def winograd_forward_kernel(input_chwn, workspace, output_khwn, N, C, H, W, K, *, precision, kernel, stream=0,

@@ -31,8 +31,9 @@ def test_python_enums_match_the_header():
     assert enums["OPENCNN_FP32"] == api.PRECISIONS["fp32"] and enums["OPENCNN_TF32"] == api.PRECISIONS["tf32"]
     assert enums["OPENCNN_BF16"] == api.PRECISIONS["bf16"]
     header_kernels = {"auto": "OPENCNN_TC_AUTO", "single": "OPENCNN_TC_SINGLE_CTA", "pair_local": "OPENCNN_TC_PAIR_LOCAL",
-                      "stacked": "OPENCNN_TC_STACKED_BLOCKS"}
+                      "stacked": "OPENCNN_TC_STACKED_BLOCKS", "image_rows": "OPENCNN_TC_IMAGE_ROWS"}
     assert set(api.TC_KERNELS) == set(header_kernels)
+    assert set(header_kernels.values()) == {name for name in enums if name.startswith("OPENCNN_TC_")}
     for name, enumerator in header_kernels.items():
         assert api.TC_KERNELS[name] == enums[enumerator], name
 

@@ -48,3 +48,31 @@ def test_a_kernel_that_does_not_fit_is_not_chosen(choose):
         got = choose([("fits", (pairs, img_pairs, 0, 0, 0)), *problems])[1:]
         assert never not in got and set(got) & {"pair_local", "image_rows"}
     assert not set(choose([("fits", (0, 0, 0, 0, 0)), *problems])) & {"pair_local", "image_rows"}
+
+
+KERNELS = {"single", "packed", "pair_local", "stacked", "image_rows"}
+
+
+def test_the_gpu_tests_reach_the_kernels_that_they_name(choose):
+    """What tests/test_tensorcore_gpu.py and test_parity_gpu.py say of the kernels that their sizes take."""
+    import test_parity_gpu as parity
+    import test_tensorcore_gpu as tc
+    routes = {}
+    for precision in ("tf32", "bf16"):
+        ask = lambda shapes: choose([(precision, shape) for shape in shapes])
+        assert set(ask(tc.CHOICES)) == KERNELS, precision
+        assert set(ask(tc.SHAPES)) == {"single", "pair_local"}
+        others = [shape for shape, route in zip(tc.PACKED, ask(tc.PACKED)) if route != "packed"]
+        expect = [(40, 20, 64, 35, 31)] + ([(72, 24, 64, 33, 30), (40, 24, 64, 41, 33), (104, 100, 64, 30, 30)] if precision == "tf32" else [])
+        assert others == expect, precision
+        contained = [shape for kernel, shape in tc.CONTAINED if kernel == "auto"]
+        assert ask(contained) == ["stacked" if precision == "bf16" else "image_rows", "pair_local", "packed", "packed", "stacked"]
+        for name in ("ORDERED", "REWRITTEN"):
+            problems = [(p, shape) for p, shape in getattr(tc, name) if p == precision]
+            routes.setdefault(name, set()).update(choose(problems))
+    assert routes["ORDERED"] == routes["REWRITTEN"] == KERNELS
+    for name in ("ORDERED", "REWRITTEN"):
+        fp32 = choose([("fp32", shape) for p, shape in getattr(tc, name) if p in ("fp32", "noalloc")])
+        assert {"packed", "packed halves"} <= set(fp32) and any(r.startswith("filled") for r in fp32)
+    fp32 = choose([("fp32", shape) for shape in parity.PACKED])
+    assert {"packed", "packed halves"} <= set(fp32) and any(r.startswith("filled") for r in fp32)

@@ -16,7 +16,8 @@ from opencnn_b200 import api  # noqa: E402
 pytestmark = pytest.mark.gpu
 
 # These small maps are one round of tiles: the deep ones take the CTA-pair kernel in both types, also with an odd number of 32-image
-# blocks, with K not a multiple of 128 and with 64 filters, the others the single-CTA kernel.
+# blocks, with K not a multiple of 128 and with 64 filters, the others the single-CTA kernel.  (test_dispatch_cpu.py checks what the
+# comments here say of the automatic choice.)
 SHAPES = [(32, 16, 128, 8, 8), (32, 8, 64, 7, 7), (64, 40, 192, 5, 9), (32, 64, 64, 14, 14), (96, 32, 256, 6, 6),
           (64, 512, 128, 4, 4), (96, 512, 192, 3, 5), (128, 520, 64, 2, 2), (64, 1024, 128, 3, 3), (96, 1040, 192, 2, 3)]
 MODEL_REL = 2e-4                     # device vs model: fp32 accumulation order inside the tensor core
@@ -234,7 +235,7 @@ def test_pair_kernel_gives_the_bits_of_the_single_cta_kernel(libs, precision, sh
     assert torch.equal(out["single"], out["pair_local"])
 
 
-# The kernel with the images in the accumulator rows (code 4 of the C ABI), likewise: one block of columns (three quarters of the
+# The kernel with the images in the accumulator rows, likewise: one block of columns (three quarters of the
 # pair's tile empty), five, a tile that spans two output tiles, more filter blocks than one, fewer K-steps than ring stages, more
 # tiles than pairs fit on the device at once.
 IMAGE_ROWS_SHAPES = [(8, 16, 64, 2, 2), (32, 24, 128, 5, 5), (40, 3, 192, 3, 5), (96, 72, 64, 3, 3), (24, 100, 320, 9, 4), (160, 40, 64, 17, 23),
@@ -250,16 +251,18 @@ def test_image_rows_kernel_gives_the_bits_of_the_single_cta_kernel(libs, precisi
     assert api.filter_transform(torch.randn((C, 3, 3, K), device="cuda") * 0.05, ws, C, K, precision=precision) == 0
     single, rows = (torch.full((K, H, W, N), float("nan"), device="cuda") for _ in range(2))
     assert api.winograd_forward_kernel(x, ws, single, N, C, H, W, K, precision=precision, kernel="single") == 0
-    assert libs["OPTSTS64"].opencnn_winograd_forward_kernel(x.data_ptr(), ws.data_ptr(), rows.data_ptr(), N, C, H, W, K,
-                                                            api.PRECISIONS[precision], 4, None) == 0
+    assert api.winograd_forward_kernel(x, ws, rows, N, C, H, W, K, precision=precision, kernel="image_rows") == 0
     assert api.last_device_status() == 0
     assert bool(torch.isfinite(single).all().item())
     assert torch.equal(single, rows)
 
 
 # Batches that are not a multiple of 32 and whose blocks of columns the automatic choice packs (single-CTA kernel): the bits that the
-# same images have in a batch filled up to a multiple of 32.  Blocks within one tile, across two and across four; odd maps.
-PACKED = [(8, 40, 128, 28, 28), (8, 3, 64, 57, 56), (16, 66, 192, 39, 38), (24, 64, 128, 28, 28), (40, 20, 64, 35, 31), (72, 24, 64, 33, 30)]
+# same images have in a batch filled up to a multiple of 32.  Blocks within one tile, across two and across four; odd maps.  The batches of 40 and
+# more have blocks within a tile, which TMA loads, between others; of these (40, 20, 64, 35, 31), and in TF32 the others with 64 filters but
+# (40, 3, 64, 13, 21), are another kernel's.
+PACKED = [(8, 40, 128, 28, 28), (8, 3, 64, 57, 56), (16, 66, 192, 39, 38), (24, 64, 128, 28, 28), (40, 20, 64, 35, 31), (72, 24, 64, 33, 30),
+          (40, 20, 192, 41, 37), (72, 8, 192, 35, 33), (104, 12, 192, 21, 27), (40, 24, 64, 41, 33), (104, 100, 64, 30, 30), (40, 3, 64, 13, 21)]
 
 
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
@@ -283,9 +286,16 @@ def test_packed_columns_give_the_bits_of_a_full_batch(libs, precision, shape):
 
 
 # The fused kernel is launched so that its set-up overlaps the filter transform: back-to-back calls that reuse one
-# workspace with other filters, and the same under stream capture, give what a transform waited for gives.
-@pytest.mark.parametrize("precision,shape", [("fp32", (32, 16, 64, 9, 9)), ("fp32", (36, 5, 68, 6, 5)), ("bf16", (64, 16, 64, 30, 30)),
-                                             ("bf16", (32, 256, 256, 6, 6)), ("tf32", (64, 64, 192, 7, 7)), ("tf32", (8, 3, 64, 4, 4))])
+# workspace with other filters, and the same under stream capture, give what a transform waited for gives.  Every kernel of the
+# automatic choice, the packed ones of both paths too.
+ORDERED = [("fp32", (32, 16, 64, 9, 9)), ("fp32", (36, 5, 68, 6, 5)), ("bf16", (64, 16, 64, 30, 30)), ("bf16", (32, 256, 256, 6, 6)),
+           ("tf32", (64, 64, 192, 7, 7)), ("tf32", (8, 3, 64, 4, 4)),
+           ("fp32", (20, 64, 64, 31, 45)), ("fp32", (4, 20, 20, 49, 11)), ("bf16", (8, 64, 64, 27, 21)), ("bf16", (40, 20, 192, 41, 37)),
+           ("tf32", (72, 20, 192, 17, 5)), ("bf16", (64, 16, 192, 25, 5)), ("tf32", (64, 64, 64, 21, 13)), ("tf32", (128, 8, 64, 5, 29)),
+           ("bf16", (32, 64, 64, 6, 6))]
+
+
+@pytest.mark.parametrize("precision,shape", ORDERED)
 def test_transform_and_kernel_stay_ordered(libs, precision, shape):
     N, C, K, H, W = shape
     x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
@@ -352,11 +362,16 @@ def test_nonfinite_values_are_not_lost(libs, precision, bits):
 
 # Every image is a convolution of its own: an infinity or a NaN in one leaves the bits of all others as they are, whichever
 # of a tile's two image blocks it sits in and whether the tile's other rows are another block's (K = 64, stacked), a
-# repetition of the same filters (K = 64, single) or filters that do not exist (K = 192).  The large maps take the device
-# four rounds of tiles, enough for the automatic choice to take the stacked kernel and the CTA pair.
+# repetition of the same filters (K = 64, single) or filters that do not exist (K = 192).  The automatic choice: stacked (image rows in TF32),
+# CTA pair, packed columns twice, with more than 64 filters and with 64, and stacked.
+CONTAINED = [("single", (64, 16, 64, 5, 6)), ("pair_local", (64, 24, 192, 5, 6)), ("stacked", (96, 24, 64, 5, 6)),
+             ("image_rows", (96, 24, 64, 5, 6)), ("image_rows", (72, 24, 128, 5, 6)),
+             ("auto", (64, 16, 64, 31, 30)), ("auto", (64, 40, 128, 31, 30)), ("auto", (72, 20, 192, 17, 5)), ("auto", (104, 8, 64, 15, 9)),
+             ("auto", (128, 8, 64, 5, 29))]
+
+
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
-@pytest.mark.parametrize("kernel,shape", [("single", (64, 16, 64, 5, 6)), ("pair_local", (64, 24, 192, 5, 6)), ("stacked", (96, 24, 64, 5, 6)),
-                                          ("auto", (64, 16, 64, 31, 30)), ("auto", (64, 40, 128, 31, 30))])
+@pytest.mark.parametrize("kernel,shape", CONTAINED)
 def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
     N, C, K, H, W = shape
     x = torch.rand((C, H, W, N), device="cuda") * 2 - 1
@@ -379,13 +394,10 @@ def test_nonfinite_values_stay_in_their_image(libs, precision, kernel, shape):
         assert torch.equal(y[..., others], clean[..., others]), (image, value)
 
 
-# The automatic choice on both sides of its cut-offs (148 SMs, 16 / 8 channels per K-step in BF16 / TF32; rounds of tiles in the
-# comment): the bits of the single-CTA kernel whatever it takes.  In BF16 / TF32 these are the single-CTA kernel for 5 / 1 of them (packed
-# columns for 2 / 0 more), the CTA pair for 2 / 5, the stacked kernel for 4 / 0 and the image-rows kernel for 0 / 7.
-CHOICES = [(32, 48, 128, 24, 12), (32, 128, 128, 24, 12), (64, 64, 192, 14, 20),                    # 1, 1, 2
-           (128, 16, 128, 41, 38), (128, 15, 256, 41, 39),                                        # 11, 23
-           (64, 64, 64, 16, 36), (64, 33, 64, 26, 26), (64, 33, 64, 30, 30), (200, 24, 64, 17, 23),  # 2 / 1, 3 / 2, 4 / 2, 6 / 3 stacked
-           (104, 100, 64, 30, 30), (160, 16, 64, 30, 30), (40, 400, 64, 30, 30), (8, 200, 64, 7, 5)]         # 7 / 4, 8 / 5, 4 / 2, 1 / 1
+# The automatic choice: the bits of the single-CTA kernel whatever it takes, which in each type is each of the kernels at some of these sizes.
+CHOICES = [(32, 48, 128, 24, 12), (32, 128, 128, 24, 12), (64, 64, 192, 14, 20), (128, 16, 128, 41, 38), (128, 15, 256, 41, 39),
+           (64, 64, 64, 16, 36), (64, 33, 64, 26, 26), (64, 33, 64, 30, 30), (200, 24, 64, 17, 23), (104, 100, 64, 30, 30), (160, 16, 64, 30, 30),
+           (40, 400, 64, 30, 30), (8, 200, 64, 7, 5), (128, 8, 64, 5, 29), (24, 64, 128, 28, 28)]
 
 
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
@@ -406,10 +418,14 @@ def test_automatic_choice_gives_the_bits_of_the_single_cta_kernel(libs, precisio
 
 # The fused kernel reads its input before the transform it overlaps is over, so what it reads must be older than that
 # transform: on one stream and without synchronisation the input buffer is rewritten before every call, and every call's
-# output is the next one's input.  Sizes that reach each fused kernel (single CTA, CTA pair, stacked, fp32), ragged ones too.
-@pytest.mark.parametrize("precision,shape", [("fp32", (32, 64, 64, 9, 9)), ("fp32", (36, 20, 20, 6, 5)), ("bf16", (32, 64, 64, 6, 6)),
-                                             ("tf32", (40, 64, 64, 5, 5)), ("bf16", (64, 128, 128, 14, 20)), ("tf32", (72, 128, 128, 15, 20)),
-                                             ("bf16", (64, 64, 64, 31, 30)), ("tf32", (56, 64, 64, 31, 30)), ("noalloc", (32, 64, 64, 9, 9))])
+# output is the next one's input.  Sizes that reach each fused kernel, the packed ones too (those read the input with other instructions).
+REWRITTEN = [("fp32", (32, 64, 64, 9, 9)), ("fp32", (36, 20, 20, 6, 5)), ("bf16", (32, 64, 64, 6, 6)), ("tf32", (40, 64, 64, 5, 5)),
+             ("bf16", (64, 128, 128, 14, 20)), ("tf32", (72, 128, 128, 15, 20)), ("bf16", (64, 64, 64, 31, 30)), ("tf32", (56, 64, 64, 31, 30)),
+             ("noalloc", (32, 64, 64, 9, 9)), ("fp32", (20, 64, 64, 31, 45)), ("fp32", (4, 20, 20, 49, 11)), ("bf16", (8, 64, 64, 27, 21)),
+             ("bf16", (8, 128, 128, 28, 28)), ("tf32", (8, 64, 64, 21, 27)), ("bf16", (64, 64, 64, 29, 9)), ("noalloc", (20, 64, 64, 31, 45))]
+
+
+@pytest.mark.parametrize("precision,shape", REWRITTEN)
 def test_input_written_just_before_the_call(libs, precision, shape):
     N, C, K, H, W = shape
     sources = [torch.rand((C, H, W, N), device="cuda") * 2 - 1 for _ in range(4)]
