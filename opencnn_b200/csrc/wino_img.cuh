@@ -18,9 +18,10 @@
 // leader, all waits are bounded, and a thread whose wait gave up reports nothing more to the leader.
 //
 // What bounds it: on shallow layers the latency of a tile's own patches, of which the ring holds two K-steps, and the epilogue
-// warps' stores; both cost about their DRAM time on top of the rest (128x64x64x56x56 BF16 66 us: without stores 48, without patch
-// loads 47, without the transform 59, without MMAs 62).  On deep ones the ring of two filter slices, the transform and the MMAs'
-// hand-off: 0.70 us per K-step in BF16, 0.48 in TF32, where the tensor pipe needs 0.26.
+// warps' stores; both cost about their DRAM time on top of the rest (128x64x64x56x56 BF16 64 us: without stores 45, without patch
+// loads 46, without the transform 58, without MMAs 58; TF32 69: 56, 61, 64, 62).  On deep ones the ring of two filter slices, the
+// transform and the MMAs' hand-off (128x512x64x14x14 BF16 27.5 us: without the transform 22.6, without MMAs 25.3, without stores or
+// patch loads 26 to 27): 0.72 us per K-step in BF16, 0.48 in TF32, where the tensor pipe needs 0.26.
 #pragma once
 #include "wino_pair.cuh"
 

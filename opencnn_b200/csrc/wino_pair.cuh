@@ -38,8 +38,9 @@ namespace ocb {
 // tile loses (256x8x128x56x56 91.0 -> 93.4 and 87.1 -> 90.8).  Handing the patches back as soon as they are in
 // registers, with a proxy fence of its own, gained nothing (203 / 323).  Since TF32 operands are rounded by one instruction:
 // 64x1024x1024x14x14 195 / 317, 128x256x256x14x14 34 / 43, 128x64x128x56x56 90 / 109, 256x8x128x56x56 92 / 88.
-// Eight accumulator columns per load, handed back before they are folded: 128x256x256x14x14 34.6 -> 33.4 in BF16, 256x32x64x112x112
-// 485 -> 477 in TF32.  16 transform warps, or BF16 K-steps taken in turn by two groups of four, need rings that leave the filters
+// Eight accumulator columns per load, handed back before they are folded, against four in two halves: BF16 128x256x256x14x14 31.8 -> 31.2,
+// 128x64x128x56x56 90.5 -> 88.0, 64x1024x1024x14x14 200 -> 198; TF32 128x64x128x56x56 111.8 -> 110.4, the deep ones the same.  With one K-step per
+// tile it may lose 1 to 3 % (BF16 8x9x256x62x68 28.0 -> 28.8).  16 transform warps, or BF16 K-steps taken in turn by two groups of four, need rings that leave the filters
 // two stages: 64x1024x1024x14x14 200 -> 234 us in BF16, nothing in TF32.
 // Five warpgroups: warps 0 and 1 load patches and filter slices, 2 and 3 issue the MMAs; warps 4-11 transform;
 // warps 12-19 are the epilogue.  Registers are shared out with setmaxnreg.
