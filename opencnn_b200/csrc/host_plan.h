@@ -4,7 +4,12 @@
 //     cudaError_t transform_filter(filter, workspace, C, K, precision, stream)
 //     cudaError_t convolve_rows(input, workspace, output, N, C, H, W, K, precision, stream, rows)               some rows of tiles
 #pragma once
+#include <cuda_runtime.h>
 #include <functional>
+#include <mutex>
+#include <new>
+
+#include "../../include/opencnn_b200.h"
 
 namespace {
 
