@@ -595,7 +595,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   for (int seq = 0; seq < my_tiles; ++seq) {
     int groups;
     const int item = (int)blockIdx.x + seq * (int)gridDim.x;
-    const int tile = S < 4 && !PACKED ? pinned_item_tile<RAGGED>(p, item, groups) : item_tile<RAGGED>(p, item, groups);
+    const int tile = !PACKED && (S < 4 || RAGGED) ? pinned_item_tile<RAGGED>(p, item, groups) : item_tile<RAGGED>(p, item, groups);
     if ((groups >> role.gi) & 1) {
       // ---- this group computes the item ----
       for (int ci = 0; ci < cpt; ++ci, ++g) {
@@ -631,7 +631,8 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       }
       // (Where this arithmetic stands and what of it the compiler moves decides how it schedules the main loop: with the packed kernel's
       // places in the others' epilogue as well, the others were 1 to 2.5 % slower, OPTSTS64 152x55x108x83x85 1400 -> 1381 us, 128x8x448x7x7
-      // 14.8 -> 14.4.  With three stages pinned registers are better still, BASE 64x512x512x14x14 542 -> 529, with four they are worse by 1 %.)
+      // 14.8 -> 14.4.  Pinned registers, items and place, are better still with three stages, BASE 64x512x512x14x14 542 -> 529; with four,
+      // pinned items are in the ragged kernel, 184x21x116x34x34 145.2 -> 144.1, and cost the exact one 0.8 %.)
       TileCoord tc = output_place<V, PACKED>(p, tile);
       if (S < 4) asm volatile("" : "+r"(tc.nb), "+r"(tc.tx), "+r"(tc.ty), "+r"(tc.kb));
       epilogue<V, SHAPE>(acc, my_stg, p, tc, role);
