@@ -523,22 +523,26 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     if (warp == kConsumerThreads / 32) {
       if (PACKED) {
         load_packed(p, &tm_in, &tm_u, stages, bar_full, bar_empty, S, my_tiles, dead);
-      } else if (lane == 0) {
-        // ---- TMA issuer: one lane keeps the ring full ----
-        tma_prefetch_descriptor(&tm_in);
-        tma_prefetch_descriptor(&tm_u);
+      } else {
+        // ---- TMA issuer: one warp keeps the ring full ----
+        if (elect_one()) {
+          tma_prefetch_descriptor(&tm_in);
+          tma_prefetch_descriptor(&tm_u);
+        }
         int seq = 0, ci = 0, groups_unused, issued = 0;
         TileCoord tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x, groups_unused));
         for (int g = 0; g < total_chunks; ++g) {
           const int s = g % S;
           // A wait that gave up: stop issuing - the stage may still be in use.
-          if (g >= S && !mbar_wait(smem_u32(bar_empty + s), ((g / S) - 1) & 1, dead, p.status)) break;
+          if (g >= S && !mbar_wait_warp(smem_u32(bar_empty + s), ((g / S) - 1) & 1, dead, p.status)) break;
           const uint32_t bar = smem_u32(bar_full + s);
           const uint32_t dst = smem_u32(stages + s * kStageFloats);
-          mbar_arrive_expect_tx(bar, kStageBytes);
-          tma_load_4d(dst, &tm_in, bar, tc.nb * kBN, 2 * tc.tx - 1, 2 * tc.ty - 1, ci * kBC);
-          if (g == 0) grid_dependency_wait();       // U is all that the kernel before this one writes
-          tma_load_3d(dst + kVStageFloats * 4u, &tm_u, bar, tc.kb * kBK, 0, ci * kBC);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar, kStageBytes);
+            tma_load_4d(dst, &tm_in, bar, tc.nb * kBN, 2 * tc.tx - 1, 2 * tc.ty - 1, ci * kBC);
+            if (g == 0) grid_dependency_wait();       // U is all that the kernel before this one writes
+            tma_load_3d(dst + kVStageFloats * 4u, &tm_u, bar, tc.kb * kBK, 0, ci * kBC);
+          }
           issued = g + 1;
           if (++ci == cpt) {
             ci = 0;

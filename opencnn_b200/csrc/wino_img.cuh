@@ -232,13 +232,12 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kIssueRegs));
     if (warp == 0) {
       // ===================================== patches =============================================
-      if (lane == 0)
         load_patches<KC, SR, 2>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
                            [&](int seq, int i) { return 4 * ((cid + seq * n_clusters) % quads) + 2 * (int)rank + i; });
     } else if (warp == 1) {
       // ===================================== filter slices =======================================
-      if (lane == 0) {
-        tma_prefetch_descriptor(&tm_u);
+      {
+        if (elect_one()) tma_prefetch_descriptor(&tm_u);
         grid_dependency_wait();   // U is all that the kernel before this one writes
         int g = 0;
         bool ok = true;
@@ -247,7 +246,8 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
           for (int ci = 0; ci < cpt; ++ci, ++g) {
             const int s = g % SU;
             const uint32_t use = g / SU;
-            if (use > 0 && !mbar_wait(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+            if (use > 0 && !mbar_wait_warp(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+            if (!elect_one()) continue;
             if (rank == 0) mbar_arrive_expect_tx(smem_u32(u_full + s), 2 * Cfg::kUBytes);
             // U viewed as {32 filters, channel, block of 32 filters, position}
             tma_load_4d_pair(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, map_to_rank(smem_u32(u_full + s), 0), 0, ci * KC,
@@ -274,8 +274,8 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
         for (int g = 0; g < total_steps; ++g) {
           const int su = g % SU, sv = g % SV;
           // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-          if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + su), (g / SU) & 1, dead, p.status))) break;
-          if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status))) break;
+          if (!mbar_wait_warp(smem_u32(u_full + su), (g / SU) & 1, dead, p.status)) break;
+          if (!mbar_wait_warp(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status)) break;
           tc_fence_after();
           const uint64_t ad = a_desc0 + (uint64_t)(sv * (Cfg::kVBytes >> 4)) + (uint64_t)(col0 * (2048 >> 4)),
                          bd = b_desc0 + (uint64_t)(su * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
@@ -285,7 +285,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
           for (int xo = 0; xo < 8; ++xo) {
             const int xr = 4 * (xo & 3) + (xo >> 2);     // position relative to col0: row xo & 3, column xo >> 2
             if ((xo & 3) == 0 && ci == 0 && seq > 0) {   // first write to a column of a new tile: drained in both CTAs?
-              if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
+              if (!mbar_wait_warp(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status)) { ok = false; break; }
               tc_fence_after();
             }
             if (elect_one()) tc_mma_pair<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (2048 >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc,

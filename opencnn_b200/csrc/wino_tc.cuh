@@ -410,7 +410,7 @@ template <int DT> __device__ __forceinline__ bool tile_repeats_filters(const Win
   return DT == kTcBf16 && p.K - kb * kTcM <= 64;
 }
 
-// The loader of the raw patches (one thread), which is the same in all tensor-core kernels: every K-step of KC channels of
+// The loader of the raw patches (one warp), which is the same in all tensor-core kernels: every K-step of KC channels of
 // each of this CTA's `my_tiles` tiles takes the patches of PER_STEP blocks of 32 columns, block_of(tile, i), into a ring of SR stages.
 template <int KC, int SR, int PER_STEP, class BlockOf>
 __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensorMap *tm_in, uint8_t *raw_s, uint64_t *raw_full,
@@ -418,7 +418,7 @@ __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensor
   constexpr uint32_t kBytes = KC * 16 * kTcN * 4;
   static_assert(PER_STEP == 1 || PER_STEP == 2, "blocks of a K-step");
   const int cpt = p.chunks_per_tile;
-  tma_prefetch_descriptor(tm_in);
+  if (elect_one()) tma_prefetch_descriptor(tm_in);
   int g = 0;
   bool ok = true;
   for (int seq = 0; seq < my_tiles && ok; ++seq) {
@@ -428,7 +428,8 @@ __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensor
       const uint32_t use = g / SR;
       const ColumnQuad &b = i % PER_STEP ? b1 : b0;
       // A wait that gave up: stop issuing - the stage may still be in use.
-      if (use > 0 && !mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+      if (use > 0 && !mbar_wait_warp(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+      if (!elect_one()) continue;
       mbar_arrive_expect_tx(smem_u32(raw_full + s), kBytes);
       // (A block past the last one reads what lies there: image rows of the next tile row, which in a run of some rows may be arriving at this
       // moment, or zeros below the image.  Its columns are not stored, and no kernel mixes columns.  To load zeros instead costs this thread a
@@ -455,7 +456,7 @@ __device__ __forceinline__ void load_packed_patches(const WinoParams &p, const C
     for (int ci = 0; ci < p.chunks_per_tile; ++ci, ++g) {
       const int s = g % SR;
       const uint32_t use = g / SR;
-      if (use > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status))) { ok = false; break; }
+      if (use > 0 && !mbar_wait_warp(smem_u32(raw_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
       patches.chunk<KC>(p, tm_in, smem_u32(raw_s + s * kBytes), smem_u32(raw_full + s), ci * KC);
     }
   }
@@ -518,23 +519,25 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
     // raw patches, the next one U.
     if (PACKED)
       load_packed_patches<KC, SR>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead);
-    else if (lane == 0)
+    else
       load_patches<KC, SR, 1>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
                               [&](int seq, int) { return ((int)blockIdx.x + seq * (int)gridDim.x) % p.blocks; });
   } else if (warp == kTcULoaderWarp) {
     // ===================================== filter slices =======================================
-    if (lane == 0) {
-      tma_prefetch_descriptor(&tm_u);
+    {
+      if (elect_one()) tma_prefetch_descriptor(&tm_u);
       grid_dependency_wait();   // U is all that the kernel before this one writes
       int seq = 0, ci = 0, issued = 0, kb = (int)blockIdx.x / p.blocks;
       for (int g = 0; g < total_chunks; ++g) {
         const int s = g % kTcStages;
         const uint32_t use = g / kTcStages;
         // A wait that gave up: stop issuing - the stage may still be in use.
-        if (use > 0 && !mbar_wait(smem_u32(uv_empty + s), (use - 1) & 1, dead, p.status)) break;
-        mbar_arrive_expect_tx(smem_u32(u_full + s), Cfg::kUBytes);
+        if (use > 0 && !mbar_wait_warp(smem_u32(uv_empty + s), (use - 1) & 1, dead, p.status)) break;
         // U viewed as {filters within a 128-byte row, channel, 128-byte row of the filter axis, position}
-        tma_load_4d(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, kb * (DT == kTcBf16 ? 2 : 4), 0);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(smem_u32(u_full + s), Cfg::kUBytes);
+          tma_load_4d(smem_u32(u_s + s * Cfg::kUBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, kb * (DT == kTcBf16 ? 2 : 4), 0);
+        }
         issued = g + 1;
         if (++ci == cpt) {
           ci = 0;
@@ -605,7 +608,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         const int s = g % kTcStages;
         const uint32_t use = g / kTcStages;
         // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + s), use & 1, dead, p.status))) break;      // U landed and V written
+        if (!mbar_wait_warp(smem_u32(u_full + s), use & 1, dead, p.status)) break;      // U landed and V written
         tc_fence_after();
         const uint64_t ad = ((dup || HU) ? a_desc0_dup : a_desc0) + (uint64_t)(s * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (Cfg::kUPosBytes >> 4)),
                        bd = b_desc0 + (uint64_t)(s * (kTcVBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
@@ -615,7 +618,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
         for (int xo = 0; xo < kPer; ++xo) {
           const int xr = 4 * (xo & 3) + (xo >> 2);                          // position relative to col0: row xo & 3, column xo >> 2
           if ((xo & 3) == 0 && ci == 0 && seq > 0) {                         // first write to a column of a new tile: drained?
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status)) { ok = false; break; }
             tc_fence_after();
           }
           if (elect_one()) tc_mma<DT>(d0 + xr * kTcN, ad + (uint64_t)(xr * (Cfg::kUPosBytes >> 4)), bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate);

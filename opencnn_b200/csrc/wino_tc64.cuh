@@ -135,22 +135,23 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
 
   if (warp == 0) {
     // ===================================== patches: one block per sub-step =====================
-    if (lane == 0)
         load_patches<KC, SR, 2>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
                          [&](int seq, int i) { return 2 * ((int)blockIdx.x + seq * (int)gridDim.x) + i; });
   } else if (warp == kTcULoaderWarp) {
     // ===================================== filter slices: one per K-step =======================
-    if (lane == 0) {
-      tma_prefetch_descriptor(&tm_u);
+    {
+      if (elect_one()) tma_prefetch_descriptor(&tm_u);
       grid_dependency_wait();   // U is all that the kernel before this one writes
       int ci = 0, issued = 0;
       for (int g = 0; g < total_steps; ++g) {
         const int s = g % SU;
         const uint32_t use = g / SU;
         // A wait that gave up: stop issuing - the stage may still be in use.
-        if (use > 0 && !mbar_wait(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) break;
-        mbar_arrive_expect_tx(smem_u32(u_full + s), kT64UBytes);
-        tma_load_4d(smem_u32(u_s + s * kT64UBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, 0, 0);
+        if (use > 0 && !mbar_wait_warp(smem_u32(u_empty + s), (use - 1) & 1, dead, p.status)) break;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(smem_u32(u_full + s), kT64UBytes);
+          tma_load_4d(smem_u32(u_s + s * kT64UBytes), &tm_u, smem_u32(u_full + s), 0, ci * KC, 0, 0);
+        }
         issued = g + 1;
         if (++ci == cpt) ci = 0;
       }
@@ -205,8 +206,8 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       for (int g = 0; g < total_sub; ++g) {
         const int b = g & 1, su = (g >> 1) % SU, sv = g % SV;
         // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-        if (b == 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(u_full + su), ((g >> 1) / SU) & 1, dead, p.status))) break;
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status))) break;
+        if (b == 0 && !mbar_wait_warp(smem_u32(u_full + su), ((g >> 1) / SU) & 1, dead, p.status)) break;
+        if (!mbar_wait_warp(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status)) break;
         tc_fence_after();
         const uint64_t astep = b == 0 ? kTopPos : kBotPos;
         const uint64_t ad = (b == 0 ? a_top0 + (uint64_t)su * kTopStage : a_bot0 + (uint64_t)su * kBotStage) + (uint64_t)col0 * astep;
@@ -218,7 +219,7 @@ wino_tc64_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
         for (int xo = 0; xo < 8; ++xo) {
           const int xr = 4 * (xo & 3) + (xo >> 2);     // position relative to col0: row xo & 3, column xo >> 2
           if ((xo & 3) == 0 && b == 0 && ci == 0 && seq > 0) {   // first write to a column of a new tile: drained?
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status))) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(acc_empty + col0 + (xo >> 2)), (seq - 1) & 1, dead, p.status)) { ok = false; break; }
             tc_fence_after();
           }
           if (elect_one()) tc_mma_half<DT>(d0 + xr * kTcN, ad + (uint64_t)xr * astep, bd + (uint64_t)(xr * (1024 >> 4)), idesc, accumulate, skip_lo, skip_hi);

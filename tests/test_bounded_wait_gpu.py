@@ -78,3 +78,17 @@ def test_wait_that_runs_out_in_one_cta_of_a_pair_ends_the_other(oracle, libs, pr
     assert api.winograd_forward_kernel(torch.from_numpy(x).cuda(), ws, dy, N, C, H, W, K, precision="bf16", kernel="pair_local") == 0
     assert api.last_device_status() == 0
     assert np.array_equal(dy.cpu().numpy().astype(np.float64), oracle.direct_f64(x, g))
+
+
+@pytest.mark.parametrize("skip_arrive", [False, True])
+def test_wait_of_a_whole_warp(probe, skip_arrive):
+    """All lanes get the same answer; the wait that nobody ends runs out after its limit, or at once where one before it has."""
+    out = (ctypes.c_longlong * 4)()
+    assert probe.wait_probe_warp_run(int(skip_arrive), LIMIT_NS, out) == 0
+    first_ok, second_ok, first_ns, second_ns = list(out)
+    assert probe.wait_probe_last_status() == 1 and probe.wait_probe_last_status() == 0
+    assert (first_ok, second_ok) == (0 if skip_arrive else 32, 0)
+    waited_ns = first_ns if skip_arrive else second_ns
+    assert LIMIT_NS <= waited_ns < 50 * LIMIT_NS
+    if skip_arrive:
+        assert second_ns < LIMIT_NS

@@ -1,4 +1,4 @@
-// Test-only kernels for the bounded waits of opencnn_b200/csrc/ptx.cuh (mbar_wait, mbar_wait_drain, mbar_wait_reporting).
+// Test-only kernels for the bounded waits of opencnn_b200/csrc/ptx.cuh (mbar_wait, mbar_wait_warp, mbar_wait_drain, mbar_wait_reporting).
 // The library's kernels never wait for ever: a wait that runs out sets the CTA's `dead` word and a
 // device status word, the thread that issues asynchronous work stops and drains, everybody else
 // falls through their later waits, and the kernel returns.  None of that can be seen in a
@@ -118,7 +118,56 @@ wait_probe_pair_kernel(PairProbeOut *out, int skip_arrive, unsigned long long li
   ocb::cluster_sync_all();                           // every thread gets here whatever the waits did
 }
 
+// One warp that waits as a whole (mbar_wait_warp): for a barrier on which another warp arrives unless `skip_arrive`, then for one on which nobody
+// ever does.  ok: how many lanes each wait told that it succeeded.
+struct WarpProbeOut {
+  int first_ok, second_ok;
+  long long first_ns, second_ns;
+};
+__global__ void __launch_bounds__(64, 1) wait_probe_warp_kernel(WarpProbeOut *out, int skip_arrive, unsigned long long limit_ns, int *status) {
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ int dead_word;
+  volatile int *dead = &dead_word;
+  if (threadIdx.x == 0) {
+    dead_word = 0;
+    ocb::mbar_init(ocb::smem_u32(bars + 0), 1);
+    ocb::mbar_init(ocb::smem_u32(bars + 1), 1);
+    ocb::mbar_fence_init();
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const uint64_t t0 = ocb::global_timer_ns();
+    const int first = __popc(__ballot_sync(0xFFFFFFFFu, ocb::mbar_wait_warp(ocb::smem_u32(bars + 0), 0, dead, status, limit_ns)));
+    const uint64_t t1 = ocb::global_timer_ns();
+    const int second = __popc(__ballot_sync(0xFFFFFFFFu, ocb::mbar_wait_warp(ocb::smem_u32(bars + 1), 0, dead, status, limit_ns)));
+    const uint64_t t2 = ocb::global_timer_ns();
+    if (threadIdx.x == 0) *out = {first, second, (long long)(t1 - t0), (long long)(t2 - t1)};
+  } else if (threadIdx.x == 32 && !skip_arrive) {
+    ocb::mbar_arrive(ocb::smem_u32(bars + 0));
+  }
+}
+
 }  // namespace
+
+// Runs the whole-warp probe once, synchronously.  out[4]: first_ok, second_ok, first_ns, second_ns.  Returns a cudaError_t code.
+extern "C" int wait_probe_warp_run(int skip_arrive, unsigned long long limit_ns, long long *out4) {
+  if (!out4 || limit_ns == 0 || limit_ns > 100000000ull) return (int)cudaErrorInvalidValue;   // at most 0.1 s per wait
+  WarpProbeOut *d = nullptr;
+  int *status = nullptr;
+  cudaError_t e = cudaMalloc(&d, sizeof(WarpProbeOut));
+  if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void **>(&status), g_status);
+  if (e == cudaSuccess) {
+    wait_probe_warp_kernel<<<1, 64>>>(d, skip_arrive, limit_ns, status);
+    e = cudaGetLastError();
+  }
+  WarpProbeOut h;
+  if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) {
+    out4[0] = h.first_ok; out4[1] = h.second_ok; out4[2] = h.first_ns; out4[3] = h.second_ns;
+  }
+  if (d) cudaFree(d);
+  return (int)e;
+}
 
 // Runs the two-CTA probe once, synchronously.  out[3]: worker_ok, leader_ok, leader_wait_ns.  Returns a cudaError_t code.
 extern "C" int wait_probe_pair_run(int skip_arrive, unsigned long long limit_ns, long long *out3) {
