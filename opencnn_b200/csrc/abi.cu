@@ -225,6 +225,17 @@ bool encode_patches(EncodeTiledFn enc, CUtensorMap *map, const float *input, int
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same for the 4x6 patches of two tiles beside each other, with the channels of a pixel one behind the other.
+bool encode_tile_pairs(EncodeTiledFn enc, CUtensorMap *map, const float *input, int N, int C, int H, int W, int channels) {
+  cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H};
+  cuuint64_t strides[3] = {(cuuint64_t)H * W * N * 4, (cuuint64_t)N * 4, (cuuint64_t)W * N * 4};
+  cuuint32_t box[4] = {32, (cuuint32_t)channels, 6, 4};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Tensor map of the workspace [C][16][K] of a tensor-core precision, viewed as {filter within a row of `row_bytes`, channel, row,
 // position}: boxes of one K-step of channels, `rows` rows of filters and all positions, swizzled over a row.
 template <int DT>
@@ -403,12 +414,17 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   const int max_clusters = st->img_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
   CUtensorMap tm_in, tm_u;
-  if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  if (!encode_tile_pairs(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
+  const long long blocks = tile_pair_blocks(N, rows, W);
+  if (blocks > 0x7fffffffll / 16) return cudaErrorInvalidValue;
+  p.blocks = (int)blocks;
+  p.tiles_w = (p.tiles_w + 1) / 2;
+  p.n_blocks = (N + kColumns - 1) / kColumns;
   p.k_blocks = K / ocb::kImgFilters;
-  const long long tiles = ((long long)p.blocks + 3) / 4 * p.k_blocks;
+  const long long tiles = (blocks + 1) / 2 * p.k_blocks;
   if (tiles > 0x7fffffffll / 8) return cudaErrorInvalidValue;
   p.total_tiles = (int)tiles;
   p.total_items = p.total_tiles;

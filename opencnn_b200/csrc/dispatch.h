@@ -28,6 +28,11 @@ Columns columns_of(int N, TileRows rows, int W, bool packed) {
   return c;
 }
 
+// Blocks of two tiles beside each other and 32 images (image-rows kernel).
+long long tile_pair_blocks(int N, TileRows rows, int W) {
+  return (long long)rows.count * (((W + 1) / 2 + 1) / 2) * ((N + kColumns - 1) / kColumns);
+}
+
 // ---- fp32 ----
 // An SM's items are item, item + grid, ...: the first SM has most.  The last round of this schedule is usually only partly filled; cutting its
 // whole tiles in two (one item per consumer group) pays if the halves still fit on the SMs (see item_tile in wino_fp32.cuh), and the
@@ -135,7 +140,7 @@ TcChoice choose_tc_kernel(bool bf16, int N, int C, TileRows rows, int W, int K, 
   if (N % kColumns) consider(OPENCNN_TC_SINGLE_CTA, true, K <= 64 ? costs.packed64 : costs.packed, columns_of(N, rows, W, true).blocks * wide, sms);
   consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, pairs);
   if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, false, costs.stacked, (blocks + 1) / 2, sms);
-  consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (blocks + 3) / 4 * (K / kImgRowFilters), img_pairs);
+  consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (tile_pair_blocks(N, rows, W) + 1) / 2 * (K / kImgRowFilters), img_pairs);
   return best;
 }
 

@@ -29,74 +29,83 @@ namespace ocb {
 
 template <int DT> struct ImgCfg {
   static constexpr int kKC = DT == kTcBf16 ? 16 : 8;                       // channels per K-step
-  static constexpr uint32_t kRawBytes = kKC * 16 * kTcN * 4;               // one block: [c][4 h][4 w][32 columns] fp32
+  static constexpr int kRows = kKC * 128;                                  // a pixel, or a position, of a stage: one row per channel
+  static constexpr uint32_t kRawBytes = 24 * kRows;                        // 4x6 patch: [h][w][c][32 images] fp32
   static constexpr uint32_t kUBytes = 16 * 1024;                           // 16 positions x (32 filters x one K-step)
   static constexpr uint32_t kVBytes = 16 * 2048;                           // 16 positions x (64 columns x one K-step)
-  static constexpr int kRawStages = DT == kTcBf16 ? 4 : 8;
+  static constexpr uint32_t kStageBytes = kRawBytes > kVBytes ? kRawBytes : kVBytes;
+  static constexpr int kStages = DT == kTcBf16 ? 4 : 6;
   static constexpr int kUStages = 2;
-  static constexpr int kVStages = 2;
-  // Transform warps: four per block of columns, a thread one channel and column pair (BF16, 16 channels: two).  In TF32 a second set of
-  // eight takes every other K-step (256x32x64x112x112 325 -> 302 us); in BF16 that gains nothing on shallow layers, and the registers
-  // are better spent on an epilogue that reads 16 accumulator columns at a time (276 -> 266, 128x512x64x14x14 30.8 -> 29.0).
-  static constexpr int kBlockWarps = 4;
-  static constexpr int kTransformWarps = DT == kTcBf16 ? 8 : 16, kFirstEpilogueWarp = kPairFirstTransformWarp + kTransformWarps;
+  // Transform warps: a thread takes the two tiles of one channel and image pair.  BF16 (16 channels): all eight share a K-step; TF32 (8 channels):
+  // two groups of four take the K-steps in turn.
+  static constexpr int kTransformWarps = 8, kStepWarps = kKC / 2, kFirstEpilogueWarp = kPairFirstTransformWarp + kTransformWarps;
   static constexpr int kThreads = (kFirstEpilogueWarp + kTcEpilogueWarps) * 32;
-  static constexpr int kEpilogueLoad = DT == kTcBf16 ? 16 : 8;       // accumulator columns per load
-  static constexpr int kLaunchRegs = DT == kTcBf16 ? 96 : 72, kIssueRegs = DT == kTcBf16 ? 64 : 72,
-                       kTransformRegs = 48, kEpilogueRegs = DT == kTcBf16 ? 160 : 120;
+  static constexpr int kEpilogueLoad = 8;                            // accumulator columns per load
+  static constexpr int kLaunchRegs = 96, kIssueRegs = 40, kTransformRegs = 80, kEpilogueRegs = 136;
   static_assert(4 * kIssueRegs + kTransformWarps * kTransformRegs + kTcEpilogueWarps * kEpilogueRegs <= kThreads / 32 * kLaunchRegs,
                 "setmaxnreg budgets exceed the registers the CTA was launched with");
-  static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kUStages * kUBytes +
-                                       (size_t)kVStages * kVBytes + 512;
+  static constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + (size_t)kUStages * kUBytes + 512;
   static_assert(kSmemBytes <= 232448, "shared memory");
-  // Transform groups of a block that take K-steps in turn.  A group has to come back to the same stages (see PairCfg::kGroups).
-  static constexpr int kStepGroups = kTransformWarps / kBlockWarps / 2;
-  static_assert(kRawStages % (2 * kStepGroups) == 0 && kVStages % kStepGroups == 0, "ring depths are multiples of the group count");
+  // Transform groups that take K-steps in turn.  A group has to come back to the same stages (see PairCfg::kGroups).
+  static constexpr int kGroups = kTransformWarps / kStepWarps;
+  static_assert(kStages % kGroups == 0, "the ring's depth is a multiple of the group count");
 };
 constexpr int kImgFilters = 64;                  // per tile
-// Transformed values of a column pair in the operand layout: as finish_v_bf16 / finish_v_tf32, but a position holds 64 columns
-// (2 KB).  BF16: rows of 128 bytes, 128-byte swizzle (16-byte chunk index ^= c & 7).  TF32: the two blocks' rows of 128 bytes
-// are 1 KB apart.
+
+// A pair of tiles beside each other and 32 images: what a CTA computes of a pair tile.
+struct TilePair { int tx, ty, n; };              // the left tile, the first image
+__device__ __forceinline__ TilePair tile_pair(const WinoParams &p, int block) {
+  const int t = block / p.n_blocks, ty = t / p.tiles_w;
+  return {2 * (t - ty * p.tiles_w), ty + p.ty0, (block - t * p.n_blocks) * kTcN};
+}
+
+// Transforms the two tiles of channel `c` and images 2 np, 2 np + 1 of a stage, whose 4x6 patch they share, and writes them where the patch was.  A
+// warp has all pixels of its two channels in registers before it writes, and a position's row of a channel lies in a pixel's row
+// of the same channel (or behind the patch), so that no other warp's data is touched.
+// V: a position holds 64 columns (2 KB), tile 0 first.  BF16: rows of 128 bytes, 128-byte swizzle (16-byte chunk index ^= c & 7).  TF32: the two
+// tiles' rows of 128 bytes are 1 KB apart, 128-byte swizzle with 32-byte atoms.
 template <int DT>
-__device__ __forceinline__ void finish_v_wide(const uint64_t (&d)[16], uint8_t *__restrict__ vst, int block, int c, int np) {
-  uint64_t b[16];
+__device__ __forceinline__ void transform_tile_pair(uint8_t *stage, int c, int np) {
+  constexpr int kRows = ImgCfg<DT>::kRows;
+  uint64_t d[24];                                  // [h][w]
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    b[j] = sub2(d[j], d[8 + j]);
-    b[4 + j] = add2(d[4 + j], d[8 + j]);
-    b[8 + j] = sub2(d[8 + j], d[4 + j]);
-    b[12 + j] = sub2(d[4 + j], d[12 + j]);
+  for (int q = 0; q < 24; ++q) d[q] = *reinterpret_cast<const uint64_t *>(stage + q * kRows + c * 128 + np * 8);
+  __syncwarp();
+#pragma unroll
+  for (int w = 0; w < 6; ++w) {
+    const uint64_t b0 = sub2(d[w], d[12 + w]), b1 = add2(d[6 + w], d[12 + w]), b2 = sub2(d[12 + w], d[6 + w]), b3 = sub2(d[6 + w], d[18 + w]);
+    d[w] = b0; d[6 + w] = b1; d[12 + w] = b2; d[18 + w] = b3;
   }
   const int n = 2 * np;
-  uint8_t *dst = DT == kTcBf16 ? vst + c * 128 + ((((4 * block + (np >> 2)) ^ c) & 7) << 4) + ((np & 3) << 2)
-                               : vst + block * 1024 + c * 128 + ((((n >> 3) ^ c) & 3) << 5) + ((n & 7) << 2);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint64_t o[4];
-    o[0] = sub2(b[4 * i + 0], b[4 * i + 2]);
-    o[1] = add2(b[4 * i + 1], b[4 * i + 2]);
-    o[2] = sub2(b[4 * i + 2], b[4 * i + 1]);
-    o[3] = sub2(b[4 * i + 1], b[4 * i + 3]);
+  for (int t = 0; t < 2; ++t) {
+    uint8_t *dst = DT == kTcBf16 ? stage + c * 128 + ((((4 * t + (np >> 2)) ^ c) & 7) << 4) + ((np & 3) << 2)
+                                 : stage + t * 1024 + c * 128 + ((((n >> 3) ^ c) & 3) << 5) + ((n & 7) << 2);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float lo, hi;
-      unpack2(o[j], lo, hi);
-      if (DT == kTcBf16) *reinterpret_cast<uint32_t *>(dst + (4 * i + j) * 2048) = pack_bf16x2(lo, hi);
-      else               *reinterpret_cast<float2 *>(dst + (4 * i + j) * 2048) = make_float2(round_tf32_rne(lo), round_tf32_rne(hi));
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t *b = d + 6 * i + 2 * t;
+      const uint64_t o[4] = {sub2(b[0], b[2]), add2(b[1], b[2]), sub2(b[2], b[1]), sub2(b[1], b[3])};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float lo, hi;
+        unpack2(o[j], lo, hi);
+        if (DT == kTcBf16) *reinterpret_cast<uint32_t *>(dst + (4 * i + j) * 2048) = pack_bf16x2(lo, hi);
+        else               *reinterpret_cast<float2 *>(dst + (4 * i + j) * 2048) = make_float2(round_tf32_rne(lo), round_tf32_rne(hi));
+      }
     }
   }
 }
 
-// Epilogue of one warp: 32 columns (its tensor-memory lanes; `q` is the quad of this lane's, `n` its image) x 16 filters
+// Epilogue of one warp: 32 columns (its tensor-memory lanes; images of one tile, of which this lane's is `n`) x 16 filters
 // (accumulator columns from `tcol`, filters from `k0`).  The same operations in the same order as tc_epilogue; every store is
 // 32 lanes of one output row.
 template <int W, class Release>
-__device__ __forceinline__ void img_epilogue(uint32_t tcol, bool active, const WinoParams &p, int k0, const ColumnQuad &q, int n,
+__device__ __forceinline__ void img_epilogue(uint32_t tcol, bool active, const WinoParams &p, int k0, int tx, int ty, int n,
                                              Release release) {
   float y[4][4][4];                                                  // [filter quad][output position][filter]
   read_accumulators<W>(tcol, active, y, release);
-  if (active && q.valid) {
-    const int oh0 = 2 * q.ty, ow0 = 2 * q.tx;
+  if (active && n < p.N) {
+    const int oh0 = 2 * ty, ow0 = 2 * tx;
     const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
     const size_t dW = (size_t)p.N, dH = (size_t)p.W * p.N, plane = (size_t)p.H * dH;
     float *dst = p.y + (size_t)k0 * plane + ((size_t)oh0 * p.W + ow0) * p.N + n;
@@ -112,47 +121,42 @@ __device__ __forceinline__ void img_epilogue(uint32_t tcol, bool active, const W
   }
 }
 
-// p.k_blocks counts 64-filter blocks, p.blocks blocks of 32 columns, p.total_tiles pair tiles (k_blocks times a quarter of
-// those).
+// p.k_blocks counts 64-filter blocks, p.tiles_w pairs of tile columns, p.blocks blocks of a pair of tiles and 32 images, p.total_tiles pair tiles
+// (k_blocks times half of those).
 template <int DT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ImgCfg<DT>::kThreads, 1)
 wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
   using Cfg = ImgCfg<DT>;
-  constexpr int SR = Cfg::kRawStages, SU = Cfg::kUStages, SV = Cfg::kVStages, KC = Cfg::kKC;
+  constexpr int S = Cfg::kStages, SU = Cfg::kUStages, KC = Cfg::kKC;
   extern __shared__ __align__(1024) uint8_t ismem[];
-  uint8_t *raw_s = ismem;
-  uint8_t *v_s = raw_s + SR * Cfg::kRawBytes;
-  uint8_t *u_s = v_s + SV * Cfg::kVBytes;
+  uint8_t *v_s = ismem;                                                // the stages: patches, then V
+  uint8_t *u_s = v_s + S * Cfg::kStageBytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(u_s + SU * Cfg::kUBytes);
-  uint64_t *raw_full = bars, *raw_empty = raw_full + SR, *u_full = raw_empty + SR, *u_empty = u_full + SU,
-           *v_ready = u_empty + SU, *v_empty = v_ready + SV;
-  uint64_t *acc_full = v_empty + SV, *mma_done = acc_full + 1, *acc_empty = acc_full + 3;   // mma_done[2], acc_empty[4]
+  uint64_t *raw_full = bars, *v_ready = raw_full + S, *v_empty = v_ready + S, *u_full = v_empty + S, *u_empty = u_full + SU;
+  uint64_t *acc_full = u_empty + SU, *mma_done = acc_full + 1, *acc_empty = acc_full + 3;   // mma_done[2], acc_empty[4]
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 7);
   volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 8);
   uint64_t *nowhere = acc_full + 9;                    // [4]: nobody waits for these; where a thread that gave up arrives
-  static_assert(SV <= 4 && (2 * SR + 2 * SU + 2 * SV + 13) * 8 <= 512, "barriers");
+  static_assert((3 * S + 2 * SU + 13) * 8 <= 512, "barriers");
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
   const uint32_t rank = cluster_ctarank();
   const int cid = (int)blockIdx.x >> 1, n_clusters = (int)gridDim.x >> 1;
   const int my_tiles = (p.total_tiles - cid + n_clusters - 1) / n_clusters;
-  const int quads = (p.blocks + 3) / 4;                // pair tiles per filter block
+  const int halves = (p.blocks + 1) / 2;               // pair tiles per filter block
   const int cpt = p.chunks_per_tile;
   const int total_steps = my_tiles * cpt;
 
   if (tid == 0) {
     *dead = 0;
-    for (int s = 0; s < SR; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(smem_u32(raw_full + s), 1);
-      mbar_init(smem_u32(raw_empty + s), Cfg::kBlockWarps);
+      mbar_init(smem_u32(v_ready + s), 2 * Cfg::kStepWarps);           // leader only: the transform warps of both CTAs
+      mbar_init(smem_u32(v_empty + s), 2);                             // one commit per issuing warp
     }
     for (int s = 0; s < SU; ++s) {
       mbar_init(smem_u32(u_full + s), 1);                              // leader only: its loader, with both CTAs' bytes
       mbar_init(smem_u32(u_empty + s), 2);                             // one commit per issuing warp
-    }
-    for (int s = 0; s < SV; ++s) {
-      mbar_init(smem_u32(v_ready + s), 2 * 8);       // leader only: the transform warps of both CTAs
-      mbar_init(smem_u32(v_empty + s), 2);
     }
     mbar_init(smem_u32(acc_full), 2);
     for (int j = 0; j < 4; ++j) mbar_init(smem_u32(acc_empty + j), 2 * kTcEpilogueWarps);   // leader only
@@ -177,63 +181,54 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     const uint32_t tcol = tmem_base + ((uint32_t)(quarter * 32) << 16) + 16 * sub;
     uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
     for (int seq = 0; seq < my_tiles; ++seq) {
-      const int t = cid + seq * n_clusters, kb = t / quads;
-      const int block = 4 * (t - kb * quads) + 2 * (int)rank + (quarter & 1);
-      const ColumnQuad q = column_quad(p, 8 * block + (lane >> 2));
+      const int t = cid + seq * n_clusters, kb = t / halves, block = 2 * (t - kb * halves) + (int)rank;
+      const TilePair at = tile_pair(p, block);
+      const int tx = at.tx + (quarter & 1);
       mbar_wait_reporting(smem_u32(acc_full), seq & 1, dead, p.status, acc_empty0, smem_u32(nowhere));
       tc_fence_after();
-      img_epilogue<Cfg::kEpilogueLoad>(tcol, block < p.blocks, p, kb * kImgFilters + 32 * (quarter >> 1) + 16 * sub, q, q.n + (lane & 3),
+      img_epilogue<Cfg::kEpilogueLoad>(tcol, block < p.blocks && 2 * tx < p.W, p, kb * kImgFilters + 32 * (quarter >> 1) + 16 * sub, tx, at.ty, at.n + lane,
                    [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
     }
   } else if (warp >= kPairFirstTransformWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kTransformRegs));
     // ===================================== input transform =====================================
-    const int t = (tid - 32 * kPairFirstTransformWarp) % (32 * Cfg::kBlockWarps), np = t & 15;   // column pair
+    const int t = (tid - 32 * kPairFirstTransformWarp) % (32 * Cfg::kStepWarps), np = t & 15;   // image pair
     // BF16: the two channels of a warp are four apart, so that their 64-byte halves of a row lie in different banks.
-    const int c = DT == kTcBf16 ? (t >> 5) + 4 * ((t >> 4) & 1) : t >> 4;
+    const int c = DT == kTcBf16 ? 8 * (t >> 7) + ((t >> 5) & 3) + 4 * ((t >> 4) & 1) : t >> 4;
     uint32_t v_ready0 = map_to_rank(smem_u32(v_ready), 0);
-    // Groups of kBlockWarps: one for each block of a K-step (TF32: of every other K-step).
-    const int group = (warp - kPairFirstTransformWarp) / Cfg::kBlockWarps, b = group & 1;
-    constexpr int kStepGroups = Cfg::kStepGroups;
-    for (int g = group >> 1; g < total_steps; g += kStepGroups) {
-      const int sv = g % SV, r = 2 * g + b, sr = r % SR;
-      const uint32_t use = g / SV;
-      mbar_wait_reporting(smem_u32(raw_full + sr), (r / SR) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
-      const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
-      uint8_t *vst = v_s + sv * Cfg::kVBytes;
-      const auto wait_for_stage = [&] {              // V stage free again
-        if (use > 0) mbar_wait_reporting(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
-      };
-      if (KC == 8) {
-        uint64_t d[16];
-        load_patch_pair(raw, c, np, d);
-        wait_for_stage();                            // (before the load: 36 -> 40 us on 128x128x64x28x28)
-        finish_v_wide<DT>(d, vst, b, c, np);
-      } else {
-        wait_for_stage();
-#pragma unroll 1                                     // (unrolled, the second patch's registers spill: 266 -> 277 us on 256x32x64x112x112)
-        for (int i = 0; i < KC; i += 8) {
-          uint64_t d[16];
-          load_patch_pair(raw, c + i, np, d);
-          finish_v_wide<DT>(d, vst, b, c + i, np);
-        }
-      }
-      fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
+    for (int g = (warp - kPairFirstTransformWarp) / Cfg::kStepWarps; g < total_steps; g += Cfg::kGroups) {
+      const int s = g % S;
+      mbar_wait_reporting(smem_u32(raw_full + s), (g / S) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
+      transform_tile_pair<DT>(v_s + s * Cfg::kStageBytes, c, np);
+      fence_proxy_async_smem();          // V is read by the tensor core through the async proxy, which writes the next patch here, too
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(smem_u32(raw_empty + sr));     // behind the fence: TMA refills the stage
-        mbar_arrive_cluster(v_ready0 + 8 * sv);
-      }
+      if (lane == 0) mbar_arrive_cluster(v_ready0 + 8 * s);
     }
     // the leader's commits arrive here until the end: do not leave before the last ones have
-    for (int i = total_steps > SV ? total_steps - SV : 0; i < total_steps; ++i)
-      mbar_wait(smem_u32(v_empty + i % SV), (i / SV) & 1, dead, p.status);
+    for (int i = total_steps > S ? total_steps - S : 0; i < total_steps; ++i)
+      mbar_wait(smem_u32(v_empty + i % S), (i / S) & 1, dead, p.status);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kIssueRegs));
     if (warp == 0) {
       // ===================================== patches =============================================
-        load_patches<KC, SR, 2>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,
-                           [&](int seq, int i) { return 4 * ((cid + seq * n_clusters) % quads) + 2 * (int)rank + i; });
+      if (elect_one()) tma_prefetch_descriptor(&tm_in);
+      int g = 0;
+      bool ok = true;
+      for (int seq = 0; seq < my_tiles && ok; ++seq) {
+        const TilePair at = tile_pair(p, 2 * ((cid + seq * n_clusters) % halves) + (int)rank);
+        for (int ci = 0; ci < cpt; ++ci, ++g) {
+          const int s = g % S;
+          const uint32_t use = g / S;
+          // A wait that gave up: stop issuing - the stage may still be in use.
+          if (use > 0 && !mbar_wait_warp(smem_u32(v_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
+          if (!elect_one()) continue;
+          mbar_arrive_expect_tx(smem_u32(raw_full + s), Cfg::kRawBytes);
+          // (A block past the last one: see load_patches.)
+          tma_load_4d(smem_u32(v_s + s * Cfg::kStageBytes), &tm_in, smem_u32(raw_full + s), at.n, ci * KC, 2 * at.tx - 1, 2 * at.ty - 1);
+        }
+      }
+      // No exit with bulk copies in flight (after a complete run these phases are long over).
+      for (int i = g > S ? g - S : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % S), (i / S) & 1);
     } else if (warp == 1) {
       // ===================================== filter slices =======================================
       {
@@ -242,7 +237,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
         int g = 0;
         bool ok = true;
         for (int seq = 0; seq < my_tiles && ok; ++seq) {
-          const int kb = (cid + seq * n_clusters) / quads;
+          const int kb = (cid + seq * n_clusters) / halves;
           for (int ci = 0; ci < cpt; ++ci, ++g) {
             const int s = g % SU;
             const uint32_t use = g / SU;
@@ -272,12 +267,12 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
         const uint64_t b_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(u_s), 512, 512, 4) : smem_desc(smem_u32(u_s), 1024, 512, 1);
         int ci = 0, seq = 0;
         for (int g = 0; g < total_steps; ++g) {
-          const int su = g % SU, sv = g % SV;
+          const int su = g % SU, sv = g % S;
           // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
           if (!mbar_wait_warp(smem_u32(u_full + su), (g / SU) & 1, dead, p.status)) break;
-          if (!mbar_wait_warp(smem_u32(v_ready + sv), (g / SV) & 1, dead, p.status)) break;
+          if (!mbar_wait_warp(smem_u32(v_ready + sv), (g / S) & 1, dead, p.status)) break;
           tc_fence_after();
-          const uint64_t ad = a_desc0 + (uint64_t)(sv * (Cfg::kVBytes >> 4)) + (uint64_t)(col0 * (2048 >> 4)),
+          const uint64_t ad = a_desc0 + (uint64_t)(sv * (Cfg::kStageBytes >> 4)) + (uint64_t)(col0 * (2048 >> 4)),
                          bd = b_desc0 + (uint64_t)(su * (Cfg::kUBytes >> 4)) + (uint64_t)(col0 * (1024 >> 4));
           const uint32_t accumulate = ci > 0 ? 1u : 0u, d0 = tmem_base + col0 * kTcN;
           bool ok = true;
