@@ -12,6 +12,7 @@
 #include "../../include/opencnn_b200.h"
 #include "fx.cuh"
 #include "layout.cuh"
+#include "launch.cuh"
 #include "wino_fp32.cuh"
 #include "wino_tc.cuh"
 #include "wino_pair.cuh"
@@ -191,29 +192,6 @@ cudaError_t check_shape(int N, int C, int H, int W, int K, ShapeRule rule) {
   return cudaSuccess;
 }
 
-// Launches a kernel that reads the transformed filter.  `after_fx`: the filter transform was the launch before it on this
-// stream, by this call, so its set-up (barriers, tensor memory, descriptors, the first patches) may overlap it; the
-// kernels wait for the transform's completion before their first load of U, and all other data is older than the
-// transform, which itself is launched the ordinary way.  Whole calls: fp32 32x16x64x9x9 12.3 -> 10.2 us,
-// 32x64x64x56x56 81.9 -> 79.7; TF32 128x128x128x28x28 63.0 -> 59.8 - with calls queued one behind the other.  On an idle
-// stream the transform is over before the host has encoded the tensor maps and launched the second kernel, and a small call
-// takes what it took: 9x9 27.1 -> 27.0 us from the call to the end of a synchronise.
-template <class... P, class... A>
-cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, bool after_fx, const A &...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = after_fx ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-  return cudaGetLastError();
-}
-
 // Tensor map of the input for the 4x4 patches of 32 images and `channels` channels.
 bool encode_patches(EncodeTiledFn enc, CUtensorMap *map, const float *input, int N, int C, int H, int W, int channels) {
   cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)C};
@@ -252,16 +230,46 @@ bool encode_filter(EncodeTiledFn enc, CUtensorMap *map, const float *workspace, 
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-cudaError_t launch_fx(const float *filter, float *workspace, int C, int K, cudaStream_t stream) {
+// `early`: see launch_early.
+cudaError_t transform_filter(const float *filter, float *workspace, int C, int K, int precision, cudaStream_t stream, bool early = false) {
   const int k4 = K / 4;
-  const int total = C * k4;
-  ocb::fx_kernel<<<(total + 127) / 128, 128, 0, stream>>>(reinterpret_cast<const float4 *>(filter),
-                                                        reinterpret_cast<float4 *>(workspace), C, k4);
-  return cudaGetLastError();
+  const unsigned blocks = ((unsigned)C * k4 + ocb::kFxThreads - 1) / ocb::kFxThreads;
+  const auto launch = [&](auto kernel, auto u) {
+    return ocb::launch(kernel, blocks, dim3(ocb::kFxThreads), 0, stream, early, reinterpret_cast<const float4 *>(filter), u, C, k4);
+  };
+  if (precision == OPENCNN_BF16) return launch(ocb::fx_tc_kernel<ocb::kTcBf16>, static_cast<void *>(workspace));
+  if (precision == OPENCNN_TF32) return launch(ocb::fx_tc_kernel<ocb::kTcTf32>, static_cast<void *>(workspace));
+  return launch(ocb::fx_kernel, reinterpret_cast<float4 *>(workspace));
 }
 
-cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *output, int N, int C, int H,
-                             int W, int K, cudaStream_t stream, bool after_fx, TileRows rows) {
+// The filter of a call: as it is, to be transformed into `workspace`, or null where the workspace holds it transformed already.
+struct Filter {
+  const float *filter;
+  float *workspace;
+  int precision;
+};
+
+// Launches the filter's transform, if there is one, and the kernel that reads it, which may start early: it sets itself up meanwhile, waits for
+// the transform before it loads U, and without one waits for the kernel before it on the stream before it loads its patches.  (The transform's
+// blocks let it start only when all that came before them is complete, so that the patches, which are older, need not wait for the transform.)
+// The transform itself starts early where its blocks, four to an SM, find room beside a kernel like this call's, which in a stream of such
+// calls is what runs before it: 32x16x64x9x9 8.2 -> 6.3 us a call, TF32 32x128x128x14x14 14.4 -> 12.2.  Where there is no room for them, they would
+// come to the SMs one by one as that kernel ends, and this call's kernel after them: fp32 32x64x64x56x56 79.3 -> 81.9 us, TF32 128x128x128x28x28
+// 55.1 -> 58.2.
+template <class... P>
+cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, const Filter &filter, int sms,
+                        const CUtensorMap &tm_in, const CUtensorMap &tm_u, ocb::WinoParams p) {
+  if (filter.filter) {
+    const long long blocks = ((long long)p.C * p.K / 4 + ocb::kFxThreads - 1) / ocb::kFxThreads;
+    const cudaError_t e = transform_filter(filter.filter, filter.workspace, p.C, p.K, filter.precision, stream, blocks <= 4ll * (sms - grid));
+    if (e != cudaSuccess) return e;
+  }
+  p.input_ready = filter.filter != nullptr;
+  return ocb::launch(kernel, (unsigned)grid, dim3((unsigned)threads), smem, stream, true, tm_in, tm_u, p);
+}
+
+cudaError_t launch_wino_fp32(const float *input, float *output, int N, int C, int H,
+                             int W, int K, cudaStream_t stream, const Filter &filter, TileRows rows) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -275,7 +283,7 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
     cuuint64_t strides[2] = {(cuuint64_t)K * 4, (cuuint64_t)K * 16 * 4};
     cuuint32_t box[3] = {(cuuint32_t)ocb::kBK, 16, (cuuint32_t)ocb::kBC};
     cuuint32_t estr[3] = {1, 1, 1};
-    if (enc(&tm_u, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(workspace), dims, strides, box, estr,
+    if (enc(&tm_u, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, filter.workspace, dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cudaErrorInvalidValue;
@@ -307,7 +315,7 @@ cudaError_t launch_wino_fp32(const float *input, const float *workspace, float *
   const auto kernel = packed   ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>
                       : ragged ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>
                                : ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>;
-  return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, after_fx, tm_in, tm_u, p);
+  return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
 }
 
 bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K, TileRows rows,
@@ -324,18 +332,9 @@ bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, i
   return c.blocks <= 0x7fffffffll / 16;
 }
 
-// Tensor-core path: filter transform rounded to the operand type, then the tcgen05 kernel.
 template <int DT>
-cudaError_t launch_fx_tc(const float *filter, float *workspace, int C, int K, cudaStream_t stream) {
-  const int k4 = K / 4;
-  const int total = C * k4;
-  ocb::fx_tc_kernel<DT><<<(total + 127) / 128, 128, 0, stream>>>(reinterpret_cast<const float4 *>(filter), workspace, C, k4);
-  return cudaGetLastError();
-}
-
-template <int DT>
-cudaError_t launch_wino_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                           int K, cudaStream_t stream, bool after_fx, TileRows rows, bool packed) {
+cudaError_t launch_wino_tc(const float *input, float *output, int N, int C, int H, int W,
+                           int K, cudaStream_t stream, const Filter &filter, TileRows rows, bool packed) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -348,7 +347,7 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   CUtensorMap tm_in, tm_u;
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   // BF16 with at most 64 filters: only the first 64-filter row block is loaded (wino_tc.cuh, "half U")
-  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 && K <= 64 ? 1 : ocb::kTcM * esz / 128)) return cudaErrorInvalidValue;
+  if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, 128, bf16 && K <= 64 ? 1 : ocb::kTcM * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, packed)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
@@ -363,16 +362,16 @@ cudaError_t launch_wino_tc(const float *input, const float *workspace, float *ou
   if constexpr (bf16) {
     if (K <= 64)
       return launch_main(packed ? ocb::wino_tc_kernel<DT, true, true> : ocb::wino_tc_kernel<DT, true>, grid, threads, ocb::TcCfg<DT, true>::kSmemBytes, stream,
-                         after_fx, tm_in, tm_u, p);
+                         filter, st->sm_count, tm_in, tm_u, p);
   }
-  return launch_main(packed ? ocb::wino_tc_kernel<DT, false, true> : ocb::wino_tc_kernel<DT>, grid, threads, ocb::TcCfg<DT>::kSmemBytes, stream, after_fx,
-                     tm_in, tm_u, p);
+  return launch_main(packed ? ocb::wino_tc_kernel<DT, false, true> : ocb::wino_tc_kernel<DT>, grid, threads, ocb::TcCfg<DT>::kSmemBytes, stream, filter,
+                     st->sm_count, tm_in, tm_u, p);
 }
 
 // CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).
 template <int DT>
-cudaError_t launch_wino_pair(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                            int K, cudaStream_t stream, bool after_fx, TileRows rows) {
+cudaError_t launch_wino_pair(const float *input, float *output, int N, int C, int H, int W,
+                            int K, cudaStream_t stream, const Filter &filter, TileRows rows) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -386,7 +385,7 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
 
   CUtensorMap tm_in, tm_u;
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
-  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, ocb::kPairFilters * esz / 128)) return cudaErrorInvalidValue;
+  if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, 128, ocb::kPairFilters * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
   p.k_blocks = (K + ocb::kTcM - 1) / ocb::kTcM;
@@ -397,13 +396,13 @@ cudaError_t launch_wino_pair(const float *input, const float *workspace, float *
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  return launch_main(ocb::wino_pair_kernel<DT>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+  return launch_main(ocb::wino_pair_kernel<DT>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
 }
 
 // Image columns in the accumulator rows: 64 filters x four blocks of 32 columns per cluster of two (wino_img.cuh).
 template <int DT>
-cudaError_t launch_wino_img(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                            int K, cudaStream_t stream, bool after_fx, TileRows rows) {
+cudaError_t launch_wino_img(const float *input, float *output, int N, int C, int H, int W,
+                            int K, cudaStream_t stream, const Filter &filter, TileRows rows) {
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
   if (e != cudaSuccess) return e;
@@ -415,7 +414,7 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   if (max_clusters <= 0) return cudaErrorNotSupported;
   CUtensorMap tm_in, tm_u;
   if (!encode_tile_pairs(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
-  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
+  if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
   const long long blocks = tile_pair_blocks(N, rows, W);
@@ -431,13 +430,13 @@ cudaError_t launch_wino_img(const float *input, const float *workspace, float *o
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  return launch_main(ocb::wino_img_kernel<DT>, 2 * clusters, ocb::ImgCfg<DT>::kThreads, ocb::ImgCfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+  return launch_main(ocb::wino_img_kernel<DT>, 2 * clusters, ocb::ImgCfg<DT>::kThreads, ocb::ImgCfg<DT>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
 }
 
 // Layers with at most 64 filters: two 32-image blocks share the 128 accumulator rows (wino_tc64.cuh).
 template <int DT>
-cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *output, int N, int C, int H, int W,
-                             int K, cudaStream_t stream, bool after_fx, TileRows rows) {
+cudaError_t launch_wino_tc64(const float *input, float *output, int N, int C, int H, int W,
+                             int K, cudaStream_t stream, const Filter &filter, TileRows rows) {
   if (K > 64) return cudaErrorInvalidValue;
   DeviceState *st = nullptr;
   cudaError_t e = device_state(&st);
@@ -450,7 +449,7 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
   // BF16: one row block of 64 filters.  TF32: a box of four row blocks of 32 filters, of which two exist -
   // the hardware fills the other two with zeros, which the kernel uses as the empty half of its A operand.
-  if (!encode_filter<DT>(enc, &tm_u, workspace, C, K, 128, bf16 ? 1 : 4)) return cudaErrorInvalidValue;
+  if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, 128, bf16 ? 1 : 4)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
   p.k_blocks = 1;
@@ -459,12 +458,12 @@ cudaError_t launch_wino_tc64(const float *input, const float *workspace, float *
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
-  return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, after_fx, tm_in, tm_u, p);
+  return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
 }
 
 template <int DT>
-cudaError_t launch_tc(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K,
-                      cudaStream_t stream, bool after_fx, TileRows rows, int kernel = OPENCNN_TC_AUTO) {
+cudaError_t launch_tc(const float *input, float *output, int N, int C, int H, int W, int K,
+                      cudaStream_t stream, const Filter &filter, TileRows rows, int kernel = OPENCNN_TC_AUTO) {
   bool packed = false;
   if (kernel == OPENCNN_TC_AUTO) {
     DeviceState *st = nullptr;
@@ -476,13 +475,22 @@ cudaError_t launch_tc(const float *input, const float *workspace, float *output,
     packed = choice.packed;
   }
   switch (kernel) {
-    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows, packed);
-    case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows);
-    case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows);
-    case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, workspace, output, N, C, H, W, K, stream, after_fx, rows);
+    case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, output, N, C, H, W, K, stream, filter, rows, packed);
+    case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, output, N, C, H, W, K, stream, filter, rows);
+    case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, output, N, C, H, W, K, stream, filter, rows);
+    case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, output, N, C, H, W, K, stream, filter, rows);
     default: return cudaErrorInvalidValue;
   }
 }
+
+cudaError_t convolve(const float *input, const Filter &filter, float *output, int N, int C, int H, int W, int K, cudaStream_t stream, TileRows rows,
+                     int kernel = OPENCNN_TC_AUTO) {
+  if (filter.precision == OPENCNN_BF16) return launch_tc<ocb::kTcBf16>(input, output, N, C, H, W, K, stream, filter, rows, kernel);
+  if (filter.precision == OPENCNN_TF32) return launch_tc<ocb::kTcTf32>(input, output, N, C, H, W, K, stream, filter, rows, kernel);
+  return launch_wino_fp32(input, output, N, C, H, W, K, stream, filter, rows);
+}
+// A workspace that is only read: its filter is transformed already.
+Filter transformed(const float *workspace, int precision) { return {nullptr, const_cast<float *>(workspace), precision}; }
 
 cudaError_t forward(const float *input, const float *filter, float *output, float *workspace, int N, int C, int H,
                     int W, int K, int precision, cudaStream_t stream, ShapeRule rule) {
@@ -492,20 +500,7 @@ cudaError_t forward(const float *input, const float *filter, float *output, floa
   if (!output_aligned(output, precision)) return cudaErrorInvalidValue;
   cudaError_t e = check_shape(N, C, H, W, K, rule);
   if (e != cudaSuccess) return e;
-  if (precision == OPENCNN_BF16) {
-    e = launch_fx_tc<ocb::kTcBf16>(filter, workspace, C, K, stream);
-    if (e != cudaSuccess) return e;
-    return launch_tc<ocb::kTcBf16>(input, workspace, output, N, C, H, W, K, stream, true, all_rows(H));
-  }
-  if (precision == OPENCNN_TF32) {
-    e = launch_fx_tc<ocb::kTcTf32>(filter, workspace, C, K, stream);
-    if (e != cudaSuccess) return e;
-    return launch_tc<ocb::kTcTf32>(input, workspace, output, N, C, H, W, K, stream, true, all_rows(H));
-  }
-  if (precision != OPENCNN_FP32) return cudaErrorInvalidValue;
-  e = launch_fx(filter, workspace, C, K, stream);
-  if (e != cudaSuccess) return e;
-  return launch_wino_fp32(input, workspace, output, N, C, H, W, K, stream, true, all_rows(H));
+  return convolve(input, {filter, workspace, precision}, output, N, C, H, W, K, stream, all_rows(H));
 }
 
 // Scratch for opencnn_convolutionForward_noalloc: the transformed filter, [C][16][K] floats, for
@@ -536,18 +531,9 @@ cudaError_t noalloc_workspace(float **out) {
   return st.error;
 }
 
-cudaError_t transform_filter(const float *filter, float *workspace, int C, int K, int precision, cudaStream_t stream) {
-  if (precision == OPENCNN_BF16) return launch_fx_tc<ocb::kTcBf16>(filter, workspace, C, K, stream);
-  if (precision == OPENCNN_TF32) return launch_fx_tc<ocb::kTcTf32>(filter, workspace, C, K, stream);
-  return launch_fx(filter, workspace, C, K, stream);
-}
-
 cudaError_t convolve_rows(const float *input, const float *workspace, float *output, int N, int C, int H, int W, int K, int precision,
                           cudaStream_t stream, TileRows rows) {
-  const auto run = [&](auto launch) { return launch(input, workspace, output, N, C, H, W, K, stream, false, rows); };
-  if (precision == OPENCNN_BF16) return run([](auto... a) { return launch_tc<ocb::kTcBf16>(a...); });
-  if (precision == OPENCNN_TF32) return run([](auto... a) { return launch_tc<ocb::kTcTf32>(a...); });
-  return run([](auto... a) { return launch_wino_fp32(a...); });
+  return convolve(input, transformed(workspace, precision), output, N, C, H, W, K, stream, rows);
 }
 
 }  // namespace
@@ -590,10 +576,8 @@ int opencnn_filter_transform_p(const float *filter, float *workspace, int in_c, 
                                opencnn_stream_t stream) {
   if (!filter || !workspace || !aligned16(filter) || !aligned16(workspace)) return (int)cudaErrorInvalidValue;
   if (in_c <= 0 || filt_k <= 0 || filt_k % 4) return (int)cudaErrorInvalidValue;
-  if (precision == OPENCNN_BF16) return (int)launch_fx_tc<ocb::kTcBf16>(filter, workspace, in_c, filt_k, (cudaStream_t)stream);
-  if (precision == OPENCNN_TF32) return (int)launch_fx_tc<ocb::kTcTf32>(filter, workspace, in_c, filt_k, (cudaStream_t)stream);
-  if (precision != OPENCNN_FP32) return (int)cudaErrorInvalidValue;
-  return (int)launch_fx(filter, workspace, in_c, filt_k, (cudaStream_t)stream);
+  if (precision != OPENCNN_FP32 && precision != OPENCNN_TF32 && precision != OPENCNN_BF16) return (int)cudaErrorInvalidValue;
+  return (int)transform_filter(filter, workspace, in_c, filt_k, precision, (cudaStream_t)stream);
 }
 
 int opencnn_winograd_forward(const float *input, const float *workspace, float *output, int in_n, int in_c,
@@ -604,12 +588,7 @@ int opencnn_winograd_forward(const float *input, const float *workspace, float *
   if (!output_aligned(output, precision)) return (int)cudaErrorInvalidValue;
   cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
   if (e != cudaSuccess) return (int)e;
-  if (precision == OPENCNN_BF16)
-    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h));
-  if (precision == OPENCNN_TF32)
-    return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h));
-  if (precision != OPENCNN_FP32) return (int)cudaErrorInvalidValue;
-  return (int)launch_wino_fp32(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h));
+  return (int)convolve(input, transformed(workspace, precision), output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, all_rows(in_h));
 }
 
 int opencnn_winograd_forward_kernel(const float *input, const float *workspace, float *output, int in_n, int in_c,
@@ -620,9 +599,7 @@ int opencnn_winograd_forward_kernel(const float *input, const float *workspace, 
   if (!output_aligned(output, precision)) return (int)cudaErrorInvalidValue;
   cudaError_t e = check_shape(in_n, in_c, in_h, in_w, filt_k, shape_rule(precision));
   if (e != cudaSuccess) return (int)e;
-  if (precision == OPENCNN_BF16)
-    return (int)launch_tc<ocb::kTcBf16>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h), kernel);
-  return (int)launch_tc<ocb::kTcTf32>(input, workspace, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, false, all_rows(in_h), kernel);
+  return (int)convolve(input, transformed(workspace, precision), output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, all_rows(in_h), kernel);
 }
 
 int opencnn_convolutionForward_noalloc(const float *input, const float *filter, float *output, int in_n,
@@ -641,9 +618,7 @@ int opencnn_convolutionForward_noalloc(const float *input, const float *filter, 
   float *ws = nullptr;
   e = noalloc_workspace(&ws);
   if (e != cudaSuccess) return (int)e;
-  e = launch_fx(filter, ws, in_c, filt_k, (cudaStream_t)stream);
-  if (e != cudaSuccess) return (int)e;
-  return (int)launch_wino_fp32(input, ws, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, true, all_rows(in_h));
+  return (int)convolve(input, {filter, ws, OPENCNN_FP32}, output, in_n, in_c, in_h, in_w, filt_k, (cudaStream_t)stream, all_rows(in_h));
 }
 
 int opencnn_nchw_to_chwn(const float *src, float *dst, int n, int c, int h, int w, opencnn_stream_t stream) {

@@ -12,6 +12,8 @@
 
 namespace ocb {
 
+constexpr int kFxThreads = 128;             // per block of both filter transforms, a thread four filters of one channel
+
 __device__ __forceinline__ float fx_half_sum(float a, float c, float b) {
   return __fmul_rn(0.5f, __fadd_rn(__fadd_rn(a, c), b));
 }
@@ -39,8 +41,9 @@ __device__ __forceinline__ void fx_one(const float (&w)[9], float (&u)[16]) {
 }
 
 // grid: ceil(C*K/4 / 128) blocks of 128 threads.  k4 = K/4.
-__global__ void __launch_bounds__(128) fx_kernel(const float4 *__restrict__ g, float4 *__restrict__ U, int C, int k4) {
-  grid_launch_dependents();                // the kernel that reads U may set itself up meanwhile
+__global__ void __launch_bounds__(kFxThreads) fx_kernel(const float4 *__restrict__ g, float4 *__restrict__ U, int C, int k4) {
+  grid_dependency_wait();                  // the filter may be new, and U still in use
+  grid_launch_dependents();                // the kernel that reads U may set itself up meanwhile, and read its input, which is older
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= C * k4) return;
   const int c = idx / k4, kq = idx - c * k4;

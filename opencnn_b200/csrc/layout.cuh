@@ -15,12 +15,17 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "launch.cuh"
+#include "ptx.cuh"
+
 namespace ocb {
 
 // dst[c][r] = src[r][c] for a rows x cols matrix.  1-D grid of 32x32 tiles (column tiles fastest), block (32, 8).
 __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict__ src, float *__restrict__ dst,
                                                        long long rows, long long cols, long long tiles_x) {
   __shared__ float tile[32][33];
+  grid_dependency_wait();
+  grid_launch_dependents();
   const long long t = blockIdx.x;
   const long long c0 = (t % tiles_x) * 32, r0 = (t / tiles_x) * 32;
 #pragma unroll
@@ -43,6 +48,8 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict_
 __global__ void __launch_bounds__(256) transpose4_kernel(const float *__restrict__ src, float *__restrict__ dst,
                                                         long long rows, long long cols, long long tiles_x) {
   __shared__ float tile[64][65];
+  grid_dependency_wait();
+  grid_launch_dependents();
   const long long t = blockIdx.x;
   const long long c0 = (t % tiles_x) * 64, r0 = (t / tiles_x) * 64;
   const int a = threadIdx.x >> 4, b4 = (threadIdx.x & 15) * 4;
@@ -73,9 +80,8 @@ inline cudaError_t launch_transpose(const float *src, float *dst, long long rows
   const long long edge = vec ? 64 : 32;
   const long long gx = (cols + edge - 1) / edge, gy = (rows + edge - 1) / edge;
   if (gx * gy > 2147483647ll) return cudaErrorInvalidValue;
-  if (vec) transpose4_kernel<<<(unsigned)(gx * gy), 256, 0, stream>>>(src, dst, rows, cols, gx);
-  else     transpose_kernel<<<(unsigned)(gx * gy), dim3(32, 8), 0, stream>>>(src, dst, rows, cols, gx);
-  return cudaGetLastError();
+  if (vec) return launch(transpose4_kernel, (unsigned)(gx * gy), dim3(256), 0, stream, true, src, dst, rows, cols, gx);
+  return launch(transpose_kernel, (unsigned)(gx * gy), dim3(32, 8), 0, stream, true, src, dst, rows, cols, gx);
 }
 
 }  // namespace ocb

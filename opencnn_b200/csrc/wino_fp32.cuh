@@ -89,6 +89,7 @@ struct WinoParams {
   int ty0;             // first tile row (tiles_h of them are computed)
   int blocks;          // 32-column blocks of all tiles: n_blocks * tiles_w * tiles_h, or the packed count (see ColumnQuad)
   int *status;         // device status word
+  bool input_ready;    // the input may be read at once; else only after the kernels before this one (see launch)
 };
 
 struct TileCoord { int nb, tx, ty, kb; };
@@ -457,6 +458,7 @@ __device__ __forceinline__ void load_packed(const WinoParams &p, const CUtensorM
     tma_prefetch_descriptor(tm_in);
     tma_prefetch_descriptor(tm_u);
   }
+  if (!p.input_ready) grid_dependency_wait();
   int g = 0;
   bool ok = true;
   for (int seq = 0; seq < my_tiles && ok; ++seq) {
@@ -501,6 +503,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   uint64_t *bar_full = bars, *bar_ready = bars + S, *bar_empty = bars + 2 * S;   // per stage
   volatile int *dead = reinterpret_cast<volatile int *>(bars + 3 * S);
 
+  grid_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int my_tiles = (p.total_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // work items
   const int cpt = p.chunks_per_tile;
@@ -529,6 +532,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
           tma_prefetch_descriptor(&tm_in);
           tma_prefetch_descriptor(&tm_u);
         }
+        if (!p.input_ready) grid_dependency_wait();
         int seq = 0, ci = 0, groups_unused, issued = 0;
         TileCoord tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x, groups_unused));
         for (int g = 0; g < total_chunks; ++g) {

@@ -139,6 +139,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
   uint64_t *nowhere = acc_full + 9;                    // [4]: nobody waits for these; where a thread that gave up arrives
   static_assert((3 * S + 2 * SU + 13) * 8 <= 512, "barriers");
 
+  grid_launch_dependents();
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
   const uint32_t rank = cluster_ctarank();
   const int cid = (int)blockIdx.x >> 1, n_clusters = (int)gridDim.x >> 1;
@@ -212,6 +213,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     if (warp == 0) {
       // ===================================== patches =============================================
       if (elect_one()) tma_prefetch_descriptor(&tm_in);
+      if (!p.input_ready) grid_dependency_wait();
       int g = 0;
       bool ok = true;
       for (int seq = 0; seq < my_tiles && ok; ++seq) {

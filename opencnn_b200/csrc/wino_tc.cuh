@@ -154,7 +154,8 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // Same arithmetic as fx_kernel, then one rounding to the operand type.  Output [C][16][K]:
 // BF16 packed, or fp32 words holding TF32 values (low 13 mantissa bits zero).
 template <int DT>
-__global__ void __launch_bounds__(128) fx_tc_kernel(const float4 *__restrict__ g, void *__restrict__ U, int C, int k4) {
+__global__ void __launch_bounds__(kFxThreads) fx_tc_kernel(const float4 *__restrict__ g, void *__restrict__ U, int C, int k4) {
+  grid_dependency_wait();                  // the filter may be new, and U still in use
   grid_launch_dependents();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= C * k4) return;
@@ -419,6 +420,7 @@ __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensor
   static_assert(PER_STEP == 1 || PER_STEP == 2, "blocks of a K-step");
   const int cpt = p.chunks_per_tile;
   if (elect_one()) tma_prefetch_descriptor(tm_in);
+  if (!p.input_ready) grid_dependency_wait();
   int g = 0;
   bool ok = true;
   for (int seq = 0; seq < my_tiles && ok; ++seq) {
@@ -448,6 +450,7 @@ __device__ __forceinline__ void load_packed_patches(const WinoParams &p, const C
   constexpr uint32_t kBytes = KC * 16 * kTcN * 4;
   const int lane = threadIdx.x & 31;
   if (lane == 0) tma_prefetch_descriptor(tm_in);
+  if (!p.input_ready) grid_dependency_wait();
   int g = 0;
   bool ok = true;
   for (int seq = 0; seq < my_tiles && ok; ++seq) {
@@ -486,6 +489,7 @@ wino_tc_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant_
   volatile int *dead = reinterpret_cast<volatile int *>(u_full + 9);
   uint64_t *mma_done = u_full + 10;                    // one per MMA-issuing thread: "all my MMAs have completed"
 
+  grid_launch_dependents();
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
   const int my_tiles = (p.total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int cpt = p.chunks_per_tile;
