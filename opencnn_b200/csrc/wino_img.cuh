@@ -34,8 +34,8 @@ template <int DT> struct ImgCfg {
   static constexpr uint32_t kUBytes = 16 * 1024;                           // 16 positions x (32 filters x one K-step)
   static constexpr uint32_t kVBytes = 16 * 2048;                           // 16 positions x (64 columns x one K-step)
   static constexpr uint32_t kStageBytes = kRawBytes > kVBytes ? kRawBytes : kVBytes;
-  static constexpr int kStages = DT == kTcBf16 ? 4 : 6;
-  static constexpr int kUStages = 2;
+  static constexpr int kStages = DT == kTcBf16 ? 4 : 5;
+  static constexpr int kUStages = DT == kTcBf16 ? 2 : 4;
   // Transform warps: a thread takes the two tiles of one channel and image pair.  BF16 (16 channels): all eight share a K-step; TF32 (8 channels):
   // two groups of four take the K-steps in turn.
   static constexpr int kTransformWarps = 8, kStepWarps = kKC / 2, kFirstEpilogueWarp = kPairFirstTransformWarp + kTransformWarps;
@@ -46,9 +46,9 @@ template <int DT> struct ImgCfg {
                 "setmaxnreg budgets exceed the registers the CTA was launched with");
   static constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + (size_t)kUStages * kUBytes + 512;
   static_assert(kSmemBytes <= 232448, "shared memory");
-  // Transform groups that take K-steps in turn.  A group has to come back to the same stages (see PairCfg::kGroups).
-  static constexpr int kGroups = kTransformWarps / kStepWarps;
-  static_assert(kStages % kGroups == 0, "the ring's depth is a multiple of the group count");
+  // Transform groups that take K-steps in turn.  "Patch landed" has a barrier for each of kStages * kGroups steps: on one that a group shared with
+  // another it could wait two phases ahead of the other, which the parity does not tell from the phase before.
+  static constexpr int kGroups = kTransformWarps / kStepWarps, kFullBars = kStages * kGroups;
 };
 constexpr int kImgFilters = 64;                  // per tile
 
@@ -132,12 +132,14 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
   uint8_t *v_s = ismem;                                                // the stages: patches, then V
   uint8_t *u_s = v_s + S * Cfg::kStageBytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(u_s + SU * Cfg::kUBytes);
-  uint64_t *raw_full = bars, *v_ready = raw_full + S, *v_empty = v_ready + S, *u_full = v_empty + S, *u_empty = u_full + SU;
+  constexpr int SF = Cfg::kFullBars;
+  uint64_t *raw_full = bars, *v_ready = raw_full + SF, *v_empty = v_ready + S, *u_full = v_empty + S, *u_empty = u_full + SU;
   uint64_t *acc_full = u_empty + SU, *mma_done = acc_full + 1, *acc_empty = acc_full + 3;   // mma_done[2], acc_empty[4]
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 7);
   volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 8);
-  uint64_t *nowhere = acc_full + 9;                    // [4]: nobody waits for these; where a thread that gave up arrives
-  static_assert((3 * S + 2 * SU + 13) * 8 <= 512, "barriers");
+  constexpr int kNowhere = S > 4 ? S : 4;
+  uint64_t *nowhere = acc_full + 9;                    // [kNowhere]: nobody waits for these; where a thread that gave up arrives
+  static_assert((SF + 2 * S + 2 * SU + 9 + kNowhere) * 8 <= 512, "barriers");
 
   grid_launch_dependents();
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
@@ -147,21 +149,22 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
   const int halves = (p.blocks + 1) / 2;               // pair tiles per filter block
   const int cpt = p.chunks_per_tile;
   const int total_steps = my_tiles * cpt;
+  const bool u_stays = p.k_blocks == 1 && cpt <= SU;   // all tiles need the same few filter slices, which are loaded once
 
   if (tid == 0) {
     *dead = 0;
     for (int s = 0; s < S; ++s) {
-      mbar_init(smem_u32(raw_full + s), 1);
       mbar_init(smem_u32(v_ready + s), 2 * Cfg::kStepWarps);           // leader only: the transform warps of both CTAs
       mbar_init(smem_u32(v_empty + s), 2);                             // one commit per issuing warp
     }
+    for (int s = 0; s < SF; ++s) mbar_init(smem_u32(raw_full + s), 1);
     for (int s = 0; s < SU; ++s) {
       mbar_init(smem_u32(u_full + s), 1);                              // leader only: its loader, with both CTAs' bytes
       mbar_init(smem_u32(u_empty + s), 2);                             // one commit per issuing warp
     }
     mbar_init(smem_u32(acc_full), 2);
     for (int j = 0; j < 4; ++j) mbar_init(smem_u32(acc_empty + j), 2 * kTcEpilogueWarps);   // leader only
-    for (int j = 0; j < 4; ++j) mbar_init(smem_u32(nowhere + j), 1);
+    for (int j = 0; j < kNowhere; ++j) mbar_init(smem_u32(nowhere + j), 1);
     mbar_init(smem_u32(mma_done + 0), 1);
     mbar_init(smem_u32(mma_done + 1), 1);
     mbar_fence_init();
@@ -199,7 +202,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     uint32_t v_ready0 = map_to_rank(smem_u32(v_ready), 0);
     for (int g = (warp - kPairFirstTransformWarp) / Cfg::kStepWarps; g < total_steps; g += Cfg::kGroups) {
       const int s = g % S;
-      mbar_wait_reporting(smem_u32(raw_full + s), (g / S) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
+      mbar_wait_reporting(smem_u32(raw_full + g % SF), (g / SF) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
       transform_tile_pair<DT>(v_s + s * Cfg::kStageBytes, c, np);
       fence_proxy_async_smem();          // V is read by the tensor core through the async proxy, which writes the next patch here, too
       __syncwarp();
@@ -224,13 +227,13 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
           // A wait that gave up: stop issuing - the stage may still be in use.
           if (use > 0 && !mbar_wait_warp(smem_u32(v_empty + s), (use - 1) & 1, dead, p.status)) { ok = false; break; }
           if (!elect_one()) continue;
-          mbar_arrive_expect_tx(smem_u32(raw_full + s), Cfg::kRawBytes);
+          mbar_arrive_expect_tx(smem_u32(raw_full + g % SF), Cfg::kRawBytes);
           // (A block past the last one: see load_patches.)
-          tma_load_4d(smem_u32(v_s + s * Cfg::kStageBytes), &tm_in, smem_u32(raw_full + s), at.n, ci * KC, 2 * at.tx - 1, 2 * at.ty - 1);
+          tma_load_4d(smem_u32(v_s + s * Cfg::kStageBytes), &tm_in, smem_u32(raw_full + g % SF), at.n, ci * KC, 2 * at.tx - 1, 2 * at.ty - 1);
         }
       }
       // No exit with bulk copies in flight (after a complete run these phases are long over).
-      for (int i = g > S ? g - S : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % S), (i / S) & 1);
+      for (int i = g > S ? g - S : 0; i < g; ++i) mbar_wait_drain(smem_u32(raw_full + i % SF), (i / SF) & 1);
     } else if (warp == 1) {
       // ===================================== filter slices =======================================
       {
@@ -238,7 +241,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
         grid_dependency_wait();   // U is all that the kernel before this one writes
         int g = 0;
         bool ok = true;
-        for (int seq = 0; seq < my_tiles && ok; ++seq) {
+        for (int seq = 0; seq < (u_stays ? 1 : my_tiles) && ok; ++seq) {
           const int kb = (cid + seq * n_clusters) / halves;
           for (int ci = 0; ci < cpt; ++ci, ++g) {
             const int s = g % SU;
@@ -252,7 +255,8 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
           }
         }
         // The slices land before the MMAs that read them, whose completion is what these phases stand for.  (After a
-        // give-up nothing completes them: their limit, in both CTAs of the pair, is the time the copies get to land.)
+        // give-up nothing completes them: their limit, in both CTAs of the pair, is the time the copies get to land.  Slices that
+        // stay are given back once, by the last tile.)
         for (int i = g > SU ? g - SU : 0; i < g; ++i) mbar_wait_drain(smem_u32(u_empty + i % SU), (i / SU) & 1);
       }
     } else {
@@ -269,9 +273,9 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
         const uint64_t b_desc0 = DT == kTcBf16 ? smem_desc(smem_u32(u_s), 512, 512, 4) : smem_desc(smem_u32(u_s), 1024, 512, 1);
         int ci = 0, seq = 0;
         for (int g = 0; g < total_steps; ++g) {
-          const int su = g % SU, sv = g % S;
+          const int su = u_stays ? ci : g % SU, sv = g % S;
           // A wait that gave up: stop issuing (the operands or the accumulators are not ready).
-          if (!mbar_wait_warp(smem_u32(u_full + su), (g / SU) & 1, dead, p.status)) break;
+          if (!mbar_wait_warp(smem_u32(u_full + su), u_stays ? 0 : (g / SU) & 1, dead, p.status)) break;
           if (!mbar_wait_warp(smem_u32(v_ready + sv), (g / S) & 1, dead, p.status)) break;
           tc_fence_after();
           const uint64_t ad = a_desc0 + (uint64_t)(sv * (Cfg::kStageBytes >> 4)) + (uint64_t)(col0 * (2048 >> 4)),
@@ -290,7 +294,8 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
           }
           if (!ok) break;
           if (elect_one()) tc_commit_both(smem_u32(v_empty + sv));
-          if (elect_one()) tc_commit_both(smem_u32(u_empty + su));
+          if (!u_stays || seq == my_tiles - 1)
+            if (elect_one()) tc_commit_both(smem_u32(u_empty + su));
           if (++ci == cpt) {
             if (elect_one()) tc_commit_both(smem_u32(acc_full));              // tile finished
             ci = 0;
