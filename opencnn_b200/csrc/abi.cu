@@ -104,8 +104,10 @@ cudaError_t device_state(DeviceState **out) {
       if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcTf32>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcBf16>);
       if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
-      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcTf32>);
-      if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      for (const auto kernel : {ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::wino_pair_kernel<ocb::kTcTf32, true>}) {
+        if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, kernel);
+        if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      }
     }
     const auto large_smem = [&](auto kernel, size_t bytes) {
       if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -119,9 +121,8 @@ cudaError_t device_state(DeviceState **out) {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_pair_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ocb::PairCfg<ocb::kTcBf16>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_pair_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::PairCfg<ocb::kTcTf32>::kSmemBytes);
+    large_smem(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes);
+    large_smem(ocb::wino_pair_kernel<ocb::kTcTf32, true>, ocb::PairCfg<ocb::kTcTf32, true>::kSmemBytes);
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_img_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes);
@@ -143,7 +144,10 @@ cudaError_t device_state(DeviceState **out) {
         if (err == cudaSuccess) err = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
       };
       pairs(ocb::wino_pair_kernel<ocb::kTcBf16>, ocb::PairCfg<ocb::kTcBf16>::kSmemBytes, st.pair_clusters[0]);
+      int in_place = 0;
       pairs(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes, st.pair_clusters[1]);
+      pairs(ocb::wino_pair_kernel<ocb::kTcTf32, true>, ocb::PairCfg<ocb::kTcTf32, true>::kSmemBytes, in_place);
+      if (in_place < st.pair_clusters[1]) st.pair_clusters[1] = in_place;
       cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcBf16>::kThreads);
       pairs(ocb::wino_img_kernel<ocb::kTcBf16>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.img_clusters[0]);
       cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcTf32>::kThreads);
@@ -203,15 +207,15 @@ bool encode_patches(EncodeTiledFn enc, CUtensorMap *map, const float *input, int
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The same for the 4x6 patches of two tiles beside each other, with the channels of a pixel one behind the other.
-bool encode_tile_pairs(EncodeTiledFn enc, CUtensorMap *map, const float *input, int N, int C, int H, int W, int channels) {
+// The same for patches of h x w pixels with the channels of a pixel one behind the other.
+bool encode_pixels(EncodeTiledFn enc, CUtensorMap *map, const float *input, int N, int C, int H, int W, int channels, int h, int w,
+                   CUtensorMapSwizzle swizzle) {
   cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H};
   cuuint64_t strides[3] = {(cuuint64_t)H * W * N * 4, (cuuint64_t)N * 4, (cuuint64_t)W * N * 4};
-  cuuint32_t box[4] = {32, (cuuint32_t)channels, 6, 4};
+  cuuint32_t box[4] = {32, (cuuint32_t)channels, (cuuint32_t)w, (cuuint32_t)h};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(input), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Tensor map of the workspace [C][16][K] of a tensor-core precision, viewed as {filter within a row of `row_bytes`, channel, row,
@@ -369,7 +373,7 @@ cudaError_t launch_wino_tc(const float *input, float *output, int N, int C, int 
 }
 
 // CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).
-template <int DT>
+template <int DT, bool IN_PLACE>
 cudaError_t launch_wino_pair(const float *input, float *output, int N, int C, int H, int W,
                             int K, cudaStream_t stream, const Filter &filter, TileRows rows) {
   DeviceState *st = nullptr;
@@ -377,14 +381,16 @@ cudaError_t launch_wino_pair(const float *input, float *output, int N, int C, in
   if (e != cudaSuccess) return e;
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  constexpr int KC = ocb::PairCfg<DT>::kKC;
+  constexpr int KC = ocb::TcCfg<DT>::kKC;
   constexpr bool bf16 = DT == ocb::kTcBf16;
   constexpr int esz = bf16 ? 2 : 4;
   const int max_clusters = st->pair_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
 
   CUtensorMap tm_in, tm_u;
-  if (!encode_patches(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  if (!(IN_PLACE ? encode_pixels(enc, &tm_in, input, N, C, H, W, KC, 4, 4, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)
+                 : encode_patches(enc, &tm_in, input, N, C, H, W, KC)))
+    return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, 128, ocb::kPairFilters * esz / 128)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
@@ -396,7 +402,7 @@ cudaError_t launch_wino_pair(const float *input, float *output, int N, int C, in
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  return launch_main(ocb::wino_pair_kernel<DT>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
+  return launch_main(ocb::wino_pair_kernel<DT, IN_PLACE>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT, IN_PLACE>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
 }
 
 // Image columns in the accumulator rows: 64 filters x four blocks of 32 columns per cluster of two (wino_img.cuh).
@@ -413,7 +419,7 @@ cudaError_t launch_wino_img(const float *input, float *output, int N, int C, int
   const int max_clusters = st->img_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
   CUtensorMap tm_in, tm_u;
-  if (!encode_tile_pairs(enc, &tm_in, input, N, C, H, W, KC)) return cudaErrorInvalidValue;
+  if (!encode_pixels(enc, &tm_in, input, N, C, H, W, KC, 4, 6, CU_TENSOR_MAP_SWIZZLE_NONE)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
@@ -476,7 +482,10 @@ cudaError_t launch_tc(const float *input, float *output, int N, int C, int H, in
   }
   switch (kernel) {
     case OPENCNN_TC_SINGLE_CTA: return launch_wino_tc<DT>(input, output, N, C, H, W, K, stream, filter, rows, packed);
-    case OPENCNN_TC_PAIR_LOCAL: return launch_wino_pair<DT>(input, output, N, C, H, W, K, stream, filter, rows);
+    case OPENCNN_TC_PAIR_LOCAL:
+      if constexpr (DT == ocb::kTcTf32)
+        if (pair_in_place(N, C, rows, W, K)) return launch_wino_pair<DT, true>(input, output, N, C, H, W, K, stream, filter, rows);
+      return launch_wino_pair<DT, false>(input, output, N, C, H, W, K, stream, filter, rows);
     case OPENCNN_TC_STACKED_BLOCKS: return launch_wino_tc64<DT>(input, output, N, C, H, W, K, stream, filter, rows);
     case OPENCNN_TC_IMAGE_ROWS: return launch_wino_img<DT>(input, output, N, C, H, W, K, stream, filter, rows);
     default: return cudaErrorInvalidValue;

@@ -105,6 +105,15 @@ constexpr TcCosts kTcCosts[2] = {   // BF16, TF32
      {3.45, 0.947, 0.896, 0.866, 4.1, 0, 0}, {4.83, 1.128, 0.542, 0.482, 5.1, 0, 0}, {3.94, 1.320, 0, 0.585, 2.9, 0.226, 0.012},
      {3.61, 1.210, 0, 0.555, 2.9, 0.078, 0.027}},
 };
+// Which of its two forms the TF32 CTA pair takes: in place, with four filter slices in flight instead of three but one ring for patches and
+// operand, where input and transformed filter are more than about half of L2, so that slices and patches come from far away; us, three slices :
+// in place, MB of both:
+//   64x1024x1024x14x14 314 : 285 (118)      128x512x128x20x20 77.4 : 75.7 (109)     128x1024x1024x7x7 231 : 224 (93)
+//   128x512x256x14x14  78.4 : 75.8 (60)     128x1024x512x7x7  107 : 103 (59)        128x512x512x14x14 142.6 : 146.8 (68)
+//   128x512x128x14x14  46.2 : 51.6 (56)     128x1024x256x7x7  45.6 : 50.4 (42)      128x128x128x28x28 45.6 : 46.2 (52)
+//   128x256x256x14x14  38.3 : 41.7 (30)
+bool pair_in_place(int N, int C, TileRows rows, int W, int K) { return 4e-6 * C * (2.0 * N * rows.count * W + 16.0 * K) > 58; }
+
 // Share of packed blocks of eight quads that run from one tile into the next, a tile having `quads` of them.
 double crossing_share(int quads) {
   int unit = quads;                        // the common divisor of eight and the quads: where in a tile blocks may begin

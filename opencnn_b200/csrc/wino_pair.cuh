@@ -50,16 +50,22 @@ constexpr int kPairLaunchRegs = 96, kPairIssueRegs = 64, kPairTransformRegs = 80
 static_assert(kPairIssueRegs + 2 * kPairTransformRegs + 2 * kPairEpilogueRegs <= 5 * kPairLaunchRegs,
               "setmaxnreg budgets exceed the registers the CTA was launched with");
 constexpr int kPairFilters = 64;                 // per CTA
-template <int DT> struct PairCfg {
+template <int DT, bool IN_PLACE = false> struct PairCfg {
   static constexpr int kKC = DT == kTcBf16 ? 16 : 8;                       // channels per K-step
   static constexpr uint32_t kRawBytes = kKC * 16 * kTcN * 4;               // [c][4 h][4 w][32 n] fp32
   static constexpr uint32_t kUPosBytes = 2048;                             // 64 filters x one K-step
   static constexpr uint32_t kUBytes = 16 * kUPosBytes;
   // Ring depths: what fits in 227 KB.  Fewer than three stages of patches starve the BF16 kernel (two: 229-270 us
   // instead of 208 on 64x1024x1024x14x14), fewer than three of filters the TF32 kernel (two: 467 instead of 330).
-  static constexpr int kRawStages = DT == kTcBf16 ? 3 : 4;
-  static constexpr int kUStages = 3;
-  static constexpr int kVStages = DT == kTcBf16 ? 2 : 4;
+  // IN_PLACE (TF32, where a patch is as large as what becomes of it): the patch arrives with its channels one behind the other and in the operand's
+  // swizzle, so that a thread finds its 16 pixels where its 16 positions belong.  One ring for both leaves room for a fourth slice of
+  // filters, which pays where slices come from beyond L2 (see pair_in_place in dispatch.h).
+  static constexpr bool kInPlace = IN_PLACE;
+  static_assert(!IN_PLACE || DT == kTcTf32, "a BF16 operand is half a patch");
+  static constexpr int kRawStages = kInPlace ? 6 : DT == kTcBf16 ? 3 : 4;
+  static constexpr int kUStages = kInPlace ? 4 : 3;
+  static constexpr int kVStages = kInPlace ? kRawStages : DT == kTcBf16 ? 2 : 4;
+  static_assert(!kInPlace || kRawBytes == kTcVBytes, "a patch and its transform are the same size");
   // Transform warps that share a K-step: all eight in BF16 (16 channels x 16 image pairs, one item per thread); in
   // TF32 (8 channels) two groups of four take the K-steps in turn.
   static constexpr int kStepWarps = DT == kTcBf16 ? 8 : 4;
@@ -68,7 +74,7 @@ template <int DT> struct PairCfg {
   static constexpr int kGroups = kPairTransformWarps / kStepWarps;
   static_assert(kRawStages % kGroups == 0 && kVStages % kGroups == 0, "ring depths are multiples of the group count");
   static constexpr size_t kSmemBytes = (size_t)kRawStages * kRawBytes + (size_t)kUStages * kUBytes +
-                                       (size_t)kVStages * kTcVBytes + 512;
+                                       (kInPlace ? 0 : (size_t)kVStages * kTcVBytes) + 512;
   static_assert(kSmemBytes <= 232448, "shared memory");
 };
 
@@ -112,23 +118,24 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uin
 }
 
 // p.k_blocks counts 128-filter blocks, p.blocks blocks of 32 columns, p.total_tiles pair tiles (k_blocks times half of those).
-template <int DT>
+template <int DT, bool IN_PLACE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
-  using Cfg = PairCfg<DT>;
+  using Cfg = PairCfg<DT, IN_PLACE>;
   constexpr int SR = Cfg::kRawStages, SU = Cfg::kUStages, SV = Cfg::kVStages, KC = Cfg::kKC;
   extern __shared__ __align__(1024) uint8_t psmem[];
   uint8_t *raw_s = psmem;
   uint8_t *u_s = raw_s + SR * Cfg::kRawBytes;
-  uint8_t *v_s = u_s + SU * Cfg::kUBytes;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(v_s + SV * kTcVBytes);
+  uint8_t *v_s = Cfg::kInPlace ? raw_s : u_s + SU * Cfg::kUBytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(psmem + Cfg::kSmemBytes - 512);
   uint64_t *raw_full = bars, *raw_empty = raw_full + SR, *u_full = raw_empty + SR, *u_empty = u_full + SU,
            *v_ready = u_empty + SU, *v_empty = v_ready + SV;
   uint64_t *acc_full = v_empty + SV, *mma_done = acc_full + 1, *acc_empty = acc_full + 3;   // mma_done[2], acc_empty[4]
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 7);
   volatile int *dead = reinterpret_cast<volatile int *>(acc_full + 8);
-  uint64_t *nowhere = acc_full + 9;                    // [4]: nobody waits for these; where a thread that gave up arrives
-  static_assert(SV <= 4 && (2 * SR + 2 * SU + 2 * SV + 13) * 8 <= 512, "barriers");
+  constexpr int kNowhere = SV > 4 ? SV : 4;
+  uint64_t *nowhere = acc_full + 9;                    // [kNowhere]: nobody waits for these; where a thread that gave up arrives
+  static_assert((2 * SR + 2 * SU + 2 * SV + 9 + kNowhere) * 8 <= 512, "barriers");
 
   grid_launch_dependents();
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform, as the compiler can see
@@ -155,7 +162,7 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     }
     mbar_init(smem_u32(acc_full), 2);
     for (int j = 0; j < 4; ++j) mbar_init(smem_u32(acc_empty + j), 2 * kTcEpilogueWarps);   // leader only
-    for (int j = 0; j < 4; ++j) mbar_init(smem_u32(nowhere + j), 1);
+    for (int j = 0; j < kNowhere; ++j) mbar_init(smem_u32(nowhere + j), 1);
     mbar_init(smem_u32(mma_done + 0), 1);
     mbar_init(smem_u32(mma_done + 1), 1);
     mbar_fence_init();
@@ -198,15 +205,22 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
       const float *raw = reinterpret_cast<const float *>(raw_s + sr * Cfg::kRawBytes);
       uint8_t *vst = v_s + sv * kTcVBytes;
       uint64_t d[16];
-      load_patch_pair(raw, t >> 4, t & 15, d);
-      if (use > 0)                       // V stage free again
-        mbar_wait_reporting(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
+      if (Cfg::kInPlace) {
+        const int n = 2 * (t & 15), c = t >> 4;
+        const uint8_t *mine = vst + c * 128 + ((((n >> 3) ^ c) & 3) << 5) + ((n & 7) << 2);     // as in finish_v_tf32
+#pragma unroll
+        for (int q = 0; q < 16; ++q) d[q] = *reinterpret_cast<const volatile uint64_t *>(mine + q * 1024);
+      } else {
+        load_patch_pair(raw, t >> 4, t & 15, d);
+        if (use > 0)                     // V stage free again
+          mbar_wait_reporting(smem_u32(v_empty + sv), (use - 1) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
+      }
       if (DT == kTcBf16) finish_v_bf16(d, vst, t >> 4, t & 15);
       else               finish_v_tf32(d, vst, t >> 4, t & 15);
       fence_proxy_async_smem();          // V is read by the tensor core through the async proxy
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(smem_u32(raw_empty + sr));     // behind the fence: TMA refills the stage
+        if (!Cfg::kInPlace) mbar_arrive(smem_u32(raw_empty + sr));     // behind the fence: TMA refills the stage
         mbar_arrive_cluster(v_ready0 + 8 * sv);
       }
     }
@@ -217,7 +231,8 @@ wino_pair_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPairIssueRegs));
     if (warp == 0) {
       // ===================================== patches =============================================
-        load_patches<KC, SR, 1>(p, &tm_in, raw_s, raw_full, raw_empty, my_tiles, dead,      // an odd last block is paired with one that does not exist
+      // (An odd last block is paired with one that does not exist.)  In place, a stage is free when its products are done.
+        load_patches<KC, SR, 1, Cfg::kInPlace>(p, &tm_in, raw_s, raw_full, Cfg::kInPlace ? v_empty : raw_empty, my_tiles, dead,
                            [&](int seq, int) { return 2 * ((cid + seq * n_clusters) % pairs) + (int)rank; });
     } else if (warp == 1) {
       // ===================================== filter slices =======================================

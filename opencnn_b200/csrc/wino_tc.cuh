@@ -412,8 +412,9 @@ template <int DT> __device__ __forceinline__ bool tile_repeats_filters(const Win
 }
 
 // The loader of the raw patches (one warp), which is the same in all tensor-core kernels: every K-step of KC channels of
-// each of this CTA's `my_tiles` tiles takes the patches of PER_STEP blocks of 32 columns, block_of(tile, i), into a ring of SR stages.
-template <int KC, int SR, int PER_STEP, class BlockOf>
+// each of this CTA's `my_tiles` tiles takes the patches of PER_STEP blocks of 32 columns, block_of(tile, i), into a ring of SR stages.  PIXELS: the
+// tensor map's order is that of encode_pixels.
+template <int KC, int SR, int PER_STEP, bool PIXELS = false, class BlockOf>
 __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensorMap *tm_in, uint8_t *raw_s, uint64_t *raw_full,
                                              uint64_t *raw_empty, int my_tiles, volatile int *dead, BlockOf block_of) {
   constexpr uint32_t kBytes = KC * 16 * kTcN * 4;
@@ -436,7 +437,9 @@ __device__ __forceinline__ void load_patches(const WinoParams &p, const CUtensor
       // (A block past the last one reads what lies there: image rows of the next tile row, which in a run of some rows may be arriving at this
       // moment, or zeros below the image.  Its columns are not stored, and no kernel mixes columns.  To load zeros instead costs this thread a
       // choice per copy: BF16 128x20x64x12x12 5.75 -> 6.25 us, 256x32x64x112x112 263 -> 267.)
-      tma_load_4d(smem_u32(raw_s + s * kBytes), tm_in, smem_u32(raw_full + s), b.n, 2 * b.tx - 1, 2 * b.ty - 1, i / PER_STEP * KC);
+      const uint32_t dst = smem_u32(raw_s + s * kBytes), full = smem_u32(raw_full + s);
+      if (PIXELS) tma_load_4d(dst, tm_in, full, b.n, i / PER_STEP * KC, 2 * b.tx - 1, 2 * b.ty - 1);
+      else        tma_load_4d(dst, tm_in, full, b.n, 2 * b.tx - 1, 2 * b.ty - 1, i / PER_STEP * KC);
     }
   }
   // No exit with bulk copies in flight (after a complete run these phases are long over).
