@@ -40,6 +40,9 @@ namespace {
 static_assert(kColumns == ocb::kBN && kColumns == ocb::kTcN && kFp32Filters == ocb::kBK && kTcFilters == ocb::kTcM && kTcFilters == 2 * ocb::kPairFilters &&
               kImgRowFilters == ocb::kImgFilters && kStepBf16 == ocb::TcCfg<ocb::kTcBf16>::kKC && kStepTf32 == ocb::TcCfg<ocb::kTcTf32>::kKC, "block sizes");
 
+// The kernel for batches and filters that fill their blocks, where four warps transform if the ring is deep enough.
+constexpr int kFourWarps = ocb::SmemLayout<OCB_VARIANT>::kStages >= 4 ? ocb::kExactFour : ocb::kExact;
+
 __device__ int g_status = 0;
 
 constexpr int kMaxDevices = 64;
@@ -83,7 +86,7 @@ cudaError_t device_state(DeviceState **out) {
     cudaError_t err = cudaDeviceGetAttribute(&st.sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (err == cudaSuccess)
       for (const auto kernel : {ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>, ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>,
-                                ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>})
+                                ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>, ocb::wino_fp32_kernel<OCB_VARIANT, kFourWarps>})
         if (err == cudaSuccess)
           err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ocb::SmemLayout<OCB_VARIANT>::kBytes);
     if (err == cudaSuccess) {
@@ -93,7 +96,7 @@ cudaError_t device_state(DeviceState **out) {
       constexpr int kBudget = ocb::kConsumerThreads * ocb::kConsumerRegs + ocb::kProducerThreads * ocb::kProducerRegs;
       cudaFuncAttributes fa;
       for (const auto kernel : {ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>, ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>,
-                                ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>}) {
+                                ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>, ocb::wino_fp32_kernel<OCB_VARIANT, kFourWarps>}) {
         if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, kernel);
         if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
       }
@@ -318,7 +321,9 @@ cudaError_t launch_wino_fp32(const float *input, float *output, int N, int C, in
   const int grid = p.total_items < st->sm_count ? p.total_items : st->sm_count;
   const auto kernel = packed   ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>
                       : ragged ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>
-                               : ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>;
+                      : p.chunks_per_tile >= 8 || p.total_items <= st->sm_count
+                          ? ocb::wino_fp32_kernel<OCB_VARIANT, kFourWarps>        // (see kFourTransform)
+                          : ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>;
   return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
 }
 

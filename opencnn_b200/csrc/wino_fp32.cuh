@@ -16,8 +16,8 @@
 //   * the 4x4 input patch (with its halo) and the 64-filter slice of the transformed filter
 //     arrive by TMA; out-of-range coordinates are zero-filled by the hardware, which replaces
 //     the reference's halo masks and predicated loads;
-//   * the input transform runs in place in shared memory on three producer warps (a fourth
-//     only issues TMA), one thread per (image, channel);
+//   * the input transform runs in place in shared memory on the producer warps: all four, the first of which
+//     also issues TMA, one thread per (image pair, channel), or three beside one that only loads (see kFourTransform);
 //   * a batch that is not a multiple of 32 is packed into the 32 columns of the tiles across output tiles (ColumnQuad);
 //   * the consumers form two groups of four warps, each owning 32 of the 64 filters and all 16
 //     positions, so a group transposes, transforms and stores its outputs on its own (named
@@ -35,8 +35,9 @@ namespace ocb {
 
 // Exact: the batch and the filters fill the blocks of 32 images and 64 filters.  Ragged: one of them does not; missing images
 // and filters are loaded as zeros and not stored.  Packed: the batch does not, and its images are packed (see ColumnQuad).
-// (Channels beyond the end are loaded as zeros by all three.)
-enum Shape : int { kExact = 0, kRagged = 1, kPacked = 2 };
+// (Channels beyond the end are loaded as zeros by all of them.)  ExactFour: as Exact, with four warps for the input transform (see kFourTransform).
+enum Shape : int { kExact = 0, kRagged = 1, kPacked = 2, kExactFour = 3 };
+template <int SHAPE> constexpr bool kIsRagged = SHAPE == kRagged || SHAPE == kPacked;
 
 enum Variant : int { kBase = 0, kOptSts64 = 1, kOptSts64Cmp = 2, kOptLds64 = 3 };
 
@@ -45,8 +46,8 @@ constexpr int kBK = 64;                     // filters per CTA tile
 constexpr int kBC = 8;                      // channels per pipeline stage
 constexpr int kGroupThreads = 128;          // one consumer group: 4 warps, 32 filters, 16 positions
 constexpr int kConsumerThreads = 256;       // warps 0-3 group 0, warps 4-7 group 1
-constexpr int kProducerThreads = 128;       // warp 8 issues TMA, warps 9-11 transform
-constexpr int kTransformThreads = 96;
+constexpr int kProducerThreads = 128;       // warp 8 issues TMA, warps 9-11 (or 8-11) transform
+constexpr int kTransformThreads = 96;       // of warps 9-11
 constexpr int kThreads = kConsumerThreads + kProducerThreads;
 // setmaxnreg budgets.  The CTA owns what it was launched with, 384 threads x 168 registers =
 // 64512, and can only redistribute that: 256*216 + 128*72 = 64512.  Asking for more than the
@@ -295,7 +296,7 @@ __device__ __forceinline__ void epilogue(uint64_t (&acc)[8][8], float *stg, cons
                                          const TileCoord &tc, const LaneRole &role) {
   const int lane = threadIdx.x & 31;
   constexpr int RF = Staging<V>::kRowFloats;
-  constexpr bool RAGGED = SHAPE != kExact, PACKED = SHAPE == kPacked;
+  constexpr bool RAGGED = kIsRagged<SHAPE>, PACKED = SHAPE == kPacked;
   const int col = V == kOptLds64 ? 2 * (lane & 15) : lane;            // first column that this lane reads back and stores
   const int oh0 = 2 * tc.ty, ow0 = 2 * tc.tx;
   const bool row1 = (oh0 + 1) < p.H, col1 = (ow0 + 1) < p.W;
@@ -418,6 +419,28 @@ __device__ __forceinline__ void transform_patch(float *vstage, int patch) {
     R[(4 * i + 3) * kBN] = __fsub_rn(b[4 * i + 1], b[4 * i + 3]);
   }
 }
+// The same for two images at once (`np`: the pair) of channel `c`.
+__device__ __forceinline__ void transform_patch_pair(float *vstage, int c, int np) {
+  uint64_t *R = reinterpret_cast<uint64_t *>(vstage + c * 16 * kBN) + np;
+  constexpr int P = kBN / 2;
+  uint64_t d[16], b[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) d[q] = R[q * P];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    b[j] = sub2(d[j], d[8 + j]);
+    b[4 + j] = add2(d[4 + j], d[8 + j]);
+    b[8 + j] = sub2(d[8 + j], d[4 + j]);
+    b[12 + j] = sub2(d[4 + j], d[12 + j]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    R[(4 * i + 0) * P] = sub2(b[4 * i + 0], b[4 * i + 2]);
+    R[(4 * i + 1) * P] = add2(b[4 * i + 1], b[4 * i + 2]);
+    R[(4 * i + 2) * P] = sub2(b[4 * i + 2], b[4 * i + 1]);
+    R[(4 * i + 3) * P] = sub2(b[4 * i + 1], b[4 * i + 3]);
+  }
+}
 // Operands of one channel for one lane: 16 images as 8 pairs, 8 filters.
 struct Frag {
   ulonglong2 v[4];
@@ -495,7 +518,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u,
                  const WinoParams p) {
   constexpr int S = SmemLayout<V>::kStages;
-  constexpr bool RAGGED = SHAPE != kExact, PACKED = SHAPE == kPacked;
+  constexpr bool RAGGED = kIsRagged<SHAPE>, PACKED = SHAPE == kPacked;
+  // Who transforms: three producer warps beside one that only loads, or all four, the first of which loads as well.  Four share the additions evenly
+  // between the schedulers, whose FMA pipes they are taken from: 64x1024x1024x14x14 1993 -> 1917 us, 128x512x512x7x7 330 -> 325, 128x128x128x28x28
+  // 265 -> 261.  Not where the loads have to run far ahead: tiles of fewer than eight chunks on SMs with several tiles
+  // (256x32x64x112x112 1178 -> 1208), a ring of three stages (OPTSTS64_CMP, the same layer 1205 -> 1280), packed columns; and not in the
+  // ragged kernel, whose consumers the compiler then schedules worse (184x21x116x34x34 143 -> 153).
+  constexpr bool kFourTransform = SHAPE == kExactFour;
+  static_assert(!kFourTransform || S >= 4, "see above");
   extern __shared__ __align__(1024) float smem[];
   float *stages = smem;
   float *stg = smem + S * kStageFloats;
@@ -513,7 +543,7 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
     *dead = 0;
     for (int s = 0; s < S; ++s) {
       mbar_init(smem_u32(bar_full + s), PACKED ? 32 : 1);         // the TMA issuer and its bytes; packed: each lane of the loader
-      mbar_init(smem_u32(bar_ready + s), kTransformThreads / 32);  // one arrive per transform warp
+      mbar_init(smem_u32(bar_ready + s), kFourTransform ? kProducerThreads / 32 : kTransformThreads / 32);   // one arrive per transform warp
       mbar_init(smem_u32(bar_empty + s), kConsumerThreads / 32);   // one arrive per consumer warp
     }
     mbar_fence_init();
@@ -523,55 +553,117 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   if (warp >= kConsumerThreads / 32) {
     // =============================== producers ===============================================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
-    if (warp == kConsumerThreads / 32) {
-      if (PACKED) {
-        load_packed(p, &tm_in, &tm_u, stages, bar_full, bar_empty, S, my_tiles, dead);
+    if (!kFourTransform) {
+      if (warp == kConsumerThreads / 32) {
+        if (PACKED) {
+          load_packed(p, &tm_in, &tm_u, stages, bar_full, bar_empty, S, my_tiles, dead);
+        } else {
+          // ---- TMA issuer: one warp keeps the ring full ----
+          if (elect_one()) {
+            tma_prefetch_descriptor(&tm_in);
+            tma_prefetch_descriptor(&tm_u);
+          }
+          if (!p.input_ready) grid_dependency_wait();
+          int seq = 0, ci = 0, groups_unused, issued = 0;
+          TileCoord tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x, groups_unused));
+          for (int g = 0; g < total_chunks; ++g) {
+            const int s = g % S;
+            // A wait that gave up: stop issuing - the stage may still be in use.
+            if (g >= S && !mbar_wait_warp(smem_u32(bar_empty + s), ((g / S) - 1) & 1, dead, p.status)) break;
+            const uint32_t bar = smem_u32(bar_full + s);
+            const uint32_t dst = smem_u32(stages + s * kStageFloats);
+            if (elect_one()) {
+              mbar_arrive_expect_tx(bar, kStageBytes);
+              tma_load_4d(dst, &tm_in, bar, tc.nb * kBN, 2 * tc.tx - 1, 2 * tc.ty - 1, ci * kBC);
+              if (g == 0) grid_dependency_wait();       // U is all that the kernel before this one writes
+              tma_load_3d(dst + kVStageFloats * 4u, &tm_u, bar, tc.kb * kBK, 0, ci * kBC);
+            }
+            issued = g + 1;
+            if (++ci == cpt) {
+              ci = 0;
+              ++seq;
+              if (seq < my_tiles) tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused));
+            }
+          }
+          // The CTA must not exit with bulk copies in flight.  After a complete run the last loads
+          // were consumed long ago and these waits return at once; after a give-up they let what
+          // was issued land (with a limit of their own).
+          for (int g = issued > S ? issued - S : 0; g < issued; ++g)
+            mbar_wait_drain(smem_u32(bar_full + g % S), (g / S) & 1);
+        }
       } else {
-        // ---- TMA issuer: one warp keeps the ring full ----
+        // ---- transform warps: raw patch -> V, in place, as soon as a stage has landed ----
+        const int t = tid - kConsumerThreads - 32;                  // 0..95
+        for (int g = 0; g < total_chunks; ++g) {
+          const int s = g % S;
+          mbar_wait(smem_u32(bar_full + s), (g / S) & 1, dead, p.status);
+          float *vst = stages + s * kStageFloats;
+          for (int patch = t; patch < kBC * kBN; patch += kTransformThreads) transform_patch(vst, patch);
+          fence_proxy_async_smem();     // these generic writes precede the TMA that refills the stage
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(bar_ready + s));
+        }
+      }
+    } else {
+      // ---- four warps transform, a thread two images of a channel; the first of them keeps the ring full as well ----
+      const bool issuer = warp == kConsumerThreads / 32;
+      const int t = tid - kConsumerThreads;                       // channel t >> 4, image pair t & 15
+      int seq = 0, ci = 0, groups_unused, issued = 0;
+      TileCoord tc = decode_tile(p, item_tile<false>(p, (int)blockIdx.x, groups_unused));
+      const auto load = [&] {                                     // the next chunk
+        const int s = issued % S;
+        const uint32_t bar = smem_u32(bar_full + s), dst = smem_u32(stages + s * kStageFloats);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar, kStageBytes);
+          tma_load_4d(dst, &tm_in, bar, tc.nb * kBN, 2 * tc.tx - 1, 2 * tc.ty - 1, ci * kBC);
+          if (issued == 0) grid_dependency_wait();  // U is all that the kernel before this one writes
+          tma_load_3d(dst + kVStageFloats * 4u, &tm_u, bar, tc.kb * kBK, 0, ci * kBC);
+        }
+        ++issued;
+      };
+      const auto advance = [&] {                                  // (with divisions, which the others' next stage is not to wait for)
+        if (++ci == cpt) {
+          ci = 0;
+          ++seq;
+          if (seq < my_tiles) tc = decode_tile(p, item_tile<false>(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused));
+        }
+      };
+      if (issuer) {
         if (elect_one()) {
           tma_prefetch_descriptor(&tm_in);
           tma_prefetch_descriptor(&tm_u);
         }
         if (!p.input_ready) grid_dependency_wait();
-        int seq = 0, ci = 0, groups_unused, issued = 0;
-        TileCoord tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x, groups_unused));
-        for (int g = 0; g < total_chunks; ++g) {
-          const int s = g % S;
-          // A wait that gave up: stop issuing - the stage may still be in use.
-          if (g >= S && !mbar_wait_warp(smem_u32(bar_empty + s), ((g / S) - 1) & 1, dead, p.status)) break;
-          const uint32_t bar = smem_u32(bar_full + s);
-          const uint32_t dst = smem_u32(stages + s * kStageFloats);
-          if (elect_one()) {
-            mbar_arrive_expect_tx(bar, kStageBytes);
-            tma_load_4d(dst, &tm_in, bar, tc.nb * kBN, 2 * tc.tx - 1, 2 * tc.ty - 1, ci * kBC);
-            if (g == 0) grid_dependency_wait();       // U is all that the kernel before this one writes
-            tma_load_3d(dst + kVStageFloats * 4u, &tm_u, bar, tc.kb * kBK, 0, ci * kBC);
-          }
-          issued = g + 1;
-          if (++ci == cpt) {
-            ci = 0;
-            ++seq;
-            if (seq < my_tiles) tc = decode_tile(p, item_tile<RAGGED>(p, (int)blockIdx.x + seq * (int)gridDim.x, groups_unused));
-          }
+        while (issued < S && issued < total_chunks) {
+          load();
+          advance();
         }
-        // The CTA must not exit with bulk copies in flight.  After a complete run the last loads
-        // were consumed long ago and these waits return at once; after a give-up they let what
-        // was issued land (with a limit of their own).
-        for (int g = issued > S ? issued - S : 0; g < issued; ++g)
-          mbar_wait_drain(smem_u32(bar_full + g % S), (g / S) & 1);
       }
-    } else {
-      // ---- transform warps: raw patch -> V, in place, as soon as a stage has landed ----
-      const int t = tid - kConsumerThreads - 32;                  // 0..95
+      // A chunk is asked for as soon as its stage is free, which is when the issuer has transformed the chunk before it and waits.  Deep tiles ask for it
+      // before that chunk is waited for, so that two loads are under way: their filters come from beyond L2, and a load may take longer than a
+      // chunk (64x1024x1024x14x14 1962 -> 1937 us, cached 128x512x512x7x7 337 -> 328); shallow ones lose by it, since the transform is then one
+      // chunk less ahead when the consumers come back from a tile's epilogue (256x32x64x112x112 1185 -> 1240).
+      const int ahead = cpt >= 64 ? 1 : 0;
       for (int g = 0; g < total_chunks; ++g) {
         const int s = g % S;
+        const bool refill = issuer && issued < total_chunks && issued == g + ahead;
+        if (refill) {
+          // A wait that gave up: stop issuing - the stage may still be in use.
+          if (!mbar_wait_warp(smem_u32(bar_empty + issued % S), ((issued / S) - 1) & 1, dead, p.status)) break;
+          load();
+        }
         mbar_wait(smem_u32(bar_full + s), (g / S) & 1, dead, p.status);
-        float *vst = stages + s * kStageFloats;
-        for (int patch = t; patch < kBC * kBN; patch += kTransformThreads) transform_patch(vst, patch);
-        fence_proxy_async_smem();     // these generic writes precede the TMA that refills the stage
+        transform_patch_pair(stages + s * kStageFloats, t >> 4, t & 15);
+        fence_proxy_async_smem();       // these generic writes precede the TMA that refills the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(bar_ready + s));
+        if (refill) advance();
       }
+      // The CTA must not exit with bulk copies in flight.  After a complete run the last loads
+      // were consumed long ago and these waits return at once; after a give-up they let what
+      // was issued land (with a limit of their own).
+      for (int g = issued > S ? issued - S : 0; g < issued; ++g)
+        mbar_wait_drain(smem_u32(bar_full + g % S), (g / S) & 1);
     }
     return;
   }

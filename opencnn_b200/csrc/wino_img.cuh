@@ -6,22 +6,31 @@
 // has no tensor-core path).  wino_pair.cuh has filters as the M dimension and 128 of them per pair, of which a layer with 64
 // filters leaves half empty; and its accumulator rows are filters, so a warp's stores go to 32 output planes at once.  Here
 //     D[xi] (128 image columns x 64 filters)  +=  V[xi] (128 x KC) * U[xi] (KC x 64),   M = 128, N = 64 over two SMs:
-// CTA r transforms the patches of blocks 4q + 2r and 4q + 2r + 1 of 32 columns (see ColumnQuad), loads the filters
+// CTA r's 64 columns are 32 images of two tiles beside each other (TilePair), block 2q + r of their list; it loads the filters
 // 32*r .. 32*r+31 of the tile's 64, and its tensor memory receives
 //     lanes  0-63   its 64 columns x filters  0-31 of the tile      32 accumulator columns per position
 //     lanes 64-127  the same 64 columns x filters 32-63
 // (the M = 128 data-path layout of cta_group::2).  Each SM computes the same 64 x 64 share as in wino_pair.cuh for half the
 // filters and twice the patches, and an epilogue warp stores whole 128-byte lines: 32 images of one filter.
 //
-// Barriers and roles are those of wino_pair.cuh: the patches' ring is each CTA's own; "filter slice landed" and "V written"
-// are barriers of the leading CTA, the tensor core's commits reach both, a drained accumulator column is reported to the
-// leader, all waits are bounded, and a thread whose wait gave up reports nothing more to the leader.
+// Two tiles share a 4x6 patch: 48 KB per BF16 K-step instead of 64 for two patches of their own, a quarter fewer bytes from L2 and reads of shared memory.
+// And the transform writes the operand where the patch was (transform_tile_pair), so that shared memory holds one ring of four (BF16) or five (TF32)
+// K-steps.  With a patch per tile and an operand ring of its own there was room for two and four, and a K-step could not be shorter than a
+// part of a load's way to DRAM, 3000 to 4400 cycles on layers that stream; us, then -> now: BF16 128x64x64x56x56 63.5 -> 47, 256x32x64x112x112 263 -> 228,
+// 128x128x128x28x28 53 -> 43; TF32 69 -> 62, 297 -> 257, 64 -> 56.  The list has whole pairs of tile columns, so that maps with an odd number compute a
+// column of tiles for nothing: 128x512x64x14x14 BF16 26.1 -> 27, 128x256x256x14x14 41 -> 49 (the CTA pair takes 30).
 //
-// What bounds it: on shallow layers the latency of a tile's own patches, of which the ring holds two K-steps, and the epilogue
-// warps' stores; both cost about their DRAM time on top of the rest (128x64x64x56x56 BF16 64 us: without stores 45, without patch
-// loads 46, without the transform 58, without MMAs 58; TF32 69: 56, 61, 64, 62).  On deep ones the ring of two filter slices, the
-// transform and the MMAs' hand-off (128x512x64x14x14 BF16 27.5 us: without the transform 22.6, without MMAs 25.3, without stores or
-// patch loads 26 to 27): 0.72 us per K-step in BF16, 0.48 in TF32, where the tensor pipe needs 0.26.
+// Barriers and roles are those of wino_pair.cuh, less those between patches and operand: a stage lands, is transformed ("V written", on the leading
+// CTA), and is free when the tensor core's commits say so, in both CTAs; "filter slice landed" is the leader's, a drained accumulator column is reported
+// to the leader, all waits are bounded, and a thread whose wait gave up reports nothing more to the leader.
+//
+// What bounds it: BF16, the transform - 48 KB read, 32 KB written and 64 KB of operands read by the MMAs per K-step, all in shared memory, 1000 to 1400
+// cycles - and the epilogue: an SM stores 32 bytes per clock at most, whatever the instruction, so 2048 cycles for a tile's 64 KB, behind 1500
+// for reading the accumulators, during which no store is on its way (256x32x64x112x112: period of a tile 4600 cycles, 4280 of them the HBM time
+// of its bytes; without accumulator reads and stores 144 us, without loads and transform 177).  16 transform warps gain 2 to 8 % on deep layers and
+// lose as much on shallow ones; three stages and five filter slices lose everywhere.  TF32, the filters' turnover: a slice of 8 channels takes 1900
+// cycles from its stage's release to the next one; with two in flight instead of four 128x512x64x28x28 takes 128 us instead of 96.  A layer with one filter block and
+// no more K-steps than slices loads them once (256x32x64x112x112 BF16 234 -> 228).
 #pragma once
 #include "wino_pair.cuh"
 

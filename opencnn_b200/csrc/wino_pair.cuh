@@ -14,7 +14,7 @@
 //     lanes  0-63   filters 64*r .. +63 of image block 0      32 columns per position
 //     lanes 64-127  the same filters of image block 1
 // (the M = 128 data-path layout of cta_group::2).  A square 64 x 64 share per CTA instead of 128 x 32:
-// the filter slice of a K-step is 32 KB instead of 64 KB, three or four of them fit, and nothing is
+// the filter slice of a K-step is 32 KB instead of 64 KB, three of them fit (four in place), and nothing is
 // exchanged by the threads - each CTA has all 16 positions of its outputs and stores them on its own.
 //
 // The two image blocks need not belong together: block q of the list (tile row, tile column, image
@@ -31,8 +31,8 @@
 
 namespace ocb {
 
-// What bounds it: the bytes in flight per SM - patches and filter slices of a K-step are 64 KB (BF16), the three-deep rings
-// of 96 KB each turn over in one load latency - and the transform's shared-memory round trip.  Kernel alone, four
+// What bounds it: no one part of a K-step, but their chain through rings of two and three stages.  64x1024x1024x14x14 BF16, cycles per K-step of 64 KB:
+// all 950, loads alone 710, the transform alone 650, MMAs alone 505, any two of them 820 to 850, barriers alone 300.  Kernel alone, four
 // transform warps (512 threads) -> eight: 64x1024x1024x14x14 199 -> 196 us in BF16 and 355 -> 321 in TF32,
 // 128x256x256x14x14 36.2 -> 35.4 and 56.0 -> 46.2, 128x64x128x56x56 93.5 -> 91.3 and 124 -> 115; a single K-step per
 // tile loses (256x8x128x56x56 91.0 -> 93.4 and 87.1 -> 90.8).  Handing the patches back as soon as they are in

@@ -76,3 +76,11 @@ def test_the_gpu_tests_reach_the_kernels_that_they_name(choose):
         assert {"packed", "packed halves"} <= set(fp32) and any(r.startswith("filled") for r in fp32)
     fp32 = choose([("fp32", shape) for shape in parity.PACKED])
     assert {"packed", "packed halves"} <= set(fp32) and any(r.startswith("filled") for r in fp32)
+
+
+def test_the_form_of_the_tf32_pair(choose):
+    """Both sides of the line, and what tests/test_overlap_gpu.py says of its sizes."""
+    import test_overlap_gpu as overlap
+    sizes = [(64, 1024, 1024, 14, 14), (128, 512, 256, 14, 14), (128, 512, 128, 14, 14), (128, 128, 128, 28, 28)]
+    assert choose([("form", s) for s in sizes]) == ["in place", "in place", "two rings", "two rings"]
+    assert set(choose([("form", s) for kernel, s in overlap.DEPTHS if kernel == "pair_local"])) == {"in place"}

@@ -1,0 +1,138 @@
+"""Kernels start while the one before them on the stream ends (opencnn_b200/csrc/launch.cuh): whatever a kernel reads was written by then, and nothing that
+an earlier one still reads is overwritten.  And the forms of the kernels that depend on the depth of a tile, against others that do not have them."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from opencnn_b200 import api  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _random(*shape, scale=1.0):
+    return (torch.rand(shape, device="cuda") * 2 - 1) * scale
+
+
+# A chain of layers with fixed weights and then with weights that are transformed in every call, ping-pong between two buffers: every call
+# reads what the one before it writes, and writes what the one before it reads.  Kernels of all kinds: (N, C = K, H, W).
+CHAINS = [("fp32", (32, 64, 9, 9)), ("fp32", (20, 64, 31, 45)), ("fp32", (32, 512, 5, 5)), ("bf16", (32, 64, 6, 6)), ("bf16", (64, 64, 30, 30)),
+          ("bf16", (32, 256, 12, 12)), ("tf32", (64, 64, 21, 13)), ("tf32", (64, 192, 7, 7)), ("tf32", (8, 64, 27, 21))]
+
+
+@pytest.mark.parametrize("precision,shape", CHAINS)
+@pytest.mark.parametrize("cached", [True, False])
+def test_a_chain_of_calls_is_ordered(libs, precision, shape, cached):
+    N, C, H, W = shape
+    layers = 6
+    stream = torch.cuda.Stream()
+    x = _random(C, H, W, N)
+    filters = [_random(C, 3, 3, C, scale=(C * 9) ** -0.5) for _ in range(layers)]
+    shared = torch.empty((C, 4, 4, C), device="cuda")
+    weights = [torch.empty_like(shared) for _ in range(layers)]
+    for g, w in zip(filters, weights):
+        assert api.filter_transform(g, w, C, C, precision=precision) == 0
+    buffers = [torch.empty_like(x), torch.empty_like(x)]
+
+    def run(wait):
+        for i in range(layers):
+            src, dst = buffers[i % 2], buffers[1 - i % 2]
+            if cached:
+                err = api.winograd_forward(src, weights[i], dst, N, C, H, W, C, precision=precision, stream=stream.cuda_stream)
+            else:
+                err = api.conv3x3(src, filters[i], dst, shared, N, C, H, W, C, precision=precision, stream=stream.cuda_stream)
+            assert err == 0
+            if wait:
+                torch.cuda.synchronize()
+
+    def result(go):
+        torch.cuda.synchronize()
+        buffers[0].copy_(x)
+        buffers[1].fill_(float("nan"))
+        torch.cuda.synchronize()
+        go()
+        torch.cuda.synchronize()
+        return buffers[layers % 2].clone()
+
+    expect = result(lambda: run(True))
+    assert bool(torch.isfinite(expect).all())
+    for _ in range(3):
+        assert torch.equal(result(lambda: run(False)), expect)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        run(False)
+    assert torch.equal(result(graph.replay), expect)
+    assert api.last_device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(128, 16, 64, 14, 14), (36, 5, 68, 7, 9)])
+def test_layout_adapters_and_the_operator_are_ordered(libs, shape):
+    """NCHW in, NCHW out, all of it queued, with inputs that another library's kernel has just written."""
+    N, C, K, H, W = shape
+    stream = torch.cuda.Stream()
+    inputs = [_random(N, C, H, W) for _ in range(4)]
+    g = _random(C, 3, 3, K, scale=0.05)
+    ws, chwn, y = (torch.empty(s, device="cuda") for s in ((C, 4, 4, K), (C, H, W, N), (K, H, W, N)))
+    staged = torch.empty_like(inputs[0])
+
+    def run(wait):
+        out = []
+        with torch.cuda.stream(stream):
+            for x in inputs:
+                staged.copy_(x)
+                nkhw = torch.full((N, K, H, W), float("nan"), device="cuda")
+                for err in (lambda: api.nchw_to_chwn(staged, chwn, N, C, H, W, stream=stream.cuda_stream),
+                            lambda: api.conv3x3(chwn, g, y, ws, N, C, H, W, K, stream=stream.cuda_stream),
+                            lambda: api.khwn_to_nkhw(y, nkhw, N, K, H, W, stream=stream.cuda_stream)):
+                    assert err() == 0
+                    if wait:
+                        torch.cuda.synchronize()
+                out.append(nkhw)
+        torch.cuda.synchronize()
+        return out
+
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(run(False), run(True)))
+
+
+# The fp32 kernel's four-stage ring is filled by a warp that transforms as well, deep tiles (64 chunks of 8 channels) one chunk further ahead; BASE has three
+# stages and a warp that only loads.  Fewer chunks than stages, as many, more; tiles on both sides of 64 chunks; several items per SM, the last round split.
+RINGS = [(32, 8, 64, 4, 4), (32, 24, 64, 26, 26), (32, 32, 128, 25, 25), (32, 33, 64, 31, 30), (32, 504, 64, 26, 26), (32, 512, 64, 26, 26),
+         (32, 520, 128, 19, 19), (64, 1024, 64, 5, 5)]
+
+
+@pytest.mark.parametrize("shape", RINGS)
+def test_ring_orders_give_the_same_bits(libs, shape):
+    N, C, K, H, W = shape
+    x, ws = _random(C, H, W, N), torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(_random(C, 3, 3, K, scale=0.05), ws, C, K) == 0
+    out = {}
+    for variant in ("BASE", "OPTSTS64", "OPTLDS64"):
+        out[variant] = torch.full((K, H, W, N), float("nan"), device="cuda")
+        assert api.winograd_forward(x, ws, out[variant], N, C, H, W, K, variant=variant) == 0
+        assert api.last_device_status(variant) == 0
+    assert bool(torch.isfinite(out["BASE"]).all())
+    assert torch.equal(out["OPTSTS64"], out["BASE"]) and torch.equal(out["OPTLDS64"], out["BASE"])
+
+
+# The image-rows kernel: filter slices that stay (as many K-steps as ring stages or fewer, one filter block, several tiles per pair) and their neighbours that do
+# not; one tile column, an odd number, a single pair; batches that leave blocks part empty.  And the TF32 CTA pair in place (input and filters
+# beyond 58 MB), with an odd number of blocks, channels that fill no step and filters that fill half a block.
+DEPTHS = [("image_rows", (32, 32, 64, 40, 40)), ("image_rows", (32, 33, 64, 41, 38)), ("image_rows", (64, 32, 128, 30, 29)), ("image_rows", (8, 5, 64, 33, 2)),
+          ("image_rows", (40, 16, 64, 21, 3)), ("image_rows", (72, 64, 192, 9, 5)), ("image_rows", (32, 9, 64, 1, 1)),
+          ("pair_local", (64, 1024, 128, 15, 14)), ("pair_local", (40, 1021, 192, 19, 21)), ("pair_local", (104, 515, 64, 21, 17))]
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("kernel,shape", DEPTHS)
+def test_forms_by_depth_give_the_bits_of_the_single_cta_kernel(libs, precision, kernel, shape):
+    N, C, K, H, W = shape
+    x, ws = _random(C, H, W, N), torch.empty((C, 4, 4, K), device="cuda")
+    assert api.filter_transform(_random(C, 3, 3, K, scale=0.05), ws, C, K, precision=precision) == 0
+    out = {}
+    for name in ("single", kernel):
+        out[name] = torch.full((K, H, W, N), float("nan"), device="cuda")
+        assert api.winograd_forward_kernel(x, ws, out[name], N, C, H, W, K, precision=precision, kernel=name) == 0
+        assert api.last_device_status() == 0
+    assert bool(torch.isfinite(out["single"]).all())
+    assert torch.equal(out[kernel], out["single"])
