@@ -101,10 +101,14 @@ cudaError_t device_state(DeviceState **out) {
         if (err == cudaSuccess && fa.numRegs * ocb::kThreads < kBudget) err = cudaErrorLaunchOutOfResources;
       }
       // the same for the CTA-pair kernels
-      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_img_kernel<ocb::kTcBf16>);
-      if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcBf16>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
-      if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_img_kernel<ocb::kTcTf32>);
-      if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcTf32>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      for (const auto kernel : {ocb::wino_img_kernel<ocb::kTcBf16, false>, ocb::wino_img_kernel<ocb::kTcBf16, true>}) {
+        if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, kernel);
+        if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcBf16>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      }
+      for (const auto kernel : {ocb::wino_img_kernel<ocb::kTcTf32, false>, ocb::wino_img_kernel<ocb::kTcTf32, true>}) {
+        if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, kernel);
+        if (err == cudaSuccess && fa.numRegs < ocb::ImgCfg<ocb::kTcTf32>::kLaunchRegs) err = cudaErrorLaunchOutOfResources;
+      }
       if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, ocb::wino_pair_kernel<ocb::kTcBf16>);
       if (err == cudaSuccess && fa.numRegs < ocb::kPairLaunchRegs) err = cudaErrorLaunchOutOfResources;
       for (const auto kernel : {ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::wino_pair_kernel<ocb::kTcTf32, true>}) {
@@ -126,12 +130,10 @@ cudaError_t device_state(DeviceState **out) {
                                  (int)ocb::PairCfg<ocb::kTcBf16>::kSmemBytes);
     large_smem(ocb::wino_pair_kernel<ocb::kTcTf32>, ocb::PairCfg<ocb::kTcTf32>::kSmemBytes);
     large_smem(ocb::wino_pair_kernel<ocb::kTcTf32, true>, ocb::PairCfg<ocb::kTcTf32, true>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_img_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(ocb::wino_img_kernel<ocb::kTcTf32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes);
+    large_smem(ocb::wino_img_kernel<ocb::kTcBf16, false>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes);
+    large_smem(ocb::wino_img_kernel<ocb::kTcBf16, true>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes);
+    large_smem(ocb::wino_img_kernel<ocb::kTcTf32, false>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes);
+    large_smem(ocb::wino_img_kernel<ocb::kTcTf32, true>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes);
     if (err == cudaSuccess) {
       // how many CTA pairs fit on the device at once (pairs must sit in one GPC)
       cudaLaunchConfig_t cfg = {};
@@ -152,9 +154,15 @@ cudaError_t device_state(DeviceState **out) {
       pairs(ocb::wino_pair_kernel<ocb::kTcTf32, true>, ocb::PairCfg<ocb::kTcTf32, true>::kSmemBytes, in_place);
       if (in_place < st.pair_clusters[1]) st.pair_clusters[1] = in_place;
       cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcBf16>::kThreads);
-      pairs(ocb::wino_img_kernel<ocb::kTcBf16>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.img_clusters[0]);
+      int odd0 = 0;
+      pairs(ocb::wino_img_kernel<ocb::kTcBf16, false>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, st.img_clusters[0]);
+      pairs(ocb::wino_img_kernel<ocb::kTcBf16, true>, ocb::ImgCfg<ocb::kTcBf16>::kSmemBytes, odd0);
+      if (odd0 < st.img_clusters[0]) st.img_clusters[0] = odd0;
       cfg.blockDim = dim3(ocb::ImgCfg<ocb::kTcTf32>::kThreads);
-      pairs(ocb::wino_img_kernel<ocb::kTcTf32>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, st.img_clusters[1]);
+      int odd1 = 0;
+      pairs(ocb::wino_img_kernel<ocb::kTcTf32, false>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, st.img_clusters[1]);
+      pairs(ocb::wino_img_kernel<ocb::kTcTf32, true>, ocb::ImgCfg<ocb::kTcTf32>::kSmemBytes, odd1);
+      if (odd1 < st.img_clusters[1]) st.img_clusters[1] = odd1;
     }
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(ocb::wino_tc64_kernel<ocb::kTcBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -263,16 +271,16 @@ struct Filter {
 // calls is what runs before it: 32x16x64x9x9 8.2 -> 6.3 us a call, TF32 32x128x128x14x14 14.4 -> 12.2.  Where there is no room for them, they would
 // come to the SMs one by one as that kernel ends, and this call's kernel after them: fp32 32x64x64x56x56 79.3 -> 81.9 us, TF32 128x128x128x28x28
 // 55.1 -> 58.2.
-template <class... P>
-cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, const Filter &filter, int sms,
-                        const CUtensorMap &tm_in, const CUtensorMap &tm_u, ocb::WinoParams p) {
+template <class... P, class... Maps>
+cudaError_t launch_main(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, const Filter &filter, int sms, ocb::WinoParams p,
+                        const Maps &...maps) {
   if (filter.filter) {
     const long long blocks = ((long long)p.C * p.K / 4 + ocb::kFxThreads - 1) / ocb::kFxThreads;
     const cudaError_t e = transform_filter(filter.filter, filter.workspace, p.C, p.K, filter.precision, stream, blocks <= 4ll * (sms - grid));
     if (e != cudaSuccess) return e;
   }
   p.input_ready = filter.filter != nullptr;
-  return ocb::launch(kernel, (unsigned)grid, dim3((unsigned)threads), smem, stream, true, tm_in, tm_u, p);
+  return ocb::launch(kernel, (unsigned)grid, dim3((unsigned)threads), smem, stream, true, maps..., p);
 }
 
 cudaError_t launch_wino_fp32(const float *input, float *output, int N, int C, int H,
@@ -324,7 +332,7 @@ cudaError_t launch_wino_fp32(const float *input, float *output, int N, int C, in
                       : p.chunks_per_tile >= 8 || p.total_items <= st->sm_count
                           ? ocb::wino_fp32_kernel<OCB_VARIANT, kFourWarps>        // (see kFourTransform)
                           : ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>;
-  return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
+  return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, filter, st->sm_count, p, tm_in, tm_u);
 }
 
 bool set_problem(ocb::WinoParams &p, const float *input, float *output, int N, int C, int H, int W, int K, TileRows rows,
@@ -371,10 +379,10 @@ cudaError_t launch_wino_tc(const float *input, float *output, int N, int C, int 
   if constexpr (bf16) {
     if (K <= 64)
       return launch_main(packed ? ocb::wino_tc_kernel<DT, true, true> : ocb::wino_tc_kernel<DT, true>, grid, threads, ocb::TcCfg<DT, true>::kSmemBytes, stream,
-                         filter, st->sm_count, tm_in, tm_u, p);
+                         filter, st->sm_count, p, tm_in, tm_u);
   }
   return launch_main(packed ? ocb::wino_tc_kernel<DT, false, true> : ocb::wino_tc_kernel<DT>, grid, threads, ocb::TcCfg<DT>::kSmemBytes, stream, filter,
-                     st->sm_count, tm_in, tm_u, p);
+                     st->sm_count, p, tm_in, tm_u);
 }
 
 // CTA-pair kernel: 128 filters x two 32-image blocks per cluster of two (wino_pair.cuh).
@@ -407,7 +415,7 @@ cudaError_t launch_wino_pair(const float *input, float *output, int N, int C, in
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  return launch_main(ocb::wino_pair_kernel<DT, IN_PLACE>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT, IN_PLACE>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
+  return launch_main(ocb::wino_pair_kernel<DT, IN_PLACE>, 2 * clusters, ocb::kPairThreads, ocb::PairCfg<DT, IN_PLACE>::kSmemBytes, stream, filter, st->sm_count, p, tm_in, tm_u);
 }
 
 // Image columns in the accumulator rows: 64 filters x four blocks of 32 columns per cluster of two (wino_img.cuh).
@@ -423,15 +431,18 @@ cudaError_t launch_wino_img(const float *input, float *output, int N, int C, int
   constexpr bool bf16 = DT == ocb::kTcBf16;
   const int max_clusters = st->img_clusters[bf16 ? 0 : 1];
   if (max_clusters <= 0) return cudaErrorNotSupported;
-  CUtensorMap tm_in, tm_u;
+  const bool odd = image_rows_odd(N, rows, W, K, max_clusters);
+  CUtensorMap tm_in, tm_above, tm_u;
   if (!encode_pixels(enc, &tm_in, input, N, C, H, W, KC, 4, 6, CU_TENSOR_MAP_SWIZZLE_NONE)) return cudaErrorInvalidValue;
+  if (!odd) tm_above = tm_in;                       // not used
+  else if (!encode_pixels(enc, &tm_above, input, N, C, H, W, KC, 6, 4, CU_TENSOR_MAP_SWIZZLE_NONE)) return cudaErrorInvalidValue;
   if (!encode_filter<DT>(enc, &tm_u, filter.workspace, C, K, bf16 ? 64 : 128, 1)) return cudaErrorInvalidValue;
   ocb::WinoParams p;
   if (!set_problem(p, input, output, N, C, H, W, K, rows, false)) return cudaErrorInvalidValue;
-  const long long blocks = tile_pair_blocks(N, rows, W);
+  const long long blocks = tile_pair_blocks(N, rows, W, odd);
   if (blocks > 0x7fffffffll / 16) return cudaErrorInvalidValue;
   p.blocks = (int)blocks;
-  p.tiles_w = (p.tiles_w + 1) / 2;
+  p.tiles_w = odd ? p.tiles_w / 2 : (p.tiles_w + 1) / 2;
   p.n_blocks = (N + kColumns - 1) / kColumns;
   p.k_blocks = K / ocb::kImgFilters;
   const long long tiles = (blocks + 1) / 2 * p.k_blocks;
@@ -441,7 +452,8 @@ cudaError_t launch_wino_img(const float *input, float *output, int N, int C, int
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int clusters = p.total_tiles < max_clusters ? p.total_tiles : max_clusters;
-  return launch_main(ocb::wino_img_kernel<DT>, 2 * clusters, ocb::ImgCfg<DT>::kThreads, ocb::ImgCfg<DT>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
+  return launch_main(odd ? ocb::wino_img_kernel<DT, true> : ocb::wino_img_kernel<DT, false>, 2 * clusters, ocb::ImgCfg<DT>::kThreads,
+                     ocb::ImgCfg<DT>::kSmemBytes, stream, filter, st->sm_count, p, tm_in, tm_u, tm_above);
 }
 
 // Layers with at most 64 filters: two 32-image blocks share the 128 accumulator rows (wino_tc64.cuh).
@@ -469,7 +481,7 @@ cudaError_t launch_wino_tc64(const float *input, float *output, int N, int C, in
   p.chunks_per_tile = (C + KC - 1) / KC;
   p.status = st->status_ptr;
   const int grid = p.total_tiles < st->sm_count ? p.total_tiles : st->sm_count;
-  return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, filter, st->sm_count, tm_in, tm_u, p);
+  return launch_main(ocb::wino_tc64_kernel<DT>, grid, ocb::kT64Threads, ocb::T64Cfg<DT>::kSmemBytes, stream, filter, st->sm_count, p, tm_in, tm_u);
 }
 
 template <int DT>

@@ -28,9 +28,23 @@ Columns columns_of(int N, TileRows rows, int W, bool packed) {
   return c;
 }
 
-// Blocks of two tiles beside each other and 32 images (image-rows kernel).
-long long tile_pair_blocks(int N, TileRows rows, int W) {
-  return (long long)rows.count * (((W + 1) / 2 + 1) / 2) * ((N + kColumns - 1) / kColumns);
+// Blocks of two tiles and 32 images (image-rows kernel).  The tiles lie beside each other; with `odd` an odd last column's one above the other.
+long long tile_pair_blocks(int N, TileRows rows, int W, bool odd) {
+  const long long tiles_w = (W + 1) / 2;
+  const long long pairs = odd ? tiles_w / 2 * rows.count + tiles_w % 2 * ((rows.count + 1) / 2) : (tiles_w + 1) / 2 * rows.count;
+  return pairs * ((N + kColumns - 1) / kColumns);
+}
+long long image_rows_tiles(int N, TileRows rows, int W, int K, bool odd) {
+  return (tile_pair_blocks(N, rows, W, odd) + 1) / 2 * (K / kImgRowFilters);
+}
+// Whether the image-rows kernel pairs an odd last column's tiles.  That form is 3 to 6 % slower per tile (`clusters`: CTA pairs at once); us, BF16 / TF32, a
+// column beside one that is not stored : its tiles paired, rounds of tiles:
+//   136x301x64x19x9  28.5 : 19.1 / 38.9 : 23.6  2 : 1     80x103x64x101x5   19.5 : 15.7 / 23.5 : 18.1  4 : 3
+//   128x256x256x14x14 47.7 : 42.7 / 65.8 : 53.4 4 : 3     128x512x64x22x22  50.6 : 52.9 (BF16)         2 : 2
+bool image_rows_odd(int N, TileRows rows, int W, int K, int clusters) {
+  if ((W + 1) / 2 % 2 == 0) return false;
+  const auto rounds = [&](bool odd) { return (image_rows_tiles(N, rows, W, K, odd) + clusters - 1) / clusters; };
+  return 106 * rounds(true) < 100 * rounds(false);
 }
 
 // ---- fp32 ----
@@ -73,19 +87,18 @@ Fp32Schedule schedule_fp32(int N, TileRows rows, int W, int K, int sms) {
 // packed blocks that lie in more than one tile (they are copied by threads); and a problem much larger than L2 no less than its bytes at
 // the rate the kernel's stores and loads were seen to reach.  The constants are least squares through the fused kernels' times, back to
 // back in a graph, at 1800 random sizes per type (8 to 256 images, 64 to 1024 filters, 1 to 1024 channels, maps of 4 to 112), on
-// 148 SMs at 1.9 GHz; the estimates are 3 to 6 % off in the mean.  At 1600 other sizes the kernel chosen by them was 0.35 % behind the fastest
-// one in the mean, and more than 10 % at 8.  Those are layers of one or two K-steps with an output that is many times L2, which the CTA
-// pair may write at 3.3 instead of 4.1 MB per us, for a reason not found (TF32 104x6x1024x54x54 377 us against 265, BF16 104x7x256x111x111 483
-// against 347), and small ones where two kernels' rounds end at about the same time (BF16 232x4x128x23x23 23.9 against 21.5).  Both sides of it, us,
+// 148 SMs at 1.9 GHz, before launches overlapped (which takes 1.4 us from all of them alike) and before the image-rows kernel became what it is; with
+// constants fitted to that, the choice gains nothing in BF16 and 0.3 % in TF32.  At 1600 other sizes the kernel chosen is 0.4 % (BF16) and 1.0 % (TF32) behind
+// the fastest one in the mean, and more than 10 % at 41: layers of one or two K-steps with an output that is many times L2, which the CTA
+// pair may write at 3.3 instead of 4.1 MB per us (its stores are runs of 64 bytes, TF32 104x6x1024x54x54 377 us against 265), and
+// small ones where two kernels' rounds end at about the same time (BF16 232x4x128x23x23 23.9 against 21.5).  Both sides of it, us,
 // single : pair : stacked : image rows:
-//   few K-steps or rounds      128x32x128x28x28  BF16 20.3 : 19.8 : - : 22.0    TF32 26.0 : 22.1 : - : 25.8
-//                              128x64x64x14x14   BF16 10.1 : 11.4 : 9.2 : 9.2   TF32 14.1 : 13.1 : 12.3 : 10.4
-//   64 filters                 128x64x64x56x56   BF16 80.9 : 80.6 : 68.6 : 63.6  TF32 124 : 103 : 112 : 70.4
-//                              256x32x64x112x112 BF16 811 : 415 : 390 : 265      TF32 570 : 497 : 506 : 308
-//                              128x512x64x14x14  BF16 41.2 : 38.4 : 39.3 : 27.1  TF32 74.7 : 48.0 : 58.4 : 36.3
-//   more filters, deep         128x256x256x14x14 BF16 38.5 : 31.3 : - : 40.4    TF32 60.0 : 40.1 : - : 54.7
-//                              64x1024x1024x14x14 BF16 275 : 194 : - : 275      TF32 524 : 328 : - : 468
-//   more filters, large output 96x4x128x99x99    BF16 182 : 135 : - : 110       TF32 192 : 132 : - : 105
+//   64 filters                 128x64x64x56x56   BF16 80.1 : 78.6 : 66.1 : 47.0  TF32 116 : 95.9 : 106 : 62.5
+//                              256x32x64x112x112 BF16 808 : 406 : 381 : 230      TF32 539 : 459 : 484 : 258
+//                              128x512x64x14x14  BF16 37.4 : 34.9 : 36.6 : 27.1  TF32 69.3 : 43.9 : 56.3 : 35.3
+//   more filters, deep         128x256x256x14x14 BF16 36.6 : 29.6 : - : 42.5    TF32 57.8 : 38.7 : - : 53.5
+//                              64x1024x1024x14x14 BF16 266 : 188 : - : 295      TF32 502 : 287 : - : 379
+//   more filters, large output 96x4x128x99x99    BF16 183 : 126 : - : 110       TF32 188 : 126 : - : 105
 // Packed columns (single-CTA kernel, batch not a multiple of 32), filled up : packed : the best of the others
 //                              8x66x192x38x38    BF16 22.9 : 16.5 : 20.8        TF32 32.1 : 18.1 : 23.9
 //                              48x83x64x9x39     BF16 11.7 : 12.3 : 10.2        TF32 17.2 : 17.8 : 11.5
@@ -149,7 +162,8 @@ TcChoice choose_tc_kernel(bool bf16, int N, int C, TileRows rows, int W, int K, 
   if (N % kColumns) consider(OPENCNN_TC_SINGLE_CTA, true, K <= 64 ? costs.packed64 : costs.packed, columns_of(N, rows, W, true).blocks * wide, sms);
   consider(OPENCNN_TC_PAIR_LOCAL, false, costs.pair, (blocks + 1) / 2 * wide, pairs);
   if (K <= 64) consider(OPENCNN_TC_STACKED_BLOCKS, false, costs.stacked, (blocks + 1) / 2, sms);
-  consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, (tile_pair_blocks(N, rows, W) + 1) / 2 * (K / kImgRowFilters), img_pairs);
+  if (img_pairs > 0)
+    consider(OPENCNN_TC_IMAGE_ROWS, false, costs.image_rows, image_rows_tiles(N, rows, W, K, image_rows_odd(N, rows, W, K, img_pairs)), img_pairs);
   return best;
 }
 

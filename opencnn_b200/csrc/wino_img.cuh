@@ -17,8 +17,8 @@
 // And the transform writes the operand where the patch was (transform_tile_pair), so that shared memory holds one ring of four (BF16) or five (TF32)
 // K-steps.  With a patch per tile and an operand ring of its own there was room for two and four, and a K-step could not be shorter than a
 // part of a load's way to DRAM, 3000 to 4400 cycles on layers that stream; us, then -> now: BF16 128x64x64x56x56 63.5 -> 47, 256x32x64x112x112 263 -> 228,
-// 128x128x128x28x28 53 -> 43; TF32 69 -> 62, 297 -> 257, 64 -> 56.  The list has whole pairs of tile columns, so that maps with an odd number compute a
-// column of tiles for nothing: 128x512x64x14x14 BF16 26.1 -> 27, 128x256x256x14x14 41 -> 49 (the CTA pair takes 30).
+// 128x128x128x28x28 53 -> 43; TF32 69 -> 62, 297 -> 257, 64 -> 56.  An odd number of tile columns leaves one
+// that is computed beside nothing, or whose tiles are paired one above the other where that saves a round (image_rows_odd in dispatch.h).
 //
 // Barriers and roles are those of wino_pair.cuh, less those between patches and operand: a stage lands, is transformed ("V written", on the leading
 // CTA), and is free when the tensor core's commits say so, in both CTAs; "filter slice landed" is the leader's, a drained accumulator column is reported
@@ -61,29 +61,35 @@ template <int DT> struct ImgCfg {
 };
 constexpr int kImgFilters = 64;                  // per tile
 
-// A pair of tiles beside each other and 32 images: what a CTA computes of a pair tile.
-struct TilePair { int tx, ty, n; };              // the left tile, the first image
+// Two tiles and 32 images: what a CTA computes of a pair tile.  The tiles lie beside each other; the kernel for an odd number of tile columns (ODD) takes
+// the last column's one above the other, behind all others in the list, the other kernel beside a column that is not stored.  Image blocks fastest.
+struct TilePair { int tx, ty, n; bool vertical; };   // the left or upper tile, the first image
+template <bool ODD>
 __device__ __forceinline__ TilePair tile_pair(const WinoParams &p, int block) {
-  const int t = block / p.n_blocks, ty = t / p.tiles_w;
-  return {2 * (t - ty * p.tiles_w), ty + p.ty0, (block - t * p.n_blocks) * kTcN};
+  const int t = block / p.n_blocks, n = (block - t * p.n_blocks) * kTcN, beside = t - p.tiles_w * p.tiles_h;
+  if (ODD && beside >= 0) return {2 * p.tiles_w, 2 * beside + p.ty0, n, true};
+  const int ty = t / p.tiles_w;
+  return {2 * (t - ty * p.tiles_w), ty + p.ty0, n, false};
 }
 
-// Transforms the two tiles of channel `c` and images 2 np, 2 np + 1 of a stage, whose 4x6 patch they share, and writes them where the patch was.  A
-// warp has all pixels of its two channels in registers before it writes, and a position's row of a channel lies in a pixel's row
+// Transforms the two tiles of channel `c` and images 2 np, 2 np + 1 of a stage, whose 4x6 (VERTICAL: 6x4) patch they share, and writes them where the patch
+// was.  A warp has all pixels of its two channels in registers before it writes, and a position's row of a channel lies in a pixel's row
 // of the same channel (or behind the patch), so that no other warp's data is touched.
 // V: a position holds 64 columns (2 KB), tile 0 first.  BF16: rows of 128 bytes, 128-byte swizzle (16-byte chunk index ^= c & 7).  TF32: the two
 // tiles' rows of 128 bytes are 1 KB apart, 128-byte swizzle with 32-byte atoms.
-template <int DT>
+template <int DT, bool VERTICAL>
 __device__ __forceinline__ void transform_tile_pair(uint8_t *stage, int c, int np) {
   constexpr int kRows = ImgCfg<DT>::kRows;
   uint64_t d[24];                                  // [h][w]
 #pragma unroll
   for (int q = 0; q < 24; ++q) d[q] = *reinterpret_cast<const uint64_t *>(stage + q * kRows + c * 128 + np * 8);
   __syncwarp();
+  if (!VERTICAL) {
 #pragma unroll
-  for (int w = 0; w < 6; ++w) {
-    const uint64_t b0 = sub2(d[w], d[12 + w]), b1 = add2(d[6 + w], d[12 + w]), b2 = sub2(d[12 + w], d[6 + w]), b3 = sub2(d[6 + w], d[18 + w]);
-    d[w] = b0; d[6 + w] = b1; d[12 + w] = b2; d[18 + w] = b3;
+    for (int w = 0; w < 6; ++w) {
+      const uint64_t b0 = sub2(d[w], d[12 + w]), b1 = add2(d[6 + w], d[12 + w]), b2 = sub2(d[12 + w], d[6 + w]), b3 = sub2(d[6 + w], d[18 + w]);
+      d[w] = b0; d[6 + w] = b1; d[12 + w] = b2; d[18 + w] = b3;
+    }
   }
   const int n = 2 * np;
 #pragma unroll
@@ -92,7 +98,15 @@ __device__ __forceinline__ void transform_tile_pair(uint8_t *stage, int c, int n
                                  : stage + t * 1024 + c * 128 + ((((n >> 3) ^ c) & 3) << 5) + ((n & 7) << 2);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint64_t *b = d + 6 * i + 2 * t;
+      uint64_t v[4];
+      if (VERTICAL) {                              // row i of the columns of tile t, whose patch begins in row 2 t
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint64_t *col = d + 8 * t + w;
+          v[w] = i == 0 ? sub2(col[0], col[8]) : i == 1 ? add2(col[4], col[8]) : i == 2 ? sub2(col[8], col[4]) : sub2(col[4], col[12]);
+        }
+      }
+      const uint64_t *b = VERTICAL ? v : d + 6 * i + 2 * t;
       const uint64_t o[4] = {sub2(b[0], b[2]), add2(b[1], b[2]), sub2(b[2], b[1]), sub2(b[1], b[3])};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -130,11 +144,13 @@ __device__ __forceinline__ void img_epilogue(uint32_t tcol, bool active, const W
   }
 }
 
-// p.k_blocks counts 64-filter blocks, p.tiles_w pairs of tile columns, p.blocks blocks of a pair of tiles and 32 images, p.total_tiles pair tiles
-// (k_blocks times half of those).
-template <int DT>
+// p.k_blocks counts 64-filter blocks, p.tiles_w pairs of tile columns, p.blocks blocks of two tiles and 32 images (see TilePair), p.total_tiles pair
+// tiles (k_blocks times half of those).  tm_in, tm_above: 4x6 patches and 6x4 ones.  ODD: see image_rows_odd in dispatch.h; an instantiation of its own, since
+// a kernel that holds both transforms is 3 to 6 % slower.
+template <int DT, bool ODD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ImgCfg<DT>::kThreads, 1)
-wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const WinoParams p) {
+wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_above,
+                const WinoParams p) {
   using Cfg = ImgCfg<DT>;
   constexpr int S = Cfg::kStages, SU = Cfg::kUStages, KC = Cfg::kKC;
   extern __shared__ __align__(1024) uint8_t ismem[];
@@ -195,11 +211,12 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
     for (int seq = 0; seq < my_tiles; ++seq) {
       const int t = cid + seq * n_clusters, kb = t / halves, block = 2 * (t - kb * halves) + (int)rank;
-      const TilePair at = tile_pair(p, block);
-      const int tx = at.tx + (quarter & 1);
+      const TilePair at = tile_pair<ODD>(p, block);
+      const int second = quarter & 1, tx = at.tx + (ODD && at.vertical ? 0 : second), ty = at.ty + (ODD && at.vertical ? second : 0);
       mbar_wait_reporting(smem_u32(acc_full), seq & 1, dead, p.status, acc_empty0, smem_u32(nowhere));
       tc_fence_after();
-      img_epilogue<Cfg::kEpilogueLoad>(tcol, block < p.blocks && 2 * tx < p.W, p, kb * kImgFilters + 32 * (quarter >> 1) + 16 * sub, tx, at.ty, at.n + lane,
+      img_epilogue<Cfg::kEpilogueLoad>(tcol, block < p.blocks && (ODD ? ty < p.ty0 + p.tiles_h : 2 * tx < p.W), p,
+                   kb * kImgFilters + 32 * (quarter >> 1) + 16 * sub, tx, ty, at.n + lane,
                    [&](int j) { mbar_arrive_cluster(acc_empty0 + 8 * j); });
     }
   } else if (warp >= kPairFirstTransformWarp) {
@@ -209,10 +226,17 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
     // BF16: the two channels of a warp are four apart, so that their 64-byte halves of a row lie in different banks.
     const int c = DT == kTcBf16 ? 8 * (t >> 7) + ((t >> 5) & 3) + 4 * ((t >> 4) & 1) : t >> 4;
     uint32_t v_ready0 = map_to_rank(smem_u32(v_ready), 0);
+    const int first_vertical = p.tiles_w * p.tiles_h * p.n_blocks;     // block
+    int tile = cid, tile_end = cpt;                                      // the K-step's pair tile within a filter block, and the first step behind it
     for (int g = (warp - kPairFirstTransformWarp) / Cfg::kStepWarps; g < total_steps; g += Cfg::kGroups) {
       const int s = g % S;
+      if (ODD) {
+        for (; g >= tile_end; tile_end += cpt) tile += n_clusters;
+        while (tile >= halves) tile -= halves;
+      }
       mbar_wait_reporting(smem_u32(raw_full + g % SF), (g / SF) & 1, dead, p.status, v_ready0, smem_u32(nowhere));
-      transform_tile_pair<DT>(v_s + s * Cfg::kStageBytes, c, np);
+      if (!ODD || 2 * tile + (int)rank < first_vertical) transform_tile_pair<DT, false>(v_s + s * Cfg::kStageBytes, c, np);
+      else                                                transform_tile_pair<DT, true>(v_s + s * Cfg::kStageBytes, c, np);
       fence_proxy_async_smem();          // V is read by the tensor core through the async proxy, which writes the next patch here, too
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(v_ready0 + 8 * s);
@@ -229,7 +253,7 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
       int g = 0;
       bool ok = true;
       for (int seq = 0; seq < my_tiles && ok; ++seq) {
-        const TilePair at = tile_pair(p, 2 * ((cid + seq * n_clusters) % halves) + (int)rank);
+        const TilePair at = tile_pair<ODD>(p, 2 * ((cid + seq * n_clusters) % halves) + (int)rank);
         for (int ci = 0; ci < cpt; ++ci, ++g) {
           const int s = g % S;
           const uint32_t use = g / S;
@@ -238,7 +262,8 @@ wino_img_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant
           if (!elect_one()) continue;
           mbar_arrive_expect_tx(smem_u32(raw_full + g % SF), Cfg::kRawBytes);
           // (A block past the last one: see load_patches.)
-          tma_load_4d(smem_u32(v_s + s * Cfg::kStageBytes), &tm_in, smem_u32(raw_full + g % SF), at.n, ci * KC, 2 * at.tx - 1, 2 * at.ty - 1);
+          tma_load_4d(smem_u32(v_s + s * Cfg::kStageBytes), ODD && at.vertical ? &tm_above : &tm_in, smem_u32(raw_full + g % SF), at.n, ci * KC,
+                      2 * at.tx - 1, 2 * at.ty - 1);
         }
       }
       // No exit with bulk copies in flight (after a complete run these phases are long over).

@@ -1,5 +1,5 @@
 // The rules of opencnn_b200/csrc/dispatch.h from the command line: `fp32 N C K H W` prints "filled" or "packed" and the rounds of items,
-// `tf32 | bf16 N C K H W` the kernel; `form N C K H W` the form of the TF32 CTA pair; `fits P I 0 0 0`: from here on P CTA pairs of the pair kernel and I of the image-rows kernel fit on the
+// `tf32 | bf16 N C K H W` the kernel; `form N C K H W` the form of the TF32 CTA pair and `odd N C K H W` that of the image-rows kernel; `fits P I 0 0 0`: from here on P CTA pairs of the pair kernel and I of the image-rows kernel fit on the
 // device, which has 148 SMs (74 of each).
 #include <cstdio>
 #include <cstdlib>
@@ -24,6 +24,10 @@ int main(int argc, char **argv) {
     }
     if (!strcmp(argv[i], "form")) {
       std::printf("%s\n", pair_in_place(N, C, all_rows(H), W, K) ? "in place" : "two rings");
+      continue;
+    }
+    if (!strcmp(argv[i], "odd")) {
+      std::printf("%s\n", image_rows_odd(N, all_rows(H), W, K, img_pairs) ? "paired" : "beside");
       continue;
     }
     const TcChoice c = choose_tc_kernel(!strcmp(argv[i], "bf16"), N, C, all_rows(H), W, K, 148, pairs, img_pairs);

@@ -84,3 +84,12 @@ def test_the_form_of_the_tf32_pair(choose):
     sizes = [(64, 1024, 1024, 14, 14), (128, 512, 256, 14, 14), (128, 512, 128, 14, 14), (128, 128, 128, 28, 28)]
     assert choose([("form", s) for s in sizes]) == ["in place", "in place", "two rings", "two rings"]
     assert set(choose([("form", s) for kernel, s in overlap.DEPTHS if kernel == "pair_local"])) == {"in place"}
+
+
+def test_the_form_of_the_image_rows_kernel(choose):
+    """An odd last column of tiles is paired where that saves a round; an even number of columns has none to pair."""
+    import test_overlap_gpu as overlap
+    sizes = [(136, 301, 64, 19, 9), (128, 256, 256, 14, 14), (128, 512, 64, 22, 22), (128, 512, 64, 14, 14), (136, 301, 64, 19, 8), (128, 64, 64, 56, 56)]
+    assert choose([("odd", s) for s in sizes]) == ["paired", "paired", "beside", "beside", "beside", "beside"]
+    forms = choose([("odd", s) for kernel, s in overlap.DEPTHS if kernel == "image_rows"])
+    assert forms.count("paired") == 4
