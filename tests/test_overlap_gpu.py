@@ -14,9 +14,11 @@ def _random(*shape, scale=1.0):
 
 
 # A chain of layers with fixed weights and then with weights that are transformed in every call, ping-pong between two buffers: every call
-# reads what the one before it writes, and writes what the one before it reads.  Kernels of all kinds: (N, C = K, H, W).
+# reads what the one before it writes, and writes what the one before it reads.  Kernels of all kinds, and transforms that start early
+# with one, two and four blocks to an SM, or the ordinary way (the last): (N, C = K, H, W).
 CHAINS = [("fp32", (32, 64, 9, 9)), ("fp32", (20, 64, 31, 45)), ("fp32", (32, 512, 5, 5)), ("bf16", (32, 64, 6, 6)), ("bf16", (64, 64, 30, 30)),
-          ("bf16", (32, 256, 12, 12)), ("tf32", (64, 64, 21, 13)), ("tf32", (64, 192, 7, 7)), ("tf32", (8, 64, 27, 21))]
+          ("bf16", (32, 256, 12, 12)), ("bf16", (32, 320, 4, 4)), ("tf32", (64, 64, 21, 13)), ("tf32", (64, 192, 7, 7)), ("tf32", (8, 64, 27, 21)),
+          ("tf32", (32, 576, 9, 9))]
 
 
 @pytest.mark.parametrize("precision,shape", CHAINS)
