@@ -338,7 +338,7 @@ cudaError_t launch_wino_fp32(const float *input, float *output, int N, int C, in
   const int grid = p.total_items < st->sm_count ? p.total_items : st->sm_count;
   const auto kernel = packed   ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kPacked>
                       : ragged ? ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kRagged>
-                      : p.chunks_per_tile >= 8 || p.total_items <= st->sm_count
+                      : (p.total_items <= st->sm_count ? p.chunks_per_tile <= 16 : p.chunks_per_tile >= 8)
                           ? ocb::wino_fp32_kernel<OCB_VARIANT, kFourWarps>        // (see kFourTransform)
                           : ocb::wino_fp32_kernel<OCB_VARIANT, ocb::kExact>;
   return launch_main(kernel, grid, ocb::kThreads, ocb::SmemLayout<OCB_VARIANT>::kBytes, stream, filter, st->sm_count, p, tm_in, tm_u);

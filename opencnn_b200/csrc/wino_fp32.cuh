@@ -522,7 +522,9 @@ wino_fp32_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constan
   // Who transforms: three producer warps beside one that only loads, or all four, the first of which loads as well.  Four share the additions evenly
   // between the schedulers, whose FMA pipes they are taken from: 64x1024x1024x14x14 1993 -> 1917 us, 128x512x512x7x7 330 -> 325, 128x128x128x28x28
   // 265 -> 261.  Not where the loads have to run far ahead: tiles of fewer than eight chunks on SMs with several tiles
-  // (256x32x64x112x112 1178 -> 1208), a ring of three stages (OPTSTS64_CMP, the same layer 1205 -> 1280), packed columns; and not in the
+  // (256x32x64x112x112 1178 -> 1208); tiles of more than 16 chunks with an SM each, whose ring starts empty and is all that hides the way to a
+  // filter that was just transformed (32x256x64x14x14 32.6 us a call with three warps, 34.4 with four; 32x128x128x14x14 27.7 and 27.8,
+  // 32x64x64x14x14 11.8 and 11.7); a ring of three stages (OPTSTS64_CMP, 256x32x64x112x112 1205 -> 1280); packed columns; and not in the
   // ragged kernel, whose consumers the compiler then schedules worse (184x21x116x34x34 143 -> 153).
   constexpr bool kFourTransform = SHAPE == kExactFour;
   static_assert(!kFourTransform || S >= 4, "see above");

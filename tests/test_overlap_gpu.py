@@ -99,8 +99,9 @@ def test_layout_adapters_and_the_operator_are_ordered(libs, shape):
 
 # The fp32 kernel's four-stage ring is filled by a warp that transforms as well, deep tiles (64 chunks of 8 channels) one chunk further ahead; BASE has three
 # stages and a warp that only loads.  Fewer chunks than stages, as many, more; tiles on both sides of 64 chunks; several items per SM, the last round split.
+# With an item per SM, tiles of up to 16 chunks and deeper ones, which leave the loads to a warp of their own.
 RINGS = [(32, 8, 64, 4, 4), (32, 24, 64, 26, 26), (32, 32, 128, 25, 25), (32, 33, 64, 31, 30), (32, 504, 64, 26, 26), (32, 512, 64, 26, 26),
-         (32, 520, 128, 19, 19), (64, 1024, 64, 5, 5)]
+         (32, 520, 128, 19, 19), (64, 1024, 64, 5, 5), (32, 128, 64, 12, 12), (32, 129, 64, 12, 12), (32, 136, 64, 12, 12)]
 
 
 @pytest.mark.parametrize("shape", RINGS)
