@@ -25,7 +25,6 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict_
                                                        long long rows, long long cols, long long tiles_x) {
   __shared__ float tile[32][33];
   grid_dependency_wait();
-  grid_launch_dependents();
   const long long t = blockIdx.x;
   const long long c0 = (t % tiles_x) * 32, r0 = (t / tiles_x) * 32;
 #pragma unroll
@@ -49,7 +48,6 @@ __global__ void __launch_bounds__(256) transpose4_kernel(const float *__restrict
                                                         long long rows, long long cols, long long tiles_x) {
   __shared__ float tile[64][65];
   grid_dependency_wait();
-  grid_launch_dependents();
   const long long t = blockIdx.x;
   const long long c0 = (t % tiles_x) * 64, r0 = (t / tiles_x) * 64;
   const int a = threadIdx.x >> 4, b4 = (threadIdx.x & 15) * 4;
@@ -80,8 +78,13 @@ inline cudaError_t launch_transpose(const float *src, float *dst, long long rows
   const long long edge = vec ? 64 : 32;
   const long long gx = (cols + edge - 1) / edge, gy = (rows + edge - 1) / edge;
   if (gx * gy > 2147483647ll) return cudaErrorInvalidValue;
-  if (vec) return launch(transpose4_kernel, (unsigned)(gx * gy), dim3(256), 0, stream, true, src, dst, rows, cols, gx);
-  return launch(transpose_kernel, (unsigned)(gx * gy), dim3(32, 8), 0, stream, true, src, dst, rows, cols, gx);
+  // Early (see launch) up to 80 MB: whole NCHW calls of 64x64x128x30x30 TF32 41.0 -> 36.7 us, 8x64x64x112x112 fp32 131.4 -> 126.8, 128x32x96x40x40 BF16
+  // (79 MB) 39.2 -> 34.9.  Beyond that a transpose that starts so runs slower, for a reason not found: 40x222x448x97x12 BF16 (83 MB) 188.3 -> 190.1,
+  // 44x4x112x97x97 fp32 (185 MB) 229 -> 240, 64x3x64x96x96 BF16 (151 MB) 94.1 -> 100.9.  Neither kernel lets the next one start before it ends: doing so
+  // cost 1.5 % at 128x128x128x28x28 fp32 and 7 % at 64x64x128x30x30 TF32.
+  const bool early = rows * cols <= 20'000'000;
+  if (vec) return launch(transpose4_kernel, (unsigned)(gx * gy), dim3(256), 0, stream, early, src, dst, rows, cols, gx);
+  return launch(transpose_kernel, (unsigned)(gx * gy), dim3(32, 8), 0, stream, early, src, dst, rows, cols, gx);
 }
 
 }  // namespace ocb

@@ -67,9 +67,10 @@ def test_a_chain_of_calls_is_ordered(libs, precision, shape, cached):
     assert api.last_device_status() == 0
 
 
-@pytest.mark.parametrize("shape", [(128, 16, 64, 14, 14), (36, 5, 68, 7, 9)])
+@pytest.mark.parametrize("shape", [(128, 16, 64, 14, 14), (36, 5, 68, 7, 9), (64, 4, 80, 62, 63), (64, 4, 80, 62, 64)])
 def test_layout_adapters_and_the_operator_are_ordered(libs, shape):
-    """NCHW in, NCHW out, all of it queued, with inputs that another library's kernel has just written."""
+    """NCHW in, NCHW out, all of it queued, with inputs that another library's kernel has just written.  The last two: a transpose
+    of just under 80 MB and one of just over, which start early and do not."""
     N, C, K, H, W = shape
     stream = torch.cuda.Stream()
     inputs = [_random(N, C, H, W) for _ in range(4)]
